@@ -7,10 +7,13 @@ first call raises ``RuntimeError`` telling the user to build it.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 from ctypes import c_char_p, c_int, c_int64, c_size_t, c_void_p, POINTER
 from pathlib import Path
 
 LIB_PATH = Path(__file__).resolve().parent / "libfp8lin.so"
+HOST_PATH = LIB_PATH.parent / "_fp8host.so"
 
 W8A16 = 0
 W8A8_STATIC = 1
@@ -84,6 +87,22 @@ def load() -> ctypes.CDLL:
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native binding of the per-step calls (csrc/host.cpp), loaded once; it calls the same library."""
+    global _host
+    if _host is None:
+        load()
+        if not HOST_PATH.exists():
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python {HOST_PATH.parent / 'build.py'}`")
+        loader = importlib.machinery.ExtensionFileLoader("_fp8host", str(HOST_PATH))
+        _host = importlib.util.module_from_spec(importlib.machinery.ModuleSpec("_fp8host", loader, origin=str(HOST_PATH)))
+        loader.exec_module(_host)
+    return _host
 
 
 def last_error() -> str:

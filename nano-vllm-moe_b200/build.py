@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -19,6 +20,7 @@ HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
 OBJ = HERE / "build"
 LIB = HERE / "libfp8lin.so"
+HOST = HERE / "_fp8host.so"            # the Python binding of the per-step calls (csrc/host.cpp)
 SOURCES = ["api.cu", "rmsnorm_quant.cu", "stream_kernel.cu", "elementwise.cu", "umma_gemm.cu", "umma_pair_gemm.cu", "umma_swap.cu", "umma_swap_w8a16.cu", "umma_grouped.cu", "umma_grouped_rows.cu", "moe_kernels.cu", "static_scratch.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
@@ -40,6 +42,23 @@ def _stale(target: Path, deps) -> bool:
     return any(Path(d).stat().st_mtime > t for d in deps)
 
 
+def _compile_host(force: bool) -> tuple[Path, Path]:
+    """csrc/host.cpp against this interpreter's and torch's headers; returns the object and torch's library folder."""
+    import importlib.util
+    root = Path(importlib.util.find_spec("torch").submodule_search_locations[0])
+    src, obj = CSRC / "host.cpp", OBJ / "host.cpp.o"
+    if force or _stale(obj, [src, HERE.parent / "include" / "fp8lin.h"]):
+        cuda = Path(_nvcc()).resolve().parent.parent
+        cmd = [shutil.which("g++") or "g++", "-O2", "-fPIC", "-std=c++17", "-fvisibility=hidden", "-D_GLIBCXX_USE_CXX11_ABI=1", "-c", str(src), "-o", str(obj),
+               "-isystem", str(root / "include"), "-isystem", str(root / "include" / "torch" / "csrc" / "api" / "include"),
+               "-isystem", str(cuda / "include"), "-isystem", sysconfig.get_paths()["include"]]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        (OBJ / "host.cpp.log").write_text(r.stdout + r.stderr)
+        if r.returncode != 0:
+            raise RuntimeError(f"g++ failed for host.cpp:\n{r.stdout}\n{r.stderr}")
+    return obj, root / "lib"
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     nvcc = _nvcc()
     OBJ.mkdir(exist_ok=True)
@@ -58,10 +77,18 @@ def build(force: bool = False, verbose: bool = False) -> Path:
                 print(r.stderr)
         return obj
 
-    with ThreadPoolExecutor(max_workers=min(len(sources), os.cpu_count() or 1)) as ex:
+    with ThreadPoolExecutor(max_workers=min(len(sources) + 1, os.cpu_count() or 1)) as ex:
+        host = ex.submit(_compile_host, force)
         objs = list(ex.map(compile_one, sources))
     if force or _stale(LIB, objs):
         cmd = [nvcc, "-shared", "-o", str(LIB), *map(str, objs), "-lcudart"]
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    host_obj, torch_lib = host.result()
+    if force or _stale(HOST, [host_obj, LIB]):
+        cmd = [shutil.which("g++") or "g++", "-shared", "-o", str(HOST), str(host_obj), f"-L{HERE}", "-l:libfp8lin.so", f"-L{torch_lib}", "-ltorch_python",
+               "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN"]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")

@@ -16,7 +16,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from ..quantization import kernels
+from .. import _lib
 
 
 class QuantizedActivation:
@@ -40,22 +40,16 @@ class RMSNorm(nn.Module):
         self.eps = eps
         self.weight = nn.Parameter(torch.ones(hidden_size))
 
-    def _weight_bf16(self, device) -> torch.Tensor:
-        w = self.weight.data
-        if w.dtype != torch.bfloat16 or w.device != device:
-            w = w.to(device=device, dtype=torch.bfloat16)
-        return w.contiguous()
-
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None):
         if not x.is_cuda:
             raise RuntimeError("fp8lin RMSNorm requires CUDA")
-        x2 = x.reshape(-1, x.shape[-1])
+        norm = _lib.host().rmsnorm_quant
         if residual is None:
-            _, y = kernels.rmsnorm_quant(x2, self._weight_bf16(x.device), self.eps)
-            return y.view(x.shape)
-        res = residual.reshape(-1, x.shape[-1]).clone()       # the reference returns a new residual tensor
-        _, y = kernels.rmsnorm_quant(x2, self._weight_bf16(x.device), self.eps, residual=res)
-        return y.view(x.shape), res.view(x.shape)
+            return norm(x, self._parameters["weight"], self.eps, None, None, True, None, None)[1]
+        res = residual.clone(memory_format=torch.contiguous_format)          # the reference returns a new residual tensor
+        if res.shape != x.shape:
+            res = res.view(x.shape)
+        return norm(x, self._parameters["weight"], self.eps, None, res, True, None, None)[1], res
 
     def forward_quant(self, x: torch.Tensor, input_scale: torch.Tensor, residual: torch.Tensor | None = None,
                       inplace_residual: bool = True):
@@ -63,11 +57,13 @@ class RMSNorm(nn.Module):
         residual tensor is updated in place, as a decode loop replayed from a CUDA graph needs."""
         if not x.is_cuda:
             raise RuntimeError("fp8lin RMSNorm requires CUDA")
-        x2 = x.reshape(-1, x.shape[-1])
-        res = None
-        if residual is not None:
-            res = residual.reshape(-1, x.shape[-1])
+        res = residual
+        if res is not None:
             if not inplace_residual:
-                res = res.clone()
-        xq, _ = kernels.rmsnorm_quant(x2, self._weight_bf16(x.device), self.eps, input_scale=input_scale, residual=res)
-        return QuantizedActivation(xq.view(*x.shape[:-1], x.shape[-1]), input_scale), (res.view(x.shape) if res is not None else None)
+                res = res.clone(memory_format=torch.contiguous_format)
+            if res.shape != x.shape:
+                res = res.reshape(x.shape)
+            if res.dim() != 2 and not res.is_contiguous():
+                res = res.contiguous()
+        xq, _ = _lib.host().rmsnorm_quant(x, self._parameters["weight"], self.eps, input_scale, res, False, None, None)
+        return QuantizedActivation(xq, input_scale), res

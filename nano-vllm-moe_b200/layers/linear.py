@@ -55,6 +55,11 @@ class LinearBase(nn.Module):
             return F.linear(x, self.weight, bias)
         return self.quant_method.apply(self, x, bias)
 
+    def _own_bias(self) -> torch.Tensor | None:
+        """``self.bias`` without nn.Module's attribute fallback (a call per layer and step)."""
+        params = self._parameters
+        return params["bias"] if "bias" in params else self.bias
+
     def _make_params(self, k_part: int, n_parts: list[int], bias: bool) -> None:
         n_part = sum(n_parts)
         if self.quant_method is None:
@@ -103,7 +108,7 @@ class ColumnParallelLinear(LinearBase):
         param.data.copy_(loaded_weight.narrow(self.tp_dim, self.tp_rank * rows, rows))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        return self.apply_linear(x, self.bias)
+        return self.apply_linear(x, self._own_bias())
 
 
 class MergedColumnParallelLinear(ColumnParallelLinear):
@@ -391,7 +396,9 @@ class RowParallelLinear(LinearBase):
         return y.view(*x.shape[:-1], self.output_size)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        bias = self.bias if self.tp_rank == 0 else None
+        bias = self._own_bias() if self.tp_rank == 0 else None
+        if self.tp_size == 1:
+            return self.apply_linear(x, bias)
         reduce = self.tp_size > 1 and bool(self.reduce_results)
         rows = x.numel() // x.shape[-1] if x.dim() > 0 else 0
         if reduce and (self._use_peer_rs(x, rows) or self._use_peer_reduce(x, rows)):

@@ -13,6 +13,7 @@ import torch
 import torch.distributed as dist
 from torch import nn
 
+from .. import _lib
 from ..quantization import kernels
 from .linear import MergedColumnParallelLinear, RowParallelLinear
 
@@ -49,17 +50,16 @@ class FusedFp8MLP(nn.Module):
 
     def forward(self, x) -> torch.Tensor:
         """``x``: bfloat16 [.., H], or a ``QuantizedActivation`` made with gate_up_proj's input scale."""
-        codes = getattr(x, "codes", None)
-        if codes is not None:
-            x = codes
+        if not isinstance(x, torch.Tensor):
+            x = x.codes
         if not x.is_cuda:
             raise RuntimeError("FP8 W8A8 static requires CUDA")
-        down = self.down_proj
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, x.shape[-1])
-        bias = down.bias if (getattr(down, "bias", None) is not None and down.tp_rank == 0) else None   # as layers/linear.py:259
-        y = kernels.launch_mlp_w8a8(x2, self.gate_up_packed, self.gate_up_scale, self.gate_up_proj.input_scale, self.gate_up_bias,
-                                    down.qweight_packed, down.weight_scale, down.input_scale, bias)
+        modules, buffers = self._modules, self._buffers
+        down, gate_up = modules["down_proj"], modules["gate_up_proj"]
+        down_buffers = down._buffers
+        bias = down._own_bias() if down.tp_rank == 0 else None        # as layers/linear.py:259
+        y = _lib.host().mlp(x, buffers["gate_up_packed"], buffers["gate_up_scale"], gate_up._buffers["input_scale"], self.gate_up_bias,
+                            down_buffers["qweight_packed"], down_buffers["weight_scale"], down_buffers["input_scale"], bias, None)
         if down.tp_size > 1 and down.reduce_results:
             dist.all_reduce(y, group=down.tp_group)
-        return y.reshape(*lead, y.shape[-1])
+        return y

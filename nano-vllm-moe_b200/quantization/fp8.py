@@ -76,6 +76,7 @@ class Fp8LinearMethod(QuantizeMethodBase):
     def __init__(self, quant_config: Fp8Config, prefix: str = "") -> None:
         self.quant_config = quant_config
         self.prefix = prefix
+        self._scheme = _lib.W8A8_STATIC if self.is_w8a8 else _lib.W8A16
 
     @property
     def is_w8a8(self) -> bool:
@@ -148,37 +149,27 @@ class Fp8LinearMethod(QuantizeMethodBase):
               out: torch.Tensor | None = None) -> torch.Tensor:
         """``out`` (optional, bf16 [M, N], row stride a multiple of 8) receives the result in place;
         the row-parallel layer uses it to compute M in chunks into one buffer."""
-        backend = getattr(layer, "_fp8_backend", None)
-        codes = getattr(x, "codes", None)
-        if codes is not None:
-            # activations already quantised by the producer (layers/layernorm.py RMSNorm.forward_quant)
-            if not self.is_w8a8:
-                raise ValueError("pre-quantised activations need the fp8_w8a8_static scheme")
-            if backend is None:
-                raise RuntimeError("FP8 backend is not initialized: call process_weights_after_loading first")
-            if (x.scale.data_ptr() != layer.input_scale.data_ptr() and not torch.cuda.is_current_stream_capturing()
-                    and not torch.equal(x.scale.reshape(()), layer.input_scale.reshape(()))):
-                raise ValueError("the activations were quantised with a scale other than this layer's input_scale")
-            if bias is not None and bias.dtype != torch.bfloat16:
-                bias = bias.to(torch.bfloat16)
-            y = kernels.launch_w8a8_preq(codes.reshape(-1, codes.shape[-1]), layer.qweight_packed, layer.input_scale,
-                                         layer.weight_scale, bias, out=out)
-            return out if out is not None else y.view(*codes.shape[:-1], y.shape[-1])
+        if not isinstance(x, torch.Tensor):
+            return self._apply_codes(layer, x, bias, out)
         if not x.is_cuda:
             scheme = "FP8 W8A8 static" if self.is_w8a8 else "FP8 W8A16"
             raise RuntimeError(f"{scheme} requires CUDA")
-        if backend is None:
+        if getattr(layer, "_fp8_backend", None) is None:
             raise RuntimeError("FP8 backend is not initialized: call process_weights_after_loading first")
-        k = x.shape[-1]
-        x2 = x.reshape(-1, k)
-        if x2.dtype != torch.bfloat16:
-            x2 = x2.to(torch.bfloat16)
-        if bias is not None and bias.dtype != torch.bfloat16:
-            bias = bias.to(torch.bfloat16)
-        if self.is_w8a8:
-            y = kernels.launch_w8a8_gemm(x2, layer.qweight_packed, layer.input_scale, layer.weight_scale, bias, out=out)
-        else:
-            y = kernels.launch_w8a16_gemm(x2, layer.qweight_packed, layer.weight_scale, bias, out=out)
-        if out is not None:
-            return out
-        return y.view(*x.shape[:-1], y.shape[-1]).to(x.dtype)
+        # (the buffer dict directly: nn.Module's attribute lookup costs as much as the rest of this function)
+        buffers = layer._buffers
+        return _lib.host().linear(self._scheme, x, buffers["qweight_packed"], buffers["weight_scale"], buffers.get("input_scale"),
+                                  bias, out)
+
+    def _apply_codes(self, layer: nn.Module, x, bias: torch.Tensor | None, out: torch.Tensor | None) -> torch.Tensor:
+        """Activations already quantised by the producer (layers/layernorm.py RMSNorm.forward_quant)."""
+        if not self.is_w8a8:
+            raise ValueError("pre-quantised activations need the fp8_w8a8_static scheme")
+        if getattr(layer, "_fp8_backend", None) is None:
+            raise RuntimeError("FP8 backend is not initialized: call process_weights_after_loading first")
+        buffers = layer._buffers
+        scale = buffers["input_scale"]
+        if (x.scale is not scale and x.scale.data_ptr() != scale.data_ptr() and not torch.cuda.is_current_stream_capturing()
+                and not torch.equal(x.scale.reshape(()), scale.reshape(()))):
+            raise ValueError("the activations were quantised with a scale other than this layer's input_scale")
+        return _lib.host().linear_codes(x.codes, buffers["qweight_packed"], buffers["weight_scale"], scale, bias, out)

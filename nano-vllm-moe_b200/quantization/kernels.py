@@ -16,10 +16,6 @@ import torch
 
 from .. import _lib
 
-_workspaces: dict[tuple[int, int], torch.Tensor] = {}
-_retired: list[torch.Tensor] = []       # outgrown scratch buffers, kept alive (see workspace())
-
-
 def _require_cuda(*tensors: torch.Tensor) -> None:
     for t in tensors:
         if t is not None and not t.is_cuda:
@@ -44,20 +40,8 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     CAPTURE, before the capture starts.  ``torch.cuda.graph`` captures on a side stream, so the
     warm-up belongs inside ``with torch.cuda.stream(side):`` too.  Graphs captured on the same
     stream share one scratch buffer; replay them on one stream at a time."""
-    key = (device.index if device.index is not None else torch.cuda.current_device(), _stream_ptr(device))
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        if torch.cuda.is_current_stream_capturing():
-            raise RuntimeError(
-                f"fp8lin scratch for this stream must grow to {nbytes} bytes during a CUDA graph capture; "
-                "run the shape once (or call reserve_workspace) on the capturing stream before the capture")
-        size = max(nbytes, _lib.WS_HEADER_BYTES)
-        if ws is not None:
-            size = max(size, 2 * ws.numel())
-            _retired.append(ws)
-        ws = torch.zeros(size, dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return _lib.host().workspace(index, _stream_ptr(device), nbytes)
 
 
 def reserve_workspace(device: torch.device, nbytes: int) -> None:
@@ -69,8 +53,7 @@ def release_workspaces() -> None:
     """Free every scratch buffer, retired ones included.  Only when no kernel of this library is
     in flight and no CUDA graph that captured one of its calls will be replayed again."""
     torch.cuda.synchronize()
-    _workspaces.clear()
-    _retired.clear()
+    _lib.host().release_workspaces()
 
 
 def workspace_bytes(scheme: int, m: int, k: int, n: int) -> int:
@@ -147,64 +130,39 @@ def _check_linear_args(x, w_packed, weight_scale, bias):
     return x, n, k
 
 
+def _check_bias(bias) -> None:
+    """The functional launchers take bf16 biases only (the layers convert theirs)."""
+    if bias is not None and bias.dtype != torch.bfloat16:
+        raise ValueError("bias must be bfloat16 [N]")
+
+
 def launch_w8a16_gemm(x: torch.Tensor, w_packed: torch.Tensor, weight_scale: torch.Tensor,
                       bias: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """bf16 ``(x @ W^T) * weight_scale + bias`` with packed e4m3 weights."""
-    x, n, k = _check_linear_args(x, w_packed, weight_scale, bias)
-    m = x.shape[0]
-    y = out if out is not None else torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
-        need = workspace_bytes(_lib.W8A16, m, k, n)
-        ws = workspace(x.device, need)
-        rc = _lib.load().fp8lin_w8a16(
-            x.data_ptr(), x.stride(0), w_packed.data_ptr(), weight_scale.data_ptr(),
-            bias.data_ptr() if bias is not None else None, y.data_ptr(), y.stride(0),
-            m, k, n, ws.data_ptr(), ws.numel(), _stream_ptr(x.device))
-    _lib.raise_for(rc, "fp8lin_w8a16")
-    return y
+    if x.dim() != 2 or x.dtype != torch.bfloat16:
+        raise ValueError("x must be a 2-D bfloat16 tensor [M, K]")
+    _check_bias(bias)
+    return _lib.host().linear(_lib.W8A16, x, w_packed, weight_scale, None, bias, out)
 
 
 def launch_w8a8_gemm(x: torch.Tensor, w_packed: torch.Tensor, input_scale: torch.Tensor,
                      weight_scale: torch.Tensor, bias: torch.Tensor | None = None,
                      out: torch.Tensor | None = None) -> torch.Tensor:
     """Static-scale W8A8: x is quantised to e4m3 with ``input_scale`` inside the call."""
-    x, n, k = _check_linear_args(x, w_packed, weight_scale, bias)
-    _require_cuda(input_scale)
-    if input_scale.dtype != torch.float32 or input_scale.numel() != 1:
-        raise ValueError("input_scale must be one float32 value on the device")
-    m = x.shape[0]
-    y = out if out is not None else torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
-        need = workspace_bytes(_lib.W8A8_STATIC, m, k, n)
-        ws = workspace(x.device, need)
-        rc = _lib.load().fp8lin_w8a8(
-            x.data_ptr(), x.stride(0), w_packed.data_ptr(), weight_scale.data_ptr(), input_scale.data_ptr(),
-            bias.data_ptr() if bias is not None else None, y.data_ptr(), y.stride(0),
-            m, k, n, ws.data_ptr(), ws.numel(), _stream_ptr(x.device))
-    _lib.raise_for(rc, "fp8lin_w8a8")
-    return y
+    if x.dim() != 2 or x.dtype != torch.bfloat16:
+        raise ValueError("x must be a 2-D bfloat16 tensor [M, K]")
+    _check_bias(bias)
+    return _lib.host().linear(_lib.W8A8_STATIC, x, w_packed, weight_scale, input_scale, bias, out)
 
 
 def launch_w8a8_preq(xq: torch.Tensor, w_packed: torch.Tensor, input_scale: torch.Tensor, weight_scale: torch.Tensor,
                      bias: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """W8A8 linear on activations that are already e4m3 codes (uint8 [M, K], contiguous), e.g. from
     ``rmsnorm_quant``: no quantiser pass."""
-    _require_cuda(xq, w_packed, weight_scale, input_scale, bias)
-    if xq.dtype != torch.uint8 or xq.dim() != 2 or not xq.is_contiguous():
+    if xq.dim() != 2:
         raise ValueError("xq must be a contiguous 2-D uint8 tensor of e4m3 codes [M, K]")
-    m, k = xq.shape
-    n = weight_scale.numel()
-    if k % 16 != 0 or w_packed.numel() != packed_bytes(k, n):
-        raise ValueError(f"xq has K={k}, weight_scale has N={n}, but the packed weight holds {w_packed.numel()} bytes")
-    y = out if out is not None else torch.empty((m, n), dtype=torch.bfloat16, device=xq.device)
-    with torch.cuda.device(xq.device):
-        ws = workspace(xq.device, workspace_bytes(_lib.W8A8_STATIC, m, k, n))
-        rc = _lib.load().fp8lin_w8a8_preq(
-            xq.data_ptr(), w_packed.data_ptr(), weight_scale.data_ptr(), input_scale.data_ptr(),
-            bias.data_ptr() if bias is not None else None, y.data_ptr(), y.stride(0), m, k, n,
-            ws.data_ptr(), ws.numel(), _stream_ptr(xq.device))
-    _lib.raise_for(rc, "fp8lin_w8a8_preq")
-    return y
+    _check_bias(bias)
+    return _lib.host().linear_codes(xq, w_packed, weight_scale, input_scale, bias, out)
 
 
 def rmsnorm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float, input_scale: torch.Tensor | None = None,
@@ -214,29 +172,11 @@ def rmsnorm_quant(x: torch.Tensor, weight: torch.Tensor, eps: float, input_scale
     the stream the next layer adds to) fused with the static activation quantiser.
     Returns (xq or None, y or None): e4m3 codes [M, H] when ``input_scale`` is given, the bf16 result when
     ``want_bf16`` (or when there is no ``input_scale``)."""
-    _require_cuda(x, weight, input_scale, residual)
     if x.dim() != 2 or x.dtype != torch.bfloat16 or weight.dtype != torch.bfloat16:
         raise ValueError("x must be a 2-D bfloat16 tensor and weight a bfloat16 vector")
-    if x.stride(1) != 1:
-        x = x.contiguous()
-    m, h = x.shape
-    if weight.numel() != h or not weight.is_contiguous():
+    if not weight.is_contiguous():
         raise ValueError("weight must be a contiguous vector of H elements")
-    if residual is not None and (residual.shape != x.shape or residual.dtype != torch.bfloat16 or residual.stride(1) != 1):
-        raise ValueError("residual must be a bfloat16 tensor of x's shape with contiguous rows (it is updated in place)")
-    xq = y = None
-    if input_scale is not None:
-        xq = xq_out if xq_out is not None else torch.empty((m, h), dtype=torch.uint8, device=x.device)
-    if want_bf16 or input_scale is None:
-        y = y_out if y_out is not None else torch.empty((m, h), dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
-        rc = _lib.load().fp8lin_rmsnorm_quant(
-            x.data_ptr(), x.stride(0), residual.data_ptr() if residual is not None else None,
-            residual.stride(0) if residual is not None else 0, weight.data_ptr(), float(eps),
-            input_scale.data_ptr() if input_scale is not None else None, xq.data_ptr() if xq is not None else None,
-            y.data_ptr() if y is not None else None, y.stride(0) if y is not None else 0, m, h, _stream_ptr(x.device))
-    _lib.raise_for(rc, "fp8lin_rmsnorm_quant")
-    return xq, y
+    return _lib.host().rmsnorm_quant(x, weight, eps, input_scale, residual, want_bf16, xq_out, y_out)
 
 
 def quantize_activation(x: torch.Tensor, input_scale: torch.Tensor) -> torch.Tensor:
@@ -329,39 +269,8 @@ def launch_mlp_w8a8(x: torch.Tensor, w_gate_up_il: torch.Tensor, gate_up_scale_i
     """bf16 ``down(silu(gate(x)) * up(x))`` with both projections W8A8-static; operands as produced by
     ``interleave_gate_up`` (gate_up) and ``pack_weight_nk`` / ``prepack_weight`` (down).  ``x`` is bfloat16
     [M, H], or uint8 [M, H] e4m3 codes already quantised with ``gate_up_input_scale`` (``rmsnorm_quant``)."""
-    preq = x.dtype == torch.uint8
-    if preq:
-        if x.dim() != 2 or not x.is_contiguous() or not x.is_cuda:
-            raise ValueError("pre-quantised activations must be a contiguous 2-D uint8 CUDA tensor")
-        n2, h = gate_up_scale_il.numel(), x.shape[1]
-        if h % 16 or w_gate_up_il.numel() != packed_bytes(h, n2):
-            raise ValueError("the packed gate_up weight does not match the activations' width")
-    else:
-        x, n2, h = _check_linear_args(x, w_gate_up_il, gate_up_scale_il, gate_up_bias_il)
-    inter = n2 // 2
-    n = down_scale.numel()
-    _require_cuda(w_down, down_scale, gate_up_input_scale, down_input_scale)
-    if w_down.numel() != packed_bytes(inter, n):
-        raise ValueError("w_down does not match the intermediate size of the gate_up weight")
-    if down_bias is not None and (down_bias.dtype != torch.bfloat16 or down_bias.numel() != n):
-        raise ValueError("down_bias must be bf16 [N]")
-    m = x.shape[0]
-    y = out if out is not None else torch.empty((m, n), dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
-        lib = _lib.load()
-        ws = workspace(x.device, lib.fp8lin_mlp_workspace_bytes(m, h, inter, n))
-        if preq:
-            rc = lib.fp8lin_mlp_w8a8_preq(
-                x.data_ptr(), w_gate_up_il.data_ptr(), gate_up_scale_il.data_ptr(), gate_up_input_scale.data_ptr(),
-                gate_up_bias_il.data_ptr() if gate_up_bias_il is not None else None, w_down.data_ptr(), down_scale.data_ptr(),
-                down_input_scale.data_ptr(), down_bias.data_ptr() if down_bias is not None else None, y.data_ptr(), y.stride(0),
-                m, h, inter, n, ws.data_ptr(), ws.numel(), _stream_ptr(x.device))
-            _lib.raise_for(rc, "fp8lin_mlp_w8a8_preq")
-            return y
-        rc = lib.fp8lin_mlp_w8a8(
-            x.data_ptr(), x.stride(0), w_gate_up_il.data_ptr(), gate_up_scale_il.data_ptr(), gate_up_input_scale.data_ptr(),
-            gate_up_bias_il.data_ptr() if gate_up_bias_il is not None else None, w_down.data_ptr(), down_scale.data_ptr(),
-            down_input_scale.data_ptr(), down_bias.data_ptr() if down_bias is not None else None, y.data_ptr(), y.stride(0),
-            m, h, inter, n, ws.data_ptr(), ws.numel(), _stream_ptr(x.device))
-    _lib.raise_for(rc, "fp8lin_mlp_w8a8")
-    return y
+    if x.dim() != 2:
+        raise ValueError("x must be a 2-D bfloat16 tensor [M, K] or 2-D uint8 codes")
+    _check_bias(gate_up_bias_il)
+    return _lib.host().mlp(x, w_gate_up_il, gate_up_scale_il, gate_up_input_scale, gate_up_bias_il, w_down, down_scale,
+                           down_input_scale, down_bias, out)
