@@ -281,12 +281,18 @@ int fp8lin_mlp_w8a8_preq(const void* xq, const void* w_gate_up, const float* gat
 /* Which kernel variant a shape is routed to ("stream_mma_w8a8_m16", "umma_w8a8_128x256", ...),
  * for labelling bench rows and ncu captures.  Host-only, returns a static string. */
 const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N);
+/* The kernel that a call with 16-byte aligned y (ldy a multiple of 8) runs.  Differs from fp8lin_variant_name for W8A16
+ * from 65 rows on: those calls take the CTA-pair kernel that widens the weights into tensor memory
+ * ("umma_w8a16_pair_256x224_s3"); the variant name is the route of a call that kernel does not take (other alignments,
+ * or one of the knobs of the other routes set).  Host-only, returns a static string. */
+const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N);
 
 /* Bench/ncu studies only: force a tuning knob (value < 0 restores the default).  Not thread safe.
  * Knobs: "stream_splits", "stream_max_m", "umma_bn", "umma_splits", "umma_pair" (CTA-pair GEMM on/off),
  * "swap_splits", "swap_enable", "swap_min_m", "swap_preq_min_m", "w8a16_swap_enable", "w8a16_swap_min_m", "fuse_quant" (1 = large-M W8A8 quantises most rows with warps of the GEMM
  * itself instead of a pass in front of it; n > 1 = the pass takes the first n rows), "quant_lead",
  * "w8a16_umma_min_m" (rows from which W8A16 takes the f16 GEMM route; 0 = never), "w8a16_chunk_mb", "pdl",
+ * "w8a16_pair" (0 / 1: never / always the W8A16 CTA-pair kernel), "w8a16_pair_tokens", "w8a16_pair_splits",
  * "stream_push" (0 = split-K of the mma.sync streaming kernel always through global scratch instead of a cluster),
  * "mlp_decode_fused" (1 = the fused MLP on up to 16 pre-quantised rows computes silu * up inside the gate_up kernel),
  * "moe_fused" (0 = the expert FFN keeps a separate activation pass), "moe_rows_major" (0 = prefill-sized expert

@@ -34,6 +34,9 @@ struct Tuning {
     int w8a16_swap_min_m = -1;
     int w8a16_umma_min_m = -1;  // smallest M for the dequantise-to-f16 + tcgen05 GEMM route (0 = never)
     int w8a16_chunk_mb = -1;    // size of the f16 weight chunk that route keeps in L2
+    int w8a16_pair = -1;        // 0 = never the CTA-pair kernel that widens weights into TMEM, 1 = for every M
+    int w8a16_pair_tokens = -1; // force its tokens per tile / its K slices
+    int w8a16_pair_splits = -1;
     int umma_pair = -1;         // 1 = large-M GEMMs on CTA pairs (256 x 256 tiles), 0 = never
     int fuse_quant = -1;        // large-M W8A8: <= 0 (default) = quantise x in a separate pass; 1 = the pass takes the rows
                                 // of the first round of tiles, the GEMM's own quantiser warps the rest; n > 1 = the pass
@@ -80,6 +83,17 @@ bool w8a16_swap_eligible(int64_t M, int64_t N) {
     const int wide = (N + 127) / 128 >= fp8lin::sm_count();
     const int min_m = g_tune.w8a16_swap_min_m >= 0 ? g_tune.w8a16_swap_min_m : (wide ? 33 : 17);
     return g_tune.w8a16_swap_enable != 0 && M >= min_m && M <= 64;
+}
+
+// W8A16 on CTA pairs with the weights widened into tensor memory and the caller's bf16 rows as the other operand.
+// A knob that selects one of the other W8A16 routes switches it off.
+bool w8a16_pair_eligible(int64_t M, int64_t N, int64_t ldy, const void* y) {
+    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return false;             // (two channels per store)
+    if (g_tune.w8a16_pair >= 0) return g_tune.w8a16_pair != 0;
+    if (g_tune.w8a16_umma_min_m >= 0 || g_tune.w8a16_chunk_mb > 0 || g_tune.w8a16_swap_min_m >= 0 || g_tune.w8a16_swap_enable >= 0 ||
+        g_tune.stream_splits > 0 || g_tune.swap_splits > 0)
+        return false;
+    return M >= 65;
 }
 
 // Large-M W8A16: channel chunks of the weights are widened to f16 into scratch (small enough to stay
@@ -319,6 +333,17 @@ int fp8lin_w8a16(const void* x, int64_t ldx, const void* w_nk, const float* w_sc
                  void* stream) {
     int rc = validate_common(x, ldx, w_nk, w_scale, bias, y, ldy, M, K, N);
     if (rc != FP8LIN_OK || M == 0) return rc;
+    if (workspace && workspace_bytes >= FP8LIN_WS_HEADER_BYTES && w8a16_pair_eligible(M, N, ldy, y)) {
+        const W8a16PairPlan pl = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
+        UmmaArgs a;
+        a.xq = nullptr; a.w = (const unsigned char*)w_nk; a.w_scale = w_scale; a.input_scale = nullptr;
+        a.bias = (const __nv_bfloat16*)bias; a.y = (__nv_bfloat16*)y; a.partial = nullptr; a.counters = nullptr;
+        a.status = ws_view(workspace, workspace_bytes).status; a.M = (int)M; a.K = (int)K; a.N = (int)N; a.ldy = (int)ldy;
+        const char* why = nullptr;
+        cudaError_t e = launch_w8a16_pair(pl, a, x, ldx, (cudaStream_t)stream, &why);
+        if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "tcgen05 W8A16 pair kernel launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
+        return FP8LIN_OK;
+    }
     if (w8a16_swap_eligible(M, N) && workspace) {
         SwapPlan sp = plan_swap_w8a16(M, K, N, g_tune.swap_splits);
         UmmaArgs a;
@@ -739,6 +764,16 @@ const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N) {
     return buf;
 }
 
+const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N) {
+    static thread_local char buf[64];
+    if (M > 0 && K > 0 && N > 0 && scheme == FP8LIN_W8A16 && w8a16_pair_eligible(M, N, 8, nullptr)) {
+        const W8a16PairPlan pl = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
+        snprintf(buf, sizeof(buf), "umma_w8a16_pair_256x%d_s%d", pl.tokens, pl.splits);
+        return buf;
+    }
+    return fp8lin_variant_name(scheme, M, K, N);
+}
+
 int fp8lin_set_tuning(const char* knob, int value) {
     if (!knob) return fail(FP8LIN_ERR_NULL, "knob is NULL");
     if (!strcmp(knob, "stream_splits")) g_tune.stream_splits = value;
@@ -753,6 +788,9 @@ int fp8lin_set_tuning(const char* knob, int value) {
     else if (!strcmp(knob, "w8a16_swap_min_m")) g_tune.w8a16_swap_min_m = value;
     else if (!strcmp(knob, "w8a16_umma_min_m")) g_tune.w8a16_umma_min_m = value;
     else if (!strcmp(knob, "w8a16_chunk_mb")) g_tune.w8a16_chunk_mb = value;
+    else if (!strcmp(knob, "w8a16_pair")) g_tune.w8a16_pair = value;
+    else if (!strcmp(knob, "w8a16_pair_tokens")) g_tune.w8a16_pair_tokens = value;
+    else if (!strcmp(knob, "w8a16_pair_splits")) g_tune.w8a16_pair_splits = value;
     else if (!strcmp(knob, "umma_pair")) g_tune.umma_pair = value;
     else if (!strcmp(knob, "fuse_quant")) g_tune.fuse_quant = value;
     else if (!strcmp(knob, "quant_lead")) g_tune.quant_lead = value;

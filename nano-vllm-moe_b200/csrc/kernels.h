@@ -217,6 +217,18 @@ cudaError_t launch_grouped_rows_w8a8(GroupedArgs args, const void* w_packed, int
 cudaError_t launch_grouped_w8a8(bool gather, int mp, GroupedArgs a, const void* w_packed, int num_experts,
                                 const void* xq_sorted, int64_t xq_rows, cudaStream_t stream, const char** why);
 
+// ---- W8A16 on CTA pairs, weights widened into TMEM, activations as they are (umma_w8a16_pair.cu) ----
+struct W8a16PairPlan {
+    int n_tiles, m_tiles;      // 256-channel tiles, token tiles
+    int tokens;                // tokens per tile: 32..256, a multiple of 32
+    int splits;                // K slices, 1..4 (clusters of 2 * splits CTAs; 1 = persistent pairs)
+    int kblocks_per_split;
+    int grid;
+};
+W8a16PairPlan plan_w8a16_pair(int64_t M, int64_t K, int64_t N, int force_tokens, int force_splits);
+cudaError_t launch_w8a16_pair(const W8a16PairPlan& plan, const UmmaArgs& a, const void* x, int64_t ldx, cudaStream_t stream,
+                              const char** why);
+
 // ---- swapped-operand tcgen05 kernel for W8A16, 9 <= M <= 64 (umma_swap_w8a16.cu) ----
 SwapPlan plan_swap_w8a16(int64_t M, int64_t K, int64_t N, int force_splits);
 cudaError_t launch_swap_w8a16(const SwapPlan& plan, const UmmaArgs& a, const void* x, int64_t ldx,

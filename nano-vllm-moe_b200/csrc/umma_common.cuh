@@ -84,6 +84,75 @@ __device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, ui
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(acc) : "memory");
 }
 
+// ---- issue from a converged warp ---------------------------------------------------------------------------
+// The producer and MMA warps run their loops with all 32 lanes and issue through a predicate that elect.sync gives one lane.
+// Inside `if (lane == 0)` the compiler has to treat every address and descriptor as a per-lane value and moves each one to
+// the uniform registers these instructions take: measured 92 SM cycles per tcgen05.mma and 160 per pair of commits, against
+// 16 and 60 from converged code, which made the issuing thread the limit of every kernel here with small tiles.
+// A wait inside such a loop ends in a vote, so that its exit is uniform too.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t elected, uint32_t bar, uint32_t bytes) {
+    asm volatile(
+        "{\n .reg .b64 st;\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}"
+        ::"r"(bar), "r"(bytes), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d(uint32_t elected, uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+        " @q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n}"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t elected, uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %5, 0;\n"
+        " @q cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n}"
+        ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t elected, uint32_t bar) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}"
+                 ::"r"(bar), "r"(elected) : "memory");
+}
+// arrives on the barrier at this shared-memory offset in every CTA of `mask` once the pair's MMAs issued so far are done
+__device__ __forceinline__ void umma_commit_both(uint32_t elected, uint32_t bar, uint16_t mask) {
+    asm volatile(
+        "{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n"
+        " @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n}"
+        ::"r"(bar), "h"(mask), "r"(elected) : "memory");
+}
+#define FP8LIN_UMMA_SS(NAME, GROUP, KIND)                                                                                     \
+    __device__ __forceinline__ void NAME(uint32_t elected, uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) { \
+        asm volatile(                                                                                                         \
+            "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"                                        \
+            " @q tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, p;\n}"                                     \
+            ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(elected) : "memory");                          \
+    }
+FP8LIN_UMMA_SS(umma_f8, "1", "f8f6f4")
+FP8LIN_UMMA_SS(umma_f16_ss, "1", "f16")
+FP8LIN_UMMA_SS(umma_f8_pair, "2", "f8f6f4")
+FP8LIN_UMMA_SS(umma_f16_pair, "2", "f16")
+#undef FP8LIN_UMMA_SS
+// A from tensor memory
+__device__ __forceinline__ void umma_f16_ts(uint32_t elected, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(elected) : "memory");
+}
+__device__ __forceinline__ void umma_f16_ts_pair(uint32_t elected, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p, q;\n setp.ne.b32 p, %4, 0;\n setp.ne.b32 q, %5, 0;\n"
+        " @q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(elected) : "memory");
+}
+
 // ---- CTA pairs (cta_group::2): one MMA spans the tensor cores, shared memory and TMEM of two CTAs ----
 // Every collective below is executed by the same warp of BOTH CTAs of the pair.
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t cols) {

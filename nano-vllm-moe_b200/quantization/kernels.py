@@ -69,6 +69,11 @@ def variant_name(scheme: int, m: int, k: int, n: int) -> str:
     return _lib.load().fp8lin_variant_name(scheme, m, k, n).decode()
 
 
+def kernel_name(scheme: int, m: int, k: int, n: int) -> str:
+    """The kernel an aligned call of this shape runs (``variant_name`` names the route behind it)."""
+    return _lib.load().fp8lin_kernel_name(scheme, m, k, n).decode()
+
+
 def set_tuning(knob: str, value: int) -> None:
     _lib.raise_for(_lib.load().fp8lin_set_tuning(knob.encode(), int(value)), "fp8lin_set_tuning")
 
