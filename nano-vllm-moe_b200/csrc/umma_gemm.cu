@@ -149,7 +149,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     __shared__ __align__(16) __nv_bfloat16 s_bias[BN];
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     // In split mode a cluster shares one tile: tile = cluster id, K slice = rank in the cluster.
@@ -180,9 +180,12 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         quant_worker(qjob, p.input_scale, p.M, p.K, lane);
     } else if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
+        {
+            const uint32_t el = elect_one();
+            if (el) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
+            }
             uint32_t it = 0;
             bool ok = true;
             bool waited = false;      // weight tiles of the first ring pass go out before the predecessor is done
@@ -199,46 +202,47 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     const int first_kb = min(kb1 - kb0, S);
                     for (int i = 0; i < first_kb; ++i) {
                         const uint32_t full = smem_u32(&bar_full[i]);
-                        mbar_expect_tx(full, stage_tx);
+                        mbar_expect_tx(el, full, stage_tx);
 #pragma unroll
                         for (int sub = 0; sub < nsub; ++sub) {
                             const int n_sub = wk.n0 + sub * 128;
                             const int wrow = ((n_sub >> 7) * sched.kblocks_total + kb0 + i) * 128 + (n_sub & 127);
-                            tma_load_2d(smem_base + i * Cfg::kStageBytes + Cfg::kABytes + sub * 128 * kBK, &tmap_b, 0, wrow, full);
+                            tma_load_2d(el, smem_base + i * Cfg::kStageBytes + Cfg::kABytes + sub * 128 * kBK, &tmap_b, 0, wrow, full);
                         }
                     }
                     pdl_wait();       // the quantised activations are written by the kernel before this one
-                    if (kFuseQ && !quant_wait_block(qjob, p.M, tm, p.status)) { s_abort = 1; ok = false; break; }
+                    if (kFuseQ) ok = __all_sync(0xffffffffu, quant_wait_block(qjob, p.M, tm, p.status));
+                    if (!ok) { s_abort = 1; break; }
                     if (kFuseQ && w + work_step < sched.total_work)
-                        next_ready = quant_probe_block(qjob, p.M, decode_work<BN, kNarrow>(sched, w + work_step).tm);
+                        next_ready = __all_sync(0xffffffffu, quant_probe_block(qjob, p.M, decode_work<BN, kNarrow>(sched, w + work_step).tm));
                     for (int i = 0; i < first_kb; ++i)
-                        tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_a, (kb0 + i) * kBK, tm * kBM, smem_u32(&bar_full[i]));
+                        tma_load_2d(el, smem_base + i * Cfg::kStageBytes, &tmap_a, (kb0 + i) * kBK, tm * kBM, smem_u32(&bar_full[i]));
                     waited = true;
                     it = (uint32_t)first_kb;
                     if (kb0 + first_kb >= kb1) continue;
                 } else if (kFuseQ) {
                     if (next_ready) fence_proxy_async_all();
-                    else if (s_abort || !quant_wait_block(qjob, p.M, tm, p.status)) { s_abort = 1; ok = false; break; }
-                    next_ready = w + work_step < sched.total_work &&
-                                 quant_probe_block(qjob, p.M, decode_work<BN, kNarrow>(sched, w + work_step).tm);
+                    else ok = __all_sync(0xffffffffu, !s_abort && quant_wait_block(qjob, p.M, tm, p.status));
+                    if (!ok) { s_abort = 1; break; }
+                    next_ready = __all_sync(0xffffffffu, w + work_step < sched.total_work &&
+                                 quant_probe_block(qjob, p.M, decode_work<BN, kNarrow>(sched, w + work_step).tm));
                 }
                 for (int kb = kb0 + (w == first_work ? min(kb1 - kb0, S) : 0); kb < kb1; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty));
+                    if (!ok) { s_abort = 1; break; }
                     const uint32_t full = smem_u32(&bar_full[st]);
-                    mbar_expect_tx(full, stage_tx);
+                    mbar_expect_tx(el, full, stage_tx);
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
-                    tma_load_2d(sa, &tmap_a, kb * kBK, tm * kBM, full);
+                    tma_load_2d(el, sa, &tmap_a, kb * kBK, tm * kBM, full);
                     // packed weights: the tile of channel block cb and K block kb is rows
                     // [(cb*KB + kb)*128, +128) of a [tiles*128][128-byte] matrix
 #pragma unroll
                     for (int sub = 0; sub < nsub; ++sub) {
                         const int n_sub = wk.n0 + sub * 128;
                         const int wrow = ((n_sub >> 7) * sched.kblocks_total + kb) * 128 + (n_sub & 127);
-                        tma_load_2d(sa + Cfg::kABytes + sub * 128 * kBK, &tmap_b, 0, wrow, full);
+                        tma_load_2d(el, sa + Cfg::kABytes + sub * 128 * kBK, &tmap_b, 0, wrow, full);
                     }
                 }
             }
@@ -250,7 +254,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc_full = make_idesc<BN>();
             uint32_t it = 0;
             int tl = 0;
@@ -263,17 +268,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 // a half tile is the same instruction with N = 128
                 const uint32_t idesc = (kNarrow && w >= sched.narrow_from)
                                            ? ((idesc_full & ~(0x3fu << 17)) | ((128u >> 3) << 17)) : idesc_full;
-                if (s_abort || !mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty)) {
-                    s_abort = 1; ok = false; break;
-                }
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * BN;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull));
+                    if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
                     const uint64_t da = make_smem_desc(sa);
@@ -281,12 +284,12 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
                     for (int k = 0; k < kBK / 32; ++k) {
                         // advance 32 bytes along K inside the 128-byte swizzle span: +2 in 16-byte units
-                        if (kF16) umma_f16_ss(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-                        else umma_f8(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        if (kF16) umma_f16_ss(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        else umma_f8(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    umma_commit(smem_u32(&bar_empty[st]));
+                    umma_commit(el, smem_u32(&bar_empty[st]));
                 }
-                if (ok) umma_commit(smem_u32(&bar_tfull[as]));
+                if (ok) umma_commit(el, smem_u32(&bar_tfull[as]));
             }
         }
     } else {

@@ -68,7 +68,7 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     __shared__ volatile int s_abort;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -90,34 +90,37 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     pdl_launch_dependents();
     pdl_wait();                                   // the chunk list, the rows and the outputs all come from predecessors
 
-    const int n_chunks = p.meta[0];
+    const int n_chunks = __shfl_sync(0xffffffffu, p.meta[0], 0);
     const int total = n_chunks * p.n_tiles;       // item w = chunk * n_tiles + tile
     const int KB = p.kblocks;
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-            if (!kGather) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_xq) : "memory");
+        {
+            const uint32_t el = elect_one();
+            if (el) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+                if (!kGather) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_xq) : "memory");
+            }
             uint32_t it = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-                const int4 ch = p.chunks[w / p.n_tiles];
+                const int4 chunk = p.chunks[w / p.n_tiles];
+                const int2 ch = make_int2(__shfl_sync(0xffffffffu, chunk.x, 0), __shfl_sync(0xffffffffu, chunk.y, 0));     // (uniform)
                 const int t = w % p.n_tiles;
                 const int wrow0 = (ch.x * p.w_tiles + t) * KB;        // packed tile index of (expert, tile, kb = 0)
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty));
+                    if (!ok) { s_abort = 1; break; }
                     const uint32_t full = smem_u32(&bar_full[st]);
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
-                    mbar_expect_tx(full, kGather ? Cfg::kWBytes : Cfg::kWTiles * Cfg::kWBytes + Cfg::kXqBytes);
-                    tma_load_2d(sa, &tmap_w, 0, (wrow0 + kb) * kGrpTile, full);
+                    mbar_expect_tx(el, full, kGather ? Cfg::kWBytes : Cfg::kWTiles * Cfg::kWBytes + Cfg::kXqBytes);
+                    tma_load_2d(el, sa, &tmap_w, 0, (wrow0 + kb) * kGrpTile, full);
                     // fused: the up tile of the same channels sits up_tile_offset tile rows further on in the expert's weight
-                    if (kFused) tma_load_2d(sa + Cfg::kWBytes, &tmap_w, 0, (wrow0 + p.up_tile_offset * KB + kb) * kGrpTile, full);
-                    if (!kGather) tma_load_2d(sa + Cfg::kWTiles * Cfg::kWBytes, &tmap_xq, kb * kGrpKB, ch.y, full);
+                    if (kFused) tma_load_2d(el, sa + Cfg::kWBytes, &tmap_w, 0, (wrow0 + p.up_tile_offset * KB + kb) * kGrpTile, full);
+                    if (!kGather) tma_load_2d(el, sa + Cfg::kWTiles * Cfg::kWBytes, &tmap_xq, kb * kGrpKB, ch.y, full);
                 }
             }
             if (!ok) {
@@ -127,7 +130,8 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc = make_idesc_mn(kGrpTile, MP, 0, 0);
             uint32_t it = 0;
             int tl = 0;
@@ -135,31 +139,29 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++tl) {
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
-                if (s_abort || !mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty)) {
-                    s_abort = 1; ok = false; break;
-                }
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * Cfg::kAccCols;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull) ||
-                        (kGather && !mbar_wait(smem_u32(&bar_xq[st]), ph, p.status, kDevTimeoutFull))) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull) &&
+                                                     (!kGather || mbar_wait(smem_u32(&bar_xq[st]), ph, p.status, kDevTimeoutFull)));
+                    if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
                     const uint64_t da = make_smem_desc(sa);
                     const uint64_t db = make_smem_desc(sa + Cfg::kWTiles * Cfg::kWBytes);
 #pragma unroll
                     for (int k = 0; k < kGrpKB / 32; ++k) {
-                        umma_f8(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        umma_f8(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                         if (kFused)        // the up tile against the same rows, into the second half of the accumulator stage
-                            umma_f8(d_tmem + MP, make_smem_desc(sa + Cfg::kWBytes) + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                            umma_f8(el, d_tmem + MP, make_smem_desc(sa + Cfg::kWBytes) + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     }
-                    umma_commit(smem_u32(&bar_empty[st]));
+                    umma_commit(el, smem_u32(&bar_empty[st]));
                 }
-                if (ok) umma_commit(smem_u32(&bar_tfull[as]));
+                if (ok) umma_commit(el, smem_u32(&bar_tfull[as]));
             }
         }
     } else if (warp < 2 + kGrpConvWarps) {

@@ -50,7 +50,7 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     __shared__ __align__(16) float s_scale[kColsN];
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -68,7 +68,7 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     pdl_launch_dependents();
     pdl_wait();                                   // the chunk list, the rows and the outputs all come from predecessors
 
-    const int n_chunks = p.meta[0];
+    const int n_chunks = __shfl_sync(0xffffffffu, p.meta[0], 0);
     const int n_items = p.n_tiles;                // channel items per chunk (set by the launcher)
     const int total = n_chunks * n_items;         // item w = chunk * n_items + t
     const int KB = p.kblocks;
@@ -78,27 +78,30 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_xq) : "memory");
+        {
+            const uint32_t el = elect_one();
+            if (el) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_xq) : "memory");
+            }
             uint32_t it = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
-                const int4 ch = p.chunks[w / n_items];
+                const int4 chunk = p.chunks[w / n_items];
+                const int2 ch = make_int2(__shfl_sync(0xffffffffu, chunk.x, 0), __shfl_sync(0xffffffffu, chunk.y, 0));     // (uniform)
                 const int t = w % n_items;
                 const int ns = n_sub(t);
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty));
+                    if (!ok) { s_abort = 1; break; }
                     const uint32_t full = smem_u32(&bar_full[st]);
                     const uint32_t sa = smem_base + st * kStageBytesR;
-                    mbar_expect_tx(full, (uint32_t)(kABytesR + ns * kRowsM * kKB));
-                    tma_load_2d(sa, &tmap_xq, kb * kKB, ch.y, full);
+                    mbar_expect_tx(el, full, (uint32_t)(kABytesR + ns * kRowsM * kKB));
+                    tma_load_2d(el, sa, &tmap_xq, kb * kKB, ch.y, full);
                     for (int s = 0; s < ns; ++s)
-                        tma_load_2d(sa + kABytesR + s * 128 * kKB, &tmap_w, 0, ((ch.x * p.w_tiles + sub_tile(t, s)) * KB + kb) * 128, full);
+                        tma_load_2d(el, sa + kABytesR + s * 128 * kKB, &tmap_w, 0, ((ch.x * p.w_tiles + sub_tile(t, s)) * KB + kb) * 128, full);
                 }
             }
             if (!ok) {
@@ -108,7 +111,8 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             uint32_t it = 0;
             int tl = 0;
             bool ok = true;
@@ -117,26 +121,24 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 const uint32_t idesc = make_idesc_mn(kRowsM, n_sub(t) * 128, 0, 0);
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
-                if (s_abort || !mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty)) {
-                    s_abort = 1; ok = false; break;
-                }
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * kColsN;
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull));
+                    if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + st * kStageBytesR;
                     const uint64_t da = make_smem_desc(sa);
                     const uint64_t db = make_smem_desc(sa + kABytesR);
 #pragma unroll
-                    for (int k = 0; k < kKB / 32; ++k) umma_f8(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    umma_commit(smem_u32(&bar_empty[st]));
+                    for (int k = 0; k < kKB / 32; ++k) umma_f8(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    umma_commit(el, smem_u32(&bar_empty[st]));
                 }
-                if (ok) umma_commit(smem_u32(&bar_tfull[as]));
+                if (ok) umma_commit(el, smem_u32(&bar_tfull[as]));
             }
         }
     } else {

@@ -11,7 +11,7 @@
 // Barriers (per CTA unless noted):
 //   full[s]   (used in the leader only)  both CTAs' TMA loads complete their bytes on the LEADER's
 //             barrier; the leader's producer thread arms it with the byte count of both.
-//   empty[s]  the MMA thread commits to the barrier of the same name in both CTAs (two commits), so each
+//   empty[s]  the MMA warp commits to the barrier of the same name in both CTAs (one multicast commit), so each
 //             producer refills its own stage.
 //   tfull[a]  likewise committed to both CTAs after the last K block: the epilogue warps of each CTA
 //             read their own tensor memory.
@@ -86,7 +86,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     __shared__ __align__(16) __nv_bfloat16 s_bias[kBN];
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();          // 0 = leader
     const bool leader = rank == 0;
@@ -117,9 +117,12 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         quant_worker(qjob, p.input_scale, p.M, p.K, lane);
     } else if (warp == 0) {
         // ================= TMA producer (both CTAs) =================
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
+        {
+            const uint32_t el = elect_one();
+            if (el) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_a) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_b) : "memory");
+            }
             pdl_wait();            // the activations (and, for f16, the weight tiles) come from the kernel before
             uint32_t it = 0;
             bool ok = true;
@@ -131,29 +134,29 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 const int n_sub = tn * kBN + (int)rank * 128;             // this CTA's 128 channels
                 if (kFuseQ) {
                     if (next_ready) fence_proxy_async_all();
-                    else if (s_abort || !quant_wait_block(qjob, p.M, 2 * tmp + (int)rank, p.status)) { s_abort = 1; ok = false; break; }
+                    else ok = __all_sync(0xffffffffu, !s_abort && quant_wait_block(qjob, p.M, 2 * tmp + (int)rank, p.status));
+                    if (!ok) { s_abort = 1; break; }
                     next_ready = false;
                     if (t + tile_step < sched.total) {
                         int ntmp, ntn;
                         decode_pair_tile(sched, t + tile_step, ntmp, ntn);
-                        next_ready = quant_probe_block(qjob, p.M, 2 * ntmp + (int)rank);
+                        next_ready = __all_sync(0xffffffffu, quant_probe_block(qjob, p.M, 2 * ntmp + (int)rank));
                     }
                 }
                 for (int kb = 0; kb < sched.kblocks; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty));
+                    if (!ok) { s_abort = 1; break; }
                     const uint32_t full_local = smem_u32(&bar_full[st]);
-                    if (leader) mbar_expect_tx(full_local, 2 * kStageBytes);
-                    const uint32_t full = leader ? full_local : map_to_cta(full_local, 0);
+                    mbar_expect_tx(leader ? el : 0u, full_local, 2 * kStageBytes);
+                    const uint32_t full = map_to_cta(full_local, 0);
                     const uint32_t sa = smem_base + st * kStageBytes;
-                    tma_load_2d_pair(sa, &tmap_a, kb * kBK, row0, full);
+                    tma_load_2d_pair(el, sa, &tmap_a, kb * kBK, row0, full);
                     // packed weights: the tile of channel block cb and K block kb is rows
                     // [(cb*KB + kb)*128, +128) of a [tiles*128][128-byte] matrix
                     const int wrow = ((n_sub >> 7) * sched.kblocks + kb) * 128;
-                    tma_load_2d_pair(sa + kABytes, &tmap_b, 0, wrow, full);
+                    tma_load_2d_pair(el, sa + kABytes, &tmap_b, 0, wrow, full);
                 }
             }
             if (!ok) {
@@ -163,44 +166,37 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         }
     } else if (warp == 1) {
         // ================= MMA issuer (leader CTA only) =================
-        if (leader && lane == 0) {
+        if (leader) {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc = make_idesc_mn(2 * kBM, kBN, 0, 0);
-            const uint32_t peer = 1;
+            constexpr uint16_t both = 3;                            // the two CTAs of the pair
             uint32_t it = 0;
             int tl = 0;
             bool ok = true;
             for (int t = first_tile; t < sched.total && ok; t += tile_step, ++tl) {
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
-                if (s_abort || !mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty)) {
-                    s_abort = 1; ok = false; break;
-                }
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * kBN;
                 for (int kb = 0; kb < sched.kblocks; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull));
+                    if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + st * kStageBytes;
                     const uint64_t da = make_smem_desc(sa);
                     const uint64_t db = make_smem_desc(sa + kABytes);
 #pragma unroll
                     for (int k = 0; k < kBK / 32; ++k) {
-                        if (kF16) umma_f16_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        else umma_f8_pair(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        if (kF16) umma_f16_pair(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                        else umma_f8_pair(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     }
-                    const uint32_t e = smem_u32(&bar_empty[st]);
-                    umma_commit_pair(e);                        // this CTA's stage is free again ...
-                    umma_commit_pair(map_to_cta(e, peer));      // ... and so is the partner's
+                    umma_commit_both(el, smem_u32(&bar_empty[st]), both);      // this CTA's stage and the partner's are free again
                 }
-                if (ok) {
-                    const uint32_t f = smem_u32(&bar_tfull[as]);
-                    umma_commit_pair(f);
-                    umma_commit_pair(map_to_cta(f, peer));
-                }
+                if (ok) umma_commit_both(el, smem_u32(&bar_tfull[as]), both);
             }
         }
     } else {

@@ -117,7 +117,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     __shared__ volatile int s_abort;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     const int split_rank = kSplit ? (int)cluster_ctarank() : 0;
@@ -186,9 +186,12 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+        {
+            const uint32_t el = elect_one();
+            if (el) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+            }
             uint32_t it = 0;
             bool ok = true;
             // First pass over the ring: the weight tiles go out at once; the activation blocks
@@ -197,13 +200,13 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             if (first_tile < sched.n_tiles) {
                 for (int i = 0; i < first_kb; ++i) {
                     const uint32_t full = smem_u32(&bar_full[i]);
-                    mbar_expect_tx(full, Cfg::kWBytes + x_bytes);   // the x box holds the M real rows only
-                    tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, 0,
+                    mbar_expect_tx(el, full, Cfg::kWBytes + x_bytes);   // the x box holds the M real rows only
+                    tma_load_2d(el, smem_base + i * Cfg::kStageBytes, &tmap_w, 0,
                                 (first_tile * sched.kblocks_total + kb0 + i) * kTileN, full);   // one packed tile
                 }
                 pdl_wait();
                 for (int i = 0; i < first_kb; ++i)
-                    tma_load_2d(smem_base + i * Cfg::kStageBytes + kXDst, &tmap_x,
+                    tma_load_2d(el, smem_base + i * Cfg::kStageBytes + kXDst, &tmap_x,
                                 (kb0 + i) * kKB, 0, smem_u32(&bar_full[i]));
             }
             for (int tl = 0; ok; ++tl) {
@@ -213,14 +216,13 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     if (it < (uint32_t)first_kb) continue;                       // issued above
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty));
+                    if (!ok) { s_abort = 1; break; }
                     const uint32_t full = smem_u32(&bar_full[st]);
-                    mbar_expect_tx(full, Cfg::kWBytes + x_bytes);
+                    mbar_expect_tx(el, full, Cfg::kWBytes + x_bytes);
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
-                    tma_load_2d(sa, &tmap_w, 0, (t * sched.kblocks_total + kb) * kTileN, full);
-                    tma_load_2d(sa + kXDst, &tmap_x, kb * kKB, 0, full);
+                    tma_load_2d(el, sa, &tmap_w, 0, (t * sched.kblocks_total + kb) * kTileN, full);
+                    tma_load_2d(el, sa + kXDst, &tmap_x, kb * kKB, 0, full);
                 }
             }
             if (!ok) {
@@ -230,7 +232,8 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc = make_idesc_mn(kTileN, MP, 0, 0);
             uint32_t it = 0;
             bool ok = true;
@@ -238,28 +241,26 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 if (tile_of(tl) >= sched.n_tiles) break;
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
-                if (s_abort || !mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty)) {
-                    s_abort = 1; ok = false; break;
-                }
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * MP;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull) ||
-                        (!kPreQ && !mbar_wait(smem_u32(&bar_xq[st]), ph, p.status, kDevTimeoutFull))) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[st]), ph, p.status, kDevTimeoutFull) &&
+                                                     (kPreQ || mbar_wait(smem_u32(&bar_xq[st]), ph, p.status, kDevTimeoutFull)));
+                    if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
                     const uint64_t da = make_smem_desc(sa);
                     const uint64_t db = make_smem_desc(sa + Cfg::kWBytes);
 #pragma unroll
                     for (int k = 0; k < kKB / 32; ++k)
-                        umma_f8(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-                    umma_commit(smem_u32(&bar_empty[st]));
+                        umma_f8(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                    umma_commit(el, smem_u32(&bar_empty[st]));
                 }
-                if (ok) umma_commit(smem_u32(&bar_tfull[as]));
+                if (ok) umma_commit(el, smem_u32(&bar_tfull[as]));
             }
         }
     } else if (warp < 2 + kConvWarps) {

@@ -54,13 +54,6 @@ struct Swap16Sched {
     int n_tiles, splits, kblocks_total, kblocks_per_split;
 };
 
-__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc) : "memory");
-}
-
 // 64 consecutive 32-bit TMEM columns of this lane <- 64 registers
 __device__ __forceinline__ void tmem_st64(uint32_t taddr, const uint32_t* v) {
     asm volatile(
@@ -114,7 +107,7 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     __shared__ volatile int s_abort;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index();
     const int lane = threadIdx.x & 31;
 
     const int split_rank = kSplit ? (int)cluster_ctarank() : 0;
@@ -173,22 +166,25 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
     if (warp == 0) {
         // ================= TMA producer =================
-        if (lane == 0) {
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-            asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+        {
+            const uint32_t el = elect_one();
+            if (el) {
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_x) : "memory");
+            }
             uint32_t it = 0;
             bool ok = true;
             const int first_kb = min(kb1 - kb0, S);
             if (first_tile < sched.n_tiles) {
                 for (int i = 0; i < first_kb; ++i) {           // weights do not depend on the predecessor
                     const uint32_t full = smem_u32(&bar_full[i]);
-                    mbar_expect_tx(full, Cfg::kWBytes + x_bytes);
-                    tma_load_2d(smem_base + i * Cfg::kStageBytes, &tmap_w, 0,
+                    mbar_expect_tx(el, full, Cfg::kWBytes + x_bytes);
+                    tma_load_2d(el, smem_base + i * Cfg::kStageBytes, &tmap_w, 0,
                                 (first_tile * sched.kblocks_total + kb0 + i) * kS16Tile, full);
                 }
                 pdl_wait();
                 for (int i = 0; i < first_kb; ++i)
-                    tma_load_2d(smem_base + i * Cfg::kStageBytes + kXrawOff, &tmap_x, (kb0 + i) * kS16KB, 0,
+                    tma_load_2d(el, smem_base + i * Cfg::kStageBytes + kXrawOff, &tmap_x, (kb0 + i) * kS16KB, 0,
                                 smem_u32(&bar_full[i]));
             }
             for (int t = first_tile; t < sched.n_tiles && ok; t += tile_step) {
@@ -196,14 +192,13 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     if (it < (uint32_t)first_kb) continue;
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_empty[st]), ph ^ 1, p.status, kDevTimeoutEmpty));
+                    if (!ok) { s_abort = 1; break; }
                     const uint32_t full = smem_u32(&bar_full[st]);
-                    mbar_expect_tx(full, Cfg::kWBytes + x_bytes);
+                    mbar_expect_tx(el, full, Cfg::kWBytes + x_bytes);
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
-                    tma_load_2d(sa, &tmap_w, 0, (t * sched.kblocks_total + kb) * kS16Tile, full);
-                    tma_load_2d(sa + kXrawOff, &tmap_x, kb * kS16KB, 0, full);
+                    tma_load_2d(el, sa, &tmap_w, 0, (t * sched.kblocks_total + kb) * kS16Tile, full);
+                    tma_load_2d(el, sa + kXrawOff, &tmap_x, kb * kS16KB, 0, full);
                 }
             }
             if (!ok) {
@@ -213,7 +208,8 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
     } else if (warp == 1) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        {
+            const uint32_t el = elect_one();
             constexpr uint32_t idesc = make_idesc_mn(kS16Tile, MP, 0, 0);      // A, B = f16
             uint32_t it = 0;
             int tl = 0;
@@ -221,17 +217,15 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             for (int t = first_tile; t < sched.n_tiles && ok; t += tile_step, ++tl) {
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
-                if (s_abort || !mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty)) {
-                    s_abort = 1; ok = false; break;
-                }
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * MP;
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
-                    if (s_abort || !mbar_wait(smem_u32(&bar_conv[st]), ph, p.status, kDevTimeoutFull)) {
-                        s_abort = 1; ok = false; break;
-                    }
+                    ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_conv[st]), ph, p.status, kDevTimeoutFull));
+                    if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t xf = smem_base + st * Cfg::kStageBytes + kXfOff;
                     const uint32_t a_t = tmem_a0 + st * Cfg::kACols;
@@ -240,11 +234,11 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                         // K = 16 f16 per MMA: 8 TMEM columns of A; 32 bytes inside the 128-byte swizzle
                         // span of the B half-tile (four steps per half)
                         const uint64_t db = make_smem_desc(xf + (k >> 2) * (MP * 128)) + 2 * (k & 3);
-                        umma_f16_ts(d_tmem, a_t + k * 8, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        umma_f16_ts(el, d_tmem, a_t + k * 8, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
                     }
-                    umma_commit(smem_u32(&bar_empty[st]));
+                    umma_commit(el, smem_u32(&bar_empty[st]));
                 }
-                if (ok) umma_commit(smem_u32(&bar_tfull[as]));
+                if (ok) umma_commit(el, smem_u32(&bar_tfull[as]));
             }
         }
     } else if (warp < 2 + kS16ConvWarps) {
