@@ -205,6 +205,9 @@ int fp8lin_quantize_activation(const void* x, int64_t ldx, const float* input_sc
 int fp8lin_moe_route(const void* logits, int logits_dtype, int64_t ld, int64_t T, int E, int top_k,
                      int renormalize, float* topk_w, int32_t* topk_ids, void* stream);
 
+/* fp8lin_moe_route with 64-bit expert ids (the type torch's topk returns). */
+int fp8lin_moe_route_i64(const void* logits, int logits_dtype, int64_t ld, int64_t T, int E, int top_k, int renormalize,
+                         float* topk_w, int64_t* topk_ids, void* stream);
 /* Grouping of routed rows by expert, the first step of fp8lin_moe_experts_w8a8, also callable on its
  * own; replaces moe_align_block_size (nanovllm/utils/moe.py:4-52).  ids: int32 [rows] expert id per
  * routed row (ids outside [0, E) are dropped: another expert-parallel rank owns them).  Outputs, all
@@ -238,6 +241,15 @@ int fp8lin_moe_experts_w8a8(const void* x, int64_t ldx, int x_div, const int32_t
 /* y[t] = bf16( sum_j routed[t*top_k + j] ) in slot order; replaces the .view(T,k,H).sum(1) of
  * NoEPPrepareFinalize.finalize (no_ep.py:45) / TorchAllToAllPrepareFinalize.finalize (:90). */
 int fp8lin_moe_combine(const void* routed, void* y, int64_t T, int top_k, int64_t H, void* stream);
+/* The whole expert FFN of T tokens whose experts are all local: grouping, fp8lin_moe_experts_w8a8 on x_div = top_k and
+ * fp8lin_moe_combine in one call.  topk_ids [T][top_k] 32- or 64-bit (ids_are_i64); an id outside [0, E) adds nothing to its
+ * token.  y: bf16 [T][ld_y], 16-byte aligned, ld_y a multiple of 8. */
+size_t fp8lin_moe_block_workspace_bytes(int64_t T, int top_k, int E, int64_t H, int64_t I);
+int fp8lin_moe_block_w8a8(const void* x, int64_t ldx, const void* topk_ids, int ids_are_i64, const float* topk_w, int64_t T, int top_k,
+                          const void* w13_packed, const float* w13_scale, const float* w13_input_scale,
+                          const void* w2_packed, const float* w2_scale, const float* w2_input_scale,
+                          int E, int64_t H, int64_t I, void* y, int64_t ld_y, void* workspace, size_t workspace_bytes, void* stream);
+
 
 /* ---- exporter arithmetic -----------------------------------------------------------------
  * fp8lin_quantize_weight replaces quantize_fp8_per_output_channel of the checkpoint exporter

@@ -810,7 +810,7 @@ namespace {
 // instead of inside the gate_up GEMM (where every channel tile would redo it)
 constexpr int64_t kMoePrequantRows = 512;
 struct MoeWs {
-    size_t off_offsets, off_sorted, off_chunks, off_meta, off_gu, off_hq, off_xq, total;
+    size_t off_offsets, off_sorted, off_chunks, off_meta, off_inv, off_gu, off_hq, off_xq, total;
 };
 MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
     MoeWs w;
@@ -820,6 +820,7 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
     w.off_sorted = take((size_t)(rows > 0 ? rows : 1) * 4);
     w.off_chunks = take((size_t)(E + rows / 16 + 2) * 16);
     w.off_meta = take(16);
+    w.off_inv = take((size_t)(rows > 0 ? rows : 1) * 4);
     w.off_gu = take((size_t)rows * 2 * I * 2);
     w.off_hq = take((size_t)rows * I);
     w.off_xq = take(rows >= kMoePrequantRows ? (size_t)rows * H : 0);
@@ -828,17 +829,27 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 }
 }  // namespace
 
-int fp8lin_moe_route(const void* logits, int logits_dtype, int64_t ld, int64_t T, int E, int top_k, int renormalize,
-                     float* topk_w, int32_t* topk_ids, void* stream) {
+static int moe_route_impl(const void* logits, int logits_dtype, int64_t ld, int64_t T, int E, int top_k, int renormalize,
+                          float* topk_w, void* topk_ids, bool ids_i64, void* stream) {
     if (T < 0 || E <= 0 || E > 1024 || top_k <= 0 || top_k > 32 || top_k > E || ld < E)
         return fail(FP8LIN_ERR_SHAPE, "bad router shape T=%lld E=%d top_k=%d ld=%lld (E <= 1024, top_k <= 32)",
                     (long long)T, E, top_k, (long long)ld);
     if (logits_dtype != 0 && logits_dtype != 1) return fail(FP8LIN_ERR_ARG, "logits_dtype must be 0 (f32) or 1 (bf16)");
     if (T == 0) return FP8LIN_OK;
     if (!logits || !topk_w || !topk_ids) return fail(FP8LIN_ERR_NULL, "logits, topk_w and topk_ids must not be NULL");
-    cudaError_t e = launch_moe_route(logits, logits_dtype, ld, (int)T, E, top_k, renormalize, topk_w, topk_ids, (cudaStream_t)stream);
+    cudaError_t e = launch_moe_route(logits, logits_dtype, ld, (int)T, E, top_k, renormalize, topk_w, topk_ids, ids_i64, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "router launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
+}
+
+int fp8lin_moe_route(const void* logits, int logits_dtype, int64_t ld, int64_t T, int E, int top_k, int renormalize,
+                     float* topk_w, int32_t* topk_ids, void* stream) {
+    return moe_route_impl(logits, logits_dtype, ld, T, E, top_k, renormalize, topk_w, topk_ids, false, stream);
+}
+
+int fp8lin_moe_route_i64(const void* logits, int logits_dtype, int64_t ld, int64_t T, int E, int top_k, int renormalize,
+                         float* topk_w, int64_t* topk_ids, void* stream) {
+    return moe_route_impl(logits, logits_dtype, ld, T, E, top_k, renormalize, topk_w, topk_ids, true, stream);
 }
 
 int fp8lin_moe_align(const int32_t* ids, int64_t rows, int E, int chunk_rows, int32_t* expert_offsets, int32_t* sorted_rows,
@@ -849,7 +860,7 @@ int fp8lin_moe_align(const int32_t* ids, int64_t rows, int E, int chunk_rows, in
         return fail(FP8LIN_ERR_ARG, "chunk_rows must be 16, 32, 64 or 128");
     if (!ids || !expert_offsets || !sorted_rows || !chunks || !meta) return fail(FP8LIN_ERR_NULL, "a required pointer is NULL");
     if (!aligned16(chunks)) return fail(FP8LIN_ERR_ALIGN, "chunks must be 16-byte aligned");
-    cudaError_t e = launch_moe_align(ids, (int)rows, E, chunk_rows, expert_offsets, sorted_rows, (int4*)chunks, meta,
+    cudaError_t e = launch_moe_align(ids, false, (int)rows, E, chunk_rows, expert_offsets, sorted_rows, (int4*)chunks, meta, nullptr,
                                      (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
@@ -860,7 +871,7 @@ size_t fp8lin_moe_workspace_bytes(int64_t rows, int E, int64_t H, int64_t I) {
     return moe_ws_layout(rows, E, H, I).total;
 }
 
-int fp8lin_moe_experts_w8a8(const void* x, int64_t ldx, int x_div, const int32_t* ids, const float* topk_w, int64_t rows,
+static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* ids, bool ids_i64, const float* topk_w, int64_t rows,
                             const void* w13_packed, const float* w13_scale, const float* w13_input_scale,
                             const void* w2_packed, const float* w2_scale, const float* w2_input_scale,
                             int E, int64_t H, int64_t I, void* out_routed, int64_t ld_out,
@@ -886,10 +897,11 @@ int fp8lin_moe_experts_w8a8(const void* x, int64_t ldx, int x_div, const int32_t
     int* sorted = (int*)(ws + L.off_sorted);
     int4* chunks = (int4*)(ws + L.off_chunks);
     int* meta = (int*)(ws + L.off_meta);
+    int* inv = (int*)(ws + L.off_inv);
     __nv_bfloat16* gu = (__nv_bfloat16*)(ws + L.off_gu);
     unsigned char* hq = ws + L.off_hq;
     const int mp = grouped_chunk_rows(rows, E);
-    cudaError_t e = launch_moe_align(ids, (int)rows, E, mp, offsets, sorted, chunks, meta, st);
+    cudaError_t e = launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
     GroupedArgs a;
@@ -905,8 +917,8 @@ int fp8lin_moe_experts_w8a8(const void* x, int64_t ldx, int x_div, const int32_t
     const bool fused_act = rows >= kMoePrequantRows && I % 128 == 0 && mp >= 32 && g_tune.moe_fused != 0;
     if (rows >= kMoePrequantRows) {
         unsigned char* xq = ws + L.off_xq;
-        e = launch_moe_gather_quant((const __nv_bfloat16*)x, ldx, x_div, sorted, meta, w13_input_scale, xq, (int)rows, (int)H, st);
-        if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row gather launch: %s", cudaGetErrorString(e));
+        e = launch_moe_scatter_quant((const __nv_bfloat16*)x, ldx, x_div, inv, (int)rows, w13_input_scale, xq, (int)H, st);
+        if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row quantiser launch: %s", cudaGetErrorString(e));
         if (fused_act) {
             GroupedArgs f = a;
             f.N = (int)I; f.hq = hq; f.h_scale = w2_input_scale; f.out = nullptr;
@@ -933,12 +945,50 @@ int fp8lin_moe_experts_w8a8(const void* x, int64_t ldx, int x_div, const int32_t
     return FP8LIN_OK;
 }
 
+int fp8lin_moe_experts_w8a8(const void* x, int64_t ldx, int x_div, const int32_t* ids, const float* topk_w, int64_t rows,
+                            const void* w13_packed, const float* w13_scale, const float* w13_input_scale,
+                            const void* w2_packed, const float* w2_scale, const float* w2_input_scale,
+                            int E, int64_t H, int64_t I, void* out_routed, int64_t ld_out,
+                            void* workspace, size_t workspace_bytes, void* stream) {
+    return moe_experts_impl(x, ldx, x_div, ids, false, topk_w, rows, w13_packed, w13_scale, w13_input_scale, w2_packed, w2_scale, w2_input_scale,
+                            E, H, I, out_routed, ld_out, workspace, workspace_bytes, stream);
+}
+
 int fp8lin_moe_combine(const void* routed, void* y, int64_t T, int top_k, int64_t H, void* stream) {
     if (T < 0 || top_k <= 0 || H <= 0 || H % 8 != 0) return fail(FP8LIN_ERR_SHAPE, "bad combine shape");
     if (T == 0) return FP8LIN_OK;
     if (!routed || !y) return fail(FP8LIN_ERR_NULL, "routed and y must not be NULL");
     if (!aligned16(routed) || !aligned16(y)) return fail(FP8LIN_ERR_ALIGN, "routed and y must be 16-byte aligned");
-    cudaError_t e = launch_moe_combine((const __nv_bfloat16*)routed, (__nv_bfloat16*)y, (int)T, top_k, (int)H, (cudaStream_t)stream);
+    cudaError_t e = launch_moe_combine((const __nv_bfloat16*)routed, nullptr, (__nv_bfloat16*)y, H, (int)T, top_k, (int)H, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "combine launch: %s", cudaGetErrorString(e));
+    return FP8LIN_OK;
+}
+
+// The experts' scratch, then the routed rows that the combine reads.
+size_t fp8lin_moe_block_workspace_bytes(int64_t T, int top_k, int E, int64_t H, int64_t I) {
+    if (T < 0 || top_k <= 0 || E <= 0 || H <= 0 || I <= 0) return FP8LIN_WS_HEADER_BYTES;
+    return moe_ws_layout(T * top_k, E, H, I).total + align_up((size_t)(T * top_k) * H * 2, 256);
+}
+
+int fp8lin_moe_block_w8a8(const void* x, int64_t ldx, const void* topk_ids, int ids_are_i64, const float* topk_w, int64_t T, int top_k,
+                          const void* w13_packed, const float* w13_scale, const float* w13_input_scale,
+                          const void* w2_packed, const float* w2_scale, const float* w2_input_scale,
+                          int E, int64_t H, int64_t I, void* y, int64_t ld_y, void* workspace, size_t workspace_bytes, void* stream) {
+    if (T < 0 || top_k <= 0 || top_k > 32) return fail(FP8LIN_ERR_SHAPE, "bad MoE shape T=%lld top_k=%d (top_k <= 32)", (long long)T, top_k);
+    if (T == 0) return FP8LIN_OK;
+    if (!y) return fail(FP8LIN_ERR_NULL, "y must not be NULL");
+    if (ld_y < H || ld_y % 8 != 0 || !aligned16(y)) return fail(FP8LIN_ERR_ALIGN, "y must be 16-byte aligned, ld_y a multiple of 8 and at least H");
+    const int64_t rows = T * top_k;
+    if (rows > (1ll << 24)) return fail(FP8LIN_ERR_SHAPE, "too many routed rows");
+    const MoeWs L = moe_ws_layout(rows, E > 0 ? E : 1, H, I);
+    if (!workspace || workspace_bytes < fp8lin_moe_block_workspace_bytes(T, top_k, E, H, I))
+        return fail(FP8LIN_ERR_WORKSPACE, "workspace too small: need %zu bytes", fp8lin_moe_block_workspace_bytes(T, top_k, E, H, I));
+    __nv_bfloat16* routed = (__nv_bfloat16*)((unsigned char*)workspace + L.total);
+    int rc = moe_experts_impl(x, ldx, top_k, topk_ids, ids_are_i64 != 0, topk_w, rows, w13_packed, w13_scale, w13_input_scale, w2_packed, w2_scale,
+                              w2_input_scale, E, H, I, routed, H, workspace, L.total, stream);
+    if (rc != FP8LIN_OK) return rc;
+    cudaError_t e = launch_moe_combine(routed, (const int*)((unsigned char*)workspace + L.off_inv), (__nv_bfloat16*)y, ld_y, (int)T, top_k, (int)H,
+                                       (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "combine launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
 }

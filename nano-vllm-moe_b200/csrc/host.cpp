@@ -364,6 +364,73 @@ PyObject* py_mlp(PyObject*, PyObject* const* a, Py_ssize_t na) {
     });
 }
 
+// moe_route(logits, top_k, renormalize) -> (weights f32 [T, k], ids i64 [T, k])
+PyObject* py_moe_route(PyObject*, PyObject* const* a, Py_ssize_t na) {
+    return guarded([&]() -> PyObject* {
+        need_args(na, 3, "moe_route");
+        const at::Tensor& l0 = tensor(a[0], "router_logits");
+        const int64_t k = PyLong_AsLongLong(a[1]);
+        const int renormalize = PyObject_IsTrue(a[2]);
+        if (!l0.is_cuda()) throw ValueError("the router kernel needs CUDA tensors (there is no CPU path)");
+        if (l0.dim() != 2 || (l0.scalar_type() != at::kFloat && l0.scalar_type() != at::kBFloat16))
+            throw ValueError("router_logits must be [T, E] float32 or bfloat16");
+        const at::Tensor l = l0.stride(1) == 1 ? l0 : l0.contiguous();
+        const int64_t t = l.size(0), e = l.size(1);
+        const c10::cuda::CUDAGuard device(l.device());
+        const at::Tensor w = at::empty({t, k}, at::TensorOptions().dtype(at::kFloat).device(l.device()));
+        const at::Tensor ids = at::empty({t, k}, at::TensorOptions().dtype(at::kLong).device(l.device()));
+        const auto stream = c10::cuda::getCurrentCUDAStream();
+        const int rc = unlocked([&] {
+            return fp8lin_moe_route_i64(l.const_data_ptr(), l.scalar_type() == at::kBFloat16 ? 1 : 0, l.stride(0), t, (int)e, (int)k, renormalize,
+                                        (float*)w.mutable_data_ptr(), (int64_t*)ids.mutable_data_ptr(), stream.stream());
+        });
+        check(rc, "fp8lin_moe_route");
+        PyObject* r = PyTuple_New(2);
+        if (!r) return nullptr;
+        PyTuple_SET_ITEM(r, 0, THPVariable_Wrap(w));
+        PyTuple_SET_ITEM(r, 1, THPVariable_Wrap(ids));
+        return r;
+    });
+}
+
+// moe_block(x, topk_weights [T, k], topk_ids [T, k], w13, w13_scale, w13_input_scale, w2, w2_scale, w2_input_scale, experts, inter) -> y [T, H]
+PyObject* py_moe_block(PyObject*, PyObject* const* a, Py_ssize_t na) {
+    return guarded([&]() -> PyObject* {
+        need_args(na, 11, "moe_block");
+        const at::Tensor& x = tensor(a[0], "x");
+        const at::Tensor& w0 = tensor(a[1], "topk_weights");
+        const at::Tensor& i0 = tensor(a[2], "topk_ids");
+        const at::Tensor* wt[6];
+        for (int i = 0; i < 6; ++i) { wt[i] = &tensor(a[3 + i], "expert weights"); need_cuda(*wt[i]); }
+        const int64_t experts = PyLong_AsLongLong(a[9]), inter = PyLong_AsLongLong(a[10]);
+        if (!x.is_cuda()) throw ValueError("the expert kernels need CUDA tensors (there is no CPU path)");
+        if (x.scalar_type() != at::kBFloat16 || x.dim() != 2) throw ValueError("x must be a bfloat16 matrix [T, H]");
+        need_cuda(w0);
+        need_cuda(i0);
+        const Rows r = rows_of(x);
+        if (i0.dim() != 2 || i0.size(0) != r.m || w0.sizes() != i0.sizes()) throw ValueError("topk_weights and topk_ids must be [T, k]");
+        const int64_t k = i0.size(1);
+        const bool i64 = i0.scalar_type() == at::kLong;
+        const at::Tensor ids = i64 ? i0.contiguous() : i0.to(at::kInt).contiguous();
+        const at::Tensor w = w0.to(at::kFloat).contiguous();
+        if ((size_t)wt[0]->numel() != (size_t)experts * fp8lin_packed_bytes(r.k, 2 * inter) ||
+            (size_t)wt[3]->numel() != (size_t)experts * fp8lin_packed_bytes(inter, r.k))
+            throw ValueError("the packed expert weights do not match the number of experts, x's width and the intermediate size");
+        const c10::cuda::CUDAGuard device(x.device());
+        const at::Tensor y = at::empty({r.m, r.k}, x.options());
+        const auto stream = c10::cuda::getCurrentCUDAStream();
+        const at::Tensor scr = workspace(stream, fp8lin_moe_block_workspace_bytes(r.m, (int)k, (int)experts, r.k, inter));
+        auto f = [&](int i) { return (const float*)wt[i]->const_data_ptr(); };
+        const int rc = unlocked([&] {
+            return fp8lin_moe_block_w8a8(r.t.const_data_ptr(), r.ld, ids.const_data_ptr(), i64 ? 1 : 0, (const float*)w.const_data_ptr(), r.m, (int)k,
+                                         wt[0]->const_data_ptr(), f(1), f(2), wt[3]->const_data_ptr(), f(4), f(5), (int)experts, r.k, inter,
+                                         y.mutable_data_ptr(), r.k, scr.mutable_data_ptr(), (size_t)scr.numel(), stream.stream());
+        });
+        check(rc, "fp8lin_moe_block_w8a8");
+        return THPVariable_Wrap(y);
+    });
+}
+
 // workspace(device_index, stream_handle, nbytes) -> the stream's scratch tensor
 PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t na) {
     return guarded([&]() -> PyObject* {
@@ -392,6 +459,8 @@ PyMethodDef kMethods[] = {
     {"linear_codes", (PyCFunction)(void (*)(void))py_linear_codes, METH_FASTCALL, nullptr},
     {"rmsnorm_quant", (PyCFunction)(void (*)(void))py_rmsnorm_quant, METH_FASTCALL, nullptr},
     {"mlp", (PyCFunction)(void (*)(void))py_mlp, METH_FASTCALL, nullptr},
+    {"moe_route", (PyCFunction)(void (*)(void))py_moe_route, METH_FASTCALL, nullptr},
+    {"moe_block", (PyCFunction)(void (*)(void))py_moe_block, METH_FASTCALL, nullptr},
     {"workspace", (PyCFunction)(void (*)(void))py_workspace, METH_FASTCALL, nullptr},
     {"release_workspaces", py_release_workspaces, METH_NOARGS, nullptr},
     {nullptr, nullptr, 0, nullptr},

@@ -179,14 +179,15 @@ cudaError_t launch_swap_w8a8(const SwapPlan& plan, const UmmaArgs& a, const void
 
 // ---- MoE expert FFN (moe_kernels.cu, umma_grouped.cu) ------------------------------
 cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, int T, int E, int top_k, int renormalize,
-                             float* out_w, int* out_ids, cudaStream_t stream);
-cudaError_t launch_moe_align(const int* ids, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
-                             int4* chunks, int* meta, cudaStream_t stream);
-cudaError_t launch_moe_gather_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* sorted_rows, const int* meta,
-                                    const float* input_scale, unsigned char* xq, int max_rows, int H, cudaStream_t stream);
+                             float* out_w, void* out_ids, bool ids_i64, cudaStream_t stream);
+cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
+                             int4* chunks, int* meta, int* inv, cudaStream_t stream);
+cudaError_t launch_moe_scatter_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* inv, int rows,
+                                     const float* input_scale, unsigned char* xq, int H, cudaStream_t stream);
 cudaError_t launch_silu_mul_quant(const __nv_bfloat16* gu, const float* input_scale, unsigned char* hq, const int* meta,
                                   int max_rows, int I, cudaStream_t stream);
-cudaError_t launch_moe_combine(const __nv_bfloat16* routed, __nv_bfloat16* y, int T, int top_k, int H, cudaStream_t stream);
+cudaError_t launch_moe_combine(const __nv_bfloat16* routed, const int* inv, __nv_bfloat16* y, int64_t ld_y, int T, int top_k, int H,
+                               cudaStream_t stream);
 
 struct GroupedArgs {
     const __nv_bfloat16* x;      // gather flavour: token matrix [x_rows][ldx]

@@ -9,10 +9,10 @@ namespace fp8lin {
 // warp arg-max (ties go to the lower expert index), optional renormalisation of the k
 // weights.  Same algebra as softmax(dtype=float32) -> topk -> (w / sum w).
 // kMaxPerLane: experts per lane (E <= 32 * kMaxPerLane); small expert counts get a short unrolled loop.
-template <typename LogitT, int kMaxPerLane>
+template <typename LogitT, typename IdT, int kMaxPerLane>
 __global__ void __launch_bounds__(256)
 moe_route_kernel(const LogitT* __restrict__ logits, int64_t ld, int T, int E, int top_k, int renormalize,
-                 float* __restrict__ out_w, int* __restrict__ out_ids) {
+                 float* __restrict__ out_w, IdT* __restrict__ out_ids) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -65,25 +65,42 @@ moe_route_kernel(const LogitT* __restrict__ logits, int64_t ld, int T, int E, in
     }
 }
 
-cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, int T, int E, int top_k, int renormalize,
-                             float* out_w, int* out_ids, cudaStream_t stream) {
+// Every small kernel of the block is a programmatic dependent launch: the next one's CTAs are resident when the previous
+// one ends.
+template <typename... Params, typename... Args>
+static cudaError_t launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    cfg.numAttrs = pdl_attribute(attr);
+    cfg.attrs = attr;
+    return counted(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+}
+
+template <typename IdT>
+static cudaError_t launch_route(const void* logits, int logits_bf16, int64_t ld, int T, int E, int top_k, int renormalize,
+                                float* out_w, IdT* out_ids, cudaStream_t stream) {
     if (T == 0) return cudaSuccess;
     const int warps = 8;
-    dim3 grid((unsigned)((T + warps - 1) / warps));
-#define FP8LIN_ROUTE(PER_)                                                                                                \
-    do {                                                                                                                  \
-        if (logits_bf16)                                                                                                  \
-            moe_route_kernel<__nv_bfloat16, PER_><<<grid, warps * 32, 0, stream>>>((const __nv_bfloat16*)logits, ld, T, E, \
-                                                                                   top_k, renormalize, out_w, out_ids);   \
-        else                                                                                                              \
-            moe_route_kernel<float, PER_><<<grid, warps * 32, 0, stream>>>((const float*)logits, ld, T, E, top_k,         \
-                                                                           renormalize, out_w, out_ids);                  \
-    } while (0)
-    if (E <= 64) FP8LIN_ROUTE(2);
-    else if (E <= 256) FP8LIN_ROUTE(8);
-    else FP8LIN_ROUTE(32);
+    const unsigned grid = (unsigned)((T + warps - 1) / warps);
+#define FP8LIN_ROUTE(PER_)                                                                                                 \
+    (logits_bf16 ? launch_dependent(moe_route_kernel<__nv_bfloat16, IdT, PER_>, grid, warps * 32, 0, stream,               \
+                                    (const __nv_bfloat16*)logits, ld, T, E, top_k, renormalize, out_w, out_ids)            \
+                 : launch_dependent(moe_route_kernel<float, IdT, PER_>, grid, warps * 32, 0, stream, (const float*)logits, \
+                                    ld, T, E, top_k, renormalize, out_w, out_ids))
+    if (E <= 64) return FP8LIN_ROUTE(2);
+    if (E <= 256) return FP8LIN_ROUTE(8);
+    return FP8LIN_ROUTE(32);
 #undef FP8LIN_ROUTE
-    return counted(cudaGetLastError());
+}
+
+cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, int T, int E, int top_k, int renormalize,
+                             float* out_w, void* out_ids, bool ids_i64, cudaStream_t stream) {
+    return ids_i64 ? launch_route(logits, logits_bf16, ld, T, E, top_k, renormalize, out_w, (long long*)out_ids, stream)
+                   : launch_route(logits, logits_bf16, ld, T, E, top_k, renormalize, out_w, (int*)out_ids, stream);
 }
 
 // ---- grouping of routed rows by expert ------------------------------------------------------
@@ -93,88 +110,145 @@ cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, in
 //   expert_offsets[e]    first sorted position of expert e (E+1 entries)
 //   chunks[c]            {expert, first sorted position, rows in chunk, 0}
 //   meta[0] = number of chunks, meta[1] = number of rows that had a valid local expert id
+//   inv[r]               sorted position of routed row r, -1 if its id was not valid (only if inv is given)
 // Rows whose id is outside [0, E) are dropped (they belong to another expert-parallel rank).
+//
+// Every warp counts its own contiguous share of the rows in counters of its own (kWarps x E of them), so that the shared
+// memory atomics of a skewed or large batch collide inside a warp only; then the counters become running positions
+// (scan over experts, inside an expert over warps) and the warps place their rows.  Against one set of E counters and a
+// serial scan by one thread: 17.6 -> 5 us for 16384 rows of 60 experts, 5.7 -> 3.3 us for 256 rows.
+template <typename IdT, int kWarps>
 __global__ void __launch_bounds__(1024)
-moe_align_kernel(const int* __restrict__ ids, int rows, int E, int chunk_rows, int* __restrict__ expert_offsets,
-                 int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta) {
+moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, int* __restrict__ expert_offsets,
+                 int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta, int* __restrict__ inv) {
     pdl_launch_dependents();
-    pdl_wait();
     extern __shared__ int sh[];
-    int* count = sh;            // [E]
-    int* start = sh + E;        // [E + 1]
-    int* fill = sh + 2 * E + 1; // [E]
-    int* cstart = sh + 3 * E + 1;  // [E + 1] chunk prefix
-    for (int e = threadIdx.x; e < E; e += blockDim.x) { count[e] = 0; fill[e] = 0; }
+    int* count = sh;                       // [kWarps][E]: rows of expert e in warp w's share, then their next position
+    int* total = sh + kWarps * E;          // [E]
+    int* start = total + E;                // [E + 1]
+    int* cstart = start + E + 1;           // [E + 1] chunk prefix
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < kWarps * E; i += blockDim.x) count[i] = 0;
+    const int share = ((rows + kWarps * 32 - 1) / (kWarps * 32)) * 32;
+    const int r0 = warp * share, r1 = min(rows, r0 + share);
+    pdl_wait();
     __syncthreads();
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-        const int e = ids[r];
-        if (e >= 0 && e < E) atomicAdd(&count[e], 1);
+    if (warp < kWarps) {
+        int* mine = count + warp * E;
+#pragma unroll 4
+        for (int r = r0 + lane; r < r1; r += 32) {
+            const long long e = (long long)ids[r];
+            if (e >= 0 && e < E) atomicAdd(&mine[e], 1);
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0, cacc = 0;
-        for (int e = 0; e < E; ++e) {
-            start[e] = acc; cstart[e] = cacc;
-            acc += count[e];
-            cacc += (count[e] + chunk_rows - 1) / chunk_rows;
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        int acc = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) { const int c = count[w * E + e]; count[w * E + e] = acc; acc += c; }
+        total[e] = acc;
+    }
+    __syncthreads();
+    if (warp == 0) {                       // exclusive scans of rows and chunks over the experts
+        int row_base = 0, chunk_base = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int n = e0 + lane < E ? total[e0 + lane] : 0;
+            const int c = (n + chunk_rows - 1) / chunk_rows;
+            int sn = n, sc = c;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int pn = __shfl_up_sync(0xffffffffu, sn, o), pc = __shfl_up_sync(0xffffffffu, sc, o);
+                if (lane >= o) { sn += pn; sc += pc; }
+            }
+            if (e0 + lane < E) { start[e0 + lane] = row_base + sn - n; cstart[e0 + lane] = chunk_base + sc - c; }
+            row_base += __shfl_sync(0xffffffffu, sn, 31);
+            chunk_base += __shfl_sync(0xffffffffu, sc, 31);
         }
-        start[E] = acc; cstart[E] = cacc;
-        meta[0] = cacc; meta[1] = acc;
+        if (lane == 0) { start[E] = row_base; cstart[E] = chunk_base; meta[0] = chunk_base; meta[1] = row_base; }
     }
     __syncthreads();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = start[e];
-    for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-        const int e = ids[r];
-        if (e >= 0 && e < E) sorted_rows[start[e] + atomicAdd(&fill[e], 1)] = r;
+    if (warp < kWarps) {
+        int* mine = count + warp * E;
+#pragma unroll 4
+        for (int r = r0 + lane; r < r1; r += 32) {
+            const long long e = (long long)ids[r];
+            int pos = -1;
+            if (e >= 0 && e < E) {
+                pos = start[e] + atomicAdd(&mine[e], 1);
+                sorted_rows[pos] = r;
+            }
+            if (inv) inv[r] = pos;
+        }
     }
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int n = count[e];
+        const int n = total[e];
         for (int c = 0, pos = 0; pos < n; ++c, pos += chunk_rows)
             chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(chunk_rows, n - pos), 0);
     }
 }
 
-cudaError_t launch_moe_align(const int* ids, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
-                             int4* chunks, int* meta, cudaStream_t stream) {
-    const size_t smem = (size_t)(4 * E + 2) * sizeof(int);
-    moe_align_kernel<<<1, 1024, smem, stream>>>(ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta);
-    return counted(cudaGetLastError());
+template <typename IdT>
+static cudaError_t launch_align(const IdT* ids, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows, int4* chunks,
+                                int* meta, int* inv, cudaStream_t stream) {
+    // counters per warp: 32 sets where they fit the 48 KB of shared memory (E <= 340), one set beyond (E <= 3071)
+    auto smem = [&](int sets) { return (size_t)((sets + 3) * E + 2) * sizeof(int); };
+    if (rows > 1024 && smem(32) <= 48 * 1024)
+        return launch_dependent(moe_align_kernel<IdT, 32>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+    if (smem(8) <= 48 * 1024)
+        return launch_dependent(moe_align_kernel<IdT, 8>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+    return launch_dependent(moe_align_kernel<IdT, 1>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+}
+
+cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
+                             int4* chunks, int* meta, int* inv, cudaStream_t stream) {
+    return ids_i64 ? launch_align((const long long*)ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv, stream)
+                   : launch_align((const int*)ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv, stream);
 }
 
 // (Within an expert the rows land in the arrival order of the atomics.  Every routed row is an
 // independent column of the grouped GEMM, so the order does not change a single output bit.)
 
-// ---- gather + quantise the routed rows once (prefill-sized batches) --------------------------
-// xq[pos][:] = e4m3(x[sorted_rows[pos] / x_div][:] / scale) for every sorted position; the grouped
-// GEMM then takes its "B" tiles by TMA instead of re-quantising the rows for every channel tile.
+// ---- quantise the rows once and place them in expert order (prefill-sized batches) -------------
+// xq[inv[r]][:] = e4m3(x[r / x_div][:] / scale) for every routed row r with a valid expert; the grouped GEMM then takes its
+// rows by TMA instead of re-quantising them for every channel tile.  A thread converts 16 elements of a token once and
+// stores them to the positions of its x_div slots: 2 + x_div bytes of traffic per token element instead of the 3 x_div of
+// a gather per sorted position, and one conversion instead of x_div (16384 rows x 2048, four slots: 19.2 -> 9 us).
 __global__ void __launch_bounds__(256)
-moe_gather_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ sorted_rows,
-                        const int* __restrict__ meta, const float* __restrict__ input_scale,
-                        unsigned char* __restrict__ xq, int H) {
+moe_scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ inv, int rows,
+                         const float* __restrict__ input_scale, unsigned char* __restrict__ xq, int H) {
     pdl_launch_dependents();
     pdl_wait();
-    const int rows = meta[1];
     const ExactDiv div_scale(fmaxf(__ldg(input_scale), 1e-12f));
     const int vec_per_row = H / 16;
-    const int64_t total = (int64_t)rows * vec_per_row;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t pos = i / vec_per_row;
-        const int c = (int)(i - pos * vec_per_row) * 16;
-        const int src_row = __ldg(sorted_rows + pos) / x_div;
-        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)src_row * ldx + c);
-        const uint2 qa = quant8_e4m3(__ldg(src), div_scale);
-        const uint2 qb = quant8_e4m3(__ldg(src + 1), div_scale);
-        *reinterpret_cast<uint4*>(xq + pos * H + c) = make_uint4(qa.x, qa.y, qb.x, qb.y);
+    const int tokens = (rows + x_div - 1) / x_div;
+    // a block walks whole tokens, so no element needs a division to find its row
+    const int per = vec_per_row < 256 ? 256 / vec_per_row : 1;             // tokens a block takes at a time
+    const int sub = threadIdx.x / vec_per_row < per ? threadIdx.x / vec_per_row : per;
+    for (int64_t t0 = (int64_t)blockIdx.x * per; t0 < tokens; t0 += (int64_t)gridDim.x * per) {
+        const int64_t t = t0 + (per > 1 ? sub : 0);
+        if (sub >= per && per > 1) continue;
+        if (t >= tokens) continue;
+        for (int c = per > 1 ? (int)threadIdx.x - sub * vec_per_row : (int)threadIdx.x; c < vec_per_row; c += per > 1 ? vec_per_row : 256) {
+            const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)t * ldx + c * 16);
+            const uint2 qa = quant8_e4m3(__ldg(src), div_scale);
+            const uint2 qb = quant8_e4m3(__ldg(src + 1), div_scale);
+            const uint4 o = make_uint4(qa.x, qa.y, qb.x, qb.y);
+            for (int j = 0; j < x_div; ++j) {
+                const int64_t r = t * x_div + j;
+                const int pos = r < rows ? __ldg(inv + r) : -1;
+                if (pos >= 0) *reinterpret_cast<uint4*>(xq + (size_t)pos * H + c * 16) = o;
+            }
+        }
     }
 }
 
-cudaError_t launch_moe_gather_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* sorted_rows, const int* meta,
-                                    const float* input_scale, unsigned char* xq, int max_rows, int H, cudaStream_t stream) {
-    int64_t blocks = ((int64_t)max_rows * (H / 16) + 255) / 256;
+cudaError_t launch_moe_scatter_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* inv, int rows,
+                                     const float* input_scale, unsigned char* xq, int H, cudaStream_t stream) {
+    const int vec = H / 16, per = vec < 256 ? 256 / vec : 1;
+    int64_t blocks = ((int64_t)(rows + x_div - 1) / x_div + per - 1) / per;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
     if (blocks < 1) blocks = 1;
-    moe_gather_quant_kernel<<<(unsigned)blocks, 256, 0, stream>>>(x, ldx, x_div, sorted_rows, meta, input_scale, xq, H);
-    return counted(cudaGetLastError());
+    return launch_dependent(moe_scatter_quant_kernel, (unsigned)blocks, 256, 0, stream, x, ldx, x_div, inv, rows, input_scale, xq, H);
 }
 
 // ---- h = silu(gate) * up, quantised for the down projection ----------------------------------
@@ -213,14 +287,15 @@ cudaError_t launch_silu_mul_quant(const __nv_bfloat16* gu, const float* input_sc
     int64_t blocks = ((int64_t)max_rows * (I / 8) + 255) / 256;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
     if (blocks < 1) blocks = 1;
-    silu_mul_quant_kernel<<<(unsigned)blocks, 256, 0, stream>>>(gu, input_scale, hq, meta, I);
-    return counted(cudaGetLastError());
+    return launch_dependent(silu_mul_quant_kernel, (unsigned)blocks, 256, 0, stream, gu, input_scale, hq, meta, I);
 }
 
 // ---- combine: y[t] = bf16( sum over the k routed rows of token t ) ---------------------------
-// routed: bf16 [T*k][H] in routed-row order (slot j of token t at row t*k + j), summed in slot order.
+// routed: bf16 [T*k][H] in routed-row order (slot j of token t at row t*k + j), summed in slot order.  inv (optional): a slot
+// whose routed row had no valid expert (inv < 0) has not been written and counts as zero.
 __global__ void __launch_bounds__(256)
-moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, __nv_bfloat16* __restrict__ y, int T, int top_k, int H) {
+moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, const int* __restrict__ inv, __nv_bfloat16* __restrict__ y, int64_t ld_y, int T,
+                   int top_k, int H) {
     pdl_launch_dependents();
     pdl_wait();
     const int vec_per_row = H / 8;
@@ -229,7 +304,9 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, __nv_bfloat16* __re
         const int64_t t = i / vec_per_row;
         const int c = (int)(i - t * vec_per_row) * 8;
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
         for (int j = 0; j < top_k; ++j) {
+            if (inv && __ldg(inv + t * top_k + j) < 0) continue;
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(routed + ((size_t)t * top_k + j) * H + c));
             acc[0] += bf16_lo(v.x); acc[1] += bf16_hi(v.x); acc[2] += bf16_lo(v.y); acc[3] += bf16_hi(v.y);
             acc[4] += bf16_lo(v.z); acc[5] += bf16_hi(v.z); acc[6] += bf16_lo(v.w); acc[7] += bf16_hi(v.w);
@@ -237,17 +314,16 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, __nv_bfloat16* __re
         uint4 o;
         o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
         o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
-        *reinterpret_cast<uint4*>(y + t * H + c) = o;
+        *reinterpret_cast<uint4*>(y + t * ld_y + c) = o;
     }
 }
 
-cudaError_t launch_moe_combine(const __nv_bfloat16* routed, __nv_bfloat16* y, int T, int top_k, int H,
+cudaError_t launch_moe_combine(const __nv_bfloat16* routed, const int* inv, __nv_bfloat16* y, int64_t ld_y, int T, int top_k, int H,
                                cudaStream_t stream) {
     if (T == 0) return cudaSuccess;
     int64_t blocks = ((int64_t)T * (H / 8) + 255) / 256;
     if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    moe_combine_kernel<<<(unsigned)blocks, 256, 0, stream>>>(routed, y, T, top_k, H);
-    return counted(cudaGetLastError());
+    return launch_dependent(moe_combine_kernel, (unsigned)blocks, 256, 0, stream, routed, inv, y, ld_y, T, top_k, H);
 }
 
 }  // namespace fp8lin
