@@ -131,14 +131,24 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
     for (int i = threadIdx.x; i < kWarps * E; i += blockDim.x) count[i] = 0;
     const int share = ((rows + kWarps * 32 - 1) / (kWarps * 32)) * 32;
     const int r0 = warp * share, r1 = min(rows, r0 + share);
+    constexpr int kBatch = 8;              // ids in flight per lane
+    auto load_ids = [&](int r, int end, int* e) {
+#pragma unroll
+        for (int i = 0; i < kBatch; ++i) {
+            const long long id = r + 32 * i < end ? (long long)__ldg(ids + r + 32 * i) : -1;
+            e[i] = id >= 0 && id < E ? (int)id : -1;
+        }
+    };
     pdl_wait();
     __syncthreads();
     if (warp < kWarps) {
         int* mine = count + warp * E;
-#pragma unroll 4
-        for (int r = r0 + lane; r < r1; r += 32) {
-            const long long e = (long long)ids[r];
-            if (e >= 0 && e < E) atomicAdd(&mine[e], 1);
+        for (int r = r0 + lane; r < r1; r += 32 * kBatch) {
+            int e[kBatch];
+            load_ids(r, r1, e);
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i)
+                if (e[i] >= 0) atomicAdd(&mine[e[i]], 1);
         }
     }
     __syncthreads();
@@ -169,15 +179,20 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
     for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = start[e];
     if (warp < kWarps) {
         int* mine = count + warp * E;
-#pragma unroll 4
-        for (int r = r0 + lane; r < r1; r += 32) {
-            const long long e = (long long)ids[r];
-            int pos = -1;
-            if (e >= 0 && e < E) {
-                pos = start[e] + atomicAdd(&mine[e], 1);
-                sorted_rows[pos] = r;
+        for (int r = r0 + lane; r < r1; r += 32 * kBatch) {
+            int e[kBatch];
+            load_ids(r, r1, e);
+#pragma unroll
+            for (int i = 0; i < kBatch; ++i) {
+                const int row = r + 32 * i;
+                if (row >= r1) break;
+                int pos = -1;
+                if (e[i] >= 0) {
+                    pos = start[e[i]] + atomicAdd(&mine[e[i]], 1);
+                    sorted_rows[pos] = row;
+                }
+                if (inv) inv[row] = pos;
             }
-            if (inv) inv[r] = pos;
         }
     }
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
@@ -293,37 +308,45 @@ cudaError_t launch_silu_mul_quant(const __nv_bfloat16* gu, const float* input_sc
 // ---- combine: y[t] = bf16( sum over the k routed rows of token t ) ---------------------------
 // routed: bf16 [T*k][H] in routed-row order (slot j of token t at row t*k + j), summed in slot order.  inv (optional): a slot
 // whose routed row had no valid expert (inv < 0) has not been written and counts as zero.
+// A block walks whole rows (no division per element) and a thread has up to four slots' loads in flight.
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, const int* __restrict__ inv, __nv_bfloat16* __restrict__ y, int64_t ld_y, int T,
                    int top_k, int H) {
     pdl_launch_dependents();
     pdl_wait();
-    const int vec_per_row = H / 8;
-    const int64_t total = (int64_t)T * vec_per_row;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t t = i / vec_per_row;
-        const int c = (int)(i - t * vec_per_row) * 8;
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-        for (int j = 0; j < top_k; ++j) {
-            if (inv && __ldg(inv + t * top_k + j) < 0) continue;
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(routed + ((size_t)t * top_k + j) * H + c));
-            acc[0] += bf16_lo(v.x); acc[1] += bf16_hi(v.x); acc[2] += bf16_lo(v.y); acc[3] += bf16_hi(v.y);
-            acc[4] += bf16_lo(v.z); acc[5] += bf16_hi(v.z); acc[6] += bf16_lo(v.w); acc[7] += bf16_hi(v.w);
+    const int vec = H / 8;
+    for (int64_t t = blockIdx.x; t < T; t += gridDim.x) {
+        const __nv_bfloat16* src = routed + (size_t)t * top_k * H;
+        for (int c = threadIdx.x; c < vec; c += blockDim.x) {
+            float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int j0 = 0; j0 < top_k; j0 += 4) {
+                uint4 v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    v[j] = make_uint4(0u, 0u, 0u, 0u);
+                    if (j0 + j < top_k && (!inv || __ldg(inv + t * top_k + j0 + j) >= 0))
+                        v[j] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(j0 + j) * H + c * 8));
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[0] += bf16_lo(v[j].x); acc[1] += bf16_hi(v[j].x); acc[2] += bf16_lo(v[j].y); acc[3] += bf16_hi(v[j].y);
+                    acc[4] += bf16_lo(v[j].z); acc[5] += bf16_hi(v[j].z); acc[6] += bf16_lo(v[j].w); acc[7] += bf16_hi(v[j].w);
+                }
+            }
+            uint4 o;
+            o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
+            o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
+            *reinterpret_cast<uint4*>(y + t * ld_y + c * 8) = o;
         }
-        uint4 o;
-        o.x = pack_bf16x2(acc[0], acc[1]); o.y = pack_bf16x2(acc[2], acc[3]);
-        o.z = pack_bf16x2(acc[4], acc[5]); o.w = pack_bf16x2(acc[6], acc[7]);
-        *reinterpret_cast<uint4*>(y + t * ld_y + c) = o;
     }
 }
 
 cudaError_t launch_moe_combine(const __nv_bfloat16* routed, const int* inv, __nv_bfloat16* y, int64_t ld_y, int T, int top_k, int H,
                                cudaStream_t stream) {
     if (T == 0) return cudaSuccess;
-    int64_t blocks = ((int64_t)T * (H / 8) + 255) / 256;
-    if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    return launch_dependent(moe_combine_kernel, (unsigned)blocks, 256, 0, stream, routed, inv, y, ld_y, T, top_k, H);
+    const int64_t blocks = T < sm_count() * 16 ? T : sm_count() * 16;
+    const unsigned threads = H >= 2048 ? 256 : (H >= 1024 ? 128 : 64);
+    return launch_dependent(moe_combine_kernel, (unsigned)blocks, threads, 0, stream, routed, inv, y, ld_y, T, top_k, H);
 }
 
 }  // namespace fp8lin

@@ -26,26 +26,44 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
                      const __nv_bfloat16* __restrict__ weight, float eps, const float* __restrict__ input_scale,
                      unsigned char* __restrict__ xq, __nv_bfloat16* __restrict__ y, int64_t ldy, int H) {
     __shared__ float s_part[kNormThreads / 32];
-    __shared__ float s_inv;
-    pdl_launch_dependents();
-    pdl_wait();                                    // x and the residual come from the kernels before
-    const int64_t row = blockIdx.x;
     const int nvec = H >> 3;
+    const bool quant = xq != nullptr;
+    pdl_launch_dependents();
+    // A decode-sized call is one dependent chain: predecessor's end -> row -> sum of squares -> quantised row.  What no kernel
+    // writes (weight, scale) is fetched before the wait, all loads of the row are in flight together, and every thread adds
+    // the warps' partial sums itself (one barrier instead of two): 4.5 -> 3.6 us for one row of 3584 without the overlap of
+    // a dependent launch.
+    uint4 w[kNormMaxVec];
+#pragma unroll
+    for (int j = 0; j < kNormMaxVec; ++j) {
+        const int vec = threadIdx.x + j * kNormThreads;
+        if (vec < nvec) w[j] = __ldg(reinterpret_cast<const uint4*>(weight + vec * 8));
+    }
+    const ExactDiv div(quant ? fmaxf(__ldg(input_scale), 1e-12f) : 1.f);
+    pdl_wait();                                     // x and the residual come from the kernels before
+    const int64_t row = blockIdx.x;
     const __nv_bfloat16* xr = x + row * ldx;
     __nv_bfloat16* rr = residual ? residual + row * ld_res : nullptr;
+    uint4 xa[kNormMaxVec], ra[kNormMaxVec];
+#pragma unroll
+    for (int j = 0; j < kNormMaxVec; ++j) {
+        const int vec = threadIdx.x + j * kNormThreads;
+        if (vec < nvec) {
+            xa[j] = __ldg(reinterpret_cast<const uint4*>(xr + vec * 8));
+            if (rr) ra[j] = *reinterpret_cast<const uint4*>(rr + vec * 8);
+        }
+    }
     float v[kNormMaxVec][8];
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < kNormMaxVec; ++j) {
         const int vec = threadIdx.x + j * kNormThreads;
         if (vec < nvec) {
-            const uint4 a = __ldg(reinterpret_cast<const uint4*>(xr + vec * 8));
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+            const uint32_t aw[4] = {xa[j].x, xa[j].y, xa[j].z, xa[j].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) { v[j][2 * e] = bf16_lo(aw[e]); v[j][2 * e + 1] = bf16_hi(aw[e]); }
             if (rr) {
-                const uint4 b = *reinterpret_cast<const uint4*>(rr + vec * 8);
-                const uint32_t bw[4] = {b.x, b.y, b.z, b.w};
+                const uint32_t bw[4] = {ra[j].x, ra[j].y, ra[j].z, ra[j].w};
                 uint4 o;
                 uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
@@ -63,23 +81,15 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if ((threadIdx.x & 31) == 0) s_part[threadIdx.x >> 5] = ss;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
+    float t = 0.f;
 #pragma unroll
-        for (int i = 0; i < kNormThreads / 32; ++i) t += s_part[i];
-        const float var = __fdiv_rn(t, (float)H);
-        s_inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(var, eps)));
-    }
-    __syncthreads();
-    const float inv = s_inv;
-    const bool quant = xq != nullptr;
-    const ExactDiv div(quant ? fmaxf(__ldg(input_scale), 1e-12f) : 1.f);
+    for (int i = 0; i < kNormThreads / 32; ++i) t += s_part[i];
+    const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(t, (float)H), eps)));
 #pragma unroll
     for (int j = 0; j < kNormMaxVec; ++j) {
         const int vec = threadIdx.x + j * kNormThreads;
         if (vec < nvec) {
-            const uint4 w = __ldg(reinterpret_cast<const uint4*>(weight + vec * 8));
-            const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+            const uint32_t ww[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
             uint4 o;
             uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
