@@ -947,7 +947,7 @@ def extra_shape_rows(Kn, lib, peaks, dev, side, sampler, min_seconds):
         peak_tc = 2.0 * peaks["bf16_tflops"] if sid == lib.W8A8_STATIC else peaks["bf16_tflops"]
         bound = "hbm" if by / (peaks["hbm_gbs"] * 1e9) >= fl / (peak_tc * 1e12) else "tensor"
         mhz = sampler.median_mhz(*marks) if sampler else None
-        rows.append({"config": tag, "scheme": scheme, "m": m, "k": k, "n": n, "variant": Kn.variant_name(sid, m, k, n),
+        rows.append({"config": tag, "scheme": scheme, "m": m, "k": k, "n": n, "variant": Kn.kernel_name(sid, m, k, n),
                      "us": us, "tflops": fl / us / 1e6, "gbs": by / us / 1e3, "bound": bound,
                      "frac": (by / us / 1e3) / peaks["hbm_gbs"] if bound == "hbm" else (fl / us / 1e6) / peak_tc,
                      "sm_mhz": mhz, "kcycles": us * mhz / 1e3 if mhz else None, "weight_copies": len(ws)})
@@ -1236,7 +1236,7 @@ def main():
         mhz = sampler.median_mhz(*marks) if rank == 0 else None
         shapes.append({
             "layer": label, "m": m, "k": kl, "n": nl, "parallel": kind if tp > 1 else None,
-            "variant": Kn.variant_name(scheme_id, m, kl, nl),
+            "variant": Kn.kernel_name(scheme_id, m, kl, nl),
             "us": us, "tflops": fl / us / 1e6, "gbs": by / us / 1e3, "bound": bound,
             "frac": (by / us / 1e3) / peaks["hbm_gbs"] if bound == "hbm" else (fl / us / 1e6) / fp8_peak,
             "frac_of_sustained": None if bound == "hbm" else (fl / us / 1e6) / fp8_sustained,

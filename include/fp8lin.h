@@ -293,10 +293,10 @@ int fp8lin_mlp_w8a8_preq(const void* xq, const void* w_gate_up, const float* gat
 /* Which kernel variant a shape is routed to ("stream_mma_w8a8_m16", "umma_w8a8_128x256", ...),
  * for labelling bench rows and ncu captures.  Host-only, returns a static string. */
 const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N);
-/* The kernel that a call with 16-byte aligned y (ldy a multiple of 8) runs.  Differs from fp8lin_variant_name for W8A16
- * from 65 rows on: those calls take the CTA-pair kernel that widens the weights into tensor memory
- * ("umma_w8a16_pair_256x224_s3"); the variant name is the route of a call that kernel does not take (other alignments,
- * or one of the knobs of the other routes set).  Host-only, returns a static string. */
+/* The kernel that a call with 16-byte aligned y (ldy a multiple of 8) and one destination runs.  fp8lin_variant_name names
+ * the route by tile counts alone, which is what the multi-destination calls and calls of other alignments take; this differs
+ * for W8A16 from 65 rows on (the CTA-pair kernel that widens the weights into tensor memory, "umma_w8a16_pair_256x224_s3")
+ * and for large W8A8 calls whose rounds of tiles a model of their length gives to the other kernel.  Host-only, static string. */
 const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N);
 
 /* Bench/ncu studies only: force a tuning knob (value < 0 restores the default).  Not thread safe.

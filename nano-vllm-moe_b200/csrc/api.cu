@@ -149,12 +149,34 @@ F16Chunks plan_f16_chunks(int64_t M, int64_t K, int64_t N) {
     return c;
 }
 
-// CTA-pair GEMM (256 x 256 tiles over two SMs) instead of the one-CTA kernel.
-// Measured (W8A8, same bits as the one-CTA kernel): 4096 x 3584 -> 37888 449 vs 470 us, 16384 rows 1911 vs
-// 1980 us; but 4096 x 18944 -> 3584 (224 pair tiles = 3.03 rounds of 74 pairs) 294 vs 260 us and
-// 1024 x 2048 -> 11008 28.7 vs 26.1 us.  So: only when there are at least four rounds of pair tiles and the
-// last round is nearly full, and no worse filled than the one-CTA kernel's.
-bool pair_eligible(int64_t M, int64_t N) {
+// CTA-pair GEMM (256 x 256 tiles over two SMs) instead of the one-CTA kernel: whichever finishes its rounds of tiles first.
+// A K block of a round (74 pair tiles, or 148 tiles of 128 x 256 -- the same work) takes the pairs 0.44 us against 0.50:
+// they stage and read a third fewer shared memory bytes per multiplication, and under the power limit that is clock; a call starts and ends 2.5 us later.  The
+// pairs cannot cut a tile in two or split K, so the one-CTA kernel keeps short last rounds (half-width items, split-K tail)
+// and few-tile shapes.  Fitted to eleven row counts from 128 to 16384 on six layer shapes: of 66 choices two are more than
+// 4 % slower than the other kernel would have been, e.g. (us, pair / one CTA) 16384 x 3584 -> 3584 163 / 190, 16384 x 18944 -> 3584
+// 868 / 920, 1031 x 18944 -> 3584 65 / 72, 4096 x 3584 -> 4608 54.6 / 61; but 4096 x 18944 -> 3584 248 / 235, 1536 x
+// 18944 -> 3584 116 / 90, 256 x 3584 -> 4608 14.5 / 10.2.
+bool pair_eligible(int64_t M, int64_t K, int64_t N) {
+    if (g_tune.umma_pair >= 0) return g_tune.umma_pair != 0 && M > 64;
+    const int sms = sm_count();
+    const int64_t kblocks = (K + 127) / 128;
+    const int64_t pair_tiles = ((M + 255) / 256) * ((N + 255) / 256);
+    const int64_t pair_rounds = (pair_tiles + sms / 2 - 1) / (sms / 2);
+    const UmmaPlan pl = plan_umma(M, K, N, g_tune.umma_bn, g_tune.umma_splits);
+    if (pl.bn != 256) return false;
+    const int64_t tiles = (int64_t)pl.m_tiles * pl.n_tiles;
+    double rounds = (double)((tiles + sms - 1) / sms);
+    if (pl.splits > 1) rounds = rounds / pl.splits + 0.12;
+    else if (pl.tail_tiles) rounds += 1.0 / pl.tail_splits + 0.12 - 1.0;
+    else if (pl.narrow_tiles) rounds += 0.52 - 1.0;
+    return pair_rounds * kblocks * 0.44 + 6.0 < rounds * kblocks * 0.50 + 3.5;
+}
+
+// The same choice by how full the rounds are, without a model of their length: at least four rounds of pair tiles, the last
+// one nearly full and no worse filled than the one-CTA kernel's.  Used where the result goes to several destinations (that
+// epilogue has no split-K, so no tail to weigh), for the f16 operands of the scratch route, and in the variant name.
+bool pair_rounds_full(int64_t M, int64_t N) {
     if (g_tune.umma_pair >= 0) return g_tune.umma_pair != 0 && M > 64;
     const int64_t nt = (N + 255) / 256;
     const int64_t pt = ((M + 255) / 256) * nt;
@@ -382,7 +404,7 @@ int fp8lin_w8a16(const void* x, int64_t ldx, const void* w_nk, const float* w_sc
             a.partial = nullptr; a.counters = ws.counters; a.status = ws.status;
             a.M = (int)M; a.K = (int)K; a.N = (int)nc; a.ldy = (int)ldy;
             const char* why = nullptr;
-            e = pair_eligible(M, nc) ? launch_umma_pair(true, a, st, &why) : launch_umma_f16(pl, a, st, &why);
+            e = pair_rounds_full(M, nc) ? launch_umma_pair(true, a, st, &why) : launch_umma_f16(pl, a, st, &why);
             if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "tcgen05 f16 GEMM launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
         }
         return FP8LIN_OK;
@@ -435,7 +457,7 @@ int fp8lin_w8a8(const void* x, int64_t ldx, const void* w_nk, const float* w_sca
     a.bias = (const __nv_bfloat16*)bias; a.y = (__nv_bfloat16*)y;
     a.partial = (float*)(ws.body + xq_bytes); a.counters = ws.counters; a.status = ws.status;
     a.M = (int)M; a.K = (int)K; a.N = (int)N; a.ldy = (int)ldy;
-    const bool pair = pair_eligible(M, N);
+    const bool pair = pair_eligible(M, K, N);
     const int64_t pre = pair ? prequant_rows(M, (N + 255) / 256, 256, sm_count() / 2)
                              : (pl.splits > 1 ? M : prequant_rows(M, pl.n_tiles, 128, sm_count()));
     rc = pair ? start_quant(x, ldx, input_scale, xq, M, K, pre, ws, a, st, (N + 255) / 256, 256, sm_count() / 2)
@@ -470,7 +492,7 @@ static int w8a8_to_destinations(const void* x, int64_t ldx, const void* w_nk, co
     a.xq = ws.body; a.w = (const unsigned char*)w_nk; a.w_scale = w_scale; a.input_scale = input_scale;
     a.bias = (const __nv_bfloat16*)bias; a.y = (__nv_bfloat16*)dst_ptrs[0]; a.partial = nullptr; a.counters = ws.counters;
     a.status = ws.status; a.M = (int)M; a.K = (int)K; a.N = (int)N; a.ldy = (int)ld_dst;
-    const bool pair = pair_eligible(M, N);
+    const bool pair = pair_rounds_full(M, N);
     rc = pair ? start_quant(x, ldx, input_scale, ws.body, M, K, prequant_rows(M, (N + 255) / 256, 256, sm_count() / 2), ws, a, st,
                             (N + 255) / 256, 256, sm_count() / 2)
               : start_quant(x, ldx, input_scale, ws.body, M, K, prequant_rows(M, pl.n_tiles, 128, sm_count()), ws, a, st, pl.n_tiles, 128,
@@ -532,7 +554,7 @@ int run_w8a8_prequantised(const unsigned char* xq, const void* w, const float* w
     if (M <= 64) {
         SwapPlan sp = plan_swap(M, K, N, g_tune.swap_splits, true);
         e = launch_swap_w8a8(sp, a, nullptr, 0, st, &why);
-    } else if (pair_eligible(M, N)) {
+    } else if (pair_eligible(M, K, N)) {
         e = launch_umma_pair(false, a, st, &why);
     } else {
         UmmaPlan pl = plan_umma(M, K, N, g_tune.umma_bn, g_tune.umma_splits);
@@ -730,17 +752,21 @@ int fp8lin_quantize_activation(const void* x, int64_t ldx, const float* input_sc
     return FP8LIN_OK;
 }
 
+static const char* umma_plan_name(int64_t M, int64_t K, int64_t N, char* buf, size_t size) {
+    const UmmaPlan pl = plan_umma(M, K, N, g_tune.umma_bn, g_tune.umma_splits);
+    if (pl.tail_tiles) snprintf(buf, size, "umma_w8a8_128x%d_s1+tail%dx%d", pl.bn, pl.tail_tiles, pl.tail_splits);
+    else if (pl.narrow_tiles) snprintf(buf, size, "umma_w8a8_128x%d_s1+half%d", pl.bn, pl.narrow_tiles);
+    else snprintf(buf, size, "umma_w8a8_128x%d_s%d", pl.bn, pl.splits);
+    return buf;
+}
+
 const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N) {
     static thread_local char buf[64];
     if (M <= 0 || K <= 0 || N <= 0) return "none";
     const int max_m = g_tune.stream_max_m >= 0 ? g_tune.stream_max_m : kDefaultStreamMaxM;
-    if (scheme == FP8LIN_W8A8_STATIC && M > max_m && N % 8 == 0 && pair_eligible(M, N)) return "umma_pair_w8a8_256x256";
+    if (scheme == FP8LIN_W8A8_STATIC && M > max_m && N % 8 == 0 && pair_rounds_full(M, N)) return "umma_pair_w8a8_256x256";
     if (scheme == FP8LIN_W8A8_STATIC && M > max_m && N % 8 == 0) {
-        UmmaPlan pl = plan_umma(M, K, N, g_tune.umma_bn, g_tune.umma_splits);
-        if (pl.tail_tiles) snprintf(buf, sizeof(buf), "umma_w8a8_128x%d_s1+tail%dx%d", pl.bn, pl.tail_tiles, pl.tail_splits);
-        else if (pl.narrow_tiles) snprintf(buf, sizeof(buf), "umma_w8a8_128x%d_s1+half%d", pl.bn, pl.narrow_tiles);
-        else snprintf(buf, sizeof(buf), "umma_w8a8_128x%d_s%d", pl.bn, pl.splits);
-        return buf;
+        return umma_plan_name(M, K, N, buf, sizeof(buf));
     }
     if (scheme == FP8LIN_W8A8_STATIC && swap_eligible(M, K, N)) {
         SwapPlan pl = plan_swap(M, K, N, g_tune.swap_splits, swap_prequant(M));
@@ -771,6 +797,9 @@ const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N) {
         snprintf(buf, sizeof(buf), "umma_w8a16_pair_256x%d_s%d", pl.tokens, pl.splits);
         return buf;
     }
+    const int max_m = g_tune.stream_max_m >= 0 ? g_tune.stream_max_m : kDefaultStreamMaxM;
+    if (M > max_m && K > 0 && N > 0 && N % 8 == 0 && scheme == FP8LIN_W8A8_STATIC)
+        return pair_eligible(M, K, N) ? "umma_pair_w8a8_256x256" : umma_plan_name(M, K, N, buf, sizeof(buf));
     return fp8lin_variant_name(scheme, M, K, N);
 }
 
