@@ -76,24 +76,31 @@ int validate_common(const void* x, int64_t ldx, const void* w, const float* w_sc
     return FP8LIN_OK;
 }
 
-bool w8a16_swap_eligible(int64_t M, int64_t N) {
-    // measured (us, mma.sync kernel / tcgen05 kernel): at 32 rows 3584 -> 4608 11.4 / 10.4, 3584 -> 3584 11.4 / 9.1,
-    // 18944 -> 3584 29.8 / 23.5, 3584 -> 37888 34.1 / 34.4; at 16 rows 9.5 / 9.7, 9.4 / 8.5, 21.6 / 22.7, 26.8 / 33.6;
-    // at 64 rows on 3584 -> 37888 67 / 38.  So: from 17 rows, from 33 when there is a channel tile for every SM.
-    const int wide = (N + 127) / 128 >= fp8lin::sm_count();
-    const int min_m = g_tune.w8a16_swap_min_m >= 0 ? g_tune.w8a16_swap_min_m : (wide ? 33 : 17);
+// Layers of up to ~17 MB with a short K (qkv, o_proj): up to 8 rows the mma.sync streaming kernel -- many small CTAs, its
+// split-K slices handing their sums over inside a cluster -- starts and drains faster than the tcgen05 kernels.
+bool small_layer(int64_t K, int64_t N, int64_t max_k) { return K <= max_k && N <= 4736; }
+
+bool w8a16_swap_eligible(int64_t M, int64_t K, int64_t N) {
+    // measured (us, mma.sync kernel / tcgen05 kernel, which widens the weights on its way to TMEM): one row 3584 -> 37888
+    // 23.1 / 21.0, 18944 -> 3584 15.7 / 14.0, 2048 -> 11008 8.1 / 6.9, but 3584 -> 4608 5.7 / 6.5, 3584 -> 3584 4.7 / 6.0,
+    // 5120 -> 2560 5.4 / 6.2; 16 rows 26.9 / 22.8, 20.2 / 15.5, 10.1 / 7.8, 9.0 / 7.7, 7.8 / 6.9, 7.7 / 7.1
+    const int min_m = g_tune.w8a16_swap_min_m >= 0 ? g_tune.w8a16_swap_min_m : (small_layer(K, N, 8192) ? 9 : 1);
     return g_tune.w8a16_swap_enable != 0 && M >= min_m && M <= 64;
 }
 
 // W8A16 on CTA pairs with the weights widened into tensor memory and the caller's bf16 rows as the other operand.
 // A knob that selects one of the other W8A16 routes switches it off.
-bool w8a16_pair_eligible(int64_t M, int64_t N, int64_t ldy, const void* y) {
+bool w8a16_pair_eligible(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
     if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return false;             // (two channels per store)
     if (g_tune.w8a16_pair >= 0) return g_tune.w8a16_pair != 0;
     if (g_tune.w8a16_umma_min_m >= 0 || g_tune.w8a16_chunk_mb > 0 || g_tune.w8a16_swap_min_m >= 0 || g_tune.w8a16_swap_enable >= 0 ||
         g_tune.stream_splits > 0 || g_tune.swap_splits > 0)
         return false;
-    return M >= 65;
+    if (M >= 65) return true;
+    // 33 to 64 rows: pairs where the one-CTA kernel would not split K (it then widens every tile alone, 0.56 us per block at
+    // 64 rows): 2048 -> 11008 11.0 us against 12.3, 2560 -> 9472 10.9 / 12.1, 3584 -> 37888 33.0 / 33.8; with slices it keeps
+    // 3584 -> 4608 12.2 / 11.4, 18944 -> 3584 25.0 / 24.7
+    return M > 32 && plan_swap_w8a16(M, K, N, -1).splits == 1;
 }
 
 // Large-M W8A16: channel chunks of the weights are widened to f16 into scratch (small enough to stay
@@ -189,14 +196,11 @@ bool pair_rounds_full(int64_t M, int64_t N) {
 
 bool swap_eligible(int64_t M, int64_t K, int64_t N) {
     const int max_m = g_tune.stream_max_m >= 0 ? g_tune.stream_max_m : kDefaultStreamMaxM;
-    // The tcgen05 kernel from the first row on, except on layers of up to ~17 MB with a short K (qkv, o_proj), where up to
-    // 8 rows the mma.sync streaming kernel -- many small CTAs, its split-K slices handing their sums over inside a
-    // cluster -- starts and drains faster.  Measured at one row / eight rows, us, tcgen05 against streaming kernel:
-    // 3584 -> 4608 6.8 / 7.1 against 6.0 / 6.5, 3584 -> 3584 5.8 / 6.3 against 5.1 / 5.5, 4736 -> 3584 6.9 against 6.5
-    // (four rows), 2048 -> 2048 4.1 against 4.0; but 2048 -> 11008 7.2 / 7.4 against 9.1 / 9.7, 11008 -> 2048 8.3 against
-    // 9.6, 18944 -> 3584 14.9 / 15.2 against 16.6 / 19.0, 3584 -> 37888 21.7 against 24.0.
+    // The tcgen05 kernel from the first row on, except on small layers.  Measured, us, tcgen05 / streaming kernel, one row
+    // (eight rows): 3584 -> 4608 6.1 / 5.8 (6.4 / 6.4), 3584 -> 3584 5.4 / 4.8 (5.7 / 5.4), 2048 -> 2048 3.8 / 3.7 (4.1 / 4.0);
+    // but 5120 -> 2560 5.5 / 5.9 (5.8 / 6.4), 2048 -> 11008 6.9 / 9.1, 18944 -> 3584 13.7 / 16.6, 3584 -> 37888 20.6 / 23.7.
     int min_m = g_tune.swap_min_m >= 0 ? g_tune.swap_min_m : 1;
-    if (g_tune.swap_min_m < 0 && K <= 8192 && N <= 4736) min_m = 9;
+    if (g_tune.swap_min_m < 0 && small_layer(K, N, 4096)) min_m = 9;
     return g_tune.swap_enable != 0 && M >= min_m && M <= 64 && M <= max_m;
 }
 
@@ -355,7 +359,7 @@ int fp8lin_w8a16(const void* x, int64_t ldx, const void* w_nk, const float* w_sc
                  void* stream) {
     int rc = validate_common(x, ldx, w_nk, w_scale, bias, y, ldy, M, K, N);
     if (rc != FP8LIN_OK || M == 0) return rc;
-    if (workspace && workspace_bytes >= FP8LIN_WS_HEADER_BYTES && w8a16_pair_eligible(M, N, ldy, y)) {
+    if (workspace && workspace_bytes >= FP8LIN_WS_HEADER_BYTES && w8a16_pair_eligible(M, K, N, ldy, y)) {
         const W8a16PairPlan pl = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
         UmmaArgs a;
         a.xq = nullptr; a.w = (const unsigned char*)w_nk; a.w_scale = w_scale; a.input_scale = nullptr;
@@ -366,7 +370,7 @@ int fp8lin_w8a16(const void* x, int64_t ldx, const void* w_nk, const float* w_sc
         if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "tcgen05 W8A16 pair kernel launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
         return FP8LIN_OK;
     }
-    if (w8a16_swap_eligible(M, N) && workspace) {
+    if (w8a16_swap_eligible(M, K, N) && workspace) {
         SwapPlan sp = plan_swap_w8a16(M, K, N, g_tune.swap_splits);
         UmmaArgs a;
         a.xq = nullptr; a.w = (const unsigned char*)w_nk; a.w_scale = w_scale; a.input_scale = nullptr;
@@ -780,7 +784,7 @@ const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N) {
         snprintf(buf, sizeof(buf), "umma_w8a16_f16_128x%d_s%d_c%d", pl.bn, pl.splits, (int)c.n_chunks);
         return buf;
     }
-    if (scheme == FP8LIN_W8A16 && w8a16_swap_eligible(M, N)) {
+    if (scheme == FP8LIN_W8A16 && w8a16_swap_eligible(M, K, N)) {
         SwapPlan pl = plan_swap_w8a16(M, K, N, g_tune.swap_splits);
         snprintf(buf, sizeof(buf), "umma_swap_w8a16_m%d_s%d", pl.mp, pl.splits);
         return buf;
@@ -792,7 +796,7 @@ const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N) {
 
 const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N) {
     static thread_local char buf[64];
-    if (M > 0 && K > 0 && N > 0 && scheme == FP8LIN_W8A16 && w8a16_pair_eligible(M, N, 8, nullptr)) {
+    if (M > 0 && K > 0 && N > 0 && scheme == FP8LIN_W8A16 && w8a16_pair_eligible(M, K, N, 8, nullptr)) {
         const W8a16PairPlan pl = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
         snprintf(buf, sizeof(buf), "umma_w8a16_pair_256x%d_s%d", pl.tokens, pl.splits);
         return buf;

@@ -1,4 +1,4 @@
-// Decode-sized W8A16 linear (used for 33 <= M <= 64; works from M = 1) on tcgen05, operands swapped:
+// Decode-sized W8A16 linear (M <= 64, from the first row on layers beyond a few MB) on tcgen05, operands swapped:
 //
 //   y^T[N, M] = f16(W_e4m3[N, K]) . f16(x[M, K])^T         fp32 accumulation in TMEM
 //
@@ -414,21 +414,22 @@ SwapPlan plan_swap_w8a16(int64_t M, int64_t K, int64_t N, int force_splits) {
     for (int s = 1; s <= 8; ++s) {
         if (force_splits > 0 && s != (force_splits > 8 ? 8 : force_splits)) continue;
         if (s > kblocks) break;
-        if (force_splits <= 0 && s > 1 && kblocks / s < 4) break;
+        // (two K blocks per slice are enough when every CTA has an SM to itself: 32 rows on 1280 -> 1536 5.7 -> 4.5 us)
+        if (force_splits <= 0 && s > 1 && kblocks / s < (pl.n_tiles * s <= sm_count() ? 2 : 4)) break;
         const int kps = (kblocks + s - 1) / s;
         if ((kblocks + kps - 1) / kps != s) continue;
         int slots = sm_count();
         if (s > 1) slots = pl.mp == 16 ? swap16_max_clusters<16>(s) : (pl.mp == 32 ? swap16_max_clusters<32>(s) : swap16_max_clusters<64>(s));
         if (slots < 1) slots = 1;
-        // microseconds per wave of clusters, as in plan_swap; a CTA alone is bound by the widening of its weight
-        // tiles (0.52 us per 16 KB block), and waves do not overlap
+        // microseconds, the model of plan_swap with this kernel's constants (fitted to the same shapes, 0.2 % from the best
+        // on average): a lone CTA is bound by the chain of its converters, which grows with the rows they also convert
         const int ctas = pl.n_tiles * s;
         const int resident = ctas < slots * s ? ctas : slots * s;
-        const double shared = 16384.0 * resident / 6.5e6;
-        const double t_block = shared > 0.52 ? shared : 0.52;
+        const double alone = pl.mp == 16 ? 0.236 : (pl.mp == 32 ? 0.348 : 0.564);
+        const double shared = 16384.0 * resident / 5.46e6;
+        const double t_block = shared > alone ? shared : alone;
         const int waves = (pl.n_tiles + slots - 1) / slots;
-        const double fixed = 3.5 + (s > 1 ? 0.5 + (0.1 + 0.006 * (double)M) * s : 0.0);
-        const double cost = waves * (kps * t_block + fixed);
+        const double cost = s > 1 ? waves * (kps * t_block + 2.6 + 0.5 + (0.034 + 0.0072 * (double)M) * s) : waves * kps * t_block + 2.6;
         if (cost < best_cost) { best_cost = cost; best_s = s; }
     }
     pl.splits = best_s;
