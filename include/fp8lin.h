@@ -308,7 +308,7 @@ const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N);
  * "stream_push" (0 = split-K of the mma.sync streaming kernel always through global scratch instead of a cluster),
  * "mlp_decode_fused" (1 = the fused MLP on up to 16 pre-quantised rows computes silu * up inside the gate_up kernel),
  * "moe_fused" (0 = the expert FFN keeps a separate activation pass), "moe_rows_major" (0 = prefill-sized expert
- * batches stay on the channel-major grouped kernel), "pair_stages" (4 or 5 ring slots in the CTA-pair GEMM). */
+ * batches stay on the one-CTA grouped kernel), "pair_stages" (4 or 5 ring slots in the CTA-pair GEMM). */
 int fp8lin_set_tuning(const char* knob, int value);
 
 /* Blocking: copies the device status word out of `workspace` (after syncing

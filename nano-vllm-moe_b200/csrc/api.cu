@@ -41,7 +41,7 @@ struct Tuning {
     int fuse_quant = -1;        // large-M W8A8: <= 0 (default) = quantise x in a separate pass; 1 = the pass takes the rows
                                 // of the first round of tiles, the GEMM's own quantiser warps the rest; n > 1 = the pass
                                 // takes the first n rows (rounded up to 128)
-    int moe_rows_major = -1;    // 0 = prefill-sized expert batches stay on the channel-major grouped kernel
+    int moe_rows_major = -1;    // 0 = prefill-sized expert batches stay on the one-CTA grouped kernel
     int mlp_decode_fused = -1;  // 1 = the fused MLP on up to 16 pre-quantised rows computes silu * up in the gate_up kernel (study knob)
     int moe_fused = -1;         // 0 = the expert FFN keeps its separate silu-multiply-quantise pass for every batch size
     int quant_lead = -1;        // row blocks the in-kernel quantiser may run ahead (default: from the tile schedule)
@@ -933,7 +933,10 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     int* inv = (int*)(ws + L.off_inv);
     __nv_bfloat16* gu = (__nv_bfloat16*)(ws + L.off_gu);
     unsigned char* hq = ws + L.off_hq;
-    const int mp = grouped_chunk_rows(rows, E);
+    const int avg_mp = grouped_chunk_rows(rows, E);
+    // Prefill-sized batches with more than a few rows per expert: both projections on CTA pairs with chunks of up to 256 rows.
+    const bool pairs = rows >= kMoePrequantRows && avg_mp >= 32 && ld_out % 8 == 0 && aligned16(out_routed) && g_tune.moe_rows_major != 0;
+    const int mp = pairs ? 256 : avg_mp;
     cudaError_t e = launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
@@ -942,12 +945,9 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     a.input_scale = w13_input_scale; a.topk_w = topk_w; a.out = gu; a.status = (int*)workspace;
     a.ldx = (int)ldx; a.x_div = x_div; a.ld_out = (int)(2 * I); a.N = (int)(2 * I); a.K = (int)H; a.n_tiles = 0; a.kblocks = 0;
     a.scatter = 0;
-    // Prefill-sized batches whose experts fill 128-row chunks: both projections run with the rows as the MMA M dimension
-    // (umma_grouped_rows.cu).  Measured on 4096 tokens (60 experts, top-4, H 2048, I 1408) against the channel-major kernel.
-    const bool rows_major = rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
     // prefill-sized batches with whole 128-channel tiles: the gate_up GEMM's epilogue applies the activation and writes hq
     // (from 32-row chunks on: the epilogue reads the two accumulators 32 rows at a time)
-    const bool fused_act = rows >= kMoePrequantRows && I % 128 == 0 && mp >= 32 && g_tune.moe_fused != 0;
+    const bool fused_act = pairs || (rows >= kMoePrequantRows && I % 128 == 0 && mp >= 32 && g_tune.moe_fused != 0);
     if (rows >= kMoePrequantRows) {
         unsigned char* xq = ws + L.off_xq;
         e = launch_moe_scatter_quant((const __nv_bfloat16*)x, ldx, x_div, inv, (int)rows, w13_input_scale, xq, (int)H, st);
@@ -955,8 +955,8 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
         if (fused_act) {
             GroupedArgs f = a;
             f.N = (int)I; f.hq = hq; f.h_scale = w2_input_scale; f.out = nullptr;
-            e = rows_major ? launch_grouped_rows_w8a8(f, w13_packed, E, xq, rows, st, &why)
-                           : launch_grouped_w8a8(false, mp, f, w13_packed, E, xq, rows, st, &why);
+            e = pairs ? launch_grouped_pair_w8a8(f, w13_packed, E, xq, rows, st, &why)
+                      : launch_grouped_w8a8(false, mp, f, w13_packed, E, xq, rows, st, &why);
         } else {
             e = launch_grouped_w8a8(false, mp, a, w13_packed, E, xq, rows, st, &why);
         }
@@ -970,10 +970,7 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     }
     a.w_scale = w2_scale; a.input_scale = w2_input_scale; a.out = (__nv_bfloat16*)out_routed; a.ld_out = (int)ld_out;
     a.N = (int)H; a.K = (int)I; a.scatter = 1;
-    if (rows_major && H % 8 == 0 && ld_out % 8 == 0 && aligned16(out_routed))
-        e = launch_grouped_rows_w8a8(a, w2_packed, E, hq, rows, st, &why);
-    else
-        e = launch_grouped_w8a8(false, mp, a, w2_packed, E, hq, rows, st, &why);
+    e = pairs ? launch_grouped_pair_w8a8(a, w2_packed, E, hq, rows, st, &why) : launch_grouped_w8a8(false, mp, a, w2_packed, E, hq, rows, st, &why);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "down grouped GEMM launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
     return FP8LIN_OK;
 }

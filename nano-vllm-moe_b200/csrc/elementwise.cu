@@ -215,7 +215,7 @@ silu_mul_quant_interleaved_kernel(const __nv_bfloat16* __restrict__ gu, const fl
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float g0 = bf16_lo(gw[j]), g1 = bf16_hi(gw[j]);
-            const float s0 = g0 / (1.f + expf(-g0)), s1 = g1 / (1.f + expf(-g1));
+            const float s0 = silu_f32(g0), s1 = silu_f32(g1);
             hw[j] = pack_bf16x2(s0 * bf16_lo(uw[j]), s1 * bf16_hi(uw[j]));
         }
         *reinterpret_cast<uint2*>(hq + r * I + c) = quant8_e4m3(h, div_scale);

@@ -223,9 +223,11 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
         }
     }
     for (int e = threadIdx.x * kCtas + crank; e < E; e += blockDim.x * kCtas) {
-        const int n = total[e];
-        for (int c = 0, pos = 0; pos < n; ++c, pos += chunk_rows)
-            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(chunk_rows, n - pos), 0);
+        // chunks of 256 rows are evened out to steps of 32: 273 rows are 160 + 113, not 256 + 17
+        const int n = total[e], parts = (n + chunk_rows - 1) / chunk_rows;
+        const int size = chunk_rows == 256 && n > 0 ? (((n + parts - 1) / parts) + 31) & ~31 : chunk_rows;
+        for (int c = 0, pos = 0; pos < n; ++c, pos += size)
+            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(size, n - pos), 0);
     }
 }
 
@@ -334,7 +336,7 @@ silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, const float* __restr
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float g0 = bf16_lo(gw[j]), g1 = bf16_hi(gw[j]);
-            const uint32_t sp = pack_bf16x2(g0 / (1.f + expf(-g0)), g1 / (1.f + expf(-g1)));
+            const uint32_t sp = pack_bf16x2(silu_f32(g0), silu_f32(g1));
             hw[j] = pack_bf16x2(bf16_lo(sp) * bf16_lo(uw[j]), bf16_hi(sp) * bf16_hi(uw[j]));
         }
         *reinterpret_cast<uint2*>(hq + r * I + c) = quant8_e4m3(h, div_scale);

@@ -96,6 +96,8 @@ __device__ __forceinline__ uint32_t elect_one() {
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(r));
     return r;
 }
+// A value that all lanes hold, in a form the compiler knows to be uniform (loaded values are not, shuffled ones neither).
+__device__ __forceinline__ int uniform(int v) { return (int)__reduce_or_sync(0xffffffffu, (unsigned)v); }
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, int* status, int code) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
@@ -187,6 +189,13 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {     // bar: shared::cluster address
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Arrive on another CTA's barrier without a cluster-scope release: for what is in tensor memory, ordered by
+// tcgen05.wait and the tcgen05 fence.  (A release at cluster scope waits until the warp's earlier stores have reached L2:
+// over a thousand cycles behind an epilogue's stores.)
+__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // 32 lanes x 32 columns of fp32 from TMEM (lane i of the warp reads TMEM lane base+i); no wait.

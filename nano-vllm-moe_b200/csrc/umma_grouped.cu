@@ -90,7 +90,7 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     pdl_launch_dependents();
     pdl_wait();                                   // the chunk list, the rows and the outputs all come from predecessors
 
-    const int n_chunks = __shfl_sync(0xffffffffu, p.meta[0], 0);
+    const int n_chunks = uniform(p.meta[0]);
     const int total = n_chunks * p.n_tiles;       // item w = chunk * n_tiles + tile
     const int KB = p.kblocks;
 
@@ -106,7 +106,7 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             bool ok = true;
             for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
                 const int4 chunk = p.chunks[w / p.n_tiles];
-                const int2 ch = make_int2(__shfl_sync(0xffffffffu, chunk.x, 0), __shfl_sync(0xffffffffu, chunk.y, 0));     // (uniform)
+                const int2 ch = make_int2(uniform(chunk.x), uniform(chunk.y));
                 const int t = w % p.n_tiles;
                 const int wrow0 = (ch.x * p.w_tiles + t) * KB;        // packed tile index of (expert, tile, kb = 0)
                 for (int kb = 0; kb < KB; ++kb, ++it) {
@@ -252,7 +252,7 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                             if (c0 + j < ch.z) {
                                 const uint32_t gu = pack_bf16x2(__uint_as_float(g[j]) * wg, __uint_as_float(u[j]) * wu);   // as the bf16 gate_up row
                                 const float gv = bf16_lo(gu);
-                                const uint32_t sv = pack_bf16x2(gv / (1.f + expf(-gv)), 0.f);                              // bf16(silu(g))
+                                const uint32_t sv = pack_bf16x2(silu_f32(gv), 0.f);                              // bf16(silu(g))
                                 const uint32_t hv = pack_bf16x2(bf16_lo(sv) * bf16_hi(gu), 0.f);                           // bf16(. * u)
                                 p.hq[(size_t)(ch.y + c0 + j) * p.N + n] = (unsigned char)(cvt_e4m3x2(div_h(bf16_lo(hv)), 0.f) & 0xffu);
                             }

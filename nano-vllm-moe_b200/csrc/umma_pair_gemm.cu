@@ -16,7 +16,7 @@
 //   tfull[a]  likewise committed to both CTAs after the last K block: the epilogue warps of each CTA
 //             read their own tensor memory.
 //   tempty[a] (leader only) the eight epilogue warps of both CTAs arrive on the leader's barrier (the
-//             peer's with a cluster-scope remote arrive).
+//             peer's with a remote arrive).
 // No load in this file is a cluster broadcast: every TMA load lands in exactly one CTA.
 // Every wait is bounded (about a second); a CTA that gives up still joins the cluster barrier at the
 // end, so its partner is never left waiting for it.
@@ -270,7 +270,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                             const uint32_t up = pack_bf16x2(fmaf(__uint_as_float(u[j]), su.x, bf16_lo(bu)),
                                                             fmaf(__uint_as_float(u[j + 1]), su.y, bf16_hi(bu)));
                             const float g0 = bf16_lo(gp), g1 = bf16_hi(gp);
-                            const float s0 = g0 / (1.f + expf(-g0)), s1 = g1 / (1.f + expf(-g1));
+                            const float s0 = silu_f32(g0), s1 = silu_f32(g1);
                             hw[j / 2] = pack_bf16x2(s0 * bf16_lo(up), s1 * bf16_hi(up));
                         }
                         uint2 qv[4];
@@ -298,7 +298,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (lane == 0) {
                     const uint32_t te = smem_u32(&bar_tempty[as]);
                     if (leader) mbar_arrive(te);
-                    else mbar_arrive_cluster(map_to_cta(te, 0));
+                    else mbar_arrive_remote(map_to_cta(te, 0));
                 }
                 continue;
             }
@@ -339,7 +339,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if (lane == 0) {
                 const uint32_t te = smem_u32(&bar_tempty[as]);
                 if (leader) mbar_arrive(te);
-                else mbar_arrive_cluster(map_to_cta(te, 0));
+                else mbar_arrive_remote(map_to_cta(te, 0));
             }
         }
         if (lane == 0) tma_store_wait_all();

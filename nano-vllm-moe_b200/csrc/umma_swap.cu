@@ -375,7 +375,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                         for (int j = 0; j < 4; ++j) {
                             const uint32_t gp = r[4 * gI + j], up = u[4 * gI + j];
                             const float g0 = bf16_lo(gp), g1 = bf16_hi(gp);
-                            const float s0 = g0 / (1.f + expf(-g0)), s1 = g1 / (1.f + expf(-g1));
+                            const float s0 = silu_f32(g0), s1 = silu_f32(g1);
                             hw[j] = pack_bf16x2(s0 * bf16_lo(up), s1 * bf16_hi(up));
                         }
                         const uint2 qd = quant8_e4m3(hv, div_h);

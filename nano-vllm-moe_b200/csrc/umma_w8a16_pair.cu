@@ -75,12 +75,6 @@ struct PairSched16 {
     int kblocks, kblocks_per_split;
 };
 
-// Arrive on another CTA's barrier without a cluster-scope release: what it announces is in tensor memory, ordered by
-// tcgen05.wait::st and the tcgen05 fence.  (A release at cluster scope waits for the warp's memory traffic on every block.)
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
 // mbar_wait for a barrier that the partner CTA arrives on: acquires at cluster scope
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int* status, int code) {
     long long start = -1;
@@ -277,7 +271,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             for (int item = first_item; item < items && ok; item += item_step, ++tl) {
                 const int as = acc_stages == 2 ? (tl & 1) : 0;
                 const uint32_t aph = acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1);
-                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait_cluster(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
                 if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * T;
@@ -396,6 +390,11 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     tmem_ld16_nowait(t_lane + as * T + c, v);
                     if (c + 16 < half) tmem_ld16_nowait(t_lane + as * T + c + 16, v + 16);
                     tmem_ld_wait();
+                    if (c + 32 >= half) {                      // the accumulator is in registers: the next tile may have it
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[as]), leader_cta));
+                    }
 #pragma unroll
                     for (int j = 0; j < 32; j += 2) {
                         if (j == 16 && c + 16 >= half) break;
@@ -405,9 +404,6 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                         if (in && m0 + c + j + (odd ? 1 : 0) < p.M) *reinterpret_cast<uint32_t*>(yp + (size_t)(c + j) * p.ldy) = o;
                     }
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&bar_tempty[as]), leader_cta));
             } else {
                 // the pair's MMAs are done, so this CTA's ring is free: tell the CTAs that will push into it, wait for those
                 // this one pushes into, and send each channel's sums to the owner of its band

@@ -1,0 +1,43 @@
+"""The CTA-pair grouped GEMM of prefill-sized expert batches: intermediate sizes that put the up channels inside a weight
+tile, chunk sizes at their steps, experts without rows, ids without an expert; and silu without a general division."""
+import importlib
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import fp8_oracle as O
+from helpers import assert_parity, from_bf16, kernels, to_bf16_cuda
+from test_gpu_moe import make_moe_case, upload_weights
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("counts,H,I", [
+    ([256, 257, 0, 33], 272, 144),          # one full chunk, one row over (160 + 97), no rows, one row over 32; up rows inside a tile
+    ([31, 700, 1, 288], 512, 192),          # 64-row steps of the up channels; 3 chunks of 256 / 256 / 188
+    ([513, 64, 512, 95], 144, 16),          # the narrowest intermediate size
+])
+def test_pair_grouped_gemm_against_the_oracle(counts, H, I):
+    moe = importlib.import_module("nano-vllm-moe_b200.executor.moe")
+    E, T = len(counts), sum(counts)
+    assert T >= 512
+    c = make_moe_case(T + I, T, H, I, E, 1)
+    ids = np.repeat(np.arange(E), counts)
+    ids = np.random.default_rng(I).permutation(ids).astype(np.int64)[:, None]
+    w = np.random.default_rng(H).uniform(0.2, 1.0, (T, 1)).astype(np.float32)
+    cfg = moe.make_moe_parallel_config(tp_group=None, ep_group=None, global_num_experts=E, intermediate_size=I)
+    kern = moe.MoEKernel(prepare_finalize=moe.NoEPPrepareFinalize(cfg), experts=moe.Fp8Experts(), parallel_config=cfg)
+    ref = O.moe_experts_w8a8(c["x"], ids, w, c["w13_q"], c["w13_s"], c["in13"], c["w2_q"], c["w2_s"], c["in2"])
+    wts = upload_weights(moe, c)
+    x, wt = to_bf16_cuda(c["x"]), torch.from_numpy(w).cuda()
+    y = from_bf16(kern(x, wt, torch.from_numpy(ids).cuda(), wts, model_dtype=torch.bfloat16))
+    assert_parity(y, ref, f"pair experts {counts} H={H} I={I}", ulps=3.0, min_cos=0.9999)
+    # a token whose expert is not here gets nothing, the others the same bits
+    ids[::7] = -1
+    y2 = from_bf16(kern(x, wt, torch.from_numpy(ids).cuda(), wts, model_dtype=torch.bfloat16))
+    assert (y2[::7] == 0).all()
+    keep = np.ones(T, bool)
+    keep[::7] = False
+    np.testing.assert_array_equal(y2[keep], y[keep])
+    assert kernels().read_status(torch.device("cuda", 0)) == 0
