@@ -91,9 +91,12 @@ __device__ __forceinline__ uint32_t cvt_e4m3x2_to_f16x2(uint16_t v) {
 // that follows sees the same value as after a true division.
 struct ExactDiv {
     float s, r;
+    uint32_t plain_add;        // see quant8_e4m3: 0x8000 - (bf16 bits of the smallest magnitude that needs care), in both halves
     __device__ __forceinline__ explicit ExactDiv(float scale) {
         s = scale;
         r = __fdiv_rn(1.0f, scale);
+        const float lim = fminf(1.5e38f, 1.5e38f * scale);
+        plain_add = (0x8000u - (__float_as_uint(lim) >> 16)) * 0x00010001u;
     }
     __device__ __forceinline__ float operator()(float x) const {
         const float q0 = x * r;
@@ -116,14 +119,56 @@ __device__ __forceinline__ float silu_f32(float g) {
     return (fabsf(q0) <= 3.0e38f && q0 != 0.f) ? q1 : q0;
 }
 
+// Two lanes of fp32 arithmetic per instruction (sm_100).
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint16_t cvt_e4m3x2(uint64_t v) {
+    uint16_t r;
+    asm("{\n .reg .f32 lo, hi;\n mov.b64 {lo, hi}, %1;\n cvt.rn.satfinite.e4m3x2.f32 %0, hi, lo;\n}" : "=h"(r) : "l"(v));
+    return r;
+}
+
 // Static activation quantiser for 8 bf16 values (one 16-byte word) -> 8 e4m3 bytes;
 // the codes equal the reference's torch path (true division, RNE, clamp to +-448) bit for bit.
+//
+// The passes that quantise large activations run beside power-limited GEMMs at 1.2 GHz and are bound by instruction issue
+// there (five instructions of ExactDiv per element plus its selection).  So the quotients are refined two at a time, and
+// what ExactDiv selects per element is handled around them: a zero keeps its sign through an OR on the codes, and values so
+// large that q0 could overflow (or infinite, or NaN) send the whole word through ExactDiv.
 __device__ __forceinline__ uint2 quant8_e4m3(uint4 v, const ExactDiv& d) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint2 r;
-    uint32_t a = cvt_e4m3x2(d(bf16_lo(v.x)), d(bf16_hi(v.x)));
-    uint32_t b = cvt_e4m3x2(d(bf16_lo(v.y)), d(bf16_hi(v.y)));
-    uint32_t c = cvt_e4m3x2(d(bf16_lo(v.z)), d(bf16_hi(v.z)));
-    uint32_t e = cvt_e4m3x2(d(bf16_lo(v.w)), d(bf16_hi(v.w)));
+    const uint32_t m = __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
+    if (((m + d.plain_add) & 0x80008000u) == 0) {
+        const uint64_t rr = pack_f32x2(d.r, d.r), ns = pack_f32x2(-d.s, -d.s);
+        uint32_t c[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint64_t x = pack_f32x2(bf16_lo(w[i]), bf16_hi(w[i]));
+            const uint64_t q0 = mul_f32x2(x, rr);
+            c[i] = cvt_e4m3x2(fma_f32x2(fma_f32x2(q0, ns, x), rr, q0));
+        }
+        r.x = (c[0] | (c[1] << 16)) | (__byte_perm(w[0], w[1], 0x7531) & 0x80808080u);
+        r.y = (c[2] | (c[3] << 16)) | (__byte_perm(w[2], w[3], 0x7531) & 0x80808080u);
+        return r;
+    }
+    const uint32_t a = cvt_e4m3x2(d(bf16_lo(v.x)), d(bf16_hi(v.x)));
+    const uint32_t b = cvt_e4m3x2(d(bf16_lo(v.y)), d(bf16_hi(v.y)));
+    const uint32_t c = cvt_e4m3x2(d(bf16_lo(v.z)), d(bf16_hi(v.z)));
+    const uint32_t e = cvt_e4m3x2(d(bf16_lo(v.w)), d(bf16_hi(v.w)));
     r.x = a | (b << 16);
     r.y = c | (e << 16);
     return r;
