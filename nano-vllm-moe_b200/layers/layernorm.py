@@ -17,6 +17,7 @@ import torch
 from torch import nn
 
 from .. import _lib
+from .module import DirectModule
 
 
 class QuantizedActivation:
@@ -33,7 +34,7 @@ class QuantizedActivation:
         return self.codes.shape
 
 
-class RMSNorm(nn.Module):
+class RMSNorm(DirectModule):
     def __init__(self, hidden_size: int, eps: float = 1e-6) -> None:
         super().__init__()
         self.hidden_size = hidden_size

@@ -19,6 +19,7 @@ import torch.nn.functional as F
 from torch import nn
 
 from ..quantization.base_config import QuantizeMethodBase
+from .module import DirectModule
 
 
 def divide(numerator: int, denominator: int) -> int:
@@ -35,7 +36,7 @@ def _group_size_rank(group) -> tuple[int, int]:
     return 1, 0
 
 
-class LinearBase(nn.Module):
+class LinearBase(DirectModule):
     def __init__(self, input_size: int, output_size: int, tp_dim: int | None = None,
                  tp_group: Optional[dist.ProcessGroup] = None,
                  quant_method: QuantizeMethodBase | None = None, **kwargs):

@@ -15,10 +15,11 @@ from torch import nn
 
 from .. import _lib
 from ..quantization import kernels
+from .module import DirectModule
 from .linear import MergedColumnParallelLinear, RowParallelLinear
 
 
-class FusedFp8MLP(nn.Module):
+class FusedFp8MLP(DirectModule):
     """Wraps an already loaded and processed (gate_up_proj, down_proj) pair.
 
     ``release_unfused=True`` drops the gate_up layer's own packed weight after the interleaved copy
