@@ -945,23 +945,17 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     a.input_scale = w13_input_scale; a.topk_w = topk_w; a.out = gu; a.status = (int*)workspace;
     a.ldx = (int)ldx; a.x_div = x_div; a.ld_out = (int)(2 * I); a.N = (int)(2 * I); a.K = (int)H; a.n_tiles = 0; a.kblocks = 0;
     a.scatter = 0;
-    // prefill-sized batches with whole 128-channel tiles: the gate_up GEMM's epilogue applies the activation and writes hq
-    // (from 32-row chunks on: the epilogue reads the two accumulators 32 rows at a time)
-    const bool fused_act = pairs || (rows >= kMoePrequantRows && I % 128 == 0 && mp >= 32 && g_tune.moe_fused != 0);
+    // the gate_up GEMM's epilogue applies the activation and writes hq (the separate pass stays for comparison)
+    const bool fused_act = pairs || g_tune.moe_fused != 0;
+    GroupedArgs g = a;
+    if (fused_act) { g.N = (int)I; g.hq = hq; g.h_scale = w2_input_scale; g.out = nullptr; }
     if (rows >= kMoePrequantRows) {
         unsigned char* xq = ws + L.off_xq;
         e = launch_moe_scatter_quant((const __nv_bfloat16*)x, ldx, x_div, inv, (int)rows, w13_input_scale, xq, (int)H, st);
         if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row quantiser launch: %s", cudaGetErrorString(e));
-        if (fused_act) {
-            GroupedArgs f = a;
-            f.N = (int)I; f.hq = hq; f.h_scale = w2_input_scale; f.out = nullptr;
-            e = pairs ? launch_grouped_pair_w8a8(f, w13_packed, E, xq, rows, st, &why)
-                      : launch_grouped_w8a8(false, mp, f, w13_packed, E, xq, rows, st, &why);
-        } else {
-            e = launch_grouped_w8a8(false, mp, a, w13_packed, E, xq, rows, st, &why);
-        }
+        e = pairs ? launch_grouped_pair_w8a8(g, w13_packed, E, xq, rows, st, &why) : launch_grouped_w8a8(false, mp, g, w13_packed, E, xq, rows, st, &why);
     } else {
-        e = launch_grouped_w8a8(true, mp, a, w13_packed, E, nullptr, 0, st, &why);
+        e = launch_grouped_w8a8(true, mp, g, w13_packed, E, nullptr, 0, st, &why);
     }
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "gate_up grouped GEMM launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
     if (!fused_act) {

@@ -207,7 +207,6 @@ struct GroupedArgs {
     unsigned char* hq = nullptr;
     const float* h_scale = nullptr;
     int w_tiles = 0;             // 128-channel tile rows per expert in the packed weight (set by the launcher)
-    int up_tile_offset = 0;      // tile rows from a gate tile to the up tile of the same channels (set by the launcher)
 };
 int grouped_chunk_rows(int64_t rows, int num_experts);
 // Prefill-sized batches on CTA pairs (umma_grouped_pair.cu).  args.hq set = gate_up with the activation fused (args.N = I);

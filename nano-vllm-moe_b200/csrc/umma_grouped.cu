@@ -13,17 +13,18 @@
 //          token matrix through the sorted row index and quantised on the fly (static scale,
 //          exact division) by converter warps straight into the swizzled MMA "B" tile.
 //   false  the rows are already e4m3 and contiguous in sorted order (down projection always;
-//          gate_up after moe_gather_quant_kernel for prefill-sized batches): one TMA box.
+//          gate_up after moe_scatter_quant_kernel for prefill-sized batches): one TMA box.
 // Epilogue (run-time flag `scatter`):
 //   0      gu[sorted position][channel] = bf16(acc * in_scale * w_scale[e][channel])
 //   1      out[routed row][channel] = bf16(acc * in_scale * w_scale[e][channel] * topk_w[routed row])
 //
-// kFused (prefill-sized gate_up only, rows already e4m3): a work item covers the gate tile t AND the up tile t of the
-// expert (two weight boxes per K block against one box of rows, two accumulators), and the epilogue writes what the down
-// projection reads instead of the bf16 gate_up rows: hq[sorted position][channel] = e4m3(h / h_scale) with
-// h = bf16(bf16(silu(g)) * u) from g, u rounded to bf16 -- the values and roundings of the unfused path (the eager
-// two-rounding SiluAndMul of the reference's experts).  Half the row bytes per MAC through L2 -> SM, and the bf16 gate_up
-// tensor (rows x 2I x 2 bytes each way) and the separate activation pass disappear.
+// kFused (gate_up): the 128 rows of a weight tile are 64 gate channels and the 64 up channels of the same indices, so that a
+// work item holds both halves of 64 outputs and the epilogue writes what the down projection reads instead of bf16 gate_up
+// rows: hq[sorted position][channel] = e4m3(h / h_scale) with h = bf16(bf16(silu(g)) * u) from g, u rounded to bf16 -- the
+// values and roundings of the separate activation pass (the eager two-rounding SiluAndMul of the reference's experts).  The
+// warps of the gate lanes and of the up lanes swap half of their values through shared memory and finish half of the rows
+// each.  Any intermediate size that is a multiple of 16.  Saves the bf16 tensor and a launch of the decode step's chain
+// (64 tokens, 4 of 60 experts, hidden 2048, intermediate 1408, back to back: 101 -> 99 us per block).
 //
 // Weight-bandwidth-bound for small batches (each expert's weights are read once per chunk),
 // tensor-bound for prefill-sized batches.  All mbarrier waits are bounded.
@@ -39,23 +40,34 @@ constexpr int kGrpKB = 128;
 template <int MP, bool kFused = false>
 struct GroupedCfg {
     static constexpr int kWBytes = kGrpTile * kGrpKB;
-    static constexpr int kWTiles = kFused ? 2 : 1;                 // weight boxes per K block (gate and up)
     static constexpr int kXqBytes = MP * kGrpKB;
-    static constexpr int kStageBytes = kWTiles * kWBytes + kXqBytes;
-    static constexpr int kStagesRaw = (225 * 1024) / kStageBytes;
+    static constexpr int kStageBytes = kWBytes + kXqBytes;
+    static constexpr int kStagesRaw = (218 * 1024) / kStageBytes;
     static constexpr int kStages = kStagesRaw > 10 ? 10 : kStagesRaw;
     static constexpr int kSmemBytes = kStages * kStageBytes + 1024;
-    static constexpr int kAccCols = kWTiles * MP;                  // TMEM columns of one accumulator stage
+    static constexpr int kAccCols = MP;                            // TMEM columns of one accumulator stage
     static constexpr int kTmemCols = 2 * kAccCols < 32 ? 32 : 2 * kAccCols;
     static constexpr int kTeam = MP <= 16 ? 1 : (MP <= 32 ? 2 : 4);
     static constexpr int kPiece = MP < 32 ? MP : 32;            // accumulator columns per TMEM read
     static_assert(kStageBytes % 1024 == 0, "stage alignment");
 };
 
+__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr) : "memory");
+}
+
+// Boxes of the weights: 128 rows (plain), or 64 (fused; 16 where the up rows lie inside tiles); rows of xq: MP.
+struct GroupedMaps {
+    CUtensorMap w, w16, xq;
+};
+
 template <int MP, bool kGather, bool kFused = false>
 __global__ void __launch_bounds__(kGrpThreads, 1)
-grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_xq, GroupedArgs p) {
-    static_assert(!kFused || !kGather, "the fused activation epilogue takes pre-quantised rows");
+grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
     using Cfg = GroupedCfg<MP, kFused>;
     constexpr int S = Cfg::kStages;
     extern __shared__ unsigned char smem_raw[];
@@ -66,6 +78,9 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     __shared__ __align__(8) uint64_t bar_tempty[2];
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
+    constexpr int kSwapWords = kFused ? 2 * Cfg::kPiece * 16 : 1;              // bf16 pairs of kPiece rows x 32 channels, per warp pair
+    __shared__ __align__(16) uint32_t s_swap[kSwapWords];
+    __shared__ __align__(16) unsigned char s_code[kFused ? 2 * Cfg::kPiece * 32 : 16];
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int warp = warp_index();
@@ -99,8 +114,8 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         {
             const uint32_t el = elect_one();
             if (el) {
-                asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_w) : "memory");
-                if (!kGather) asm volatile("prefetch.tensormap [%0];" ::"l"(&tmap_xq) : "memory");
+                asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.w) : "memory");
+                if (!kGather) asm volatile("prefetch.tensormap [%0];" ::"l"(&maps.xq) : "memory");
             }
             uint32_t it = 0;
             bool ok = true;
@@ -108,7 +123,14 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 const int4 chunk = p.chunks[w / p.n_tiles];
                 const int2 ch = make_int2(uniform(chunk.x), uniform(chunk.y));
                 const int t = w % p.n_tiles;
-                const int wrow0 = (ch.x * p.w_tiles + t) * KB;        // packed tile index of (expert, tile, kb = 0)
+                // packed row of K block 0: tile t, or (fused) 64 gate channels and their up channels
+                const int wrow0 = kFused ? ((ch.x * p.w_tiles + (t >> 1)) * KB) * kGrpTile + (t & 1) * 64 : ((ch.x * p.w_tiles + t) * KB) * kGrpTile;
+                const int up_row = p.N + t * 64;
+                const bool up_whole = (p.N & 63) == 0;
+                int wrow_up[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    wrow_up[i] = ((ch.x * p.w_tiles + ((up_row + 16 * i) >> 7)) * KB) * kGrpTile + ((up_row + 16 * i) & 127);
                 for (int kb = 0; kb < KB; ++kb, ++it) {
                     const int st = it % S;
                     const uint32_t ph = (it / S) & 1;
@@ -116,11 +138,16 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     if (!ok) { s_abort = 1; break; }
                     const uint32_t full = smem_u32(&bar_full[st]);
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
-                    mbar_expect_tx(el, full, kGather ? Cfg::kWBytes : Cfg::kWTiles * Cfg::kWBytes + Cfg::kXqBytes);
-                    tma_load_2d(el, sa, &tmap_w, 0, (wrow0 + kb) * kGrpTile, full);
-                    // fused: the up tile of the same channels sits up_tile_offset tile rows further on in the expert's weight
-                    if (kFused) tma_load_2d(el, sa + Cfg::kWBytes, &tmap_w, 0, (wrow0 + p.up_tile_offset * KB + kb) * kGrpTile, full);
-                    if (!kGather) tma_load_2d(el, sa + Cfg::kWTiles * Cfg::kWBytes, &tmap_xq, kb * kGrpKB, ch.y, full);
+                    mbar_expect_tx(el, full, kGather ? Cfg::kWBytes : Cfg::kWBytes + Cfg::kXqBytes);
+                    tma_load_2d(el, sa, &maps.w, 0, wrow0 + kb * kGrpTile, full);
+                    if (kFused) {
+                        if (up_whole) tma_load_2d(el, sa + Cfg::kWBytes / 2, &maps.w, 0, wrow_up[0] + kb * kGrpTile, full);
+                        else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) tma_load_2d(el, sa + Cfg::kWBytes / 2 + i * 2048, &maps.w16, 0, wrow_up[i] + kb * kGrpTile, full);
+                        }
+                    }
+                    if (!kGather) tma_load_2d(el, sa + Cfg::kWBytes, &maps.xq, kb * kGrpKB, ch.y, full);
                 }
             }
             if (!ok) {
@@ -152,13 +179,9 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     tc_fence_after();
                     const uint32_t sa = smem_base + st * Cfg::kStageBytes;
                     const uint64_t da = make_smem_desc(sa);
-                    const uint64_t db = make_smem_desc(sa + Cfg::kWTiles * Cfg::kWBytes);
+                    const uint64_t db = make_smem_desc(sa + Cfg::kWBytes);
 #pragma unroll
-                    for (int k = 0; k < kGrpKB / 32; ++k) {
-                        umma_f8(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                        if (kFused)        // the up tile against the same rows, into the second half of the accumulator stage
-                            umma_f8(el, d_tmem + MP, make_smem_desc(sa + Cfg::kWBytes) + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < kGrpKB / 32; ++k) umma_f8(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                     umma_commit(el, smem_u32(&bar_empty[st]));
                 }
                 if (ok) umma_commit(el, smem_u32(&bar_tfull[as]));
@@ -215,8 +238,11 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const int t = w % p.n_tiles;
             const int as = tl & 1;
             const uint32_t aph = (tl >> 1) & 1;
-            const int n = t * kGrpTile + q * 32 + lane;                         // output channel of this lane
-            const float ws = (!kFused && n < p.N) ? in_scale * __ldg(p.w_scale + (size_t)ch.x * p.N + n) : 0.f;
+            // output channel of this lane and its multiplier (fused: lanes of quarters 2, 3 hold the up values of the channels
+            // of quarters 0, 1)
+            const bool up = kFused && q >= 2;
+            const int n = kFused ? t * 64 + (q & 1) * 32 + lane : t * kGrpTile + q * 32 + lane;
+            const float ws = n < p.N ? in_scale * __ldg(p.w_scale + (kFused ? (size_t)ch.x * 2 * p.N + (up ? p.N : 0) : (size_t)ch.x * p.N) + n) : 0.f;
             // routed-row index and routing weight of the chunk's rows, one row per lane and piece;
             // the inner loop gets them by shuffle instead of two dependent global loads per row
             int my_routed[(MP + 31) / 32];
@@ -230,34 +256,58 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                     my_w[i] = __ldg(p.topk_w + my_routed[i]);
                 }
             }
-            if (!mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull)) { s_abort = 1; ok = false; break; }
+            bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull);
+            if (kFused) {                         // warps that meet at barriers below leave together
+                uint32_t failed;
+                asm volatile(
+                    "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
+                    " barrier.cta.red.or.pred pout, 3, 128, pin;\n selp.u32 %0, 1, 0, pout;\n}"
+                    : "=r"(failed) : "r"(arrived ? 0u : 1u) : "memory");
+                arrived = failed == 0;
+            }
+            if (!arrived) { s_abort = 1; ok = false; break; }
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + as * Cfg::kAccCols;
-            if (kFused) {
-                // lane = gate channel n of the expert; its up channel is n + N.  One e4m3 byte per row and lane.
-                const float wu = n < p.N ? in_scale * __ldg(p.w_scale + (size_t)ch.x * 2 * p.N + p.N + n) : 0.f;
-                const float wg = n < p.N ? in_scale * __ldg(p.w_scale + (size_t)ch.x * 2 * p.N + n) : 0.f;
+            if constexpr (kFused) {
+                constexpr int kP = Cfg::kPiece, kH = kP / 4;      // rows per step; column pairs each warp of a pair finishes
                 const ExactDiv div_h(fmaxf(__ldg(p.h_scale), 1e-12f));
+                const uint32_t swap_buf = smem_u32(s_swap) + (uint32_t)(q & 1) * (kP * 64);
+                const uint32_t code_buf = smem_u32(s_code) + (uint32_t)(q & 1) * (kP * 32);
 #pragma unroll 1
-                for (int c0 = 0; c0 < MP; c0 += 32) {
-                    if (c0 >= ch.z) break;
-                    uint32_t g[32], u[32];
+                for (int c0 = 0; c0 < MP; c0 += kP) {
+                    if (c0 >= ch.z) break;                        // the same for both warps of a pair
+                    uint32_t v[kP];
                     __syncwarp();
-                    tmem_ld32_nowait(t_addr + c0, g);
-                    tmem_ld32_nowait(t_addr + MP + c0, u);
+                    if (kP == 32) tmem_ld32_nowait(t_addr + c0, v);
+                    else tmem_ld16_nowait(t_addr + c0, v);
                     tmem_ld_wait();
-                    if (n < p.N) {
+                    uint32_t own[kH], other[kH];
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            if (c0 + j < ch.z) {
-                                const uint32_t gu = pack_bf16x2(__uint_as_float(g[j]) * wg, __uint_as_float(u[j]) * wu);   // as the bf16 gate_up row
-                                const float gv = bf16_lo(gu);
-                                const uint32_t sv = pack_bf16x2(silu_f32(gv), 0.f);                              // bf16(silu(g))
-                                const uint32_t hv = pack_bf16x2(bf16_lo(sv) * bf16_hi(gu), 0.f);                           // bf16(. * u)
-                                p.hq[(size_t)(ch.y + c0 + j) * p.N + n] = (unsigned char)(cvt_e4m3x2(div_h(bf16_lo(hv)), 0.f) & 0xffu);
-                            }
-                        }
+                    for (int j = 0; j < kH; ++j) {                // as the bf16 gate_up row
+                        const uint32_t lo = pack_bf16x2(__uint_as_float(v[2 * j]) * ws, __uint_as_float(v[2 * j + 1]) * ws);
+                        const uint32_t hi = pack_bf16x2(__uint_as_float(v[kP / 2 + 2 * j]) * ws, __uint_as_float(v[kP / 2 + 2 * j + 1]) * ws);
+                        own[j] = up ? hi : lo;
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(swap_buf + (up ? 0 : kP * 32) + j * 128 + lane * 4), "r"(up ? lo : hi) : "memory");
                     }
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
+#pragma unroll
+                    for (int j = 0; j < kH; ++j)
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(swap_buf + (up ? kP * 32 : 0) + j * 128 + lane * 4) : "memory");
+                    const uint32_t code_at = code_buf + (up ? kP * 16 : 0) + lane;
+#pragma unroll
+                    for (int j = 0; j < kH; ++j) {
+                        const uint32_t g = up ? other[j] : own[j], u = up ? own[j] : other[j];
+                        const uint32_t sv = pack_bf16x2(silu_f32(bf16_lo(g)), silu_f32(bf16_hi(g)));                  // bf16(silu(g))
+                        const uint32_t hv = pack_bf16x2(bf16_lo(sv) * bf16_lo(u), bf16_hi(sv) * bf16_hi(u));          // bf16(. * u)
+                        const uint32_t code = cvt_e4m3x2(div_h(bf16_lo(hv)), div_h(bf16_hi(hv)));
+                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + 2 * j * 32), "r"(code & 0xffu) : "memory");
+                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + (2 * j + 1) * 32), "r"(code >> 8) : "memory");
+                    }
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
+                    // 32 bytes per row: thread i of the 64 stores half a row (N is a multiple of 16)
+                    const int i = (up ? 32 : 0) + lane, r = i >> 1, nh = (n - lane) + (i & 1) * 16;
+                    if (r < kP && c0 + r < ch.z && nh < p.N)
+                        *reinterpret_cast<float4*>(p.hq + (size_t)(ch.y + c0 + r) * p.N + nh) = ld_shared_f4(code_buf + r * 32 + (i & 1) * 16);
                 }
                 tc_fence_before();
                 __syncwarp();
@@ -270,13 +320,7 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 uint32_t v[Cfg::kPiece];
                 __syncwarp();
                 if (Cfg::kPiece == 32) tmem_ld32_nowait(t_addr + c0, v);
-                else {
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                        : "r"(t_addr + c0) : "memory");
-                }
+                else tmem_ld16_nowait(t_addr + c0, v);
                 tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < Cfg::kPiece; ++j) {
@@ -307,7 +351,7 @@ grouped_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 
 // ---- host side -------------------------------------------------------------------
 template <int MP, bool kGather, bool kFused = false>
-static cudaError_t launch_grouped(const GroupedArgs& a, const CUtensorMap& tw, const CUtensorMap& tx, cudaStream_t stream) {
+static cudaError_t launch_grouped(const GroupedArgs& a, const GroupedMaps& maps, cudaStream_t stream) {
     using Cfg = GroupedCfg<MP, kFused>;
     auto kern = grouped_w8a8_kernel<MP, kGather, kFused>;
     static SmemOptIn opted;
@@ -323,7 +367,7 @@ static cudaError_t launch_grouped(const GroupedArgs& a, const CUtensorMap& tw, c
     cudaLaunchAttribute attr[1];
     cfg.numAttrs = pdl_attribute(attr);
     cfg.attrs = attr;
-    return counted(cudaLaunchKernelEx(&cfg, kern, tw, tx, a));
+    return counted(cudaLaunchKernelEx(&cfg, kern, maps, a));
 }
 
 int grouped_chunk_rows(int64_t rows, int num_experts) {
@@ -333,28 +377,26 @@ int grouped_chunk_rows(int64_t rows, int num_experts) {
 
 cudaError_t launch_grouped_w8a8(bool gather, int mp, GroupedArgs a, const void* w_packed, int num_experts,
                                 const void* xq_sorted, int64_t xq_rows, cudaStream_t stream, const char** why) {
-    CUtensorMap tw, tx;
+    GroupedMaps maps;
     const bool fused = a.hq != nullptr;           // a.N = I gate channels; the expert's weight holds 2 I channels
-    a.n_tiles = (int)pack_ntiles(a.N);
-    a.w_tiles = fused ? 2 * a.n_tiles : a.n_tiles;
-    a.up_tile_offset = fused ? a.n_tiles : 0;
+    a.n_tiles = fused ? (a.N + 63) / 64 : (int)pack_ntiles(a.N);
+    a.w_tiles = (int)pack_ntiles(fused ? 2 * (int64_t)a.N : a.N);
     a.kblocks = (int)pack_kblocks(a.K);
-    if (fused && (gather || a.N % kGrpTile != 0 || mp < 32 || mp > 128)) {
-        if (why) *why = "the fused activation epilogue needs pre-quantised rows and an intermediate size that is a multiple of 128";
-        return cudaErrorInvalidValue;
-    }
-    if (!encode_u8_2d(&tw, w_packed, (uint64_t)num_experts * a.w_tiles * a.kblocks * 128, 128, kGrpTile)) {
+    const uint64_t w_rows = (uint64_t)num_experts * a.w_tiles * a.kblocks * 128;
+    if (!encode_u8_2d(&maps.w, w_packed, w_rows, 128, fused ? 64 : kGrpTile) || !encode_u8_2d(&maps.w16, w_packed, w_rows, 128, 16)) {
         if (why) *why = "cuTensorMapEncodeTiled failed for the expert weights";
         return cudaErrorInvalidValue;
     }
-    tx = tw;
-    if (!gather && !encode_u8_2d(&tx, xq_sorted, (uint64_t)xq_rows, (uint64_t)a.K, (uint32_t)mp)) {
+    maps.xq = maps.w;
+    if (!gather && !encode_u8_2d(&maps.xq, xq_sorted, (uint64_t)xq_rows, (uint64_t)a.K, (uint32_t)mp)) {
         if (why) *why = "cuTensorMapEncodeTiled failed for the quantised rows";
         return cudaErrorInvalidValue;
     }
-#define FP8LIN_GROUPED_CASE(MP_) \
-    if (mp == MP_) return fused ? launch_grouped<MP_, false, true>(a, tw, tx, stream) \
-                                : (gather ? launch_grouped<MP_, true>(a, tw, tx, stream) : launch_grouped<MP_, false>(a, tw, tx, stream));
+#define FP8LIN_GROUPED_CASE(MP_)                                                                                               \
+    if (mp == MP_) {                                                                                                           \
+        if (gather) return fused ? launch_grouped<MP_, true, true>(a, maps, stream) : launch_grouped<MP_, true>(a, maps, stream); \
+        return fused ? launch_grouped<MP_, false, true>(a, maps, stream) : launch_grouped<MP_, false>(a, maps, stream);          \
+    }
     FP8LIN_GROUPED_CASE(16)
     FP8LIN_GROUPED_CASE(32)
     FP8LIN_GROUPED_CASE(64)

@@ -41,3 +41,29 @@ def test_pair_grouped_gemm_against_the_oracle(counts, H, I):
     keep[::7] = False
     np.testing.assert_array_equal(y2[keep], y[keep])
     assert kernels().read_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("counts,H,I", [
+    ([3, 0, 16, 17], 272, 144),             # 16-row chunks, gathered rows; up rows inside a tile
+    ([30, 1, 33, 25], 144, 16),             # 32-row chunks, the narrowest intermediate size
+    ([100, 64, 65, 1], 512, 192),           # 64
+    ([200, 129], 256, 64),                  # 128
+    ([4] * 130, 144, 48),                   # 16-row chunks of pre-quantised rows
+])
+def test_fused_activation_equals_the_separate_pass(counts, H, I):
+    moe = importlib.import_module("nano-vllm-moe_b200.executor.moe")
+    Kn = kernels()
+    E, T = len(counts), sum(counts)
+    c = make_moe_case(T + I, T, H, I, E, 1)
+    ids = torch.from_numpy(np.random.default_rng(I).permutation(np.repeat(np.arange(E), counts)).astype(np.int64)[:, None]).cuda()
+    w = torch.rand((T, 1), device="cuda") + 0.2
+    cfg = moe.make_moe_parallel_config(tp_group=None, ep_group=None, global_num_experts=E, intermediate_size=I)
+    kern = moe.MoEKernel(prepare_finalize=moe.NoEPPrepareFinalize(cfg), experts=moe.Fp8Experts(), parallel_config=cfg)
+    wts, x = upload_weights(moe, c), to_bf16_cuda(c["x"])
+    y = kern(x, w, ids, wts, model_dtype=torch.bfloat16)
+    try:
+        Kn.set_tuning("moe_fused", 0)
+        assert torch.equal(y, kern(x, w, ids, wts, model_dtype=torch.bfloat16))
+    finally:
+        Kn.set_tuning("moe_fused", -1)
+    assert Kn.read_status(torch.device("cuda", 0)) == 0
