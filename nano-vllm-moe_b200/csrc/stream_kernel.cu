@@ -239,13 +239,13 @@ stream_linear_kernel(StreamArgs p) {
 
     if (n_splits > 1 && push) {
         cluster_wait();
-        const uint32_t recv = smem_u32(smem) + 2 * kBufBytes;           // behind the x double buffer: [split - 1][thread][MT][4]
+        const uint32_t recv = smem_u32(smem) + 2 * kBufBytes;           // behind the x double buffer: [split - 1][MT][thread][4]
         if (crank != 0) {
-            const uint32_t dst = map_to_cta(recv + ((crank - 1) * (NWARPS * 32) + threadIdx.x) * (MT * 16), 0);
+            const uint32_t dst = map_to_cta(recv + ((crank - 1) * (NWARPS * 32 * MT) + threadIdx.x) * 16, 0);
             const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), 0);
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
-                st_async_v4(dst + mt * 16, __float_as_uint(acc[mt][0]), __float_as_uint(acc[mt][1]), __float_as_uint(acc[mt][2]),
+                st_async_v4(dst + mt * (NWARPS * 32 * 16), __float_as_uint(acc[mt][0]), __float_as_uint(acc[mt][1]), __float_as_uint(acc[mt][2]),
                             __float_as_uint(acc[mt][3]), rbar);
             return;
         }
@@ -253,7 +253,7 @@ stream_linear_kernel(StreamArgs p) {
         for (int s = 1; s < n_splits; ++s) {
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
-                const float4 v = ld_shared_f4(recv + ((s - 1) * (NWARPS * 32) + threadIdx.x) * (MT * 16) + mt * 16);
+                const float4 v = ld_shared_f4(recv + ((s - 1) * (NWARPS * 32 * MT) + mt * (NWARPS * 32) + threadIdx.x) * 16);
                 acc[mt][0] += v.x; acc[mt][1] += v.y; acc[mt][2] += v.z; acc[mt][3] += v.w;
             }
         }

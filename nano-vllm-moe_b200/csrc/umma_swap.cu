@@ -63,9 +63,8 @@ struct SwapCfg {
     static constexpr int kRingBytes = kStages * kStageBytes;
     static constexpr int kSmemBytes = kRingBytes + 1024 + kRecvBytes;
     static constexpr int kTmemCols = 2 * MP < 32 ? 32 : 2 * MP;
-    static constexpr int kPartPitch = MP * 4 + 16;               // row pitch of the received fp32 partial sums (split-K)
     static_assert(kStageBytes % 1024 == 0, "stages must keep 1024-byte alignment for the swizzle");
-    static_assert((kTileN + 8) * kPartPitch <= kRingBytes, "the received slices of a band must fit in the ring");
+    static_assert((kTileN + 8) * MP * 4 <= kRingBytes, "the received slices of a band must fit in the ring");
 };
 
 struct SwapSched {
@@ -129,11 +128,13 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const uint32_t recv_bytes_warp = 32u * (uint32_t)((p.M + 7) >> 3) * 16u;      // what one up warp sends per pair
     const int kb0 = split_rank * sched.kblocks_per_split;
     const int kb1 = kSplit ? min(sched.kblocks_total, kb0 + sched.kblocks_per_split) : sched.kblocks_total;
-    // split-K: CTA r of the cluster finishes channels [r * band, r * band + band_rows) of the tile; a slice's partials
-    // of one channel are MP floats kPartPitch bytes apart, the slices of a band follow each other in the owner's ring
+    // split-K: CTA r of the cluster finishes channels [r * band, r * band + band_rows) of the tile; received
+    // sums lie in the owner's ring as [slice][group of four rows][channel of the band] (see st_async_v4)
     const int band = kSplit ? (kTileN + sched.splits - 1) / sched.splits : kTileN;
     const int band_rows = kSplit ? min(kTileN, (split_rank + 1) * band) - split_rank * band : 0;
     const int m_groups = (p.M + 3) >> 2;                          // rows travel in groups of four
+    const uint32_t group_bytes = (uint32_t)band * 16u;
+    const uint32_t slice_bytes = group_bytes * (MP / 4);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < S; ++i) {
@@ -420,11 +421,11 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 if (!mbar_wait(smem_u32(&bar_ready), 0, p.status, kDevTimeoutPeer)) { s_abort = 1; ok = false; break; }
                 const int c = q * 32 + lane;
                 const uint32_t owner = (uint32_t)(c / band);
-                const uint32_t dst = map_to_cta(smem_base + (uint32_t)(split_rank * band + (c - (int)owner * band)) * Cfg::kPartPitch, owner);
+                const uint32_t dst = map_to_cta(smem_base + (uint32_t)split_rank * slice_bytes + (uint32_t)(c - (int)owner * band) * 16u, owner);
                 const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), owner);
 #pragma unroll
                 for (int m = 0; m < MP; m += 4)
-                    if (m < p.M) st_async_v4(dst + m * 4, v[m], v[m + 1], v[m + 2], v[m + 3], rbar);
+                    if (m < p.M) st_async_v4(dst + (uint32_t)(m >> 2) * group_bytes, v[m], v[m + 1], v[m + 2], v[m + 3], rbar);
             }
         }
     }
@@ -443,19 +444,18 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         if ((int)threadIdx.x >= band_rows * m_groups) return;
         if (s_abort || !mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) return;
         const float in_scale = in_scale0;
-        const uint32_t slice = (uint32_t)band * Cfg::kPartPitch;
         // consecutive threads take consecutive channels, so the stores of one token coalesce
         for (int i = threadIdx.x; i < band_rows * m_groups; i += kSwapThreads) {
             const int rl = i % band_rows;
             const int mg = (i / band_rows) * 4;
             const int n = first_tile * kTileN + split_rank * band + rl;
             if (n >= p.N) continue;
-            const uint32_t local = smem_base + (uint32_t)rl * Cfg::kPartPitch + (uint32_t)mg * 4;
+            const uint32_t local = smem_base + (uint32_t)(mg >> 2) * group_bytes + (uint32_t)rl * 16u;
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int sl = 0; sl < 8; ++sl) {
                 if (sl < sched.splits) {
-                    const float4 u = ld_shared_f4(local + (uint32_t)sl * slice);
+                    const float4 u = ld_shared_f4(local + (uint32_t)sl * slice_bytes);
                     a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
                 }
             }

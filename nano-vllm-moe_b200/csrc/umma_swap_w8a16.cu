@@ -44,10 +44,9 @@ struct Swap16Cfg {
     static constexpr int kAccCols = 2 * MP < 32 ? 32 : 2 * MP;   // two accumulator stages
     static constexpr int kACols = 64;                            // one widened weight tile: 128 K / 2 per column
     static constexpr int kTmemCols = 512;
-    static constexpr int kPartPitch = MP * 4 + 16;
     static_assert(kAccCols + kStages * kACols <= kTmemCols, "TMEM budget");
     static_assert(kStageBytes % 1024 == 0, "stage alignment");
-    static_assert((kS16Tile + 8) * kPartPitch <= kRingBytes, "the received slices of a band must fit in the ring");
+    static_assert((kS16Tile + 8) * MP * 4 <= kRingBytes, "the received slices of a band must fit in the ring");
 };
 
 struct Swap16Sched {
@@ -119,6 +118,8 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const int band = kSplit ? (kS16Tile + sched.splits - 1) / sched.splits : kS16Tile;
     const int band_rows = kSplit ? min(kS16Tile, (split_rank + 1) * band) - split_rank * band : 0;
     const int m_groups = (p.M + 3) >> 2;
+    const uint32_t group_bytes = (uint32_t)band * 16u;
+    const uint32_t slice_bytes = group_bytes * (MP / 4);
     constexpr uint32_t kXfOff = Cfg::kWBytes;
     constexpr uint32_t kXrawOff = Cfg::kWBytes + Cfg::kXfBytes;
 
@@ -326,11 +327,11 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 if (!mbar_wait(smem_u32(&bar_ready), 0, p.status, kDevTimeoutPeer)) { s_abort = 1; ok = false; break; }
                 const int c = q * 32 + lane;
                 const uint32_t owner = (uint32_t)(c / band);
-                const uint32_t dst = map_to_cta(smem_base + (uint32_t)(split_rank * band + (c - (int)owner * band)) * Cfg::kPartPitch, owner);
+                const uint32_t dst = map_to_cta(smem_base + (uint32_t)split_rank * slice_bytes + (uint32_t)(c - (int)owner * band) * 16u, owner);
                 const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), owner);
 #pragma unroll
                 for (int m = 0; m < MP; m += 4)
-                    if (m < p.M) st_async_v4(dst + m * 4, v[m], v[m + 1], v[m + 2], v[m + 3], rbar);
+                    if (m < p.M) st_async_v4(dst + (uint32_t)(m >> 2) * group_bytes, v[m], v[m + 1], v[m + 2], v[m + 3], rbar);
             }
         }
     }
@@ -348,18 +349,17 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         pdl_wait();
         if ((int)threadIdx.x >= band_rows * m_groups) return;
         if (s_abort || !mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) return;
-        const uint32_t slice = (uint32_t)band * Cfg::kPartPitch;
         for (int i = threadIdx.x; i < band_rows * m_groups; i += kS16Threads) {
             const int rl = i % band_rows;
             const int mg = (i / band_rows) * 4;
             const int n = first_tile * kS16Tile + split_rank * band + rl;
             if (n >= p.N) continue;
-            const uint32_t local = smem_base + (uint32_t)rl * Cfg::kPartPitch + (uint32_t)mg * 4;
+            const uint32_t local = smem_base + (uint32_t)(mg >> 2) * group_bytes + (uint32_t)rl * 16u;
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int sl = 0; sl < 8; ++sl) {
                 if (sl < sched.splits) {
-                    const float4 u = ld_shared_f4(local + (uint32_t)sl * slice);
+                    const float4 u = ld_shared_f4(local + (uint32_t)sl * slice_bytes);
                     a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
                 }
             }

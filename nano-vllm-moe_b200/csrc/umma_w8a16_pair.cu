@@ -44,7 +44,7 @@ constexpr int kRingBytes = 216 * 1024;         // activation ring (128 T bytes p
 constexpr int kSmemBytes = kRingBytes + 1024;
 constexpr int kACols = 64;                     // 128 bf16 of a row = 64 columns
 constexpr int kTmemCols = 512;
-static_assert((kTile + 8) * (256 * 4 + 16) <= kRingBytes, "the received slices of a band must fit in the ring");
+static_assert((kTile + 4) * 256 * 4 <= kRingBytes, "the received slices of a band must fit in the ring");
 
 // Ring depths for T tokens per tile.  A slot is occupied from its TMA until its MMAs (activations) or its widening (weights)
 // are done, an L2 / HBM round trip of 1 to 1.5 us under load plus the chain through converters and tensor core, so with
@@ -75,23 +75,6 @@ struct PairSched16 {
     int kblocks, kblocks_per_split;
 };
 
-// mbar_wait for a barrier that the partner CTA arrives on: acquires at cluster scope
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int* status, int code) {
-    long long start = -1;
-    for (uint32_t it = 0;; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-        if ((it & 0x3ff) == 0x3ff) {
-            const long long now = clock64();
-            if (start < 0) start = now;
-            else if (now - start > kWaitCycles) { atomicExch(status, code); return false; }
-        }
-    }
-}
-
 // 32 consecutive TMEM columns of this lane <- 32 registers; no wait
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
     asm volatile(
@@ -105,14 +88,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
         : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t* v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr) : "memory");
-}
 
 // Two e4m3 codes, zero-extended in the two halves of p, -> bf16x2, exact.  The magnitude bits go to bits 4..10 of a bf16
 // and the sign to bit 15 (b * 16 + (b & 0x80) * 240, no carry between the halves); that bf16 is the code's value times
@@ -207,7 +182,9 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const int m_left = kSplit ? p.M - (first_item % sched.m_tiles) * T : 0;
     const int m_valid = kSplit ? min(T, m_left) : 0;
     const int m_groups = (m_valid + 3) >> 2;
-    const uint32_t pitch = (uint32_t)T * 4 + 16;
+    // received sums: [slice][group of four tokens][channel of the band] (see st_async_v4)
+    const uint32_t group_bytes = (uint32_t)band * 16u;
+    const uint32_t slice_bytes = group_bytes * (uint32_t)(T >> 2);
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxW; ++i) { mbar_init(smem_u32(&bar_wfull[i]), 1); mbar_init(smem_u32(&bar_wempty[i]), kConvWarps / 2); }
@@ -413,7 +390,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const int c0 = q * 32 + lane;
                 const int owner = c0 / band;
                 const uint32_t owner_cta = (uint32_t)(2 * owner) + rank;
-                const uint32_t dst = map_to_cta(smem_base + (uint32_t)(slice_rank * band + (c0 - owner * band)) * pitch + (uint32_t)(h * half) * 4, owner_cta);
+                const uint32_t dst = map_to_cta(smem_base + slice_rank * slice_bytes + (uint32_t)(h * half >> 2) * group_bytes + (uint32_t)(c0 - owner * band) * 16u, owner_cta);
                 const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), owner_cta);
                 for (int c = 0; c < half; c += 32) {
                     uint32_t v[32];
@@ -424,7 +401,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         if (j == 16 && c + 16 >= half) break;
-                        if (h * half + c + j < m_valid) st_async_v4(dst + (c + j) * 4, v[j], v[j + 1], v[j + 2], v[j + 3], rbar);
+                        if (h * half + c + j < m_valid) st_async_v4(dst + (uint32_t)((c + j) >> 2) * group_bytes, v[j], v[j + 1], v[j + 2], v[j + 3], rbar);
                     }
                 }
             }
@@ -438,18 +415,17 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         if (band_rows > 0 && !s_abort && mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) {
             const int n_base = (2 * (first_item / sched.m_tiles) + (int)rank) * kTile + slice_rank * band;
             const int m_base = (first_item % sched.m_tiles) * T;
-            const uint32_t slice = (uint32_t)band * pitch;
             for (int i = threadIdx.x; i < band_rows * m_groups; i += kThreads) {
                 const int rl = i % band_rows;
                 const int mg = (i / band_rows) * 4;
                 const int n = n_base + rl;
                 if (n >= p.N) continue;
-                const uint32_t local = smem_base + (uint32_t)rl * pitch + (uint32_t)mg * 4;
+                const uint32_t local = smem_base + (uint32_t)(mg >> 2) * group_bytes + (uint32_t)rl * 16u;
                 float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
                 for (int sl = 0; sl < 4; ++sl) {
                     if (sl < sched.splits) {
-                        const float4 u = ld_shared_f4(local + (uint32_t)sl * slice);
+                        const float4 u = ld_shared_f4(local + (uint32_t)sl * slice_bytes);
                         a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
                     }
                 }
