@@ -78,13 +78,13 @@ int validate_common(const void* x, int64_t ldx, const void* w, const float* w_sc
 
 // Layers of up to ~17 MB with a short K (qkv, o_proj): up to 8 rows the mma.sync streaming kernel -- many small CTAs, its
 // split-K slices handing their sums over inside a cluster -- starts and drains faster than the tcgen05 kernels.
-bool small_layer(int64_t K, int64_t N, int64_t max_k) { return K <= max_k && N <= 4736; }
+bool small_layer(int64_t K, int64_t N) { return K <= 8192 && N <= 4736; }
 
 bool w8a16_swap_eligible(int64_t M, int64_t K, int64_t N) {
     // measured (us, mma.sync kernel / tcgen05 kernel, which widens the weights on its way to TMEM): one row 3584 -> 37888
     // 23.1 / 21.0, 18944 -> 3584 15.7 / 14.0, 2048 -> 11008 8.1 / 6.9, but 3584 -> 4608 5.7 / 6.5, 3584 -> 3584 4.7 / 6.0,
     // 5120 -> 2560 5.4 / 6.2; 16 rows 26.9 / 22.8, 20.2 / 15.5, 10.1 / 7.8, 9.0 / 7.7, 7.8 / 6.9, 7.7 / 7.1
-    const int min_m = g_tune.w8a16_swap_min_m >= 0 ? g_tune.w8a16_swap_min_m : (small_layer(K, N, 8192) ? 9 : 1);
+    const int min_m = g_tune.w8a16_swap_min_m >= 0 ? g_tune.w8a16_swap_min_m : (small_layer(K, N) ? 9 : 1);
     return g_tune.w8a16_swap_enable != 0 && M >= min_m && M <= 64;
 }
 
@@ -196,11 +196,13 @@ bool pair_rounds_full(int64_t M, int64_t N) {
 
 bool swap_eligible(int64_t M, int64_t K, int64_t N) {
     const int max_m = g_tune.stream_max_m >= 0 ? g_tune.stream_max_m : kDefaultStreamMaxM;
-    // The tcgen05 kernel from the first row on, except on small layers.  Measured, us, tcgen05 / streaming kernel, one row
-    // (eight rows): 3584 -> 4608 6.1 / 5.8 (6.4 / 6.4), 3584 -> 3584 5.4 / 4.8 (5.7 / 5.4), 2048 -> 2048 3.8 / 3.7 (4.1 / 4.0);
-    // but 5120 -> 2560 5.5 / 5.9 (5.8 / 6.4), 2048 -> 11008 6.9 / 9.1, 18944 -> 3584 13.7 / 16.6, 3584 -> 37888 20.6 / 23.7.
+    // The tcgen05 kernel from the first row on, except on layers of up to ~17 MB with a short K (qkv, o_proj), where up to 8
+    // rows the mma.sync streaming kernel starts and drains faster.  Measured, us, tcgen05 / streaming kernel, one row (eight
+    // rows): 3584 -> 4608 6.1 / 5.8 (6.4 / 6.4), 3584 -> 3584 5.4 / 4.8 (5.7 / 5.4), 2048 -> 2048 3.8 / 3.7 (4.1 / 4.0); but 2048
+    // -> 11008 6.9 / 9.1, 18944 -> 3584 13.7 / 16.6, 3584 -> 37888 20.6 / 23.7.  (5120 -> 2560 5.5 / 5.9 would now go the other
+    // way; the line stays, because the two kernels add the products of an output in different orders: see plan_swap.)
     int min_m = g_tune.swap_min_m >= 0 ? g_tune.swap_min_m : 1;
-    if (g_tune.swap_min_m < 0 && small_layer(K, N, 4096)) min_m = 9;
+    if (g_tune.swap_min_m < 0 && small_layer(K, N)) min_m = 9;
     return g_tune.swap_enable != 0 && M >= min_m && M <= 64 && M <= max_m;
 }
 

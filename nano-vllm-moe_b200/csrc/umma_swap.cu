@@ -534,20 +534,20 @@ SwapPlan plan_swap(int64_t M, int64_t K, int64_t N, int force_splits, bool preq)
         // 7.9 us against 10.9 us unsplit on 2048 -> 11008), so for that kernel the figure is doubled.
         if (s > 1 && pl.mp == 16) slots *= 2;
         if (slots < 1) slots = 1;
-        // Time in microseconds: the K blocks of a slice at the rate the resident CTAs share the HBM stream (a CTA alone is bound
-        // by its ring: 0.22 us per 16 KB block, a little more with wider token tiles or rows converted in the kernel), what a
-        // launch pays once (2.2), and for slices the hand-over of the partial sums, which grows with rows x slices.  Unsplit
-        // CTAs are persistent, so their rounds ramp once; a wave of clusters does not overlap the next.  Fitted to all slice
-        // counts over nine layer shapes (2048 -> 2048 .. 18944 -> 3584 .. 3584 -> 37888, 1280 -> 1536, 5120 -> 2560) at 1 to 64
-        // rows after the issuing warps stopped bounding a block (0.32 us before): the choice is within 2 % of the best on
-        // average, e.g. 64 rows on 2560 -> 9472 unsplit 8.3 us against 10.0 with the two slices taken before.
+        // The slice count fixes the order in which the products of an output are added, so it is part of the result: another
+        // count moves a few bf16 results by their last bit, and a stack of layers spreads that through the e4m3 codes
+        // between its linears (four layers end 2 to 3 % apart).  So the counts stay what this model of the time of a wave has
+        // always given, whatever kernel adds the slices up: the K blocks of a slice at the rate the resident CTAs share the HBM
+        // stream (0.32 us per 16 KB block for a CTA alone, more with wider token tiles or rows converted in the kernel), and
+        // what a wave pays once -- ramp, hand-over of the partial sums, drain.
         const int ctas = pl.n_tiles * s;
         const int resident = ctas < slots * s ? ctas : slots * s;
-        const double alone = (pl.mp == 16 ? 0.217 : (pl.mp == 32 ? 0.228 : 0.231)) + (preq || pl.mp != 16 ? 0.0 : 0.0126 * (double)(M < 16 ? M : 16));
+        const double alone = (pl.mp == 16 ? 0.32 : (pl.mp == 32 ? 0.36 : 0.40)) + (preq ? 0.0 : 0.008 * (double)(M < 16 ? M : 16));
         const double shared = 16384.0 * resident / 6.5e6;
         const double t_block = shared > alone ? shared : alone;
         const int waves = (pl.n_tiles + slots - 1) / slots;
-        const double cost = s > 1 ? waves * (kps * t_block + 2.2 + 0.63 + 0.0095 * (double)M * s) : waves * kps * t_block + 2.2;
+        const double fixed = 3.5 + (s > 1 ? 0.5 + (0.1 + 0.006 * (double)M) * s : 0.0);
+        const double cost = waves * (kps * t_block + fixed);
         if (cost < best_cost) { best_cost = cost; best_s = s; }
     }
     // Long K over few channel tiles (18944 -> 3584: 28 tiles x 148 K blocks), two CTAs per SM: measured
