@@ -305,6 +305,8 @@ const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N);
  * itself instead of a pass in front of it; n > 1 = the pass takes the first n rows), "quant_lead",
  * "w8a16_umma_min_m" (rows from which W8A16 takes the f16 GEMM route; 0 = never), "w8a16_chunk_mb", "pdl",
  * "w8a16_pair" (0 / 1: never / always the W8A16 CTA-pair kernel), "w8a16_pair_tokens", "w8a16_pair_splits",
+ * "w8a8_pair" (0 / 1: never / always the W8A8 CTA-pair kernel with the rows as the MMA's N), "w8a8_pair_tokens",
+ * "w8a8_pair_slices", "w8a8_pair_splits",
  * "stream_push" (0 = split-K of the mma.sync streaming kernel always through global scratch instead of a cluster),
  * "mlp_decode_fused" (1 = the fused MLP on up to 16 pre-quantised rows computes silu * up inside the gate_up kernel),
  * "moe_fused" (0 = the expert FFN keeps a separate activation pass), "moe_rows_major" (0 = prefill-sized expert

@@ -37,6 +37,10 @@ struct Tuning {
     int w8a16_pair = -1;        // 0 = never the CTA-pair kernel that widens weights into TMEM, 1 = for every M
     int w8a16_pair_tokens = -1; // force its tokens per tile / its K slices
     int w8a16_pair_splits = -1;
+    int w8a8_pair = -1;         // 0 = never the CTA-pair kernel with the rows as the MMA's N, 1 = for every M
+    int w8a8_pair_tokens = -1;  // force its tokens per tile / its K slices / whether a cluster takes them (1 = no)
+    int w8a8_pair_slices = -1;
+    int w8a8_pair_splits = -1;
     int umma_pair = -1;         // 1 = large-M GEMMs on CTA pairs (256 x 256 tiles), 0 = never
     int fuse_quant = -1;        // large-M W8A8: <= 0 (default) = quantise x in a separate pass; 1 = the pass takes the rows
                                 // of the first round of tiles, the GEMM's own quantiser warps the rest; n > 1 = the pass
@@ -88,10 +92,39 @@ bool w8a16_swap_eligible(int64_t M, int64_t K, int64_t N) {
     return g_tune.w8a16_swap_enable != 0 && M >= min_m && M <= 64;
 }
 
+// Routes by shape, kept per thread: the search for a plan takes 2 to 3 us of host time, as long as a small call's launch.  A
+// fixed number of entries (a later shape replaces an earlier one); a knob that changes makes them all stale.
+unsigned g_tune_version = 0;
+template <class Route, class Make>
+const Route& route_of(int64_t M, int64_t K, int64_t N, int flavour, Make make) {
+    struct Entry {
+        int64_t M = 0, K = 0, N = 0;
+        int flavour = 0;
+        unsigned version = 0;
+        Route route;
+    };
+    static thread_local Entry table[128];
+    const uint64_t h = ((uint64_t)M * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)K * 0xc2b2ae3d27d4eb4full) ^ ((uint64_t)N * 0x165667b19e3779f9ull);
+    Entry& e = table[((h >> 40) + (uint64_t)flavour) & 127];
+    if (e.M != M || e.K != K || e.N != N || e.flavour != flavour || e.version != g_tune_version) {
+        e.route = make();
+        e.M = M; e.K = K; e.N = N; e.flavour = flavour; e.version = g_tune_version;
+    }
+    return e.route;
+}
+
+struct W8a16Route {
+    bool pair = false;
+    W8a16PairPlan plan{};
+};
+struct W8a8Route {
+    bool pair = false;
+    W8a8PairPlan plan{};
+};
+
 // W8A16 on CTA pairs with the weights widened into tensor memory and the caller's bf16 rows as the other operand.
 // A knob that selects one of the other W8A16 routes switches it off.
-bool w8a16_pair_eligible(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
-    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return false;             // (two channels per store)
+bool w8a16_pair_wanted(int64_t M, int64_t K, int64_t N) {
     if (g_tune.w8a16_pair >= 0) return g_tune.w8a16_pair != 0;
     if (g_tune.w8a16_umma_min_m >= 0 || g_tune.w8a16_chunk_mb > 0 || g_tune.w8a16_swap_min_m >= 0 || g_tune.w8a16_swap_enable >= 0 ||
         g_tune.stream_splits > 0 || g_tune.swap_splits > 0)
@@ -101,6 +134,17 @@ bool w8a16_pair_eligible(int64_t M, int64_t K, int64_t N, int64_t ldy, const voi
     // 64 rows): 2048 -> 11008 11.0 us against 12.3, 2560 -> 9472 10.9 / 12.1, 3584 -> 37888 33.0 / 33.8; with slices it keeps
     // 3584 -> 4608 12.2 / 11.4, 18944 -> 3584 25.0 / 24.7
     return M > 32 && plan_swap_w8a16(M, K, N, -1).splits == 1;
+}
+// null: another kernel's
+const W8a16PairPlan* w8a16_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
+    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (two channels per store)
+    const W8a16Route& r = route_of<W8a16Route>(M, K, N, 0, [&] {
+        W8a16Route n;
+        n.pair = w8a16_pair_wanted(M, K, N);
+        if (n.pair) n.plan = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
+        return n;
+    });
+    return r.pair ? &r.plan : nullptr;
 }
 
 // Large-M W8A16: channel chunks of the weights are widened to f16 into scratch (small enough to stay
@@ -211,6 +255,89 @@ bool swap_eligible(int64_t M, int64_t K, int64_t N) {
 bool swap_prequant(int64_t M) {
     const int min_m = g_tune.swap_preq_min_m >= 0 ? g_tune.swap_preq_min_m : 17;
     return M >= min_m;
+}
+
+// Modelled microseconds of the kernels with 128- and 256-row tiles, to weigh them against plan_w8a8_pair's: rounds of tiles
+// times K blocks, a cluster's hand-over or a last round cut in two where the plan has them; large calls of the CTA-pair GEMM
+// are bound by power (0.385 us per pair tile and K block).  Fitted to the same row counts and shapes as that plan.
+double umma_cost(const UmmaPlan& pl, int64_t K, int64_t N) {
+    static const int max_clusters[9] = {148, 148, 74, 45, 33, 26, 22, 15, 15};
+    const double kblocks = (double)pack_kblocks(K), block = pl.bn == 256 ? 0.45 : (pl.bn == 128 ? 0.254 : 0.185);
+    const int64_t tiles = (int64_t)pl.m_tiles * pl.n_tiles, sms = sm_count();
+    if (pl.splits > 1) {
+        const int64_t waves = (tiles + max_clusters[pl.splits] - 1) / max_clusters[pl.splits];
+        return (double)waves * (pl.kblocks_per_split * block + 1.17) + 1.81 * pl.bn / 128 + 3.14;
+    }
+    const double hbm = (double)K * (double)N / 5.5e6;                           // the weights, for few rows
+    if (pl.narrow_tiles) return (double)(tiles / sms) * (kblocks * block + 0.49) + kblocks * block * 0.434 + 3.14;
+    const double whole = (double)((tiles + sms - 1) / sms) * (kblocks * block + 0.49) + 3.14;
+    return whole > hbm ? whole : hbm;
+}
+double umma_pair_cost(int64_t M, int64_t K, int64_t N) {
+    const int64_t pairs = sm_count() / 2, tiles = ((M + 255) / 256) * ((N + 255) / 256);
+    const double kblocks = (double)pack_kblocks(K), load = (double)(tiles < pairs ? tiles : pairs) / (double)pairs;
+    const double chain = (double)((tiles + pairs - 1) / pairs) * (kblocks * 0.267 * (1.0 + 0.215 * load) + 0.06);
+    const double power = (double)tiles * kblocks / (double)pairs * 0.385;
+    return (chain > power ? chain : power) + 5.53;
+}
+
+// Knobs that select one of the other W8A8 routes.
+bool other_w8a8_route_forced() {
+    return g_tune.umma_pair >= 0 || g_tune.umma_bn > 0 || g_tune.umma_splits > 0 || g_tune.fuse_quant > 0 || g_tune.swap_min_m >= 0 ||
+           g_tune.swap_enable >= 0 || g_tune.swap_splits > 0 || g_tune.swap_preq_min_m >= 0 || g_tune.stream_max_m >= 0 || g_tune.mlp_decode_fused > 0;
+}
+
+// W8A8 on CTA pairs with the rows as the MMA's N (umma_w8a8_pair.cu), K in as many slices as the sums of the other kernels
+// have (see plan_swap); where the one-CTA GEMM would cut only its last tiles (its tail launch), the call stays there.
+//   17 to 64 rows: where the one-CTA decode kernel does not split K (a pair's CTAs then stage half of the rows each: 64 rows
+//     on 2048 -> 11008 6.7 us against 7.8, 3584 -> 37888 23.1 / 24.2), and where the pairs are modelled faster (64 rows on
+//     2048 -> 2048 4.5 / 4.8, 3584 -> 3584 6.2 / 6.8; not 18944 -> 3584 14.9 / 14.8, 8192 -> 1024 6.6 / 5.6).
+//   65 to 4096 rows: where modelled faster than both kernels with fixed tiles.  Over twelve layer shapes (1280 -> 1536 ..
+//     18944 -> 3584, 3584 -> 37888) and nineteen row counts the choice is 0.4 % slower than the best of the three; it is this
+//     kernel for most counts below 1500, e.g. (us, this / the other two) 256 rows on 3584 -> 3584 8.3 / 10.0, 700 on 18944 ->
+//     3584 40 / 51, 1031 on 3584 -> 37888 102 / 111, 3584 -> 4608 16.7 / 20.1; not 512 on 2560 -> 9472 13.9 / 12.6, 2048 on 3584
+//     -> 4608 25.6 / 24.5.  Above 4096 rows the 256-row tiles are as good as full and store whole lines.
+const W8a8PairPlan* w8a8_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
+    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (two channels per store)
+    if (g_tune.w8a8_pair < 0 && (M < 17 || M > 4096 || other_w8a8_route_forced())) return nullptr;
+    const W8a8Route& r = route_of<W8a8Route>(M, K, N, 0, [&] {
+        W8a8Route n;
+        if (g_tune.w8a8_pair == 0) return n;
+        int slices = g_tune.w8a8_pair_slices;
+        double other = 1e29;
+        if (M <= 64) {
+            const SwapPlan sp = plan_swap(M, K, N, -1, true);
+            if (slices < 1) slices = sp.splits;
+            other = sp.splits == 1 ? 1e29 : sp.cost;
+        } else if (pair_rounds_full(M, N)) {
+            if (slices < 1) slices = 1;
+            other = umma_pair_cost(M, K, N);
+        } else {
+            const UmmaPlan pl = plan_umma(M, K, N, 0, 0);
+            if (slices < 1) slices = pl.tail_tiles ? 0 : pl.splits;
+            if (slices > 0) other = umma_cost(pl, K, N);
+            if (pl.splits == 1 && other > umma_pair_cost(M, K, N)) other = umma_pair_cost(M, K, N);
+        }
+        n.plan = plan_w8a8_pair(M, K, N, false, slices, g_tune.w8a8_pair_tokens, g_tune.w8a8_pair_splits);
+        n.pair = n.plan.cost < (g_tune.w8a8_pair > 0 ? 1e30 : other);
+        return n;
+    });
+    return r.pair ? &r.plan : nullptr;
+}
+// The same kernel for gate_up of the fused MLP, with the activation in its epilogue.  Up to 64 rows the alternative is the
+// decode kernel and a pass over its bf16 result, whose launch it saves: wherever that kernel would not split K.
+const W8a8PairPlan* mlp_pair_route(int64_t M, int64_t H, int64_t I) {
+    if (M < 17) return nullptr;
+    if (g_tune.w8a8_pair < 0 && (M > 4096 || other_w8a8_route_forced())) return nullptr;
+    const W8a8Route& r = route_of<W8a8Route>(M, H, 2 * I, 1, [&] {
+        W8a8Route n;
+        if (g_tune.w8a8_pair == 0) return n;
+        const SwapPlan sp = M <= 64 ? plan_swap(M, H, 2 * I, -1, true) : SwapPlan{};
+        n.plan = plan_w8a8_pair(M, H, 2 * I, true, M <= 64 ? sp.splits : 1, g_tune.w8a8_pair_tokens, 1);
+        n.pair = n.plan.cost < (g_tune.w8a8_pair > 0 ? 1e30 : M <= 64 ? (sp.splits == 1 ? 1e29 : sp.cost + 2.0) : umma_pair_cost(M, H, 2 * I));
+        return n;
+    });
+    return r.pair ? &r.plan : nullptr;
 }
 
 // Large-M W8A8 with the activation quantiser inside the GEMM: a short pass quantises the rows that the first
@@ -361,14 +488,14 @@ int fp8lin_w8a16(const void* x, int64_t ldx, const void* w_nk, const float* w_sc
                  void* stream) {
     int rc = validate_common(x, ldx, w_nk, w_scale, bias, y, ldy, M, K, N);
     if (rc != FP8LIN_OK || M == 0) return rc;
-    if (workspace && workspace_bytes >= FP8LIN_WS_HEADER_BYTES && w8a16_pair_eligible(M, K, N, ldy, y)) {
-        const W8a16PairPlan pl = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
+    const W8a16PairPlan* pair = workspace && workspace_bytes >= FP8LIN_WS_HEADER_BYTES ? w8a16_pair_route(M, K, N, ldy, y) : nullptr;
+    if (pair) {
         UmmaArgs a;
         a.xq = nullptr; a.w = (const unsigned char*)w_nk; a.w_scale = w_scale; a.input_scale = nullptr;
         a.bias = (const __nv_bfloat16*)bias; a.y = (__nv_bfloat16*)y; a.partial = nullptr; a.counters = nullptr;
         a.status = ws_view(workspace, workspace_bytes).status; a.M = (int)M; a.K = (int)K; a.N = (int)N; a.ldy = (int)ldy;
         const char* why = nullptr;
-        cudaError_t e = launch_w8a16_pair(pl, a, x, ldx, (cudaStream_t)stream, &why);
+        cudaError_t e = launch_w8a16_pair(*pair, a, x, ldx, (cudaStream_t)stream, &why);
         if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "tcgen05 W8A16 pair kernel launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
         return FP8LIN_OK;
     }
@@ -419,6 +546,35 @@ int fp8lin_w8a16(const void* x, int64_t ldx, const void* w_nk, const float* w_sc
                       workspace_bytes, (cudaStream_t)stream);
 }
 
+namespace {
+
+// W8A8 linear whose activations are already e4m3 (row pitch K).
+int run_w8a8_prequantised(const unsigned char* xq, const void* w, const float* w_scale, const float* input_scale,
+                          const void* bias, void* y, int64_t ldy, int64_t M, int64_t K, int64_t N, const WsView& ws,
+                          cudaStream_t st) {
+    UmmaArgs a;
+    a.xq = xq; a.w = (const unsigned char*)w; a.w_scale = w_scale; a.input_scale = input_scale;
+    a.bias = (const __nv_bfloat16*)bias; a.y = (__nv_bfloat16*)y; a.partial = nullptr; a.counters = ws.counters;
+    a.status = ws.status; a.M = (int)M; a.K = (int)K; a.N = (int)N; a.ldy = (int)ldy;
+    const char* why = nullptr;
+    cudaError_t e;
+    if (const W8a8PairPlan* pair = w8a8_pair_route(M, K, N, ldy, y)) {
+        e = launch_w8a8_pair(*pair, a, st, &why);
+    } else if (M <= 64) {
+        SwapPlan sp = plan_swap(M, K, N, g_tune.swap_splits, true);
+        e = launch_swap_w8a8(sp, a, nullptr, 0, st, &why);
+    } else if (pair_eligible(M, K, N)) {
+        e = launch_umma_pair(false, a, st, &why);
+    } else {
+        UmmaPlan pl = plan_umma(M, K, N, g_tune.umma_bn, g_tune.umma_splits);
+        e = launch_umma_w8a8(pl, a, st, &why);
+    }
+    if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "W8A8 linear launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
+    return FP8LIN_OK;
+}
+
+}  // namespace
+
 int fp8lin_w8a8(const void* x, int64_t ldx, const void* w_nk, const float* w_scale, const float* input_scale,
                 const void* bias, void* y, int64_t ldy, int64_t M, int64_t K, int64_t N, void* workspace,
                 size_t workspace_bytes, void* stream) {
@@ -426,6 +582,14 @@ int fp8lin_w8a8(const void* x, int64_t ldx, const void* w_nk, const float* w_sca
     if (rc != FP8LIN_OK || M == 0) return rc;
     if (!input_scale) return fail(FP8LIN_ERR_NULL, "input_scale must not be NULL");
     cudaStream_t st = (cudaStream_t)stream;
+    if (w8a8_pair_route(M, K, N, ldy, y)) {
+        WsView wsv = ws_view(workspace, workspace_bytes);
+        if (!workspace || wsv.body_bytes < align_up((size_t)M * K, 256))
+            return fail(FP8LIN_ERR_WORKSPACE, "workspace too small: need %zu bytes", FP8LIN_WS_HEADER_BYTES + align_up((size_t)M * K, 256));
+        cudaError_t qe = launch_act_quant((const __nv_bfloat16*)x, ldx, input_scale, wsv.body, M, K, st);
+        if (qe != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "activation quantiser launch: %s", cudaGetErrorString(qe));
+        return run_w8a8_prequantised(wsv.body, w_nk, w_scale, input_scale, bias, y, ldy, M, K, N, wsv, st);
+    }
     if (swap_eligible(M, K, N)) {
         const bool preq = swap_prequant(M);
         SwapPlan sp = plan_swap(M, K, N, g_tune.swap_splits, preq);
@@ -547,29 +711,6 @@ MlpLayout mlp_layout(int64_t M, int64_t H, int64_t I) {
     return l;
 }
 
-// W8A8 linear whose activations are already e4m3 (row pitch K): the second half of the fused MLP.
-int run_w8a8_prequantised(const unsigned char* xq, const void* w, const float* w_scale, const float* input_scale,
-                          const void* bias, void* y, int64_t ldy, int64_t M, int64_t K, int64_t N, const WsView& ws,
-                          cudaStream_t st) {
-    UmmaArgs a;
-    a.xq = xq; a.w = (const unsigned char*)w; a.w_scale = w_scale; a.input_scale = input_scale;
-    a.bias = (const __nv_bfloat16*)bias; a.y = (__nv_bfloat16*)y; a.partial = nullptr; a.counters = ws.counters;
-    a.status = ws.status; a.M = (int)M; a.K = (int)K; a.N = (int)N; a.ldy = (int)ldy;
-    const char* why = nullptr;
-    cudaError_t e;
-    if (M <= 64) {
-        SwapPlan sp = plan_swap(M, K, N, g_tune.swap_splits, true);
-        e = launch_swap_w8a8(sp, a, nullptr, 0, st, &why);
-    } else if (pair_eligible(M, K, N)) {
-        e = launch_umma_pair(false, a, st, &why);
-    } else {
-        UmmaPlan pl = plan_umma(M, K, N, g_tune.umma_bn, g_tune.umma_splits);
-        e = launch_umma_w8a8(pl, a, st, &why);
-    }
-    if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "down projection launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
-    return FP8LIN_OK;
-}
-
 }  // namespace
 
 size_t fp8lin_mlp_workspace_bytes(int64_t M, int64_t H, int64_t I, int64_t N) {
@@ -610,6 +751,19 @@ static int mlp_w8a8_impl(const void* x, int64_t ldx, bool x_is_e4m3, const void*
         const char* why = nullptr;
         cudaError_t e = launch_swap_gate_up(a, st, &why);
         if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "decode gate_up launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
+    } else if (const W8a8PairPlan* pair = mlp_pair_route(M, H, I)) {
+        UmmaArgs a;
+        a.xq = x_is_e4m3 ? (const unsigned char*)x : ws.body; a.w = (const unsigned char*)w_gate_up; a.w_scale = gate_up_scale;
+        a.input_scale = gate_up_input_scale; a.bias = (const __nv_bfloat16*)gate_up_bias; a.y = nullptr; a.partial = nullptr;
+        a.counters = nullptr; a.status = ws.status; a.M = (int)M; a.K = (int)H; a.N = (int)(2 * I); a.ldy = 0;
+        a.hq = hq; a.h_scale = down_input_scale;
+        if (!x_is_e4m3) {
+            cudaError_t qe = launch_act_quant((const __nv_bfloat16*)x, ldx, gate_up_input_scale, ws.body, M, H, st);
+            if (qe != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "activation quantiser launch: %s", cudaGetErrorString(qe));
+        }
+        const char* why = nullptr;
+        cudaError_t e = launch_w8a8_pair(*pair, a, st, &why);
+        if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "fused gate_up launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
     } else if (M <= kDefaultStreamMaxM) {
         // small batches: gate_up through the decode kernels into a bf16 buffer, one pass for silu * up + quantise
         __nv_bfloat16* gu = (__nv_bfloat16*)(ws.body + l.gu_off);
@@ -798,10 +952,12 @@ const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N) {
 
 const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N) {
     static thread_local char buf[64];
-    if (M > 0 && K > 0 && N > 0 && scheme == FP8LIN_W8A16 && w8a16_pair_eligible(M, K, N, 8, nullptr)) {
-        const W8a16PairPlan pl = plan_w8a16_pair(M, K, N, g_tune.w8a16_pair_tokens, g_tune.w8a16_pair_splits);
-        snprintf(buf, sizeof(buf), "umma_w8a16_pair_256x%d_s%d", pl.tokens, pl.splits);
-        return buf;
+    if (M > 0 && K > 0 && N > 0) {
+        const W8a16PairPlan* p16 = scheme == FP8LIN_W8A16 ? w8a16_pair_route(M, K, N, 8, nullptr) : nullptr;
+        const W8a8PairPlan* p8 = scheme == FP8LIN_W8A8_STATIC ? w8a8_pair_route(M, K, N, 8, nullptr) : nullptr;
+        if (p16) snprintf(buf, sizeof(buf), "umma_w8a16_pair_256x%d_s%d", p16->tokens, p16->splits);
+        else if (p8) snprintf(buf, sizeof(buf), "umma_w8a8_pair_256x%d_s%d%s", p8->tokens, p8->slices, p8->splits > 1 ? "_cluster" : "");
+        if (p16 || p8) return buf;
     }
     const int max_m = g_tune.stream_max_m >= 0 ? g_tune.stream_max_m : kDefaultStreamMaxM;
     if (M > max_m && K > 0 && N > 0 && N % 8 == 0 && scheme == FP8LIN_W8A8_STATIC)
@@ -811,6 +967,7 @@ const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N) {
 
 int fp8lin_set_tuning(const char* knob, int value) {
     if (!knob) return fail(FP8LIN_ERR_NULL, "knob is NULL");
+    ++g_tune_version;
     if (!strcmp(knob, "stream_splits")) g_tune.stream_splits = value;
     else if (!strcmp(knob, "stream_max_m")) g_tune.stream_max_m = value;
     else if (!strcmp(knob, "umma_bn")) g_tune.umma_bn = value;
@@ -825,6 +982,10 @@ int fp8lin_set_tuning(const char* knob, int value) {
     else if (!strcmp(knob, "w8a16_chunk_mb")) g_tune.w8a16_chunk_mb = value;
     else if (!strcmp(knob, "w8a16_pair")) g_tune.w8a16_pair = value;
     else if (!strcmp(knob, "w8a16_pair_tokens")) g_tune.w8a16_pair_tokens = value;
+    else if (!strcmp(knob, "w8a8_pair")) g_tune.w8a8_pair = value;
+    else if (!strcmp(knob, "w8a8_pair_tokens")) g_tune.w8a8_pair_tokens = value;
+    else if (!strcmp(knob, "w8a8_pair_slices")) g_tune.w8a8_pair_slices = value;
+    else if (!strcmp(knob, "w8a8_pair_splits")) g_tune.w8a8_pair_splits = value;
     else if (!strcmp(knob, "w8a16_pair_splits")) g_tune.w8a16_pair_splits = value;
     else if (!strcmp(knob, "umma_pair")) g_tune.umma_pair = value;
     else if (!strcmp(knob, "fuse_quant")) g_tune.fuse_quant = value;

@@ -166,6 +166,7 @@ struct SwapPlan {
     int splits;        // cluster split-K factor (1 = persistent over tiles)
     int kblocks_per_split;
     int grid;
+    double cost = 0;           // modelled microseconds (plan_swap)
     int preq;          // 1 = activations pre-quantised by act_quant (a.xq), 0 = quantised in the kernel from x
 };
 
@@ -228,6 +229,19 @@ struct W8a16PairPlan {
 W8a16PairPlan plan_w8a16_pair(int64_t M, int64_t K, int64_t N, int force_tokens, int force_splits);
 cudaError_t launch_w8a16_pair(const W8a16PairPlan& plan, const UmmaArgs& a, const void* x, int64_t ldx, cudaStream_t stream,
                               const char** why);
+
+// ---- W8A8 on CTA pairs, weights as the MMA's M, rows as its N (umma_w8a8_pair.cu) ----
+struct W8a8PairPlan {
+    int n_tiles, m_tiles;      // 256-channel tiles, token tiles
+    int tokens, last_tokens;   // tokens per tile, and of the last tile: 32..256, multiples of 32
+    int slices;                // K slices that a sum is made of (accumulated apart, added in order)
+    int splits;                // 1: persistent pairs, all slices each; else = slices: clusters of 2 * slices CTAs
+    int grid;
+    double cost;               // modelled microseconds; 1e30 = no plan
+};
+// mlp: gate_up of the fused MLP (args.hq set: e4m3 h is written instead of y).  args.xq holds all rows.
+W8a8PairPlan plan_w8a8_pair(int64_t M, int64_t K, int64_t N, bool mlp, int slices, int force_tokens, int force_splits);
+cudaError_t launch_w8a8_pair(const W8a8PairPlan& plan, const UmmaArgs& args, cudaStream_t stream, const char** why);
 
 // ---- swapped-operand tcgen05 kernel for W8A16, 9 <= M <= 64 (umma_swap_w8a16.cu) ----
 SwapPlan plan_swap_w8a16(int64_t M, int64_t K, int64_t N, int force_splits);

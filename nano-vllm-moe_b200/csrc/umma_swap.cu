@@ -560,6 +560,16 @@ SwapPlan plan_swap(int64_t M, int64_t K, int64_t N, int force_splits, bool preq)
             if (kps >= 16 && (kblocks + kps - 1) / kps == s) { best_s = s; break; }
         }
     }
+    // what a call takes, microseconds: fitted like plan_w8a8_pair, against which it is weighed
+    {
+        static const int max_clusters[9] = {148, 148, 74, 45, 33, 26, 22, 15, 15};
+        const int kps = (kblocks + best_s - 1) / best_s, slots = max_clusters[best_s] * (pl.mp == 16 ? 2 : 1);
+        const int ctas = pl.n_tiles * best_s, resident = ctas < slots * best_s ? ctas : slots * best_s, waves = (pl.n_tiles + slots - 1) / slots;
+        const double alone = pl.mp == 16 ? 0.261 : (pl.mp == 32 ? 0.179 : 0.184), shared = 16384.0 * resident / 5.33e6;
+        const double t_block = shared > alone ? shared : alone;
+        pl.cost = 1.44 + 0.029 * (double)M + waves * kps * t_block +
+                  (best_s > 1 ? waves * (0.63 + (0.023 + 0.0016 * (double)M) * best_s) + (waves - 1) * 1.44 : 0.0);
+    }
     pl.splits = best_s;
     pl.kblocks_per_split = (kblocks + best_s - 1) / best_s;
     const int resident = sm_count() * (pl.mp == 16 ? 2 : 1);

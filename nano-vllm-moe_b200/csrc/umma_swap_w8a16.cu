@@ -421,15 +421,16 @@ SwapPlan plan_swap_w8a16(int64_t M, int64_t K, int64_t N, int force_splits) {
         int slots = sm_count();
         if (s > 1) slots = pl.mp == 16 ? swap16_max_clusters<16>(s) : (pl.mp == 32 ? swap16_max_clusters<32>(s) : swap16_max_clusters<64>(s));
         if (slots < 1) slots = 1;
-        // microseconds, the model of plan_swap with this kernel's constants (fitted to the same shapes, 0.2 % from the best
-        // on average): a lone CTA is bound by the chain of its converters, which grows with the rows they also convert
+        // microseconds, the model of plan_swap with this kernel's constants (fitted to twelve layer shapes with
+        // the hand-over in whole lines, 0.1 % from the best on average): a lone CTA is bound by the chain of its converters, which grows with the rows they also convert
         const int ctas = pl.n_tiles * s;
         const int resident = ctas < slots * s ? ctas : slots * s;
-        const double alone = pl.mp == 16 ? 0.236 : (pl.mp == 32 ? 0.348 : 0.564);
-        const double shared = 16384.0 * resident / 5.46e6;
+        const double alone = pl.mp == 16 ? 0.239 : (pl.mp == 32 ? 0.261 : 0.477);
+        const double shared = 16384.0 * resident / 5.8e6;
         const double t_block = shared > alone ? shared : alone;
         const int waves = (pl.n_tiles + slots - 1) / slots;
-        const double cost = s > 1 ? waves * (kps * t_block + 2.6 + 0.5 + (0.034 + 0.0072 * (double)M) * s) : waves * kps * t_block + 2.6;
+        const double cost = s > 1 ? waves * (kps * t_block + 2.0 + 0.98 + (0.123 + 0.0024 * (double)M) * s)
+                                  : waves * kps * t_block + 2.0 + 0.76 * resident / sm_count();
         if (cost < best_cost) { best_cost = cost; best_s = s; }
     }
     pl.splits = best_s;

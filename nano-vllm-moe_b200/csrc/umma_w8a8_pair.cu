@@ -1,0 +1,509 @@
+// W8A8 linear on CTA pairs (tcgen05 cta_group::2), operands swapped, for batches between decode and prefill and for row
+// counts that do not fill 256-row tiles:
+//
+//   y^T[N, M] = W_e4m3[N, K] . xq_e4m3[M, K]^T          fp32 accumulation in TMEM
+//
+// A pair of CTAs computes 256 output channels x T tokens.  CTA r of the pair owns channels [128 r, 128 r + 128) of the tile
+// (the weight tile is its half of the MMA's "A" operand) and stages T/2 of the rows of xq as its half of "B".  The rows are
+// the MMA's N, so a tile takes any multiple of 32 of them up to 256, and the last tile of the batch may be smaller than the
+// others: 1031 rows are 4 x 256 + 32 of them instead of 5 x 256.
+//
+//   warp 0        TMA producer: 16 KB of weights and T/2 x 128 bytes of xq per slot; the weights of the first ring pass go
+//                 out before the wait for the kernel that writes xq
+//   warp 1        MMA issuer (leader CTA): four tcgen05.mma.cta_group::2.kind::f8f6f4 (256 x T x 32) per K block
+//   warps 2..9    epilogue: lane = channel, y[m][n] = bf16(acc * in_scale * w_scale[n] + bias[n]); two lanes swap halves so
+//                 that a lane stores two channels of one token
+//
+// kMlp (gate_up of the fused MLP, gate and up channels in alternating tiles of 128): a CTA stages 64 gate channels and the
+// 64 up channels of the same indices, and the epilogue writes e4m3 h = bf16(silu(g) * u) / h_scale; the warps of the gate
+// lanes and of the up lanes swap half of their values and finish half of the rows each.
+//
+// The caller says into how many slices the K blocks of a sum are cut: a slice is accumulated by itself and the slices are
+// added in order, which makes the result the same bits as that of the kernel that would otherwise take the call (the decode
+// kernels up to 64 rows, the one-CTA GEMM above).  Two ways:
+//   one pair works through all slices, each into its own T columns of tensor memory, and the epilogue adds them
+//   kSplit (few tiles, long K): the 2 s CTAs of a cluster take one slice each of the same tile
+//   and push the partial sums of band r to the r-th pair's CTA of the same channels (st.async counted on its mbarrier)
+// All waits are bounded.
+#include "umma_common.cuh"
+
+namespace fp8lin {
+
+namespace {
+
+constexpr int kEpiWarps = 8;
+constexpr int kThreads = (2 + kEpiWarps) * 32;
+constexpr int kTile = 128;                     // channels per CTA
+constexpr int kKB = 128;                       // K elements per block
+constexpr int kWBytes = kTile * kKB;
+constexpr int kMaxSlots = 12;
+constexpr int kMaxT = 256;                     // columns of an accumulator stage
+constexpr int kTmemCols = 512;
+constexpr int kRingBytes = 210 * 1024;         // 16 KB + 64 T bytes per slot
+constexpr int kSwapBytes = 32 * 64;            // kMlp: bf16 values of 32 rows x 32 channels, one buffer per warp pair
+constexpr int kCodeBytes = 32 * 32;            // ... and their e4m3 results
+template <bool kMlp> constexpr int kSmemBytes = kRingBytes + (kMlp ? 4 * (kSwapBytes + kCodeBytes) : 0) + 1024;
+static_assert((kTile + 4) * kMaxT * 4 <= kRingBytes, "the received slices of a band must fit in the ring");
+
+struct PairSched8 {
+    int n_tiles;              // 256-channel tiles
+    int m_tiles;              // token tiles
+    int tokens, last_tokens;  // T of all token tiles but the last, and of the last
+    int slices;               // K slices of a sum
+    int splits;               // kSplit: = slices (cluster of 2 * slices CTAs); else 1: persistent over all tiles
+    int kblocks, kblocks_per_slice;
+};
+
+// weights (boxes of 128 rows, kMlp 64) and xq (boxes of half a full and half a last token tile)
+struct PairMaps8 {
+    CUtensorMap w, x, x_last;
+};
+
+struct Item {
+    int nt;                   // channel tile
+    int m0, half;             // first token, half of its tokens
+    bool last;
+};
+// Token tiles of a channel tile follow each other, so that its weights come from L2 after the first; every other channel tile
+// walks them backwards, or with an even number of token tiles the same pairs would always get the last, smaller ones.
+__device__ __forceinline__ Item decode_item(const PairSched8& s, int item) {
+    Item r;
+    r.nt = item / s.m_tiles;
+    int mi = item - r.nt * s.m_tiles;
+    if (r.nt & 1) mi = s.m_tiles - 1 - mi;
+    r.last = mi == s.m_tiles - 1;
+    r.m0 = mi * s.tokens;
+    r.half = (r.last ? s.last_tokens : s.tokens) >> 1;
+    return r;
+}
+
+// A sum times in_scale, then times the channel's scale: in two roundings up to 64 rows, as the decode kernels do it, in one
+// product of the scales above, as the 256-row kernels do.  The bf16 results of a row count are the same bits whichever kernel
+// takes it.  Returns the factor of the channel's scale; `pre` multiplies the sum.
+__device__ __forceinline__ float channel_factor(const UmmaArgs& p, float& pre) {
+    const float in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
+    pre = p.M <= 64 ? in_scale : 1.f;
+    return p.M <= 64 ? 1.f : in_scale;
+}
+
+template <bool kSplit, bool kMlp>
+__global__ void __launch_bounds__(kThreads, 1)
+w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 sched) {
+    static_assert(!(kSplit && kMlp), "the activation epilogue takes whole sums");
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[kMaxSlots];      // leader's: both CTAs' weights and rows landed
+    __shared__ __align__(8) uint64_t bar_empty[kMaxSlots];     // the MMAs that read the slot are done (both CTAs')
+    __shared__ __align__(8) uint64_t bar_tfull[2];
+    __shared__ __align__(8) uint64_t bar_tempty[2];            // leader's
+    __shared__ __align__(8) uint64_t bar_ready;                // split-K: every CTA of these channels is past its MMAs
+    __shared__ __align__(8) uint64_t bar_recv;                 // split-K: the partials of this CTA's band have landed
+    __shared__ uint32_t s_tmem_base;
+    __shared__ volatile int s_abort;
+
+    const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const int warp = warp_index();
+    const int lane = threadIdx.x & 31;
+    const uint32_t crank = cluster_ctarank();
+    const uint32_t rank = crank & 1;                   // inside the pair
+    const bool leader = rank == 0;
+    const uint32_t leader_cta = crank & ~1u;
+    const int slice_rank = kSplit ? (int)(crank >> 1) : 0;
+    const int items = sched.n_tiles * sched.m_tiles;
+    const int first_item = kSplit ? (int)(blockIdx.x / (2 * sched.splits)) : (int)(blockIdx.x >> 1);
+    const int item_step = kSplit ? items : (int)(gridDim.x >> 1);
+    const int kb0 = slice_rank * sched.kblocks_per_slice;
+    const int kb1 = kSplit ? min(sched.kblocks, kb0 + sched.kblocks_per_slice) : sched.kblocks;
+    // accumulators: `slices` times T columns per tile, two tiles where they fit
+    const int n_acc = kSplit ? 1 : sched.slices;
+    const int acc_cols = n_acc * sched.tokens;
+    const int acc_stages = 2 * acc_cols <= kTmemCols ? 2 : 1;
+    const uint32_t slot_bytes = kWBytes + (uint32_t)sched.tokens * 64u;
+    const int n_slots = min(kMaxSlots, (int)(kRingBytes / slot_bytes));
+    // split-K: band r of this CTA's 128 channels is finished by slice r's CTA of the same pair rank
+    const int band = kSplit ? (kTile + sched.splits - 1) / sched.splits : kTile;
+    const int band_rows = kSplit ? max(0, min(kTile, (slice_rank + 1) * band) - slice_rank * band) : 0;
+    const Item it0 = decode_item(sched, first_item);
+    const int m_valid = kSplit ? min(2 * it0.half, p.M - it0.m0) : 0;
+    const int m_groups = (m_valid + 3) >> 2;
+    // received sums: [slice][group of four tokens][channel of the band], 16 bytes each, so that the 32 lanes (channels) of a
+    // warp send 512 contiguous bytes per instruction
+    const uint32_t group_bytes = (uint32_t)band * 16u;
+    const uint32_t slice_bytes = group_bytes * (uint32_t)(sched.tokens >> 2);
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kMaxSlots; ++i) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_empty[i]), 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bar_tfull[i]), 1); mbar_init(smem_u32(&bar_tempty[i]), 2 * kEpiWarps); }
+        s_abort = 0;
+        if (kSplit) {
+            mbar_init(smem_u32(&bar_ready), (uint32_t)sched.splits);
+            mbar_init(smem_u32(&bar_recv), 1);
+            mbar_expect_tx(smem_u32(&bar_recv), (uint32_t)(sched.splits * band_rows * m_groups * 16));
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) tmem_alloc_pair(smem_u32(&s_tmem_base), kTmemCols);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();            // the other CTAs' barriers exist before anything is signalled on them
+    tc_fence_after();
+    const uint32_t tmem_base = s_tmem_base;
+    pdl_launch_dependents();
+
+    if (warp == 0) {
+        // ================= TMA producer (both CTAs) =================
+        const uint32_t el = elect_one();
+        auto load_weights = [&](const Item& it, int kb, int slot) {
+            const uint32_t full_local = smem_u32(&bar_full[slot]);
+            mbar_expect_tx(leader ? el : 0u, full_local, 2u * (kWBytes + (uint32_t)it.half * kKB));
+            const uint32_t full = map_to_cta(full_local, leader_cta);
+            const uint32_t ws = smem_base + slot * slot_bytes;
+            if (kMlp) {
+                const int row = (2 * it.nt * sched.kblocks + kb) * kTile + (int)rank * 64;
+                tma_load_2d_pair(el, ws, &maps.w, 0, row, full);
+                tma_load_2d_pair(el, ws + kWBytes / 2, &maps.w, 0, row + sched.kblocks * kTile, full);
+            } else {
+                tma_load_2d_pair(el, ws, &maps.w, 0, ((2 * it.nt + (int)rank) * sched.kblocks + kb) * kTile, full);
+            }
+        };
+        auto load_rows = [&](const Item& it, int kb, int slot) {
+            const uint32_t full = map_to_cta(smem_u32(&bar_full[slot]), leader_cta);
+            tma_load_2d_pair(el, smem_base + slot * slot_bytes + kWBytes, it.last ? &maps.x_last : &maps.x, kb * kKB, it.m0 + (int)rank * it.half, full);
+        };
+        const int pre = min(kb1 - kb0, n_slots);
+        for (int i = 0; i < pre; ++i) load_weights(it0, kb0 + i, i);
+        pdl_wait();
+        for (int i = 0; i < pre; ++i) load_rows(it0, kb0 + i, i);
+        int slot = pre == n_slots ? 0 : pre;
+        uint32_t phase = pre == n_slots ? 0 : 1;           // parity that a free slot shows (1 on its first use)
+        bool ok = true;
+        for (int item = first_item; item < items && ok; item += item_step) {
+            const Item it = decode_item(sched, item);
+            for (int kb = item == first_item ? kb0 + pre : kb0; kb < kb1; ++kb) {
+                ok = !s_abort && warp_wait(smem_u32(&bar_empty[slot]), phase, p.status, kDevTimeoutEmpty);
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; s_abort = 1; break; }
+                load_weights(it, kb, slot);
+                load_rows(it, kb, slot);
+                if (++slot == n_slots) { slot = 0; phase ^= 1; }
+            }
+        }
+        if (!ok) {
+            const long long t0 = clock64();                // let copies that are still in flight land
+            while (clock64() - t0 < 2000000) {}
+        }
+    } else if (warp == 1) {
+        // ================= MMA issuer (leader CTA only) =================
+        if (leader) {
+            const uint32_t el = elect_one();
+            const uint16_t both = (uint16_t)(3u << crank);                      // this CTA and its partner
+            int tl = 0, slot = 0;
+            uint32_t phase = 0;
+            bool ok = true;
+            for (int item = first_item; item < items && ok; item += item_step, ++tl) {
+                const Item it = decode_item(sched, item);
+                const uint32_t idesc = make_idesc_mn(2 * kTile, 2 * it.half, 0, 0);          // e4m3 x e4m3
+                const int as = acc_stages == 2 ? (tl & 1) : 0;
+                const uint32_t aph = acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1);
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                if (!ok) { s_abort = 1; break; }
+                tc_fence_after();
+                uint32_t d_tmem = tmem_base + as * acc_cols;
+                int left = sched.kblocks_per_slice;           // K blocks until the next slice's accumulator
+                bool fresh = true;
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_full[slot]), phase, p.status, kDevTimeoutFull));
+                    if (!ok) { s_abort = 1; break; }
+                    tc_fence_after();
+                    const uint64_t da = make_smem_desc(smem_base + slot * slot_bytes);
+                    const uint64_t db = make_smem_desc(smem_base + slot * slot_bytes + kWBytes);
+#pragma unroll
+                    for (int k = 0; k < kKB / 32; ++k)
+                        umma_f8_pair(el, d_tmem, da + 2 * k, db + 2 * k, idesc, (!fresh || k > 0) ? 1u : 0u);
+                    umma_commit_both(el, smem_u32(&bar_empty[slot]), both);
+                    fresh = false;
+                    if (--left == 0) { left = sched.kblocks_per_slice; d_tmem += sched.tokens; fresh = true; }
+                    if (++slot == n_slots) { slot = 0; phase ^= 1; }
+                }
+                if (ok) umma_commit_both(el, smem_u32(&bar_tfull[as]), both);
+            }
+        }
+    } else {
+        // ================= epilogue (warps 2..9 of both CTAs) =================
+        pdl_wait();                                        // the output may still be in use by the predecessor
+        const int q = warp & 3;                            // TMEM lane quarter
+        const int h = (warp - 2) >> 2;                     // which half of the tile's tokens
+        float pre;
+        const float in_scale = channel_factor(p, pre);
+        const ExactDiv div_h(kMlp ? fmaxf(__ldg(p.h_scale), 1e-12f) : 1.f);
+        const bool odd = lane & 1;
+        const bool up = kMlp && q >= 2;
+        const int pair = (q & 1) + 2 * h;                  // kMlp: the warps of quarters q and q ^ 2 share 32 channels
+        const uint32_t swap_buf = smem_base + kRingBytes + pair * (kSwapBytes + kCodeBytes);
+        const uint32_t code_buf = swap_buf + kSwapBytes;
+        int tl = 0;
+        for (int item = first_item; item < items; item += item_step, ++tl) {
+            const Item it = decode_item(sched, item);
+            const int as = acc_stages == 2 ? (tl & 1) : 0;
+            // this lane's channel as the weights are laid out
+            const int n = kMlp ? it.nt * 256 + (up ? 128 : 0) + (int)rank * 64 + (q & 1) * 32 + lane : (2 * it.nt + (int)rank) * kTile + q * 32 + lane;
+            float ws = 0.f, bs = 0.f;
+            if (!kSplit && n < p.N) {
+                ws = in_scale * __ldg(p.w_scale + n);
+                if (p.bias) bs = __bfloat162float(p.bias[n]);
+            }
+            bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1), p.status, kDevTimeoutTmemFull);
+            if (kMlp) {                                    // warps that meet at barriers below leave together
+                uint32_t failed;
+                asm volatile(
+                    "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
+                    " barrier.cta.red.or.pred pout, 5, 256, pin;\n selp.u32 %0, 1, 0, pout;\n}"
+                    : "=r"(failed) : "r"(arrived ? 0u : 1u) : "memory");
+                arrived = failed == 0;
+            }
+            if (!arrived) { s_abort = 1; break; }
+            tc_fence_after();
+            const int m0 = it.m0 + h * it.half;
+            const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16) + as * acc_cols + h * it.half;
+            auto read32 = [&](int c, uint32_t* v) {        // columns [c, c + 32) or, at the end of the tile, [c, c + 16)
+                __syncwarp();
+                tmem_ld16_nowait(t_lane + c, v);
+                if (c + 16 < it.half) tmem_ld16_nowait(t_lane + c + 16, v + 16);
+                tmem_ld_wait();
+                for (int sl = 1; sl < n_acc; ++sl) {       // the other slices, in order
+                    uint32_t u[32];
+                    tmem_ld16_nowait(t_lane + sl * sched.tokens + c, u);
+                    if (c + 16 < it.half) tmem_ld16_nowait(t_lane + sl * sched.tokens + c + 16, u + 16);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+                }
+                if (!kSplit && c + 32 >= it.half) {        // all in registers: the next tile but one may have the accumulator
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[as]), leader_cta));
+                }
+            };
+            if constexpr (kMlp) {
+                const int hc = it.nt * 128 + (int)rank * 64 + (q & 1) * 32;           // first of the 32 output channels
+                const int ld = p.N >> 1;
+                for (int c = 0; c < it.half; c += 32) {
+                    uint32_t v[32];
+                    read32(c, v);
+                    const int n_cols = min(32, it.half - c);
+                    // Gate and up as the bf16 values that a separate gate_up linear stores.  The gate warp finishes columns [0, 16)
+                    // of the 32, the up warp [16, 32): each hands the other half over.  No branches inside (a last piece of 16
+                    // columns computes 16 more that are not stored), so that the eight chains of exp and divisions overlap.
+                    uint32_t own[8], other[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t lo = pack_bf16x2(fmaf(__uint_as_float(v[2 * j]) * pre, ws, bs), fmaf(__uint_as_float(v[2 * j + 1]) * pre, ws, bs));
+                        const uint32_t hi = pack_bf16x2(fmaf(__uint_as_float(v[16 + 2 * j]) * pre, ws, bs), fmaf(__uint_as_float(v[16 + 2 * j + 1]) * pre, ws, bs));
+                        own[j] = up ? hi : lo;
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(swap_buf + (up ? 0 : 1024) + j * 128 + lane * 4), "r"(up ? lo : hi) : "memory");
+                    }
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(swap_buf + (up ? 1024 : 0) + j * 128 + lane * 4) : "memory");
+                    const uint32_t code_at = code_buf + (up ? 16 * 32 : 0) + lane;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t g = up ? other[j] : own[j], u = up ? own[j] : other[j];
+                        const uint32_t hv = pack_bf16x2(silu_f32(bf16_lo(g)) * bf16_lo(u), silu_f32(bf16_hi(g)) * bf16_hi(u));
+                        const uint32_t code = cvt_e4m3x2(div_h(bf16_lo(hv)), div_h(bf16_hi(hv)));
+                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + 2 * j * 32), "r"(code & 0xffu) : "memory");
+                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + (2 * j + 1) * 32), "r"(code >> 8) : "memory");
+                    }
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+                    const int i = (up ? 32 : 0) + lane;                               // 32 bytes per row: a thread stores half a row
+                    const int m = m0 + c + (i >> 1);
+                    if ((i >> 1) < n_cols && m < p.M)
+                        *reinterpret_cast<float4*>(p.hq + (size_t)m * ld + hc + (i & 1) * 16) = ld_shared_f4(code_buf + (i >> 1) * 32 + (i & 1) * 16);
+                }
+            } else if constexpr (!kSplit) {
+                // a lane stores two channels of one token: even lanes the even tokens, odd lanes the odd ones
+                __nv_bfloat16* yp = p.y + (size_t)m0 * p.ldy + (n & ~1) + (odd ? p.ldy : 0);
+                const bool in = (n & ~1) < p.N;                // (N is even)
+                for (int c = 0; c < it.half; c += 32) {
+                    uint32_t v[32];
+                    read32(c, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) {
+                        if (j == 16 && c + 16 >= it.half) break;
+                        const float a0 = fmaf(__uint_as_float(v[j]) * pre, ws, bs), a1 = fmaf(__uint_as_float(v[j + 1]) * pre, ws, bs);
+                        const float other = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
+                        const uint32_t o = odd ? pack_bf16x2(other, a1) : pack_bf16x2(a0, other);
+                        if (in && m0 + c + j + (odd ? 1 : 0) < p.M) *reinterpret_cast<uint32_t*>(yp + (size_t)(c + j) * p.ldy) = o;
+                    }
+                }
+            } else {
+                // the pair's MMAs are done, so this CTA's ring is free: tell the CTAs that will push into it, wait for those
+                // this one pushes into, and send each channel's sums to the owner of its band
+                if (warp == 2 && lane < sched.splits)
+                    mbar_arrive_cluster(map_to_cta(smem_u32(&bar_ready), (uint32_t)(2 * lane) + rank));
+                if (!mbar_wait_cluster(smem_u32(&bar_ready), 0, p.status, kDevTimeoutPeer)) { s_abort = 1; break; }
+                const int c0 = q * 32 + lane;
+                const int owner = c0 / band;
+                const uint32_t owner_cta = (uint32_t)(2 * owner) + rank;
+                const uint32_t dst = map_to_cta(smem_base + slice_rank * slice_bytes + (uint32_t)(h * it.half >> 2) * group_bytes + (uint32_t)(c0 - owner * band) * 16u, owner_cta);
+                const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), owner_cta);
+                for (int c = 0; c < it.half; c += 32) {
+                    uint32_t v[32];
+                    read32(c, v);
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        if (j == 16 && c + 16 >= it.half) break;
+                        if (h * it.half + c + j < m_valid) st_async_v4(dst + (uint32_t)((c + j) >> 2) * group_bytes, v[j], v[j + 1], v[j + 2], v[j + 3], rbar);
+                    }
+                }
+            }
+        }
+    }
+
+    if constexpr (kSplit) {
+        // ---- this CTA finishes its band: slices added in rank order, scaled, stored ----
+        __syncwarp();
+        pdl_wait();
+        if (band_rows > 0 && !s_abort && mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) {
+            const int n_base = (2 * it0.nt + (int)rank) * kTile + slice_rank * band;
+            float pre;
+            const float in_scale = channel_factor(p, pre);
+            for (int i = threadIdx.x; i < band_rows * m_groups; i += kThreads) {
+                const int rl = i % band_rows;
+                const int mg = i / band_rows;                  // group of four tokens
+                const int n = n_base + rl;
+                if (n >= p.N) continue;
+                const uint32_t local = smem_base + (uint32_t)mg * group_bytes + (uint32_t)rl * 16u;
+                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int sl = 0; sl < 4; ++sl) {
+                    if (sl < sched.splits) {
+                        const float4 u = ld_shared_f4(local + (uint32_t)sl * slice_bytes);
+                        a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
+                    }
+                }
+                const float ws = in_scale * __ldg(p.w_scale + n);
+                const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
+                const float o[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (4 * mg + j < m_valid) p.y[(size_t)(it0.m0 + 4 * mg + j) * p.ldy + n] = __float2bfloat16_rn(fmaf(o[j] * pre, ws, bs));
+            }
+        }
+    }
+
+    // nobody leaves while another CTA may still signal its barriers, push into its ring or read its tensor memory
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, kTmemCols);
+    }
+}
+
+template <bool kSplit, bool kMlp>
+cudaError_t launch_kernel(const W8a8PairPlan& pl, const UmmaArgs& a, const PairMaps8& maps, cudaStream_t stream) {
+    auto kern = w8a8_pair_kernel<kSplit, kMlp>;
+    static SmemOptIn opted;
+    cudaError_t e = ensure_dynamic_smem((const void*)kern, kSmemBytes<kMlp>, opted);
+    if (e != cudaSuccess) return e;
+    PairSched8 s;
+    s.n_tiles = pl.n_tiles; s.m_tiles = pl.m_tiles; s.tokens = pl.tokens; s.last_tokens = pl.last_tokens; s.splits = pl.splits; s.slices = pl.slices;
+    s.kblocks = (a.K + kKB - 1) / kKB; s.kblocks_per_slice = (s.kblocks + s.slices - 1) / s.slices;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)pl.grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmemBytes<kMlp>;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    int na = pdl_attribute(attr);
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = (unsigned)(2 * pl.splits);
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    return counted(cudaLaunchKernelEx(&cfg, kern, maps, a, s));
+}
+
+}  // namespace
+
+// Tokens per tile, and whether a cluster takes the slices: the cheapest by a model of the kernel in microseconds, fitted to
+// back-to-back calls with every T and 1 to 4 slices over twelve layer shapes (1280 -> 1536 .. 2048 -> 11008 .. 18944 -> 3584, 3584
+// -> 37888) at 16 to 4096 rows; the choice is 1 % slower than the best of the sweep on average.  A K block takes the longer
+// of the way of the operands into shared memory (0.09 + 0.0003 T: 16 KB of weights whatever T is; more when every SM loads)
+// and the tensor core's (0.03 + 0.0013 T); all blocks together at least what the power limit allows.  A call starts later the
+// more SMs it needs at once (the kernel before it is still on them), and clusters add the hand-over of the sums and their
+// start: they only pay for long K, and are only taken when all fit at once.
+W8a8PairPlan plan_w8a8_pair(int64_t M, int64_t K, int64_t N, bool mlp, int slices, int force_tokens, int force_splits) {
+    W8a8PairPlan best{};
+    best.cost = 1e30;
+    const int kblocks = (int)((K + kKB - 1) / kKB);
+    const int n_tiles = (int)((N + 255) / 256);
+    if (slices < 1 || slices > 8 || slices > kblocks) return best;
+    const int kps = (kblocks + slices - 1) / slices;
+    if ((kblocks + kps - 1) / kps != slices) return best;                     // would leave an empty slice
+    for (int pass = 0; pass < 2; ++pass) {
+        const int splits = pass == 0 ? 1 : slices;
+        if (pass == 1 && (slices == 1 || slices > 4 || mlp)) break;
+        if (force_splits > 0 && splits != force_splits) continue;
+        const void* kern = splits > 1 ? (const void*)w8a8_pair_kernel<true, false>
+                         : mlp ? (const void*)w8a8_pair_kernel<false, true> : (const void*)w8a8_pair_kernel<false, false>;
+        const int slots = max_active_clusters(kern, kThreads, mlp ? kSmemBytes<true> : kSmemBytes<false>, 2 * splits);
+        if (slots < 1) continue;
+        const int blocks = splits > 1 ? kps : kblocks;                        // K blocks of a pair
+        for (int tokens = 32; tokens <= kMaxT; tokens += 32) {
+            if (force_tokens > 0 && tokens != force_tokens) continue;
+            if (force_tokens <= 0 && tokens >= M + 32) break;
+            if (splits == 1 && slices * tokens > kTmemCols) break;
+            const int m_tiles = (int)((M + tokens - 1) / tokens);
+            const int last = (int)((M - (int64_t)(m_tiles - 1) * tokens + 31) / 32) * 32;
+            const long items = (long)n_tiles * m_tiles;
+            if (force_splits <= 0 && splits > 1 && items > slots) continue;
+            const long rounds = (items + slots - 1) / slots;
+            const double active = (double)(items < slots ? items : slots) * splits, pairs = sm_count() / 2;
+            const double load = active / pairs;
+            const double hbm = 32768.0 * active / m_tiles / 10.7e6;           // (the other token tiles find the weights in L2)
+            auto block = [&](int t) {
+                const double in = (0.0907 + 0.00029 * t) * (1.0 + 0.755 * load), mma = 0.0323 + 0.00126 * t * (1.0 + 0.175 * load);
+                const double own = in > mma ? in : mma;
+                return own > hbm ? own : hbm;
+            };
+            const double t_last = block(last), t_full = m_tiles > 1 ? block(tokens) : t_last;
+            const double mean = ((m_tiles - 1) * t_full + t_last) / m_tiles;
+            const double drain = (0.0122 + (splits > 1 ? 0.0 : 0.002 * (slices - 1))) * tokens;
+            double chain = blocks * (rounds == 1 ? t_full : rounds * mean);
+            if (splits == 1 && 2 * slices * tokens > kTmemCols) chain += (rounds - 1) * drain;      // one accumulator stage
+            const double power = (double)n_tiles * kblocks / pairs * ((m_tiles - 1) * (0.148 + 0.0009 * tokens) + 0.148 + 0.0009 * last);
+            if (power > chain) chain = power;
+            static const double cluster_start[5] = {0, 0, 0.92, 0.51, 0.67};
+            const double tail = splits > 1 ? 0.96 + cluster_start[splits] + 0.030 * tokens * (1.0 - 1.0 / splits) : drain;
+            const double cost = chain + 1.66 + 1.53 * load + tail;
+            if (cost < best.cost) {
+                best.cost = cost;
+                best.n_tiles = n_tiles; best.m_tiles = m_tiles; best.tokens = tokens; best.last_tokens = last;
+                best.slices = slices; best.splits = splits;
+                best.grid = splits > 1 ? (int)(items * 2 * splits) : 2 * (int)(items < slots ? items : slots);
+            }
+        }
+    }
+    return best;
+}
+
+cudaError_t launch_w8a8_pair(const W8a8PairPlan& pl, const UmmaArgs& a, cudaStream_t stream, const char** why) {
+    const bool mlp = a.hq != nullptr;
+    PairMaps8 maps;
+    if (pl.tokens < 32 || !encode_u8_2d(&maps.w, a.w, (uint64_t)(pack_ntiles(a.N) * pack_kblocks(a.K) * 128), 128, mlp ? kTile / 2 : kTile) ||
+        !encode_u8_2d(&maps.x, a.xq, (uint64_t)a.M, (uint64_t)a.K, (uint32_t)pl.tokens / 2) ||
+        !encode_u8_2d(&maps.x_last, a.xq, (uint64_t)a.M, (uint64_t)a.K, (uint32_t)pl.last_tokens / 2)) {
+        if (why) *why = "no plan, or cuTensorMapEncodeTiled failed";
+        return cudaErrorInvalidValue;
+    }
+    if (mlp) return launch_kernel<false, true>(pl, a, maps, stream);
+    return pl.splits > 1 ? launch_kernel<true, false>(pl, a, maps, stream) : launch_kernel<false, false>(pl, a, maps, stream);
+}
+
+}  // namespace fp8lin
