@@ -6,8 +6,8 @@ namespace fp8lin {
 
 // xq[m][k] = e4m3(clamp(x[m][k] / max(s, 1e-12), +-448)).  3 bytes of traffic per element (2 read + 1 written): HBM-bound.
 // A block takes 512 consecutive 16-element vectors of [M][K/16] at a time, two per thread, so that a thread has 64 bytes in
-// flight; their row is found with one division per block and a multiplication per thread (16384 x 18944, beside the GEMMs
-// that follow at their power-limited clock: 142 -> 125 us).
+// flight; their row is found with one division per block and a multiplication per thread (16384 x 18944 alone:
+// 142 us, 6.5 TB/s).
 __global__ void __launch_bounds__(256)
 act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* __restrict__ input_scale,
                  unsigned char* __restrict__ xq, int64_t M, int64_t K) {

@@ -31,7 +31,7 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     pdl_launch_dependents();
     // A decode-sized call is one dependent chain: predecessor's end -> row -> sum of squares -> quantised row.  What no kernel
     // writes (weight, scale) is fetched before the wait, all loads of the row are in flight together, and every thread adds
-    // the warps' partial sums itself (one barrier instead of two): 4.5 -> 3.6 us for one row of 3584 without the overlap of
+    // the warps' partial sums itself (one barrier instead of two): 4.5 -> 2.7 us for one row of 3584 without the overlap of
     // a dependent launch.
     uint4 w[kNormMaxVec];
 #pragma unroll

@@ -24,7 +24,12 @@
 //   one pair works through all slices, each into its own T columns of tensor memory, and the epilogue adds them
 //   kSplit (few tiles, long K): the 2 s CTAs of a cluster take one slice each of the same tile
 //   and push the partial sums of band r to the r-th pair's CTA of the same channels (st.async counted on its mbarrier)
-// All waits are bounded.
+//
+// What bounds it: up to T = 64 the way of 16 KB of weights per CTA and K block into shared memory (0.09 us when few SMs load,
+// 0.16 when all do), above that the tensor core (512 cycles per K block at T = 256), for large calls its power.  Per call back
+// to back, before (decode kernel, one-CTA GEMM or 256-row pairs, whichever was chosen) -> now: 3584 -> 3584 64 rows 7.2 -> 6.2
+// us, 256 rows 10.0 -> 8.3; 3584 -> 4608 1031 rows 20.1 -> 16.7; 3584 -> 37888 1031 rows 111 -> 102; 18944 -> 3584 700 rows
+// 51 -> 40, 1031 rows 59 -> 54.  Four 7B layers of 64 rows: 271 -> 239 us, two of 1031 rows: 527 -> 484.  All waits are bounded.
 #include "umma_common.cuh"
 
 namespace fp8lin {
