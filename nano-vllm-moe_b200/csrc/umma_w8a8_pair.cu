@@ -479,7 +479,7 @@ W8a8PairPlan plan_w8a8_pair(int64_t M, int64_t K, int64_t N, bool mlp, int slice
             };
             const double t_last = block(last), t_full = m_tiles > 1 ? block(tokens) : t_last;
             const double mean = ((m_tiles - 1) * t_full + t_last) / m_tiles;
-            const double drain = (0.0122 + (splits > 1 ? 0.0 : 0.002 * (slices - 1))) * tokens;
+            const double drain = 0.0122 * tokens + (splits > 1 ? 0.0 : 0.2 * (slices - 1));
             double chain = blocks * (rounds == 1 ? t_full : rounds * mean);
             if (splits == 1 && 2 * slices * tokens > kTmemCols) chain += (rounds - 1) * drain;      // one accumulator stage
             const double power = (double)n_tiles * kblocks / pairs * ((m_tiles - 1) * (0.148 + 0.0009 * tokens) + 0.148 + 0.0009 * last);
