@@ -185,7 +185,7 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // Split-K hand-overs lay the received sums out as [slice][group of four rows][channel], 16 bytes each: lanes hold channels,
 // so an instruction of a warp writes 512 contiguous bytes.  With the four-row groups of a channel side by side each lane's
 // 16 bytes travelled alone, and the hand-over was the longest part of a small call: per call back to back, before / after,
-// 3584 -> 3584 W8A16 200 rows 17.0 / 14.2 us, 64 rows 10.2 / 9.2; W8A8 3584 -> 4608 64 rows 8.6 / 7.6, 2048 -> 2048 one row
+// W8A16 64 rows on 3584 -> 3584 10.2 / 9.2 us; W8A8 3584 -> 4608 64 rows 8.6 / 7.6, 2048 -> 2048 one row
 // 3.7 / 3.2, 18944 -> 3584 64 rows 15.8 / 14.8.
 __device__ __forceinline__ void st_async_v4(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t bar) {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
@@ -415,23 +415,6 @@ __device__ __forceinline__ void store_box(const OutMaps& outs, uint32_t box, int
         return;
     }
     for (int d = 0; d < outs.n; ++d) tma_store_2d(&outs.m[d], box, col0, row0);
-}
-
-// mbar_wait for a barrier that the partner CTA arrives on: acquires at cluster scope
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, int* status, int code) {
-    long long start = -1;
-    for (uint32_t it = 0;; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-        if (done) return true;
-        if ((it & 0x3ff) == 0x3ff) {
-            const long long now = clock64();
-            if (start < 0) start = now;
-            else if (now - start > kWaitCycles) { atomicExch(status, code); return false; }
-        }
-    }
 }
 
 // 16 consecutive TMEM columns of this lane -> 16 registers; no wait

@@ -23,9 +23,9 @@
 //   warps 10..17  epilogue: lane = channel, y[m][n] = bf16(acc * w_scale[n] + bias[n]); two lanes swap halves so that a lane
 //                 stores two channels of one token
 //
-// Few tiles: the K blocks are cut into up to four slices, the 2 s CTAs of a cluster take one slice each of the same tile
-// and push the partial sums of band r to the r-th pair's CTA of the same channels (st.async counted on its mbarrier; slices
-// added in rank order, so results do not depend on timing), as in umma_swap.cu.  All waits are bounded.
+// Few tiles: the K blocks are cut into up to four slices, the 2 s CTAs of a cluster take one slice each of the same tile and
+// park their sums in shared memory, and the CTA of slice r adds up band r of its pair rank's channels, slices in rank order (so
+// results do not depend on timing).  All waits are bounded.
 #include "umma_common.cuh"
 
 namespace fp8lin {
@@ -44,7 +44,7 @@ constexpr int kRingBytes = 216 * 1024;         // activation ring (128 T bytes p
 constexpr int kSmemBytes = kRingBytes + 1024;
 constexpr int kACols = 64;                     // 128 bf16 of a row = 64 columns
 constexpr int kTmemCols = 512;
-static_assert((kTile + 4) * 256 * 4 <= kRingBytes, "the received slices of a band must fit in the ring");
+static_assert(kTile * 256 * 4 <= kRingBytes, "the parked sums must fit in the ring");
 
 // Ring depths for T tokens per tile.  A slot is occupied from its TMA until its MMAs (activations) or its widening (weights)
 // are done, an L2 / HBM round trip of 1 to 1.5 us under load plus the chain through converters and tensor core, so with
@@ -148,8 +148,6 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     __shared__ __align__(8) uint64_t bar_empty[kMaxA];    // the MMAs that read the widened weights are done (both CTAs')
     __shared__ __align__(8) uint64_t bar_tfull[2];
     __shared__ __align__(8) uint64_t bar_tempty[2];    // leader's
-    __shared__ __align__(8) uint64_t bar_ready;        // split-K: every CTA of these channels is past its MMAs
-    __shared__ __align__(8) uint64_t bar_recv;         // split-K: the partials of this CTA's band have landed
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
 
@@ -182,9 +180,11 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const int m_left = kSplit ? p.M - (first_item % sched.m_tiles) * T : 0;
     const int m_valid = kSplit ? min(T, m_left) : 0;
     const int m_groups = (m_valid + 3) >> 2;
-    // received sums: [slice][group of four tokens][channel of the band] (see st_async_v4)
-    const uint32_t group_bytes = (uint32_t)band * 16u;
-    const uint32_t slice_bytes = group_bytes * (uint32_t)(T >> 2);
+    // split-K: this CTA's raw sums lie over the (then idle) ring as [group of four tokens][channel], 16 bytes each, so that 32
+    // lanes (channels) touch 512 contiguous bytes.  The CTA that finishes a band fetches its channels from all slices.
+    // Sent to it by st.async instead (which suits the few rows of the decode kernels), 128 channels x T sums took longer: 200 rows on
+    // 3584 -> 3584 14.3 us against 12.9, on 18944 -> 3584 29.9 / 28.3, 96 rows on 3584 -> 4608 12.0 / 11.1.
+    constexpr uint32_t group_bytes = kTile * 16u;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxW; ++i) { mbar_init(smem_u32(&bar_wfull[i]), 1); mbar_init(smem_u32(&bar_wempty[i]), kConvWarps / 2); }
@@ -195,11 +195,6 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
         for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bar_tfull[i]), 1); mbar_init(smem_u32(&bar_tempty[i]), 2 * kEpiWarps); }
         s_abort = 0;
-        if (kSplit) {
-            mbar_init(smem_u32(&bar_ready), (uint32_t)sched.splits);
-            mbar_init(smem_u32(&bar_recv), 1);
-            mbar_expect_tx(smem_u32(&bar_recv), (uint32_t)(sched.splits * band_rows * m_groups * 16));
-        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -382,16 +377,8 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                     }
                 }
             } else {
-                // the pair's MMAs are done, so this CTA's ring is free: tell the CTAs that will push into it, wait for those
-                // this one pushes into, and send each channel's sums to the owner of its band
-                if (warp == 2 + kConvWarps && lane < sched.splits)
-                    mbar_arrive_cluster(map_to_cta(smem_u32(&bar_ready), (uint32_t)(2 * lane) + rank));
-                if (!mbar_wait_cluster(smem_u32(&bar_ready), 0, p.status, kDevTimeoutPeer)) { s_abort = 1; ok = false; break; }
-                const int c0 = q * 32 + lane;
-                const int owner = c0 / band;
-                const uint32_t owner_cta = (uint32_t)(2 * owner) + rank;
-                const uint32_t dst = map_to_cta(smem_base + slice_rank * slice_bytes + (uint32_t)(h * half >> 2) * group_bytes + (uint32_t)(c0 - owner * band) * 16u, owner_cta);
-                const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), owner_cta);
+                // the pair's MMAs are done, so this CTA's ring is free
+                const uint32_t dst = smem_base + (uint32_t)(h * half >> 2) * group_bytes + (uint32_t)(q * 32 + lane) * 16u;
                 for (int c = 0; c < half; c += 32) {
                     uint32_t v[32];
                     __syncwarp();
@@ -401,7 +388,8 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         if (j == 16 && c + 16 >= half) break;
-                        if (h * half + c + j < m_valid) st_async_v4(dst + (uint32_t)((c + j) >> 2) * group_bytes, v[j], v[j + 1], v[j + 2], v[j + 3], rbar);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((c + j) >> 2) * group_bytes), "r"(v[j]), "r"(v[j + 1]),
+                                     "r"(v[j + 2]), "r"(v[j + 3]) : "memory");
                     }
                 }
             }
@@ -412,7 +400,8 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         // ---- this CTA finishes its band: slices added in rank order, scaled, stored ----
         __syncwarp();
         pdl_wait();
-        if (band_rows > 0 && !s_abort && mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) {
+        cluster_sync_all();                                // every CTA's sums are parked
+        if (!s_abort) {
             const int n_base = (2 * (first_item / sched.m_tiles) + (int)rank) * kTile + slice_rank * band;
             const int m_base = (first_item % sched.m_tiles) * T;
             for (int i = threadIdx.x; i < band_rows * m_groups; i += kThreads) {
@@ -420,15 +409,14 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 const int mg = (i / band_rows) * 4;
                 const int n = n_base + rl;
                 if (n >= p.N) continue;
-                const uint32_t local = smem_base + (uint32_t)(mg >> 2) * group_bytes + (uint32_t)rl * 16u;
-                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                const uint32_t local = smem_base + (uint32_t)(mg >> 2) * group_bytes + (uint32_t)(slice_rank * band + rl) * 16u;
+                float4 u[4];                               // all slices' loads go out before the first add
 #pragma unroll
-                for (int sl = 0; sl < 4; ++sl) {
-                    if (sl < sched.splits) {
-                        const float4 u = ld_shared_f4(local + (uint32_t)sl * slice_bytes);
-                        a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
-                    }
-                }
+                for (int sl = 0; sl < 4; ++sl)
+                    u[sl] = sl < sched.splits ? ld_cluster_f4(map_to_cta(local, 2u * (uint32_t)sl + rank)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 a = u[0];
+#pragma unroll
+                for (int sl = 1; sl < 4; ++sl) { a.x += u[sl].x; a.y += u[sl].y; a.z += u[sl].z; a.w += u[sl].w; }
                 const float ws = __ldg(p.w_scale + n);
                 const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
                 const float o[4] = {a.x, a.y, a.z, a.w};

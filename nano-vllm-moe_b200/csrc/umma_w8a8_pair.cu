@@ -23,7 +23,7 @@
 // kernels up to 64 rows, the one-CTA GEMM above).  Two ways:
 //   one pair works through all slices, each into its own T columns of tensor memory, and the epilogue adds them
 //   kSplit (few tiles, long K): the 2 s CTAs of a cluster take one slice each of the same tile
-//   and push the partial sums of band r to the r-th pair's CTA of the same channels (st.async counted on its mbarrier)
+//   and park their sums in shared memory; slice r's CTA adds up band r of its pair rank's channels
 //
 // What bounds it: up to T = 64 the way of 16 KB of weights per CTA and K block into shared memory (0.09 us when few SMs load,
 // 0.16 when all do), above that the tensor core (512 cycles per K block at T = 256), for large calls its power.  Per call back
@@ -48,7 +48,7 @@ constexpr int kRingBytes = 210 * 1024;         // 16 KB + 64 T bytes per slot
 constexpr int kSwapBytes = 32 * 64;            // kMlp: bf16 values of 32 rows x 32 channels, one buffer per warp pair
 constexpr int kCodeBytes = 32 * 32;            // ... and their e4m3 results
 template <bool kMlp> constexpr int kSmemBytes = kRingBytes + (kMlp ? 4 * (kSwapBytes + kCodeBytes) : 0) + 1024;
-static_assert((kTile + 4) * kMaxT * 4 <= kRingBytes, "the received slices of a band must fit in the ring");
+static_assert(kTile * 256 * 4 <= kRingBytes, "the parked sums must fit in the ring");
 
 struct PairSched8 {
     int n_tiles;              // 256-channel tiles
@@ -100,8 +100,6 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     __shared__ __align__(8) uint64_t bar_empty[kMaxSlots];     // the MMAs that read the slot are done (both CTAs')
     __shared__ __align__(8) uint64_t bar_tfull[2];
     __shared__ __align__(8) uint64_t bar_tempty[2];            // leader's
-    __shared__ __align__(8) uint64_t bar_ready;                // split-K: every CTA of these channels is past its MMAs
-    __shared__ __align__(8) uint64_t bar_recv;                 // split-K: the partials of this CTA's band have landed
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
 
@@ -130,20 +128,16 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     const Item it0 = decode_item(sched, first_item);
     const int m_valid = kSplit ? min(2 * it0.half, p.M - it0.m0) : 0;
     const int m_groups = (m_valid + 3) >> 2;
-    // received sums: [slice][group of four tokens][channel of the band], 16 bytes each, so that the 32 lanes (channels) of a
-    // warp send 512 contiguous bytes per instruction
-    const uint32_t group_bytes = (uint32_t)band * 16u;
-    const uint32_t slice_bytes = group_bytes * (uint32_t)(sched.tokens >> 2);
+    // split-K: this CTA's raw sums lie over the (then idle) ring as [group of four tokens][channel], 16 bytes each, so that 32
+    // lanes (channels) touch 512 contiguous bytes.  The CTA that finishes a band fetches its channels from all slices.
+    // Sent to it by st.async instead (which suits the few rows of the decode kernels), 128 channels x T sums took longer: 256 rows on
+    // 18944 -> 3584 22.2 us against 20.9.
+    constexpr uint32_t group_bytes = kTile * 16u;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxSlots; ++i) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_empty[i]), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bar_tfull[i]), 1); mbar_init(smem_u32(&bar_tempty[i]), 2 * kEpiWarps); }
         s_abort = 0;
-        if (kSplit) {
-            mbar_init(smem_u32(&bar_ready), (uint32_t)sched.splits);
-            mbar_init(smem_u32(&bar_recv), 1);
-            mbar_expect_tx(smem_u32(&bar_recv), (uint32_t)(sched.splits * band_rows * m_groups * 16));
-        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -342,23 +336,16 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                     }
                 }
             } else {
-                // the pair's MMAs are done, so this CTA's ring is free: tell the CTAs that will push into it, wait for those
-                // this one pushes into, and send each channel's sums to the owner of its band
-                if (warp == 2 && lane < sched.splits)
-                    mbar_arrive_cluster(map_to_cta(smem_u32(&bar_ready), (uint32_t)(2 * lane) + rank));
-                if (!mbar_wait_cluster(smem_u32(&bar_ready), 0, p.status, kDevTimeoutPeer)) { s_abort = 1; break; }
-                const int c0 = q * 32 + lane;
-                const int owner = c0 / band;
-                const uint32_t owner_cta = (uint32_t)(2 * owner) + rank;
-                const uint32_t dst = map_to_cta(smem_base + slice_rank * slice_bytes + (uint32_t)(h * it.half >> 2) * group_bytes + (uint32_t)(c0 - owner * band) * 16u, owner_cta);
-                const uint32_t rbar = map_to_cta(smem_u32(&bar_recv), owner_cta);
+                // the pair's MMAs are done, so this CTA's ring is free
+                const uint32_t dst = smem_base + (uint32_t)(h * it.half >> 2) * group_bytes + (uint32_t)(q * 32 + lane) * 16u;
                 for (int c = 0; c < it.half; c += 32) {
                     uint32_t v[32];
                     read32(c, v);
 #pragma unroll
                     for (int j = 0; j < 32; j += 4) {
                         if (j == 16 && c + 16 >= it.half) break;
-                        if (h * it.half + c + j < m_valid) st_async_v4(dst + (uint32_t)((c + j) >> 2) * group_bytes, v[j], v[j + 1], v[j + 2], v[j + 3], rbar);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((c + j) >> 2) * group_bytes), "r"(v[j]), "r"(v[j + 1]),
+                                     "r"(v[j + 2]), "r"(v[j + 3]) : "memory");
                     }
                 }
             }
@@ -369,7 +356,8 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         // ---- this CTA finishes its band: slices added in rank order, scaled, stored ----
         __syncwarp();
         pdl_wait();
-        if (band_rows > 0 && !s_abort && mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) {
+        cluster_sync_all();                                // every CTA's sums are parked
+        if (!s_abort) {
             const int n_base = (2 * it0.nt + (int)rank) * kTile + slice_rank * band;
             float pre;
             const float in_scale = channel_factor(p, pre);
@@ -378,15 +366,14 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                 const int mg = i / band_rows;                  // group of four tokens
                 const int n = n_base + rl;
                 if (n >= p.N) continue;
-                const uint32_t local = smem_base + (uint32_t)mg * group_bytes + (uint32_t)rl * 16u;
-                float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                const uint32_t local = smem_base + (uint32_t)mg * group_bytes + (uint32_t)(slice_rank * band + rl) * 16u;
+                float4 u[4];                               // all slices' loads go out before the first add
 #pragma unroll
-                for (int sl = 0; sl < 4; ++sl) {
-                    if (sl < sched.splits) {
-                        const float4 u = ld_shared_f4(local + (uint32_t)sl * slice_bytes);
-                        a.x += u.x; a.y += u.y; a.z += u.z; a.w += u.w;
-                    }
-                }
+                for (int sl = 0; sl < 4; ++sl)
+                    u[sl] = sl < sched.splits ? ld_cluster_f4(map_to_cta(local, 2u * (uint32_t)sl + rank)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 a = u[0];
+#pragma unroll
+                for (int sl = 1; sl < 4; ++sl) { a.x += u[sl].x; a.y += u[sl].y; a.z += u[sl].z; a.w += u[sl].w; }
                 const float ws = in_scale * __ldg(p.w_scale + n);
                 const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
                 const float o[4] = {a.x, a.y, a.z, a.w};
