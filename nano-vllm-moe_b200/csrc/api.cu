@@ -133,7 +133,10 @@ bool w8a16_pair_wanted(int64_t M, int64_t K, int64_t N) {
     // 33 to 64 rows: pairs where the one-CTA kernel would not split K (it then widens every tile alone, 0.56 us per block at
     // 64 rows): 2048 -> 11008 11.0 us against 12.3, 2560 -> 9472 10.9 / 12.1, 3584 -> 37888 33.0 / 33.8; with slices it keeps
     // 3584 -> 4608 12.2 / 11.4, 18944 -> 3584 25.0 / 24.7
-    return M > 32 && plan_swap_w8a16(M, K, N, -1).splits == 1;
+    if (M > 32 && plan_swap_w8a16(M, K, N, -1).splits == 1) return true;
+    // from 49 rows also where the pairs do not split K and a third of them have a channel tile: 64 rows on 1280 -> 7168 6.2 / 8.2,
+    // 2560 -> 9472 10.4 / 11.1; not 1280 -> 1536 (six tiles) 5.5 / 5.1
+    return M > 48 && 3 * ((N + 255) / 256) >= sm_count() / 2 && plan_w8a16_pair(M, K, N, -1, -1).splits == 1;
 }
 // null: another kernel's
 const W8a16PairPlan* w8a16_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {

@@ -478,17 +478,17 @@ cudaError_t launch_kernel(const W8a16PairPlan& pl, const UmmaArgs& a, const CUte
 }  // namespace
 
 // Tokens per tile and K slices: the cheapest by a model of the kernel, microseconds, fitted to back-to-back calls with every
-// (T, slices) on eight layer shapes (1280 -> 7168, 2048 -> 11008, 8192 -> 1024 .. 3584 -> 37888, 18944 -> 3584) at 70 to 4096
-// rows; the choice is 1.2 % slower than the best of the sweep on average.  A K block takes the longer of the weights' way
-// (ring, widening, HBM: 0.42, more when every SM streams) and the tensor core's (0.12 + 0.0018 T, likewise), and all blocks
-// together what the power limit allows (0.22 + 0.0023 T per pair and block: large calls run at 1.2 GHz).  A tile adds its
-// epilogue; slices add the hand-over of T x (1 - 1/s) sums per channel and what a cluster takes to start (slices are only
-// taken when all clusters fit at once: a second wave never paid).
+// (T, slices) on twelve layer shapes (1280 -> 1536 .. 2048 -> 11008 .. 18944 -> 3584, 3584 -> 37888) at 40 to 1031 rows; the choice is
+// 0.7 % slower than the best of the sweep on average.  A K block takes the longer of the weights' way (ring, widening, HBM:
+// 0.45, a little more when every SM streams) and the tensor core's (0.19 + 0.0016 T), and all blocks together what the
+// power limit allows (0.17 + 0.0025 T per pair and block: large calls run at 1.2 GHz).  A call starts later the more SMs it
+// needs at once; a tile adds its epilogue; slices add the hand-over of T x (1 - 1/s) sums per channel and what a cluster
+// takes to start (slices are only taken when all clusters fit at once: a second wave never paid).
 W8a16PairPlan plan_w8a16_pair(int64_t M, int64_t K, int64_t N, int force_tokens, int force_splits) {
     W8a16PairPlan best{};
     const int kblocks = (int)((K + kKB - 1) / kKB);
     const int n_tiles = (int)((N + 255) / 256);
-    static const double cluster_start[5] = {0, 0, 2.1, 0.7, 0.5};
+    static const double cluster_start[5] = {0, 0, 0.24, 0.22, 1.48};
     double best_cost = 1e30;
     for (int splits = 1; splits <= 4; ++splits) {
         if (force_splits > 0 && splits != (force_splits > 4 ? 4 : force_splits)) continue;
@@ -507,13 +507,13 @@ W8a16PairPlan plan_w8a16_pair(int64_t M, int64_t K, int64_t N, int force_tokens,
             if (force_splits <= 0 && splits > 1 && items > slots) continue;
             const long rounds = (items + slots - 1) / slots;
             const double load = (double)(items < slots ? items : slots) * 2 * splits / sm_count();
-            const double weights = 0.42 * (1 + 0.154 * load), tensor = (0.12 + 0.0018 * tokens) * (1 + 0.175 * load);
+            const double weights = 0.447 * (1 + 0.08 * load), tensor = (0.193 + 0.00163 * tokens) * (1 + 0.023 * load);
             const double t_block = weights > tensor ? weights : tensor;
-            const double drain = 0.0037 * tokens;
+            const double drain = 0.0149 * tokens;
             const double chain = rounds * kps * t_block + (rounds - 1) * (0.08 + drain);
-            const double power = (double)items * splits * kps / (sm_count() / 2) * (0.22 + 0.0023 * tokens);
-            const double tail = splits > 1 ? 1.3 + cluster_start[splits] + 0.0373 * tokens * (1.0 - 1.0 / splits) : drain;
-            const double cost = (chain > power ? chain : power) + 3.3 + tail;
+            const double power = (double)items * splits * kps / (sm_count() / 2) * (0.173 + 0.00246 * tokens);
+            const double tail = splits > 1 ? 1.31 + cluster_start[splits] + 0.0303 * tokens * (1.0 - 1.0 / splits) : drain;
+            const double cost = (chain > power ? chain : power) + 2.8 * load + tail;
             if (cost < best_cost) {
                 best_cost = cost;
                 best.n_tiles = n_tiles; best.m_tiles = m_tiles; best.tokens = tokens; best.splits = splits; best.kblocks_per_split = kps;
