@@ -196,9 +196,9 @@ int fp8lin_quantize_activation(const void* x, int64_t ldx, const float* input_sc
  * w2_packed = E x packed(K=I, N=H).  Scales: w13_scale f32 [E][2I], w2_scale f32 [E][H],
  * one static activation scale per projection.
  *
- * From 512 routed rows on the rows are gathered and quantised once, the gate_up grouped GEMM applies silu(g) * u and
- * the down projection's quantiser in its epilogue (I a multiple of 128), and with more than 64 rows per expert on
- * average both grouped GEMMs run with the routed rows as the MMA M dimension (128 x 256 work items).
+ * The gate_up grouped GEMM applies silu(g) * u and the down projection's quantiser in its epilogue.  From 512 routed rows
+ * on the rows are quantised once, into expert order, before it; with more than 64 rows per expert on average the grouped
+ * GEMMs then run with the routed rows as the MMA M dimension (128 x 256 work items; gate_up where I is a multiple of 128).
  * fp8lin_moe_route replaces SoftmaxTopKRouter.select_experts (executor/moe/router.py:24-34):
  * fp32 softmax over E logits (logits_dtype 0 = f32, 1 = bf16), top-k, optional
  * renormalisation; topk_w f32 [T][k], topk_ids i32 [T][k]. */
@@ -310,7 +310,7 @@ const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N);
  * "stream_push" (0 = split-K of the mma.sync streaming kernel always through global scratch instead of a cluster),
  * "mlp_decode_fused" (1 = the fused MLP on up to 16 pre-quantised rows computes silu * up inside the gate_up kernel),
  * "moe_fused" (0 = the expert FFN keeps a separate activation pass), "moe_rows_major" (0 = prefill-sized expert
- * batches stay on the one-CTA grouped kernel), "pair_stages" (4 or 5 ring slots in the CTA-pair GEMM). */
+ * batches stay on the channel-major grouped kernel), "pair_stages" (4 or 5 ring slots in the CTA-pair GEMM). */
 int fp8lin_set_tuning(const char* knob, int value);
 
 /* Blocking: copies the device status word out of `workspace` (after syncing

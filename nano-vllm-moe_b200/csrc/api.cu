@@ -45,7 +45,7 @@ struct Tuning {
     int fuse_quant = -1;        // large-M W8A8: <= 0 (default) = quantise x in a separate pass; 1 = the pass takes the rows
                                 // of the first round of tiles, the GEMM's own quantiser warps the rest; n > 1 = the pass
                                 // takes the first n rows (rounded up to 128)
-    int moe_rows_major = -1;    // 0 = prefill-sized expert batches stay on the one-CTA grouped kernel
+    int moe_rows_major = -1;    // 0 = prefill-sized expert batches stay on the channel-major grouped kernel
     int mlp_decode_fused = -1;  // 1 = the fused MLP on up to 16 pre-quantised rows computes silu * up in the gate_up kernel (study knob)
     int moe_fused = -1;         // 0 = the expert FFN keeps its separate silu-multiply-quantise pass for every batch size
     int quant_lead = -1;        // row blocks the in-kernel quantiser may run ahead (default: from the tile schedule)
@@ -1099,10 +1099,10 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     int* inv = (int*)(ws + L.off_inv);
     __nv_bfloat16* gu = (__nv_bfloat16*)(ws + L.off_gu);
     unsigned char* hq = ws + L.off_hq;
-    const int avg_mp = grouped_chunk_rows(rows, E);
-    // Prefill-sized batches with more than a few rows per expert: both projections on CTA pairs with chunks of up to 256 rows.
-    const bool pairs = rows >= kMoePrequantRows && avg_mp >= 32 && ld_out % 8 == 0 && aligned16(out_routed) && g_tune.moe_rows_major != 0;
-    const int mp = pairs ? 256 : avg_mp;
+    const int mp = grouped_chunk_rows(rows, E);
+    // Prefill-sized batches whose experts fill 128-row chunks: the rows are the MMA M dimension (umma_grouped_rows.cu), in
+    // gate_up where the up channels start at a tile.
+    const bool rows_major = rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
     cudaError_t e = launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
@@ -1112,14 +1112,15 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     a.ldx = (int)ldx; a.x_div = x_div; a.ld_out = (int)(2 * I); a.N = (int)(2 * I); a.K = (int)H; a.n_tiles = 0; a.kblocks = 0;
     a.scatter = 0;
     // the gate_up GEMM's epilogue applies the activation and writes hq (the separate pass stays for comparison)
-    const bool fused_act = pairs || g_tune.moe_fused != 0;
+    const bool fused_act = g_tune.moe_fused != 0;
     GroupedArgs g = a;
     if (fused_act) { g.N = (int)I; g.hq = hq; g.h_scale = w2_input_scale; g.out = nullptr; }
     if (rows >= kMoePrequantRows) {
         unsigned char* xq = ws + L.off_xq;
         e = launch_moe_scatter_quant((const __nv_bfloat16*)x, ldx, x_div, inv, (int)rows, w13_input_scale, xq, (int)H, st);
         if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row quantiser launch: %s", cudaGetErrorString(e));
-        e = pairs ? launch_grouped_pair_w8a8(g, w13_packed, E, xq, rows, st, &why) : launch_grouped_w8a8(false, mp, g, w13_packed, E, xq, rows, st, &why);
+        e = rows_major && fused_act && I % 128 == 0 ? launch_grouped_rows_w8a8(g, w13_packed, E, xq, rows, st, &why)
+                                                    : launch_grouped_w8a8(false, mp, g, w13_packed, E, xq, rows, st, &why);
     } else {
         e = launch_grouped_w8a8(true, mp, g, w13_packed, E, nullptr, 0, st, &why);
     }
@@ -1130,7 +1131,8 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     }
     a.w_scale = w2_scale; a.input_scale = w2_input_scale; a.out = (__nv_bfloat16*)out_routed; a.ld_out = (int)ld_out;
     a.N = (int)H; a.K = (int)I; a.scatter = 1;
-    e = pairs ? launch_grouped_pair_w8a8(a, w2_packed, E, hq, rows, st, &why) : launch_grouped_w8a8(false, mp, a, w2_packed, E, hq, rows, st, &why);
+    e = rows_major && ld_out % 8 == 0 && aligned16(out_routed) ? launch_grouped_rows_w8a8(a, w2_packed, E, hq, rows, st, &why)
+                                                               : launch_grouped_w8a8(false, mp, a, w2_packed, E, hq, rows, st, &why);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "down grouped GEMM launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
     return FP8LIN_OK;
 }

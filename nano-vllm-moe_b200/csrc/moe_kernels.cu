@@ -1,7 +1,6 @@
 // Small kernels around the MoE expert FFN: router, row grouping, activation, combine.
 #include "common.cuh"
 #include "kernels.h"
-#include "umma_common.cuh"
 
 namespace fp8lin {
 
@@ -118,9 +117,8 @@ cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, in
 // memory atomics of a skewed or large batch collide inside a warp only; then the counters become running positions
 // (scan over experts, inside an expert over warps) and the warps place their rows.  Against one set of E counters and a
 // serial scan by one thread: 5.7 -> 2.8 us for 256 rows of 60 experts.  A single SM's shared memory atomics bound it from a
-// few thousand rows on (16384 rows: 14.7 us, with the cluster 7.2), so from kAlignClusterRows rows a cluster of eight CTAs shares the rows
-// (kCluster): each counts its own part, reads the other CTAs' totals through distributed shared memory and places its rows.
-template <typename IdT, int kWarps, bool kCluster>
+// few thousand rows on (16384 rows: 14.7 us).
+template <typename IdT, int kWarps>
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, int* __restrict__ expert_offsets,
                  int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta, int* __restrict__ inv) {
@@ -132,10 +130,8 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
     int* cstart = start + E + 1;           // [E + 1] chunk prefix
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < kWarps * E; i += blockDim.x) count[i] = 0;
-    const int crank = kCluster ? (int)cluster_ctarank() : 0;
-    constexpr int kCtas = kCluster ? 8 : 1;
-    const int share = ((rows + kCtas * kWarps * 32 - 1) / (kCtas * kWarps * 32)) * 32;
-    const int r0 = min(rows, (crank * kWarps + warp) * share), r1 = min(rows, r0 + share);
+    const int share = ((rows + kWarps * 32 - 1) / (kWarps * 32)) * 32;
+    const int r0 = min(rows, warp * share), r1 = min(rows, r0 + share);
     constexpr int kBatch = 8;              // ids in flight per lane
     auto load_ids = [&](int r, int end, int* e) {
 #pragma unroll
@@ -164,24 +160,6 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
         total[e] = acc;
     }
     __syncthreads();
-    if constexpr (kCluster) {              // total becomes the whole batch's, the positions move up by the CTAs in front
-        cluster_sync_all();
-        for (int e = threadIdx.x; e < E; e += blockDim.x) {
-            int before = 0, all = 0;
-#pragma unroll
-            for (int c = 0; c < kCtas; ++c) {
-                int v;
-                asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(map_to_cta(smem_u32(total + e), (uint32_t)c)));
-                if (c < crank) before += v;
-                all += v;
-            }
-            start[e] = all;                // (parked: the other CTAs still read total)
-            for (int w = 0; w < kWarps; ++w) count[w * E + e] += before;
-        }
-        cluster_sync_all();
-        for (int e = threadIdx.x; e < E; e += blockDim.x) total[e] = start[e];
-        __syncthreads();
-    }
     if (warp == 0) {                       // exclusive scans of rows and chunks over the experts
         int row_base = 0, chunk_base = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
@@ -198,12 +176,11 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
         }
         if (lane == 0) {
             start[E] = row_base; cstart[E] = chunk_base;
-            if (crank == 0) { meta[0] = chunk_base; meta[1] = row_base; }
+            meta[0] = chunk_base; meta[1] = row_base;
         }
     }
     __syncthreads();
-    if (crank == 0)
-        for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = start[e];
+    for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = start[e];
     if (warp < kWarps) {
         int* mine = count + warp * E;
         for (int r = r0 + lane; r < r1; r += 32 * kBatch) {
@@ -222,42 +199,23 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
             }
         }
     }
-    for (int e = threadIdx.x * kCtas + crank; e < E; e += blockDim.x * kCtas) {
-        // chunks of 256 rows are evened out to steps of 32: 273 rows are 160 + 113, not 256 + 17
-        const int n = total[e], parts = (n + chunk_rows - 1) / chunk_rows;
-        const int size = chunk_rows == 256 && n > 0 ? (((n + parts - 1) / parts) + 31) & ~31 : chunk_rows;
-        for (int c = 0, pos = 0; pos < n; ++c, pos += size)
-            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(size, n - pos), 0);
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        const int n = total[e];
+        for (int c = 0, pos = 0; pos < n; ++c, pos += chunk_rows)
+            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(chunk_rows, n - pos), 0);
     }
 }
-
-constexpr int kAlignClusterRows = 2048;
 
 template <typename IdT>
 static cudaError_t launch_align(const IdT* ids, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows, int4* chunks,
                                 int* meta, int* inv, cudaStream_t stream) {
     // counters per warp: 32 sets where they fit the 48 KB of shared memory (E <= 340), one set beyond (E <= 3071)
     auto smem = [&](int sets) { return (size_t)((sets + 3) * E + 2) * sizeof(int); };
-    if (rows >= kAlignClusterRows && smem(32) <= 48 * 1024) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(8);
-        cfg.blockDim = dim3(1024);
-        cfg.dynamicSmemBytes = smem(32);
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[2];
-        int na = pdl_attribute(attr);
-        attr[na].id = cudaLaunchAttributeClusterDimension;
-        attr[na].val.clusterDim.x = 8;
-        attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = na + 1;
-        return counted(cudaLaunchKernelEx(&cfg, moe_align_kernel<IdT, 32, true>, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv));
-    }
     if (rows > 1024 && smem(32) <= 48 * 1024)
-        return launch_dependent(moe_align_kernel<IdT, 32, false>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+        return launch_dependent(moe_align_kernel<IdT, 32>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
     if (smem(8) <= 48 * 1024)
-        return launch_dependent(moe_align_kernel<IdT, 8, false>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
-    return launch_dependent(moe_align_kernel<IdT, 1, false>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+        return launch_dependent(moe_align_kernel<IdT, 8>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+    return launch_dependent(moe_align_kernel<IdT, 1>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
 }
 
 cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,

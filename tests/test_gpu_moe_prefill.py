@@ -1,5 +1,5 @@
-"""The CTA-pair grouped GEMM of prefill-sized expert batches: intermediate sizes that put the up channels inside a weight
-tile, chunk sizes at their steps, experts without rows, ids without an expert; and silu without a general division."""
+"""Prefill-sized expert batches: intermediate sizes that put the up channels inside a weight tile, chunk sizes at their
+steps, experts without rows, ids without an expert; many passes in flight at once; and the activation in the epilogue."""
 import importlib
 
 import numpy as np
@@ -14,11 +14,12 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("counts,H,I", [
-    ([256, 257, 0, 33], 272, 144),          # one full chunk, one row over (160 + 97), no rows, one row over 32; up rows inside a tile
-    ([31, 700, 1, 288], 512, 192),          # 64-row steps of the up channels; 3 chunks of 256 / 256 / 188
+    ([256, 257, 0, 33], 272, 144),          # full chunks, one row over, no rows, a part of a chunk; up rows inside a tile
+    ([31, 700, 1, 288], 512, 192),          # 64-row steps of the up channels
     ([513, 64, 512, 95], 144, 16),          # the narrowest intermediate size
+    ([128, 129, 400, 0], 272, 128),         # up channels at a tile: rows as the MMA's M in both projections, an odd last tile in down
 ])
-def test_pair_grouped_gemm_against_the_oracle(counts, H, I):
+def test_prefill_experts_against_the_oracle(counts, H, I):
     moe = importlib.import_module("nano-vllm-moe_b200.executor.moe")
     E, T = len(counts), sum(counts)
     assert T >= 512
@@ -32,7 +33,7 @@ def test_pair_grouped_gemm_against_the_oracle(counts, H, I):
     wts = upload_weights(moe, c)
     x, wt = to_bf16_cuda(c["x"]), torch.from_numpy(w).cuda()
     y = from_bf16(kern(x, wt, torch.from_numpy(ids).cuda(), wts, model_dtype=torch.bfloat16))
-    assert_parity(y, ref, f"pair experts {counts} H={H} I={I}", ulps=3.0, min_cos=0.9999)
+    assert_parity(y, ref, f"prefill experts {counts} H={H} I={I}", ulps=3.0, min_cos=0.9999)
     # a token whose expert is not here gets nothing, the others the same bits
     ids[::7] = -1
     y2 = from_bf16(kern(x, wt, torch.from_numpy(ids).cuda(), wts, model_dtype=torch.bfloat16))
@@ -40,6 +41,34 @@ def test_pair_grouped_gemm_against_the_oracle(counts, H, I):
     keep = np.ones(T, bool)
     keep[::7] = False
     np.testing.assert_array_equal(y2[keep], y[keep])
+    assert kernels().read_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("T,H,E,I,k", [(1024, 512, 8, 384, 4), (700, 272, 5, 144, 4)])       # rows as M; channels as M
+def test_passes_in_flight_give_the_bits_of_single_passes(T, H, E, I, k):
+    """A serving loop never waits between blocks: every kernel of the chain starts under its predecessor, in the next pass too."""
+    moe = importlib.import_module("nano-vllm-moe_b200.executor.moe")
+    cfg = moe.make_moe_parallel_config(tp_group=None, ep_group=None, global_num_experts=E, intermediate_size=I)
+    kern = moe.MoEKernel(prepare_finalize=moe.NoEPPrepareFinalize(cfg), experts=moe.Fp8Experts(), parallel_config=cfg)
+    router = moe.SoftmaxTopKRouter(k, False)
+    c = make_moe_case(T + I, T, H, I, E, k)
+    wts = upload_weights(moe, c)
+    gen = torch.Generator(device="cuda").manual_seed(T)
+    inputs = [(torch.randn(T, H, generator=gen, device="cuda").bfloat16(), torch.randn(T, E, generator=gen, device="cuda").bfloat16())
+              for _ in range(3)]
+
+    def one_pass(x, logits):
+        w, ids = router.select_experts(x, logits)
+        return kern(x, w, ids, wts, model_dtype=torch.bfloat16)
+
+    single = []
+    for x, logits in inputs:
+        single.append(one_pass(x, logits))
+        torch.cuda.synchronize()
+    last = [one_pass(*inputs[i % 3]) for i in range(300)][-6:]
+    torch.cuda.synchronize()
+    for i, y in enumerate(last):
+        assert torch.equal(y, single[(294 + i) % 3])
     assert kernels().read_status(torch.device("cuda", 0)) == 0
 
 
