@@ -179,6 +179,34 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+// Tensor memory of a CTA pair, from warp 1 of every CTA.  The allocation and its release reach into the partner CTA, so the
+// first waits until every CTA of the cluster runs, and none ends before all are through the second.  Between the two, every
+// CTA's mbarriers exist (initialised before the call) and its tensor memory is allocated before a leader's MMA writes there;
+// nobody releases while a partner may still signal its barriers or the leader's MMAs may still use its memory.
+__device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_base, uint32_t cols) {
+    cluster_sync_all();
+    if (warp == 1) {
+        __syncwarp();
+        tmem_alloc_pair(smem_u32(s_base), cols);
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    tc_fence_after();
+    return *s_base;
+}
+__device__ __forceinline__ void pair_tmem_end(int warp, uint32_t tmem_base, uint32_t cols) {
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        tmem_dealloc_pair(tmem_base, cols);
+    }
+    cluster_sync_all();
+}
 // 16 bytes into a CTA of the cluster (dst and bar are shared::cluster addresses of the same CTA); the store is
 // asynchronous and counts its bytes on that CTA's barrier when it lands
 //

@@ -100,12 +100,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc_pair(smem_u32(&s_tmem_base), kTmemCols);
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();            // the partner's barriers exist before anything is signalled on them
-    tc_fence_after();
-    const uint32_t tmem_base = s_tmem_base;
+    const uint32_t tmem_base = pair_tmem_begin(warp, &s_tmem_base, kTmemCols);
     pdl_launch_dependents();
     static_assert(!kFuseQ || !kF16, "in-kernel quantisation: e4m3 operands only");
     QuantJob qjob;
@@ -345,16 +340,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (lane == 0) tma_store_wait_all();
     }
 
-    // nobody leaves while its partner may still signal its barriers or the leader's MMAs may still
-    // read its shared memory and write its tensor memory
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();
-    if (warp == 1) {
-        __syncwarp();
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, kTmemCols);
-    }
+    pair_tmem_end(warp, tmem_base, kTmemCols);
     if (kFuseQ && threadIdx.x == 0) quant_ctrl_release(qjob, p.M);
 }
 

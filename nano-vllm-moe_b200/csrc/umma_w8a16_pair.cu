@@ -198,12 +198,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc_pair(smem_u32(&s_tmem_base), kTmemCols);
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();            // the other CTAs' barriers exist before anything is signalled on them
-    tc_fence_after();
-    const uint32_t tmem_base = s_tmem_base;
+    const uint32_t tmem_base = pair_tmem_begin(warp, &s_tmem_base, kTmemCols);
     pdl_launch_dependents();
 
     if (warp == 0) {
@@ -427,15 +422,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
     }
 
-    // nobody leaves while another CTA may still signal its barriers, push into its ring or read its tensor memory
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();
-    if (warp == 1) {
-        __syncwarp();
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, kTmemCols);
-    }
+    pair_tmem_end(warp, tmem_base, kTmemCols);
 }
 
 bool encode_x_tokens(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows) {

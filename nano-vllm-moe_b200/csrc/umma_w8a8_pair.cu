@@ -141,12 +141,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc_pair(smem_u32(&s_tmem_base), kTmemCols);
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();            // the other CTAs' barriers exist before anything is signalled on them
-    tc_fence_after();
-    const uint32_t tmem_base = s_tmem_base;
+    const uint32_t tmem_base = pair_tmem_begin(warp, &s_tmem_base, kTmemCols);
     pdl_launch_dependents();
 
     if (warp == 0) {
@@ -384,15 +379,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         }
     }
 
-    // nobody leaves while another CTA may still signal its barriers, push into its ring or read its tensor memory
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();
-    if (warp == 1) {
-        __syncwarp();
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, kTmemCols);
-    }
+    pair_tmem_end(warp, tmem_base, kTmemCols);
 }
 
 template <bool kSplit, bool kMlp>

@@ -1,0 +1,31 @@
+"""Orders that a wait in a kernel depends on and that no output shows: read from the kernels' sources."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "nano-vllm-moe_b200" / "csrc"
+SOURCES = {p.name: re.sub(r"//[^\n]*", "", p.read_text()) for p in sorted(CSRC.iterdir()) if p.suffix in (".cu", ".cuh")}
+
+
+def body(source, function):
+    """The text between the braces of one function of a source."""
+    at = source.index("{", source.index(f" {function}("))
+    depth = 0
+    for i in range(at, len(source)):
+        depth += {"{": 1, "}": -1}.get(source[i], 0)
+        if depth == 0:
+            return source[at:i]
+    raise AssertionError(f"{function} does not end")
+
+
+def test_pair_tensor_memory_is_taken_and_released_between_cluster_barriers():
+    """tcgen05.alloc / dealloc of a CTA pair are collective over both CTAs: the partner has to run, and has to be there still."""
+    common = SOURCES["umma_common.cuh"]
+    begin, end = body(common, "pair_tmem_begin"), body(common, "pair_tmem_end")
+    assert begin.index("cluster_sync_all") < begin.index("tmem_alloc_pair") < begin.rindex("cluster_sync_all")
+    assert end.index("cluster_sync_all") < end.index("tmem_dealloc_pair") < end.rindex("cluster_sync_all")
+    for name, text in SOURCES.items():
+        rest = text.replace(begin, "").replace(end, "")
+        calls = re.findall(r"(?<!void )tmem_(?:de)?alloc_pair\(", rest)
+        assert not calls, f"{name} takes or releases a pair's tensor memory by itself"
+        assert text.count("pair_tmem_begin(") == text.count("pair_tmem_end("), name
+    assert sum(t.count("= pair_tmem_begin(") for t in SOURCES.values()) == 3
