@@ -235,6 +235,57 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     return v;
 }
 
+// ---- named barriers ------------------------------------------------------------------------------------------
+// The form without .aligned: it often follows code that one lane of the warp ran, and whether the warp is together again by
+// then is the compiler's choice.
+__device__ __forceinline__ void named_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// ... with a vote: true in every thread when one of them said so
+__device__ __forceinline__ bool named_sync_any(int id, int threads, bool flag) {
+    uint32_t any;
+    asm volatile(
+        "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
+        " barrier.cta.red.or.pred pout, %2, %3, pin;\n selp.u32 %0, 1, 0, pout;\n}"
+        : "=r"(any) : "r"(flag ? 1u : 0u), "r"(id), "r"(threads) : "memory");
+    return any != 0;
+}
+
+// ---- gate_up epilogues: silu(gate) * up, quantised ---------------------------------------------------------------
+// A warp holds kP rows of 32 gate channels, another one the same rows of the up channels (a lane a channel; column pairs of
+// rows as bf16x2: lo = rows [0, kP / 2), hi the rest).  Each hands the other half of its values over through swap_buf (kP x 64
+// bytes for the two, words [pair][lane], the gate's half in front), the gate warp finishes rows [0, kP / 2), the up warp the
+// rest, and code_buf holds e4m3 [row][32 channels] when the call returns.  No branches inside (rows that do not exist are
+// computed and not stored by the caller), so that the chains of exp and divisions overlap.  kTwoRoundings: silu(gate) is
+// rounded to bf16 before the product, as the experts' eager SiluAndMul does it.
+template <int kP, bool kTwoRoundings>
+__device__ __forceinline__ void gate_up_swap(const uint32_t (&lo)[kP / 4], const uint32_t (&hi)[kP / 4], bool up, uint32_t swap_buf,
+                                             uint32_t code_buf, int barrier, int lane, const ExactDiv& div_h) {
+    constexpr int kH = kP / 4;
+#pragma unroll
+    for (int j = 0; j < kH; ++j)
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(swap_buf + (up ? 0 : kP * 32) + j * 128 + lane * 4), "r"(up ? lo[j] : hi[j]) : "memory");
+    named_sync(barrier, 64);
+    uint32_t other[kH];
+#pragma unroll
+    for (int j = 0; j < kH; ++j)
+        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(swap_buf + (up ? kP * 32 : 0) + j * 128 + lane * 4) : "memory");
+    const uint32_t code_at = code_buf + (up ? kP * 16 : 0) + lane;
+#pragma unroll
+    for (int j = 0; j < kH; ++j) {
+        const uint32_t g = up ? other[j] : lo[j], u = up ? hi[j] : other[j];
+        float s0 = silu_f32(bf16_lo(g)), s1 = silu_f32(bf16_hi(g));
+        if (kTwoRoundings) {
+            const uint32_t sv = pack_bf16x2(s0, s1);
+            s0 = bf16_lo(sv);
+            s1 = bf16_hi(sv);
+        }
+        const uint32_t hv = pack_bf16x2(s0 * bf16_lo(u), s1 * bf16_hi(u));
+        const uint32_t code = cvt_e4m3x2(div_h(bf16_lo(hv)), div_h(bf16_hi(hv)));
+        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + 2 * j * 32), "r"(code & 0xffu) : "memory");
+        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + (2 * j + 1) * 32), "r"(code >> 8) : "memory");
+    }
+    named_sync(barrier, 64);
+}
+
 // K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
     uint64_t d = 0;

@@ -326,14 +326,14 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const int n0 = wk.n0;
             const int half_cols = kNarrow ? (wk.bn >> 1) : BN / 2;   // columns of this warp's half of the item
             // every epilogue warp is done with the previous tile's multipliers before they are replaced
-            if (tl > 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (tl > 0) named_sync(1, 256);
             if (et < BN) { s_scale[et] = next_scale; s_bias[et] = next_bias; }
             // the loads for the tile after this one land while this tile's epilogue runs
             if (w + work_step < sched.total_work) fetch_columns(w + work_step);
             if (kSplit) {
                 // one tile per CTA: nothing after this loop meets at a named barrier, so each warp may give
                 // up on its own, and the barrier stays off the path between the last MMA and the reduction
-                asm volatile("bar.sync 1, 256;" ::: "memory");
+                named_sync(1, 256);
                 if (!mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull)) {
                     s_abort = 1; ok = false; break;
                 }
@@ -342,12 +342,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                 // One barrier makes the multipliers visible and takes the vote: if the wait ran out in any
                 // warp, every epilogue warp leaves here together (they meet at named barriers again on the
                 // next tile, so they must agree).
-                uint32_t any_failed;
-                asm volatile(
-                    "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
-                    " barrier.cta.red.or.pred pout, 1, 256, pin;\n selp.u32 %0, 1, 0, pout;\n}"
-                    : "=r"(any_failed) : "r"(arrived ? 0u : 1u) : "memory");
-                if (any_failed) { s_abort = 1; ok = false; break; }
+                if (named_sync_any(1, 256, !arrived)) { s_abort = 1; ok = false; break; }
             }
             tc_fence_after();
             const int row0 = tm * kBM + q * 32;
@@ -376,7 +371,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                     }
                     // the pair's previous store must have finished reading the box
                     if (h == 0 && lane == 0) tma_store_wait_read();
-                    asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+                    named_sync(2 + q, 64);
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const uint32_t dst = pbox + lane * 128 + (((uint32_t)(h * 4 + j) ^ (uint32_t)(lane & 7)) << 4);
@@ -384,7 +379,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                                      "r"(o[4 * j + 2]), "r"(o[4 * j + 3]) : "memory");
                     }
                     fence_async_smem();
-                    asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+                    named_sync(2 + q, 64);
                     if (h == 0 && lane == 0) {
                         // one store per destination: the local output, or (row-parallel scatter) this
                         // rank's slot in every rank's buffer, peers reached over NVLink

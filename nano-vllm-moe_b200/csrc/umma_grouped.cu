@@ -249,14 +249,7 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
                 }
             }
             bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull);
-            if (kFused) {                         // warps that meet at barriers below leave together
-                uint32_t failed;
-                asm volatile(
-                    "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
-                    " barrier.cta.red.or.pred pout, 3, 128, pin;\n selp.u32 %0, 1, 0, pout;\n}"
-                    : "=r"(failed) : "r"(arrived ? 0u : 1u) : "memory");
-                arrived = failed == 0;
-            }
+            if (kFused) arrived = !named_sync_any(3, 128, !arrived);              // warps that meet at barriers below leave together
             if (!arrived) { s_abort = 1; ok = false; break; }
             tc_fence_after();
             const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + as * Cfg::kAccCols;
@@ -273,29 +266,13 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
                     if (kP == 32) tmem_ld32_nowait(t_addr + c0, v);
                     else tmem_ld16_nowait(t_addr + c0, v);
                     tmem_ld_wait();
-                    uint32_t own[kH], other[kH];
-#pragma unroll
-                    for (int j = 0; j < kH; ++j) {                // as the bf16 gate_up row
-                        const uint32_t lo = pack_bf16x2(__uint_as_float(v[2 * j]) * ws, __uint_as_float(v[2 * j + 1]) * ws);
-                        const uint32_t hi = pack_bf16x2(__uint_as_float(v[kP / 2 + 2 * j]) * ws, __uint_as_float(v[kP / 2 + 2 * j + 1]) * ws);
-                        own[j] = up ? hi : lo;
-                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(swap_buf + (up ? 0 : kP * 32) + j * 128 + lane * 4), "r"(up ? lo : hi) : "memory");
-                    }
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
-#pragma unroll
-                    for (int j = 0; j < kH; ++j)
-                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(swap_buf + (up ? kP * 32 : 0) + j * 128 + lane * 4) : "memory");
-                    const uint32_t code_at = code_buf + (up ? kP * 16 : 0) + lane;
+                    uint32_t lo[kH], hi[kH];                      // as the bf16 gate_up row
 #pragma unroll
                     for (int j = 0; j < kH; ++j) {
-                        const uint32_t g = up ? other[j] : own[j], u = up ? own[j] : other[j];
-                        const uint32_t sv = pack_bf16x2(silu_f32(bf16_lo(g)), silu_f32(bf16_hi(g)));                  // bf16(silu(g))
-                        const uint32_t hv = pack_bf16x2(bf16_lo(sv) * bf16_lo(u), bf16_hi(sv) * bf16_hi(u));          // bf16(. * u)
-                        const uint32_t code = cvt_e4m3x2(div_h(bf16_lo(hv)), div_h(bf16_hi(hv)));
-                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + 2 * j * 32), "r"(code & 0xffu) : "memory");
-                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + (2 * j + 1) * 32), "r"(code >> 8) : "memory");
+                        lo[j] = pack_bf16x2(__uint_as_float(v[2 * j]) * ws, __uint_as_float(v[2 * j + 1]) * ws);
+                        hi[j] = pack_bf16x2(__uint_as_float(v[kP / 2 + 2 * j]) * ws, __uint_as_float(v[kP / 2 + 2 * j + 1]) * ws);
                     }
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
+                    gate_up_swap<kP, true>(lo, hi, up, swap_buf, code_buf, 1 + (q & 1), lane, div_h);
                     // 32 bytes per row: thread i of the 64 stores half a row (N is a multiple of 16)
                     const int i = (up ? 32 : 0) + lane, r = i >> 1, nh = (n - lane) + (i & 1) * 16;
                     if (r < kP && c0 + r < ch.z && nh < p.N)

@@ -167,7 +167,7 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const int t = w % n_items;
             const int as = tl & 1;
             const uint32_t aph = (tl >> 1) & 1;
-            if (tl > 0) asm volatile("bar.sync 1, 256;" ::: "memory");        // everybody is done with the previous multipliers
+            if (tl > 0) named_sync(1, 256);        // everybody is done with the previous multipliers
             s_scale[et] = next_scale;
             if (w + (int)gridDim.x < total) next_scale = column_scale(w + gridDim.x);
             const int r = q * 32 + lane;                                      // this thread's row of the chunk
@@ -179,12 +179,7 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
                 rw = __ldg(p.topk_w + routed);
             }
             const bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull);
-            uint32_t any_failed;                                              // publishes the multipliers and takes the vote
-            asm volatile(
-                "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
-                " barrier.cta.red.or.pred pout, 1, 256, pin;\n selp.u32 %0, 1, 0, pout;\n}"
-                : "=r"(any_failed) : "r"(arrived ? 0u : 1u) : "memory");
-            if (any_failed) { s_abort = 1; ok = false; break; }
+            if (named_sync_any(1, 256, !arrived)) { s_abort = 1; ok = false; break; }
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + as * kColsN;
             if (kFusedAct) {

@@ -224,18 +224,13 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             const int as = tl & 1;
             const uint32_t aph = (tl >> 1) & 1;
             const int n0 = tn * kBN;
-            if (tl > 0) asm volatile("bar.sync 1, 256;" ::: "memory");
+            if (tl > 0) named_sync(1, 256);
             s_scale[et] = next_scale;
             s_bias[et] = next_bias;
             if (t + tile_step < sched.total) fetch_columns(t + tile_step);
             const bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull);
             // one barrier publishes the multipliers and takes the vote: the eight warps leave together
-            uint32_t any_failed;
-            asm volatile(
-                "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
-                " barrier.cta.red.or.pred pout, 1, 256, pin;\n selp.u32 %0, 1, 0, pout;\n}"
-                : "=r"(any_failed) : "r"(arrived ? 0u : 1u) : "memory");
-            if (any_failed) { s_abort = 1; ok = false; break; }
+            if (named_sync_any(1, 256, !arrived)) { s_abort = 1; ok = false; break; }
             tc_fence_after();
             const int row0 = (2 * tmp + (int)rank) * kBM + q * 32;
             if (kMlp) {
@@ -274,7 +269,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                             qv[j] = quant8_e4m3(make_uint4(hw[4 * j], hw[4 * j + 1], hw[4 * j + 2], hw[4 * j + 3]), div_h);
                         if (sp == 0) {
                             if (h == 0 && lane == 0) tma_store_wait_read();      // the previous store has read the box
-                            asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+                            named_sync(2 + q, 64);
                         }
 #pragma unroll
                         for (int j = 0; j < 2; ++j) {
@@ -285,7 +280,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                         }
                     }
                     fence_async_smem();
-                    asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+                    named_sync(2 + q, 64);
                     if (h == 0 && lane == 0) tma_store_2d(&outs.m[0], pbox, n0 >> 1, row0);
                 }
                 tc_fence_before();
@@ -316,7 +311,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                                                fmaf(__uint_as_float(v[j + 3]), sc.w, __uint_as_float(bb.y & 0xffff0000u)));
                 }
                 if (h == 0 && lane == 0) tma_store_wait_read();      // the previous store has read the box
-                asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+                named_sync(2 + q, 64);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const uint32_t dst = pbox + lane * 128 + (((uint32_t)(h * 4 + j) ^ (uint32_t)(lane & 7)) << 4);
@@ -324,7 +319,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                                  "r"(o[4 * j + 2]), "r"(o[4 * j + 3]) : "memory");
                 }
                 fence_async_smem();
-                asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+                named_sync(2 + q, 64);
                 if (h == 0 && lane == 0) {
                     store_box(outs, pbox, n0 + col, row0);
                 }

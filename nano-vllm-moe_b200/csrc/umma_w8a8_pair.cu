@@ -246,14 +246,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                 if (p.bias) bs = __bfloat162float(p.bias[n]);
             }
             bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1), p.status, kDevTimeoutTmemFull);
-            if (kMlp) {                                    // warps that meet at barriers below leave together
-                uint32_t failed;
-                asm volatile(
-                    "{\n .reg .pred pin, pout;\n setp.ne.b32 pin, %1, 0;\n"
-                    " barrier.cta.red.or.pred pout, 5, 256, pin;\n selp.u32 %0, 1, 0, pout;\n}"
-                    : "=r"(failed) : "r"(arrived ? 0u : 1u) : "memory");
-                arrived = failed == 0;
-            }
+            if (kMlp) arrived = !named_sync_any(5, 256, !arrived);        // warps that meet at barriers below leave together
             if (!arrived) { s_abort = 1; break; }
             tc_fence_after();
             const int m0 = it.m0 + h * it.half;
@@ -284,31 +277,13 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                     uint32_t v[32];
                     read32(c, v);
                     const int n_cols = min(32, it.half - c);
-                    // Gate and up as the bf16 values that a separate gate_up linear stores.  The gate warp finishes columns [0, 16)
-                    // of the 32, the up warp [16, 32): each hands the other half over.  No branches inside (a last piece of 16
-                    // columns computes 16 more that are not stored), so that the eight chains of exp and divisions overlap.
-                    uint32_t own[8], other[8];
+                    uint32_t lo[8], hi[8];                 // the bf16 values that a separate gate_up linear stores
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const uint32_t lo = pack_bf16x2(fmaf(__uint_as_float(v[2 * j]) * pre, ws, bs), fmaf(__uint_as_float(v[2 * j + 1]) * pre, ws, bs));
-                        const uint32_t hi = pack_bf16x2(fmaf(__uint_as_float(v[16 + 2 * j]) * pre, ws, bs), fmaf(__uint_as_float(v[16 + 2 * j + 1]) * pre, ws, bs));
-                        own[j] = up ? hi : lo;
-                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(swap_buf + (up ? 0 : 1024) + j * 128 + lane * 4), "r"(up ? lo : hi) : "memory");
+                        lo[j] = pack_bf16x2(fmaf(__uint_as_float(v[2 * j]) * pre, ws, bs), fmaf(__uint_as_float(v[2 * j + 1]) * pre, ws, bs));
+                        hi[j] = pack_bf16x2(fmaf(__uint_as_float(v[16 + 2 * j]) * pre, ws, bs), fmaf(__uint_as_float(v[16 + 2 * j + 1]) * pre, ws, bs));
                     }
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        asm volatile("ld.shared.b32 %0, [%1];" : "=r"(other[j]) : "r"(swap_buf + (up ? 1024 : 0) + j * 128 + lane * 4) : "memory");
-                    const uint32_t code_at = code_buf + (up ? 16 * 32 : 0) + lane;
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const uint32_t g = up ? other[j] : own[j], u = up ? own[j] : other[j];
-                        const uint32_t hv = pack_bf16x2(silu_f32(bf16_lo(g)) * bf16_lo(u), silu_f32(bf16_hi(g)) * bf16_hi(u));
-                        const uint32_t code = cvt_e4m3x2(div_h(bf16_lo(hv)), div_h(bf16_hi(hv)));
-                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + 2 * j * 32), "r"(code & 0xffu) : "memory");
-                        asm volatile("st.shared.u8 [%0], %1;" ::"r"(code_at + (2 * j + 1) * 32), "r"(code >> 8) : "memory");
-                    }
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + pair) : "memory");
+                    gate_up_swap<32, false>(lo, hi, up, swap_buf, code_buf, 1 + pair, lane, div_h);
                     const int i = (up ? 32 : 0) + lane;                               // 32 bytes per row: a thread stores half a row
                     const int m = m0 + c + (i >> 1);
                     if ((i >> 1) < n_cols && m < p.M)

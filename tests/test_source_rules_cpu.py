@@ -29,3 +29,14 @@ def test_pair_tensor_memory_is_taken_and_released_between_cluster_barriers():
         assert not calls, f"{name} takes or releases a pair's tensor memory by itself"
         assert text.count("pair_tmem_begin(") == text.count("pair_tmem_end("), name
     assert sum(t.count("= pair_tmem_begin(") for t in SOURCES.values()) == 3
+
+
+def test_named_barriers_do_not_ask_for_a_converged_warp():
+    """The aligned form (bar.sync, or barrier.cta with .aligned) needs the whole warp at the instruction; the epilogues come there
+    out of branches that one lane took."""
+    for name, text in SOURCES.items():
+        asm = re.findall(r'"[^"\n]*\b(?:bar\.(?:sync|red|arrive)|barrier\.cta\.[a-z.]+)[^"\n]*"', text)
+        if name == "umma_common.cuh":
+            assert len(asm) == 2 and not any("bar.sync" in a or ".aligned" in a for a in asm), asm
+        else:
+            assert not asm, f"{name}: {asm}"
