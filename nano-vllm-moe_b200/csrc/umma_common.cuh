@@ -286,6 +286,36 @@ __device__ __forceinline__ void gate_up_swap(const uint32_t (&lo)[kP / 4], const
     named_sync(barrier, 64);
 }
 
+// ---- K slices of a CTA-pair tile: sums parked in shared memory ------------------------------------------------
+// Every CTA of the cluster has its raw sums at smem_base as [group of four tokens][128 channels], 16 bytes each.  This CTA
+// finishes channels [c0, c0 + rows) of its pair rank's 128 (n_base: the first of the 128): the up to four slices are added in
+// order, then y = bf16(sum * pre * (factor * w_scale[n]) + bias[n]).  After a cluster barrier; the caller keeps the memory alive.
+constexpr uint32_t kParkedGroupBytes = 128 * 16u;
+__device__ __forceinline__ void finish_parked_band(const UmmaArgs& p, uint32_t smem_base, int splits, int rank, int c0, int rows, int m_valid,
+                                                   int n_base, int m_base, float pre, float factor, int threads) {
+    const int total = rows * ((m_valid + 3) >> 2);
+    for (int i = threadIdx.x; i < total; i += threads) {
+        const int c = c0 + i % rows;
+        const int mg = i / rows;
+        const int n = n_base + c;
+        if (n >= p.N) continue;
+        const uint32_t local = smem_base + (uint32_t)mg * kParkedGroupBytes + (uint32_t)c * 16u;
+        float4 u[4];                                       // all slices' loads go out before the first add
+#pragma unroll
+        for (int sl = 0; sl < 4; ++sl)
+            u[sl] = sl < splits ? ld_cluster_f4(map_to_cta(local, 2u * (uint32_t)sl + (uint32_t)rank)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 a = u[0];
+#pragma unroll
+        for (int sl = 1; sl < 4; ++sl) { a.x += u[sl].x; a.y += u[sl].y; a.z += u[sl].z; a.w += u[sl].w; }
+        const float ws = factor * __ldg(p.w_scale + n);
+        const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
+        const float o[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (4 * mg + j < m_valid) p.y[(size_t)(m_base + 4 * mg + j) * p.ldy + n] = __float2bfloat16_rn(fmaf(o[j] * pre, ws, bs));
+    }
+}
+
 // K-major operand tile with 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
 __device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr) {
     uint64_t d = 0;

@@ -179,12 +179,11 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const int band_rows = kSplit ? max(0, min(kTile, (slice_rank + 1) * band) - slice_rank * band) : 0;
     const int m_left = kSplit ? p.M - (first_item % sched.m_tiles) * T : 0;
     const int m_valid = kSplit ? min(T, m_left) : 0;
-    const int m_groups = (m_valid + 3) >> 2;
     // split-K: this CTA's raw sums lie over the (then idle) ring as [group of four tokens][channel], 16 bytes each, so that 32
     // lanes (channels) touch 512 contiguous bytes.  The CTA that finishes a band fetches its channels from all slices.
     // Sent to it by st.async instead (which suits the few rows of the decode kernels), 128 channels x T sums took longer: 200 rows on
     // 3584 -> 3584 14.3 us against 12.9, on 18944 -> 3584 29.9 / 28.3, 96 rows on 3584 -> 4608 12.0 / 11.1.
-    constexpr uint32_t group_bytes = kTile * 16u;
+    constexpr uint32_t group_bytes = kParkedGroupBytes;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxW; ++i) { mbar_init(smem_u32(&bar_wfull[i]), 1); mbar_init(smem_u32(&bar_wempty[i]), kConvWarps / 2); }
@@ -397,28 +396,8 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         pdl_wait();
         cluster_sync_all();                                // every CTA's sums are parked
         if (!s_abort) {
-            const int n_base = (2 * (first_item / sched.m_tiles) + (int)rank) * kTile + slice_rank * band;
-            const int m_base = (first_item % sched.m_tiles) * T;
-            for (int i = threadIdx.x; i < band_rows * m_groups; i += kThreads) {
-                const int rl = i % band_rows;
-                const int mg = (i / band_rows) * 4;
-                const int n = n_base + rl;
-                if (n >= p.N) continue;
-                const uint32_t local = smem_base + (uint32_t)(mg >> 2) * group_bytes + (uint32_t)(slice_rank * band + rl) * 16u;
-                float4 u[4];                               // all slices' loads go out before the first add
-#pragma unroll
-                for (int sl = 0; sl < 4; ++sl)
-                    u[sl] = sl < sched.splits ? ld_cluster_f4(map_to_cta(local, 2u * (uint32_t)sl + rank)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 a = u[0];
-#pragma unroll
-                for (int sl = 1; sl < 4; ++sl) { a.x += u[sl].x; a.y += u[sl].y; a.z += u[sl].z; a.w += u[sl].w; }
-                const float ws = __ldg(p.w_scale + n);
-                const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
-                const float o[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (mg + j < m_valid) p.y[(size_t)(m_base + mg + j) * p.ldy + n] = __float2bfloat16_rn(fmaf(o[j], ws, bs));
-            }
+            finish_parked_band(p, smem_base, sched.splits, (int)rank, slice_rank * band, band_rows, m_valid,
+                               (2 * (first_item / sched.m_tiles) + (int)rank) * kTile, (first_item % sched.m_tiles) * T, 1.f, 1.f, kThreads);
         }
     }
 

@@ -127,12 +127,11 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     const int band_rows = kSplit ? max(0, min(kTile, (slice_rank + 1) * band) - slice_rank * band) : 0;
     const Item it0 = decode_item(sched, first_item);
     const int m_valid = kSplit ? min(2 * it0.half, p.M - it0.m0) : 0;
-    const int m_groups = (m_valid + 3) >> 2;
     // split-K: this CTA's raw sums lie over the (then idle) ring as [group of four tokens][channel], 16 bytes each, so that 32
     // lanes (channels) touch 512 contiguous bytes.  The CTA that finishes a band fetches its channels from all slices.
     // Sent to it by st.async instead (which suits the few rows of the decode kernels), 128 channels x T sums took longer: 256 rows on
     // 18944 -> 3584 22.2 us against 20.9.
-    constexpr uint32_t group_bytes = kTile * 16u;
+    constexpr uint32_t group_bytes = kParkedGroupBytes;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxSlots; ++i) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_empty[i]), 1); }
@@ -328,29 +327,10 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         pdl_wait();
         cluster_sync_all();                                // every CTA's sums are parked
         if (!s_abort) {
-            const int n_base = (2 * it0.nt + (int)rank) * kTile + slice_rank * band;
             float pre;
             const float in_scale = channel_factor(p, pre);
-            for (int i = threadIdx.x; i < band_rows * m_groups; i += kThreads) {
-                const int rl = i % band_rows;
-                const int mg = i / band_rows;                  // group of four tokens
-                const int n = n_base + rl;
-                if (n >= p.N) continue;
-                const uint32_t local = smem_base + (uint32_t)mg * group_bytes + (uint32_t)(slice_rank * band + rl) * 16u;
-                float4 u[4];                               // all slices' loads go out before the first add
-#pragma unroll
-                for (int sl = 0; sl < 4; ++sl)
-                    u[sl] = sl < sched.splits ? ld_cluster_f4(map_to_cta(local, 2u * (uint32_t)sl + rank)) : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 a = u[0];
-#pragma unroll
-                for (int sl = 1; sl < 4; ++sl) { a.x += u[sl].x; a.y += u[sl].y; a.z += u[sl].z; a.w += u[sl].w; }
-                const float ws = in_scale * __ldg(p.w_scale + n);
-                const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
-                const float o[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    if (4 * mg + j < m_valid) p.y[(size_t)(it0.m0 + 4 * mg + j) * p.ldy + n] = __float2bfloat16_rn(fmaf(o[j] * pre, ws, bs));
-            }
+            finish_parked_band(p, smem_base, sched.splits, (int)rank, slice_rank * band, band_rows, m_valid, (2 * it0.nt + (int)rank) * kTile,
+                               it0.m0, pre, in_scale, kThreads);
         }
     }
 
