@@ -317,7 +317,12 @@ int fp8lin_set_tuning(const char* knob, int value);
  * `stream`) and clears it.  0 = no kernel gave up a bounded wait.  Otherwise the code of the wait
  * that ran out (about a second): 0x101 operand tile never landed, 0x102 ring slot never freed, 0x103 /
  * 0x104 accumulator never filled / never drained, 0x105 in-kernel activation quantiser, 0x106 a peer
- * CTA of the cluster (split-K hand-over) never answered. */
+ * CTA of the cluster (split-K hand-over) never answered.
+ *
+ * The call whose kernel gave up has no valid result.  To learn of it without a blocking read, put the address of an int
+ * that the device can write and the host can read (pinned, mapped memory; initially 0) into bytes 8..15 of the workspace,
+ * once, after its zero fill: the code is stored there too.  Python callers need not: a stream's scratch is set up that way,
+ * and the next call on the stream raises. */
 int fp8lin_read_status(void* workspace, void* stream, int* status_out);
 
 /* Exercises the give-up path of the kernels' bounded waits without a fault (no counterpart in the

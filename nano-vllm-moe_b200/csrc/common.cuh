@@ -37,6 +37,18 @@ __host__ __device__ inline WsView ws_view(void* ws, size_t bytes) {
 enum : int { kDevOk = 0, kDevTimeoutFull = 0x101, kDevTimeoutEmpty = 0x102, kDevTimeoutTmemFull = 0x103,
              kDevTimeoutTmemEmpty = 0x104, kDevTimeoutQuant = 0x105, kDevTimeoutPeer = 0x106 };
 
+// A wait that gave up leaves its code in the status word, and in the host's word whose address the header holds (the words
+// behind the status: kWsHostWord; 0 = none), which a caller can look at on every call without asking the device.
+constexpr int kWsHostWord = 2;
+__device__ __forceinline__ void report_status(int* status, int code) {
+    atomicExch(status, code);
+    volatile int* host = *reinterpret_cast<int* volatile*>(status + kWsHostWord);
+    if (host) {
+        *host = code;
+        __threadfence_system();
+    }
+}
+
 // ---- packed weight layout ----------------------------------------------------------
 // Weights are stored as 128-channel x 128-byte tiles, each tile contiguous (16 KiB),
 // tiles of one channel block consecutive along K:

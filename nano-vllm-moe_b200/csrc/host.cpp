@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <cstdio>
 #include <map>
 #include <mutex>
 #include <stdexcept>
@@ -48,32 +49,62 @@ void need_cuda(const at::Tensor& t) {
 
 // ---- scratch: one zero-initialised buffer per (device, stream), grown on demand ------------------------------------
 // An outgrown buffer is kept (a captured CUDA graph has its address baked in) until release().
+// Every buffer of a stream names the same pinned word, where a kernel that gives up a wait leaves its code: the next call on
+// the stream sees it and raises, at the cost of a load from host memory.
 
+struct StreamScratch {
+    at::Tensor buffer;
+    at::Tensor gave_up;          // pinned int
+};
 struct Scratch {
     std::mutex lock;
-    std::map<std::pair<int, void*>, at::Tensor> live;
+    std::map<std::pair<int, void*>, StreamScratch> live;
     std::vector<at::Tensor> retired;
 };
+constexpr int64_t kHostWordAt = 8;           // byte of the header that names the host's word
 Scratch& scratch() { static Scratch* s = new Scratch; return *s; }      // (outlives the CUDA context's teardown)
 
-at::Tensor workspace(c10::cuda::CUDAStream stream, size_t nbytes) {
+// Raises when a kernel of an earlier call on this stream gave up a wait, and forgets it.
+void raise_if_given_up(StreamScratch& e) {
+    volatile int* word = e.gave_up.mutable_data_ptr<int>();
+    const int code = *word;
+    if (code == 0) return;
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+        *word = 0;
+        const c10::InferenceMode any_tensor(true);      // (the buffer may have been made in inference mode)
+        e.buffer.narrow(0, 0, (int64_t)sizeof(int)).zero_();
+    }
+    char hex[16];
+    snprintf(hex, sizeof(hex), "0x%x", code);
+    throw std::runtime_error(std::string("a kernel of an earlier call on this stream gave up a bounded wait (device status ") + hex +
+                             "): the result of that call is not valid");
+}
+
+at::Tensor workspace(c10::cuda::CUDAStream stream, size_t nbytes, bool raise = true) {
     Scratch& s = scratch();
     const auto key = std::make_pair((int)stream.device_index(), (void*)stream.stream());
     std::lock_guard<std::mutex> guard(s.lock);
     auto it = s.live.find(key);
-    if (it != s.live.end() && (size_t)it->second.numel() >= nbytes) return it->second;
+    if (it != s.live.end()) {
+        if (raise) raise_if_given_up(it->second);
+        if ((size_t)it->second.buffer.numel() >= nbytes) return it->second.buffer;
+    }
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
         throw std::runtime_error("fp8lin scratch for this stream must grow to " + std::to_string(nbytes) +
                                  " bytes during a CUDA graph capture; run the shape once (or call reserve_workspace) on "
                                  "the capturing stream before the capture");
     size_t size = nbytes < (size_t)FP8LIN_WS_HEADER_BYTES ? (size_t)FP8LIN_WS_HEADER_BYTES : nbytes;
     if (it != s.live.end()) {
-        if (size < 2 * (size_t)it->second.numel()) size = 2 * (size_t)it->second.numel();
-        s.retired.push_back(it->second);
+        const size_t old = (size_t)it->second.buffer.numel();
+        if (size < 2 * old) size = 2 * old;
     }
-    at::Tensor t = at::zeros({(int64_t)size}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, stream.device_index()));
-    s.live[key] = t;
-    return t;
+    StreamScratch fresh;
+    fresh.buffer = at::zeros({(int64_t)size}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, stream.device_index()));
+    fresh.gave_up = it != s.live.end() ? it->second.gave_up : at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    fresh.buffer.narrow(0, kHostWordAt, (int64_t)sizeof(int64_t)).view(at::kLong).fill_((int64_t)(intptr_t)fresh.gave_up.mutable_data_ptr());
+    if (it != s.live.end()) s.retired.push_back(it->second.buffer);
+    s.live[key] = fresh;
+    return fresh.buffer;
 }
 
 // ---- running one call of the library ---------------------------------------------------------------------------------
@@ -439,18 +470,27 @@ PyObject* py_moe_block(PyObject*, PyObject* const* a, Py_ssize_t na) {
     });
 }
 
-// workspace(device_index, stream_handle, nbytes) -> the stream's scratch tensor
+// workspace(device_index, stream_handle, nbytes, for_status) -> the stream's scratch tensor.  for_status: to read the status
+// word, so a wait that was given up is not raised here, and the host's copy of its code is forgotten.
 PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t na) {
     return guarded([&]() -> PyObject* {
-        need_args(na, 3, "workspace");
+        need_args(na, 4, "workspace");
         const long device = PyLong_AsLong(a[0]);
         void* handle = PyLong_AsVoidPtr(a[1]);
         const size_t nbytes = PyLong_AsSize_t(a[2]);
+        const bool for_status = a[3] == Py_True;
         if (PyErr_Occurred()) return nullptr;
         const c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
         const auto stream = c10::cuda::getCurrentCUDAStream();
         if ((void*)stream.stream() != handle) throw std::runtime_error("workspace: the stream is not the current one");
-        return THPVariable_Wrap(workspace(stream, nbytes));
+        const at::Tensor t = workspace(stream, nbytes, !for_status);
+        if (for_status) {
+            stream.synchronize();
+            Scratch& s = scratch();
+            std::lock_guard<std::mutex> lock(s.lock);
+            *s.live[std::make_pair((int)stream.device_index(), (void*)stream.stream())].gave_up.mutable_data_ptr<int>() = 0;
+        }
+        return THPVariable_Wrap(t);
     });
 }
 

@@ -35,7 +35,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* st
         if ((it & 0x3ff) == 0x3ff) {
             const long long now = clock64();
             if (start < 0) start = now;
-            else if (now - start > limit) { atomicExch(status, code); return false; }
+            else if (now - start > limit) { report_status(status, code); return false; }
         }
     }
 }
@@ -421,7 +421,7 @@ __device__ __forceinline__ bool quant_wait_block(const QuantJob& j, int M, int b
         if ((it & 0xff) == 0xff) {
             const long long now = clock64();
             if (start < 0) start = now;
-            else if (now - start > kWaitCycles) { atomicExch(status, (int)kDevTimeoutQuant); return false; }
+            else if (now - start > kWaitCycles) { report_status(status, kDevTimeoutQuant); return false; }
         }
         __nanosleep(64);
     }

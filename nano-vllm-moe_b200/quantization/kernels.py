@@ -39,9 +39,12 @@ def workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     shape up once (or call ``reserve_workspace`` with the largest size) ON THE STREAM THAT WILL
     CAPTURE, before the capture starts.  ``torch.cuda.graph`` captures on a side stream, so the
     warm-up belongs inside ``with torch.cuda.stream(side):`` too.  Graphs captured on the same
-    stream share one scratch buffer; replay them on one stream at a time."""
+    stream share one scratch buffer; replay them on one stream at a time.
+
+    Raises ``RuntimeError``, as every call that needs scratch does, when a kernel of an earlier call on this stream gave up
+    a bounded wait: that call's result is not valid."""
     index = device.index if device.index is not None else torch.cuda.current_device()
-    return _lib.host().workspace(index, _stream_ptr(device), nbytes)
+    return _lib.host().workspace(index, _stream_ptr(device), nbytes, False)
 
 
 def reserve_workspace(device: torch.device, nbytes: int) -> None:
@@ -80,7 +83,8 @@ def set_tuning(knob: str, value: int) -> None:
 
 def read_status(device: torch.device) -> int:
     """Blocking check of the device status word of the current stream's scratch."""
-    ws = workspace(device, _lib.WS_HEADER_BYTES)
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    ws = _lib.host().workspace(index, _stream_ptr(device), _lib.WS_HEADER_BYTES, True)
     out = ctypes.c_int(0)
     rc = _lib.load().fp8lin_read_status(ws.data_ptr(), _stream_ptr(device), ctypes.byref(out))
     _lib.raise_for(rc, "fp8lin_read_status")
