@@ -66,9 +66,11 @@ __host__ __device__ inline size_t pack_offset(int64_t n, int64_t k, int64_t KB) 
 // ---- programmatic dependent launch ------------------------------------------------
 // Every kernel lets the next kernel in the stream start launching early
 // (pdl_launch_dependents) and, before it touches memory a predecessor may still be
-// writing or reading (activations, outputs, scratch), waits for the predecessors to
-// finish (pdl_wait).  Weights are never written by a kernel, so their first loads are
-// issued before the wait.  Both are no-ops when the launch carries no such dependency.
+// writing or reading (activations, outputs, scratch, and scales or biases, which a
+// caller may have converted just before), waits for the predecessors to finish
+// (pdl_wait).  Only packed weights are read before the wait: they are packed once,
+// and who packs them waits until that is done before handing them out.
+// Both are no-ops when the launch carries no such dependency.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

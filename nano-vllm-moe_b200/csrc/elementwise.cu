@@ -12,16 +12,15 @@ __global__ void __launch_bounds__(256)
 act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* __restrict__ input_scale,
                  unsigned char* __restrict__ xq, int64_t M, int64_t K) {
     pdl_launch_dependents();       // the GEMM behind this pass may set up and prefetch its weights now
-    const ExactDiv s(fmaxf(__ldg(input_scale), 1e-12f));
     const int vec_per_row = (int)(K >> 4);
     const float inv_vpr = 1.0f / (float)vec_per_row;
     const int64_t total = M * vec_per_row;
-    pdl_wait();                    // x may come from the kernel before
-    for (int64_t base = (int64_t)blockIdx.x * 512; base < total; base += (int64_t)gridDim.x * 512) {
+    int64_t base = (int64_t)blockIdx.x * 512;
+    uint4 a[2][2];
+    unsigned char* dst[2];
+    auto load = [&]() {
         const int64_t row0 = base / vec_per_row;
         const int col0 = (int)(base - row0 * vec_per_row);
-        uint4 a[2][2];
-        unsigned char* dst[2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             // (offsets stay below 2^24 / 2: the product is off by less than half a row either way, the compare settles it)
@@ -38,6 +37,13 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
                 a[u][1] = __ldg(src + 1);
             }
         }
+    };
+    pdl_wait();                    // x may come from the kernel before, the scale too
+    if (base >= total) return;
+    const float scale = fmaxf(__ldg(input_scale), 1e-12f);
+    load();                        // (in flight beside the scale, which the first quotient needs)
+    const ExactDiv s(scale);
+    for (;;) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             if (dst[u]) {
@@ -45,6 +51,9 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
                 *reinterpret_cast<uint4*>(dst[u]) = make_uint4(qa.x, qa.y, qb.x, qb.y);
             }
         }
+        base += (int64_t)gridDim.x * 512;
+        if (base >= total) break;
+        load();
     }
 }
 

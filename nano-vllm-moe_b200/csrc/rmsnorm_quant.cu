@@ -29,30 +29,25 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     const int nvec = H >> 3;
     const bool quant = xq != nullptr;
     pdl_launch_dependents();
-    // A decode-sized call is one dependent chain: predecessor's end -> row -> sum of squares -> quantised row.  What no kernel
-    // writes (weight, scale) is fetched before the wait, all loads of the row are in flight together, and every thread adds
-    // the warps' partial sums itself (one barrier instead of two): 4.5 -> 2.7 us for one row of 3584 without the overlap of
-    // a dependent launch.
-    uint4 w[kNormMaxVec];
-#pragma unroll
-    for (int j = 0; j < kNormMaxVec; ++j) {
-        const int vec = threadIdx.x + j * kNormThreads;
-        if (vec < nvec) w[j] = __ldg(reinterpret_cast<const uint4*>(weight + vec * 8));
-    }
-    const ExactDiv div(quant ? fmaxf(__ldg(input_scale), 1e-12f) : 1.f);
-    pdl_wait();                                     // x and the residual come from the kernels before
+    // A decode-sized call is one dependent chain: predecessor's end -> row -> sum of squares -> quantised row.  All loads, of
+    // the row and of the operands it meets later, are in flight together, and every thread adds the warps' partial sums itself
+    // (one barrier instead of two).
+    pdl_wait();                                     // x and the residual come from the kernels before, perhaps a copy of the weight too
+    const float scale = quant ? fmaxf(__ldg(input_scale), 1e-12f) : 1.f;
     const int64_t row = blockIdx.x;
     const __nv_bfloat16* xr = x + row * ldx;
     __nv_bfloat16* rr = residual ? residual + row * ld_res : nullptr;
-    uint4 xa[kNormMaxVec], ra[kNormMaxVec];
+    uint4 xa[kNormMaxVec], ra[kNormMaxVec], w[kNormMaxVec];
 #pragma unroll
     for (int j = 0; j < kNormMaxVec; ++j) {
         const int vec = threadIdx.x + j * kNormThreads;
         if (vec < nvec) {
             xa[j] = __ldg(reinterpret_cast<const uint4*>(xr + vec * 8));
             if (rr) ra[j] = *reinterpret_cast<const uint4*>(rr + vec * 8);
+            w[j] = __ldg(reinterpret_cast<const uint4*>(weight + vec * 8));
         }
     }
+    const ExactDiv div(scale);
     float v[kNormMaxVec][8];
     float ss = 0.f;
 #pragma unroll

@@ -121,9 +121,8 @@ stream_linear_kernel(StreamArgs p) {
         cluster_arrive();                              // (waited for before the first remote access)
     }
 
-    float in_scale = 1.f;
-    if (SCHEME == FP8LIN_W8A8_STATIC) in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
-    const ExactDiv div_scale(in_scale);
+    float in_scale = 1.f;                              // (W8A8: read behind the wait below)
+    ExactDiv div_scale(1.f);
 
     float acc[MT][4];
 #pragma unroll
@@ -181,7 +180,11 @@ stream_linear_kernel(StreamArgs p) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) load_w_step(0, s);       // weights first: they do not depend on the predecessor
     pdl_launch_dependents();
-    pdl_wait();                                           // x, y and the split-K scratch may belong to the predecessor
+    pdl_wait();                                           // x, y and the split-K scratch may belong to the predecessor, scales and bias too
+    if (SCHEME == FP8LIN_W8A8_STATIC) {
+        in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
+        div_scale = ExactDiv(in_scale);
+    }
 #pragma unroll
     for (int part = 0; part < kParts; ++part) { load_x(0, part); store_x(0, part); }
     __syncthreads();

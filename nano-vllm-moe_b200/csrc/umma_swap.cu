@@ -172,9 +172,12 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const uint32_t tmem_base = s_tmem_base;
     pdl_launch_dependents();
     if (kSplit || kGateUp) cluster_arrive();                 // (waited for before the first remote access: the peers' barriers exist)
+    // Everything but the packed weights may come from the kernel in front -- the rows, but also a bias or a scale that the
+    // caller has just converted.  The producer warp waits by itself, between the weights and the rows.
+    if (warp != 0) pdl_wait();
     // scale and bias of the first channel this thread finishes, fetched long before they are needed
     float ws0 = 0.f, bs0 = 0.f, in_scale0 = 0.f;
-    if constexpr (kSplit) {
+    auto fetch_first = [&]() {
         in_scale0 = fmaxf(__ldg(p.input_scale), 1e-12f);
         if (band_rows > 0 && (int)threadIdx.x < band_rows * m_groups) {
             const int n0 = first_tile * kTileN + split_rank * band + (int)threadIdx.x % band_rows;
@@ -183,7 +186,8 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 if (p.bias) bs0 = __bfloat162float(p.bias[n0]);
             }
         }
-    }
+    };
+    if (kSplit && warp != 0) fetch_first();
 
     if (warp == 0) {
         // ================= TMA producer =================
@@ -209,6 +213,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 for (int i = 0; i < first_kb; ++i)
                     tma_load_2d(el, smem_base + i * Cfg::kStageBytes + kXDst, &tmap_x,
                                 (kb0 + i) * kKB, 0, smem_u32(&bar_full[i]));
+                if constexpr (kSplit) fetch_first();
             }
             for (int tl = 0; ok; ++tl) {
                 const int t = tile_of(tl);
@@ -308,7 +313,6 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
     } else {
         // ================= epilogue (warps 10..13) =================
-        pdl_wait();                                          // y may still be read by the predecessor
         const int q = warp & 3;
         const float in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
         bool ok = true;
@@ -440,7 +444,6 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             tc_fence_after();
             tmem_dealloc(tmem_base, Cfg::kTmemCols);
         }
-        pdl_wait();
         if ((int)threadIdx.x >= band_rows * m_groups) return;
         if (s_abort || !mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) return;
         const float in_scale = in_scale0;

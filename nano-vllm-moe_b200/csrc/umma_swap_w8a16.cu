@@ -153,9 +153,12 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const uint32_t tmem_a0 = tmem_base + Cfg::kAccCols;            // first widened-weight buffer
     pdl_launch_dependents();
     if (kSplit) cluster_arrive();                            // (waited for before the first remote access)
+    // Everything but the packed weights may come from the kernel in front -- the rows, but also a bias or a scale that the
+    // caller has just converted.  The producer warp waits by itself, between the weights and the rows.
+    if (warp != 0) pdl_wait();
     // scale and bias of the first channel this thread finishes, fetched long before they are needed
     float ws0 = 0.f, bs0 = 0.f;
-    if constexpr (kSplit) {
+    auto fetch_first = [&]() {
         if (band_rows > 0 && (int)threadIdx.x < band_rows * m_groups) {
             const int n0 = first_tile * kS16Tile + split_rank * band + (int)threadIdx.x % band_rows;
             if (n0 < p.N) {
@@ -163,7 +166,8 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 if (p.bias) bs0 = __bfloat162float(p.bias[n0]);
             }
         }
-    }
+    };
+    if (kSplit && warp != 0) fetch_first();
 
     if (warp == 0) {
         // ================= TMA producer =================
@@ -187,6 +191,7 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 for (int i = 0; i < first_kb; ++i)
                     tma_load_2d(el, smem_base + i * Cfg::kStageBytes + kXrawOff, &tmap_x, (kb0 + i) * kS16KB, 0,
                                 smem_u32(&bar_full[i]));
+                if constexpr (kSplit) fetch_first();
             }
             for (int t = first_tile; t < sched.n_tiles && ok; t += tile_step) {
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
@@ -292,7 +297,6 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
     } else {
         // ================= epilogue (warps 10..13) =================
-        pdl_wait();
         const int q = warp & 3;
         int tl = 0;
         bool ok = true;
@@ -346,7 +350,6 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             tc_fence_after();
             tmem_dealloc(tmem_base, Cfg::kTmemCols);
         }
-        pdl_wait();
         if ((int)threadIdx.x >= band_rows * m_groups) return;
         if (s_abort || !mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) return;
         for (int i = threadIdx.x; i < band_rows * m_groups; i += kS16Threads) {

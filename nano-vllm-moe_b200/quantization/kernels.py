@@ -95,7 +95,15 @@ def packed_bytes(k: int, n: int) -> int:
     return int(_lib.load().fp8lin_packed_bytes(k, n))
 
 
-def _pack(src: torch.Tensor, k: int, n: int, from_kn: bool) -> torch.Tensor:
+def weights_written(device: torch.device) -> None:
+    """Wait until packed weights that this stream has just written are complete (load time).  The linears read packed weights
+    before they wait for the kernel in front of them, so stream order alone does not protect them.  During a stream capture
+    there is nothing to wait for: the packing runs when the graph does, and that replay has to end first."""
+    if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
+        torch.cuda.current_stream(device).synchronize()
+
+
+def _pack(src: torch.Tensor, k: int, n: int, from_kn: bool, wait: bool = True) -> torch.Tensor:
     _require_cuda(src)
     if src.dtype not in (torch.uint8, torch.float8_e4m3fn) or src.dim() != 2:
         raise ValueError("weight codes must be a 2-D uint8/float8_e4m3fn tensor")
@@ -105,6 +113,8 @@ def _pack(src: torch.Tensor, k: int, n: int, from_kn: bool) -> torch.Tensor:
     with torch.cuda.device(src.device):
         rc = fn(src.data_ptr(), out.data_ptr(), k, n, _stream_ptr(src.device))
     _lib.raise_for(rc, "fp8lin_prepack_weight" if from_kn else "fp8lin_pack_weight_nk")
+    if wait:
+        weights_written(src.device)
     return out
 
 
@@ -114,10 +124,11 @@ def prepack_weight(qweight_kn: torch.Tensor) -> torch.Tensor:
     return _pack(qweight_kn, k, n, True)
 
 
-def pack_weight_nk(qweight_nk: torch.Tensor) -> torch.Tensor:
-    """e4m3 codes [N, K] (the checkpoint layout) -> the kernels' packed tile layout."""
+def pack_weight_nk(qweight_nk: torch.Tensor, wait: bool = True) -> torch.Tensor:
+    """e4m3 codes [N, K] (the checkpoint layout) -> the kernels' packed tile layout.  ``wait=False``: the caller sees to
+    ``weights_written`` (after packing several)."""
     n, k = qweight_nk.shape
-    return _pack(qweight_nk, k, n, False)
+    return _pack(qweight_nk, k, n, False, wait)
 
 
 def _check_linear_args(x, w_packed, weight_scale, bias):
@@ -268,6 +279,7 @@ def interleave_gate_up(w_packed: torch.Tensor, weight_scale: torch.Tensor, bias:
     w = w_packed.view(2, t, -1).transpose(0, 1).contiguous().view(-1)
     s = weight_scale.view(2, t, 128).transpose(0, 1).contiguous().view(-1)
     b = bias.view(2, t, 128).transpose(0, 1).contiguous().view(-1) if bias is not None else None
+    weights_written(w.device)
     return w, s, b
 
 

@@ -40,3 +40,19 @@ def test_named_barriers_do_not_ask_for_a_converged_warp():
             assert len(asm) == 2 and not any("bar.sync" in a or ".aligned" in a for a in asm), asm
         else:
             assert not asm, f"{name}: {asm}"
+
+
+def test_only_packed_weights_are_read_before_the_wait_for_the_kernel_in_front():
+    """A bias or a norm's weight may be a copy that the caller's last kernel wrote; only griddepcontrol.wait orders it."""
+    early = re.compile(r"\b(bias|weight|w_scale|input_scale|h_scale|topk_w|residual)\b")
+    kernels = 0
+    for name, text in SOURCES.items():
+        for head in re.finditer(r"__global__[^{;]*?\b(\w+_kernel)\(", text):
+            code = body(text[head.start():], head.group(1)) if f" {head.group(1)}(" in text[head.start():] else \
+                body(" " + text[head.start():].replace("\n" + head.group(1) + "(", "\n " + head.group(1) + "(", 1), head.group(1))
+            if "pdl_wait()" not in code:
+                continue
+            kernels += 1
+            found = early.findall(code[:code.index("pdl_wait()")])
+            assert not found, f"{name}: {head.group(1)} reads {found} too early"
+    assert kernels > 15
