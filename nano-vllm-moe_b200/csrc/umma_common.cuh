@@ -22,15 +22,22 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n}" ::"r"(bar), "r"(bytes)
                  : "memory");
 }
-// Bounded wait; false = gave up after `limit` clock cycles (status word written).
+// Bounded wait; false = gave up after `limit` clock cycles (status word written).  kTensorMemory: for a barrier that CTAs of
+// the cluster arrive on with mbar_arrive_remote; a tcgen05 fence follows.
+template <bool kTensorMemory = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status, int code,
                                           long long limit = kWaitCycles) {
     long long start = -1;
     for (uint32_t it = 0;; ++it) {
         uint32_t done;
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-            : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        if constexpr (kTensorMemory)
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+        else
+            asm volatile(
+                "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                : "=r"(done) : "r"(bar), "r"(parity) : "memory");
         if (done) return true;
         if ((it & 0x3ff) == 0x3ff) {
             const long long now = clock64();
@@ -146,11 +153,12 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {     // bar: 
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// Arrive on another CTA's barrier without a cluster-scope release: for what is in tensor memory, ordered by
-// tcgen05.wait and the tcgen05 fence.  (A release at cluster scope waits until the warp's earlier stores have reached L2:
-// over a thousand cycles behind an epilogue's stores.)
+// Arrive on a barrier of any CTA of the cluster to hand over tensor memory and nothing else: the tcgen05 accesses are ordered
+// by tcgen05.wait and the tcgen05 fences on both sides of the barrier, which take the execution order that a relaxed arrival
+// and a relaxed wait at cluster scope give; no other memory is released.  (A release at cluster scope waits until the warp's
+// earlier stores have reached L2: over a thousand cycles behind an epilogue's stores.)
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
 // 32 lanes x 32 columns of fp32 from TMEM (lane i of the warp reads TMEM lane base+i); no wait.

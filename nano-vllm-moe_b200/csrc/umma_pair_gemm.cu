@@ -171,7 +171,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             for (int t = first_tile; t < sched.total && ok; t += tile_step, ++tl) {
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
-                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait<true>(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
                 if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * kBN;
@@ -285,11 +285,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    const uint32_t te = smem_u32(&bar_tempty[as]);
-                    if (leader) mbar_arrive(te);
-                    else mbar_arrive_remote(map_to_cta(te, 0));
-                }
+                if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[as]), 0));
                 continue;
             }
             const uint32_t t_pair = tmem_base + ((uint32_t)(q * 32) << 16) + as * kBN + h * 32;
@@ -326,11 +322,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
-                const uint32_t te = smem_u32(&bar_tempty[as]);
-                if (leader) mbar_arrive(te);
-                else mbar_arrive_remote(map_to_cta(te, 0));
-            }
+            if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[as]), 0));
         }
         if (lane == 0) tma_store_wait_all();
     }

@@ -237,13 +237,13 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             for (int item = first_item; item < items && ok; item += item_step, ++tl) {
                 const int as = acc_stages == 2 ? (tl & 1) : 0;
                 const uint32_t aph = acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1);
-                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait<true>(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
                 if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + as * T;
                 for (int kb = kb0; kb < kb1; ++kb) {
                     ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_xfull[xslot]), xphase, p.status, kDevTimeoutFull) &&
-                                                     mbar_wait(smem_u32(&bar_conv[aslot]), aphase, p.status, kDevTimeoutFull));
+                                                     mbar_wait<true>(smem_u32(&bar_conv[aslot]), aphase, p.status, kDevTimeoutFull));
                     if (!ok) { s_abort = 1; break; }
                     tc_fence_after();
                     const uint32_t xs = smem_base + xslot * x_bytes;

@@ -197,7 +197,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                 const uint32_t idesc = make_idesc_mn(2 * kTile, 2 * it.half, 0, 0);          // e4m3 x e4m3
                 const int as = acc_stages == 2 ? (tl & 1) : 0;
                 const uint32_t aph = acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1);
-                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
+                ok = __all_sync(0xffffffffu, !s_abort && mbar_wait<true>(smem_u32(&bar_tempty[as]), aph ^ 1, p.status, kDevTimeoutTmemEmpty));
                 if (!ok) { s_abort = 1; break; }
                 tc_fence_after();
                 uint32_t d_tmem = tmem_base + as * acc_cols;

@@ -56,3 +56,17 @@ def test_only_packed_weights_are_read_before_the_wait_for_the_kernel_in_front():
             found = early.findall(code[:code.index("pdl_wait()")])
             assert not found, f"{name}: {head.group(1)} reads {found} too early"
     assert kernels > 15
+
+
+def test_tensor_memory_is_handed_over_at_cluster_scope():
+    """A barrier that another CTA arrives on is named at cluster scope on both sides: the arrival and the wait."""
+    common = SOURCES["umma_common.cuh"]
+    assert "mbarrier.arrive.relaxed.cluster.shared::cluster" in body(common, "mbar_arrive_remote")
+    assert "mbarrier.try_wait.parity.relaxed.cluster.shared::cta" in body(common, "mbar_wait")
+    for name in ("umma_pair_gemm.cu", "umma_w8a8_pair.cu", "umma_w8a16_pair.cu"):
+        remote = set(re.findall(r"(bar_\w+)\[", " ".join(re.findall(r"mbar_arrive_remote\([^;]*;", SOURCES[name]))))
+        remote |= {"bar_conv"} if "conv0" in SOURCES[name] else set()
+        assert "bar_tempty" in remote, name
+        for bar in remote:
+            waits = re.findall(r"(mbar_wait(?:<true>)?)\(smem_u32\(&" + bar, SOURCES[name])
+            assert waits and set(waits) == {"mbar_wait<true>"}, (name, bar, waits)
