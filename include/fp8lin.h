@@ -293,13 +293,19 @@ int fp8lin_mlp_w8a8_preq(const void* xq, const void* w_gate_up, const float* gat
                          const float* down_scale, const float* down_input_scale, const void* down_bias, void* y, int64_t ldy,
                          int64_t M, int64_t H, int64_t I, int64_t N, void* workspace, size_t workspace_bytes, void* stream);
 
-/* Which kernel variant a shape is routed to ("stream_mma_w8a8_m16", "umma_w8a8_128x256", ...),
- * for labelling bench rows and ncu captures.  Host-only, returns a static string. */
+/* The route of a shape by its tile counts alone ("stream_mma_w8a8_m16", "umma_w8a8_128x256", ...): what calls run that the
+ * CTA-pair kernels with channels as the MMA's M do not take -- several destinations, N or ldy not a multiple of 8, y not
+ * 16-byte aligned.  Not what most other calls of 17 rows and more run: see fp8lin_kernel_name.  Host-only, static string. */
 const char* fp8lin_variant_name(int scheme, int64_t M, int64_t K, int64_t N);
-/* The kernel that a call with 16-byte aligned y (ldy a multiple of 8) and one destination runs.  fp8lin_variant_name names
- * the route by tile counts alone, which is what the multi-destination calls and calls of other alignments take; this differs
- * for W8A16 from 65 rows on (the CTA-pair kernel that widens the weights into tensor memory, "umma_w8a16_pair_256x224_s3")
- * and for large W8A8 calls whose rounds of tiles a model of their length gives to the other kernel.  Host-only, static string. */
+/* The kernel that a call with 16-byte aligned y (N and ldy multiples of 8) and one destination runs; for labelling
+ * measurements.  It differs from fp8lin_variant_name
+ *   W8A16, 65 rows and more, and from 33 on where the decode kernel would not split K: the CTA-pair kernel that widens the
+ *     weights into tensor memory ("umma_w8a16_pair_256x224_s3");
+ *   W8A8, 17 to 4096 rows, wherever it is modelled faster than the others: the CTA-pair kernel with the rows as the MMA's N
+ *     ("umma_w8a8_pair_256x64_s4_cluster"; the same K slices and the same bits as the route it stands in for);
+ *   W8A8, more than 64 rows otherwise: 256 x 256 tiles or 128-row tiles by a model of their rounds, where the route's name
+ *     goes by how full the rounds are.
+ * Host-only, static string. */
 const char* fp8lin_kernel_name(int scheme, int64_t M, int64_t K, int64_t N);
 
 /* Bench/ncu studies only: force a tuning knob (value < 0 restores the default).  Not thread safe.

@@ -69,11 +69,12 @@ def launch_count() -> int:
 
 
 def variant_name(scheme: int, m: int, k: int, n: int) -> str:
+    """The route of a shape by its tile counts alone (calls with several destinations or an unaligned output)."""
     return _lib.load().fp8lin_variant_name(scheme, m, k, n).decode()
 
 
 def kernel_name(scheme: int, m: int, k: int, n: int) -> str:
-    """The kernel an aligned call of this shape runs (``variant_name`` names the route behind it)."""
+    """The kernel that a call of this shape runs (one destination, aligned output)."""
     return _lib.load().fp8lin_kernel_name(scheme, m, k, n).decode()
 
 

@@ -82,34 +82,37 @@ def run(scheme, d):
     return Kn.launch_w8a8_gemm(d["x"], d["w_nk"], d["input_scale"], d["w_scale"], d["bias"])
 
 
-# (M, K, N, forced umma_pair or None, substring expected in the variant name)
+# (M, K, N, 0 = 128-row tiles / 1 = 256-row tiles on CTA pairs, substring expected in the kernel's name)
 PREFILL = [
-    (4096, 18944, 3584, None, "+tail"),            # persistent launch + cluster split-K tail launch
-    (2048, 8192, 2560, None, "+tail"),             # the same route on a small problem
-    (16384, 18944, 3584, None, "+tail"),
-    (16384, 3584, 3584, None, "+half"),
+    (4096, 18944, 3584, 0, "+tail"),               # persistent launch + cluster split-K tail launch
+    (2048, 8192, 2560, 0, "+tail"),                # the same route on a small problem
+    (16384, 18944, 3584, 0, "+tail"),
+    (16384, 3584, 3584, 0, "+half"),
     (32640, 3584, 4608, 0, "umma_w8a8"),           # ragged M (32640 = 255 x 128), one-CTA kernel
     (32640, 3584, 4608, 1, "umma_pair"),           # ragged M on CTA pairs: the last pair has one live CTA row block
-    (4096, 3584, 37888, None, "umma_pair"),        # gate_up on CTA pairs (148 column tiles)
-    (32640, 18944, 3584, None, "umma_pair"),
-    (16384, 3584, 576, None, "umma_w8a8_128x256"), # qkv and gate_up column shards of 8 ranks (N = 4.5 and 37 tiles of 128)
-    (16384, 3584, 4736, None, "umma_pair"),
-    (16384, 2368, 3584, None, "+half"),            # down's K shard of 8 ranks: 18.5 K blocks
+    (4096, 3584, 37888, 1, "umma_pair"),           # gate_up on CTA pairs (148 column tiles)
+    (32640, 18944, 3584, 1, "umma_pair"),
+    (16384, 3584, 576, 0, "umma_w8a8_128x256"),    # qkv and gate_up column shards of 8 ranks (N = 4.5 and 37 tiles of 128)
+    (16384, 3584, 4736, 1, "umma_pair"),
+    (16384, 2368, 3584, 0, "+half"),               # down's K shard of 8 ranks: 18.5 K blocks
 ]
 
 
 @pytest.mark.parametrize("m,k,n,pair,expect", PREFILL)
 def test_prefill_shapes_sampled(m, k, n, pair, expect):
     Kn = kernels()
-    if pair is not None:
-        Kn.set_tuning("umma_pair", pair)
-    name = Kn.variant_name(1, m, k, n)
-    assert expect in name, name
+    chosen = Kn.kernel_name(1, m, k, n)
     d = big_case(m + k + n, m, k, n)
+    by_default = run("fp8_w8a8_static", d)
+    Kn.set_tuning("umma_pair", pair)
+    name = Kn.kernel_name(1, m, k, n)
+    assert expect in name, name
     y = run("fp8_w8a8_static", d)              # default: a separate pass quantises the activations
     rng = np.random.default_rng(m + n)
     rows, cols = sample(m, 48, rng), sample(n, 160, rng)
     check_sampled("fp8_w8a8_static", d, y, rows, cols, f"{name} {m}x{k}x{n}")
+    if chosen != name:                         # (a call of this shape runs the other kernel)
+        check_sampled("fp8_w8a8_static", d, by_default, rows, cols, f"{chosen} {m}x{k}x{n}")
     # every row block and column block is written: no element keeps the fill value
     assert torch.isfinite(y.float()).all()
     assert torch.equal(y, run("fp8_w8a8_static", d))
@@ -152,7 +155,7 @@ def test_decode_sweep_all_layers(scheme, layer):
     for m in (1, 4, 16, 64):
         d["x"] = full_x[:m].contiguous()
         y = run(scheme, d)
-        name = kernels().variant_name(0 if scheme == "fp8_w8a16" else 1, m, k, n)
+        name = kernels().kernel_name(0 if scheme == "fp8_w8a16" else 1, m, k, n)
         check_sampled(scheme, d, y, np.arange(m), cols, f"{scheme} {layer} M={m} [{name}]")
         assert torch.isfinite(y.float()).all()
 

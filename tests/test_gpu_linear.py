@@ -23,7 +23,7 @@ def _clean_tuning_and_status():
     Kn = kernels()
     yield
     for knob in ("stream_splits", "stream_max_m", "umma_bn", "umma_splits", "swap_splits", "swap_enable", "swap_min_m", "swap_preq_min_m", "w8a16_swap_enable",
-                 "w8a16_swap_min_m", "w8a16_umma_min_m", "w8a16_chunk_mb", "umma_pair"):
+                 "w8a16_swap_min_m", "w8a16_umma_min_m", "w8a16_chunk_mb", "umma_pair", "w8a16_pair"):
         Kn.set_tuning(knob, -1)
     torch.cuda.synchronize()
     assert Kn.read_status(torch.device("cuda", 0)) == 0
@@ -138,13 +138,13 @@ def test_streaming_kernel_parity(scheme, m, k, n):
         kernels().set_tuning("swap_enable", 0)
         kernels().set_tuning("w8a16_swap_enable", 0)
         scheme = scheme.split("/")[0]
-        assert kernels().variant_name(1 if "a8" in scheme[-10:] else 0, m, k, n).startswith("stream_mma_")
+        assert kernels().kernel_name(1 if "a8" in scheme[-10:] else 0, m, k, n).startswith("stream_mma_")
     elif scheme == "fp8_w8a16":
         kernels().set_tuning("w8a16_swap_min_m", 1)  # by default M <= 8 stays on the mma.sync kernel
-        assert kernels().variant_name(0, m, k, n).startswith("umma_swap_w8a16")
+        assert kernels().kernel_name(0, m, k, n).startswith("umma_swap_w8a16")
     elif scheme == "fp8_w8a8_static":
         kernels().set_tuning("swap_min_m", 1)        # by default M <= 8 goes to the mma.sync kernel
-        assert kernels().variant_name(1, m, k, n).startswith("umma_swap_w8a8")
+        assert kernels().kernel_name(1, m, k, n).startswith("umma_swap_w8a8")
     c = O.make_case(20260519 + m * 7 + k + n, m, k, n)
     d = upload_case(c)
     y = run_linear(scheme, d)
@@ -164,7 +164,7 @@ def test_swapped_w8a16_kernel_split_variants(m, splits):
     Kn.set_tuning("swap_splits", splits)
     c = O.make_case(1900 + m + splits, m, 2048, 640)
     d = upload_case(c)
-    assert Kn.variant_name(0, m, 2048, 640).startswith("umma_swap_w8a16")
+    assert Kn.kernel_name(0, m, 2048, 640).startswith("umma_swap_w8a16")
     y1 = run_linear("fp8_w8a16", d)
     y2 = run_linear("fp8_w8a16", d)
     np.testing.assert_array_equal(y1, y2)
@@ -231,13 +231,19 @@ UMMA_SHAPES = [
 
 @pytest.mark.parametrize("m,k,n", UMMA_SHAPES)
 def test_tcgen05_gemm_parity(m, k, n):
+    """The one-CTA GEMM, and whichever kernel takes the call by default."""
+    Kn = kernels()
     c = O.make_case(4242 + m + k + n, m, k, n)
     d = upload_case(c)
-    assert kernels().variant_name(1, m, k, n).startswith("umma_w8a8")
+    ref = oracle_linear("fp8_w8a8_static", c)
+    by_default = run_linear("fp8_w8a8_static", d)
+    assert_parity(by_default, ref, f"{Kn.kernel_name(1, m, k, n)} {m}x{k}x{n}")
+    np.testing.assert_array_equal(by_default, run_linear("fp8_w8a8_static", d))
+    Kn.set_tuning("umma_pair", 0)
+    assert Kn.kernel_name(1, m, k, n).startswith("umma_w8a8_128x")
     y = run_linear("fp8_w8a8_static", d)
-    assert_parity(y, oracle_linear("fp8_w8a8_static", c), f"umma {m}x{k}x{n}")
-    y2 = run_linear("fp8_w8a8_static", d)
-    np.testing.assert_array_equal(y, y2)
+    assert_parity(y, ref, f"umma {m}x{k}x{n}")
+    np.testing.assert_array_equal(y, run_linear("fp8_w8a8_static", d))
 
 
 @pytest.mark.parametrize("m,k,n", [(1280, 256, 4000), (1024, 2048, 11008), (2500, 144, 2056)])
@@ -247,7 +253,8 @@ def test_tcgen05_half_width_tail_items(m, k, n):
     Kn = kernels()
     c = O.make_case(808 + m + n, m, k, n)
     d = upload_case(c)
-    assert "+half" in Kn.variant_name(1, m, k, n)
+    Kn.set_tuning("umma_pair", 0)
+    assert "+half" in Kn.kernel_name(1, m, k, n)
     y = run_linear("fp8_w8a8_static", d)
     assert_parity(y, oracle_linear("fp8_w8a8_static", c), f"umma half-width tail {m}x{k}x{n}")
     Kn.set_tuning("umma_bn", 128)                       # same arithmetic on whole 128-wide tiles
@@ -264,9 +271,10 @@ def test_tcgen05_cta_pair_gemm_parity(m, k, n):
     Kn = kernels()
     c = O.make_case(6060 + m + k + n, m, k, n)
     d = upload_case(c)
+    Kn.set_tuning("umma_pair", 0)
     y1 = run_linear("fp8_w8a8_static", d)
     Kn.set_tuning("umma_pair", 1)
-    assert Kn.variant_name(1, m, k, n).startswith("umma_pair_w8a8")
+    assert Kn.kernel_name(1, m, k, n).startswith("umma_pair_w8a8")
     y = run_linear("fp8_w8a8_static", d)
     assert_parity(y, oracle_linear("fp8_w8a8_static", c), f"cta pair {m}x{k}x{n}")
     np.testing.assert_array_equal(y, run_linear("fp8_w8a8_static", d))
@@ -318,7 +326,7 @@ def test_swapped_kernel_with_and_without_prequantised_rows(m, preq_min):
     c = O.make_case(4000 + m, m, 1408, 1000)
     d = upload_case(c)
     y = run_linear("fp8_w8a8_static", d)
-    assert ("_preq" in Kn.variant_name(1, m, 1408, 1000)) == (m >= preq_min)
+    assert ("_preq" in Kn.kernel_name(1, m, 1408, 1000)) == (m >= preq_min)
     assert_parity(y, oracle_linear("fp8_w8a8_static", c), f"swap preq_min={preq_min} m={m}")
     Kn.set_tuning("swap_preq_min_m", 65 if preq_min == 1 else 1)
     np.testing.assert_array_equal(y, run_linear("fp8_w8a8_static", d))
@@ -329,19 +337,21 @@ W8A16_UMMA_SHAPES = [(129, 448, 576), (256, 3584, 4608), (300, 2368, 1000), (513
 
 @pytest.mark.parametrize("m,k,n", W8A16_UMMA_SHAPES)
 def test_w8a16_large_m_f16_gemm_parity(m, k, n):
-    """Large M (by default from 256 rows): weights widened to f16 chunk by chunk, tcgen05 f16 GEMM; against the oracle and the
-    mma.sync passes (same operand values, so only the accumulation order differs)."""
+    """Large M without the CTA-pair kernel (calls whose output it does not take): from 256 rows weights widened to f16 chunk by
+    chunk, tcgen05 f16 GEMM; against the oracle and the mma.sync passes (same operand values, so only the accumulation order
+    differs)."""
     Kn = kernels()
     c = O.make_case(5150 + m + k + n, m, k, n)
     d = upload_case(c)
-    assert Kn.variant_name(0, m, k, n).startswith("umma_w8a16_f16") == (m >= 256)     # default threshold
+    Kn.set_tuning("w8a16_pair", 0)
+    assert Kn.kernel_name(0, m, k, n).startswith("umma_w8a16_f16") == (m >= 256)      # default threshold
     Kn.set_tuning("w8a16_umma_min_m", 1)
-    assert Kn.variant_name(0, m, k, n).startswith("umma_w8a16_f16")
+    assert Kn.kernel_name(0, m, k, n).startswith("umma_w8a16_f16")
     y = run_linear("fp8_w8a16", d)
     assert_parity(y, oracle_linear("fp8_w8a16", c), f"w8a16 f16 gemm {m}x{k}x{n}")
     np.testing.assert_array_equal(y, run_linear("fp8_w8a16", d))
     Kn.set_tuning("w8a16_umma_min_m", 0)
-    assert Kn.variant_name(0, m, k, n).startswith("stream_mma_w8a16")
+    assert Kn.kernel_name(0, m, k, n).startswith("stream_mma_w8a16")
     assert_parity(y, run_linear("fp8_w8a16", d), "f16 gemm vs mma.sync passes")
 
 
@@ -356,7 +366,7 @@ def test_w8a16_large_m_chunks_and_tiles(chunk_mb, bn, splits):
     m, k, n = 260, 1408, 1928
     c = O.make_case(77 + chunk_mb + bn, m, k, n)
     d = upload_case(c)
-    name = Kn.variant_name(0, m, k, n)
+    name = Kn.kernel_name(0, m, k, n)
     assert name.startswith("umma_w8a16_f16") and not name.endswith("_c1")
     y = run_linear("fp8_w8a16", d)
     assert_parity(y, oracle_linear("fp8_w8a16", c), f"w8a16 chunks {name}")
@@ -428,12 +438,15 @@ def test_layer_end_to_end(pkg, scheme):
 
 
 CANARY_SHAPES = [
-    # (scheme, M, K, N): one shape per kernel route, with ragged M and N where the route allows them
+    # (scheme[/kernel], M, K, N): shapes of every kernel, with ragged M and N where it allows them; /pair: 256 x 256 tiles,
+    # /one_cta: the one-CTA GEMM, /f16 and /passes: W8A16 without its CTA-pair kernel
     ("fp8_w8a16", 3, 448, 576), ("fp8_w8a16", 40, 704, 72), ("fp8_w8a16", 150, 512, 264), ("fp8_w8a16", 300, 2368, 1000),
     ("fp8_w8a8_static", 1, 2048, 2048), ("fp8_w8a8_static", 7, 16, 24), ("fp8_w8a8_static", 12, 1408, 1000),
     ("fp8_w8a8_static", 33, 2368, 1000), ("fp8_w8a8_static", 64, 3584, 3584), ("fp8_w8a8_static", 130, 448, 576),
     ("fp8_w8a8_static", 300, 2368, 1000), ("fp8_w8a8_static", 1280, 256, 4000), ("fp8_w8a8_static", 2048, 8192, 2560),
     ("fp8_w8a8_static/pair", 300, 2368, 1000), ("fp8_w8a8_static/pair", 1025, 448, 520),
+    ("fp8_w8a8_static/one_cta", 130, 448, 576), ("fp8_w8a8_static/one_cta", 300, 2368, 1000), ("fp8_w8a8_static/one_cta", 1280, 256, 4000),
+    ("fp8_w8a16/passes", 150, 512, 264), ("fp8_w8a16/f16", 300, 2368, 1000),
 ]
 
 
@@ -443,9 +456,11 @@ def test_no_kernel_writes_outside_its_output_matrix(scheme, m, k, n):
     its right (row pitch > N) must come back untouched, whatever tails the tiles have (TMA stores clip at the tensor
     map's extent, the other epilogues predicate).  Stands in for a memory checker on the store side."""
     Kn = kernels()
-    if scheme.endswith("/pair"):
-        Kn.set_tuning("umma_pair", 1)
-        scheme = scheme.split("/")[0]
+    scheme, _, forced = scheme.partition("/")
+    if forced:
+        Kn.set_tuning("w8a16_pair" if scheme == "fp8_w8a16" else "umma_pair", 1 if forced == "pair" else 0)
+        assert Kn.kernel_name(0 if scheme == "fp8_w8a16" else 1, m, k, n).startswith(
+            {"pair": "umma_pair_w8a8", "one_cta": "umma_w8a8_128x", "f16": "umma_w8a16_f16", "passes": "stream_mma_w8a16"}[forced])
     c = O.make_case(777 + m + n, m, k, n, calib_rows=64)
     d = upload_case(c)
     pitch = (n + 8 + 7) // 8 * 8 + 8                       # a multiple of 8, at least 8 spare columns
