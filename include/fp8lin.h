@@ -341,6 +341,10 @@ int fp8lin_read_status(void* workspace, void* stream, int* status_out);
  * `workspace` and returns normally; the next fp8lin_read_status reports FP8LIN_ERR_DEVICE and clears it. */
 int fp8lin_debug_wait_timeout(void* workspace, int64_t limit_us, void* stream);
 
+/* For tests: fast[i] = silu(g[i]) as the activation epilogues compute it (a refined reciprocal), divided[i] the same by a
+ * division, both fp32, for n bf16 values g. */
+int fp8lin_debug_silu(const void* g, float* fast, float* divided, int64_t n, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

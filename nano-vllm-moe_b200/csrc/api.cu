@@ -1195,6 +1195,16 @@ int fp8lin_debug_wait_timeout(void* workspace, int64_t limit_us, void* stream) {
     return FP8LIN_OK;
 }
 
+int fp8lin_debug_silu(const void* g, float* fast, float* divided, int64_t n, void* stream) {
+    if (n < 0 || n > (1ll << 30)) return fail(FP8LIN_ERR_SHAPE, "n must be 0..2^30");
+    if (n == 0) return FP8LIN_OK;
+    if (!g || !fast || !divided) return fail(FP8LIN_ERR_NULL, "g, fast and divided must not be NULL");
+    if (!check_arch()) return fail(FP8LIN_ERR_ARCH, "fp8lin kernels are built for sm_100a only");
+    cudaError_t e = launch_silu_probe((const __nv_bfloat16*)g, fast, divided, n, (cudaStream_t)stream);
+    if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "probe launch: %s", cudaGetErrorString(e));
+    return FP8LIN_OK;
+}
+
 int fp8lin_read_status(void* workspace, void* stream, int* status_out) {
     if (!workspace || !status_out) return fail(FP8LIN_ERR_NULL, "workspace and status_out must not be NULL");
     cudaStream_t st = (cudaStream_t)stream;

@@ -392,4 +392,18 @@ cudaError_t launch_pack_tiles(const unsigned char* src, unsigned char* dst, int6
     return counted(cudaGetLastError());
 }
 
+// silu_f32 beside the division it stands for, for a test over every bf16 value.
+__global__ void silu_probe_kernel(const __nv_bfloat16* __restrict__ g, float* __restrict__ fast, float* __restrict__ divided, int64_t n) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const float v = __bfloat162float(g[i]);
+    fast[i] = silu_f32(v);
+    divided[i] = __fdiv_rn(v, 1.f + expf(-v));
+}
+
+cudaError_t launch_silu_probe(const __nv_bfloat16* g, float* fast, float* divided, int64_t n, cudaStream_t stream) {
+    silu_probe_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(g, fast, divided, n);
+    return counted(cudaGetLastError());
+}
+
 }  // namespace fp8lin

@@ -150,6 +150,9 @@ cudaError_t launch_sum_slots(const __nv_bfloat16* slots, int n_slots, int64_t sl
 // `limit_cycles`, writes kDevTimeoutFull to *status (and 1 to *gave_up if given) and returns.
 cudaError_t launch_wait_timeout_probe(int* status, long long limit_cycles, int* gave_up, cudaStream_t stream);
 
+// fast[i] = silu_f32(g[i]) as every activation epilogue and pass computes it, divided[i] = g[i] / (1 + e^-g[i])
+cudaError_t launch_silu_probe(const __nv_bfloat16* g, float* fast, float* divided, int64_t n, cudaStream_t stream);
+
 // The same sum written to several destinations (this rank's band of a row-parallel result stored into every rank's
 // output matrix by plain stores; peers over NVLink).
 struct SumDst {

@@ -96,3 +96,19 @@ def test_fused_activation_equals_the_separate_pass(counts, H, I):
     finally:
         Kn.set_tuning("moe_fused", -1)
     assert Kn.read_status(torch.device("cuda", 0)) == 0
+
+
+def test_silu_equals_the_division_for_every_bf16_value(pkg):
+    """The epilogues refine an approximate reciprocal instead of dividing; no value may differ, also not in the sign of a zero."""
+    L = pkg._lib
+    g = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).cuda()
+    fast, divided = torch.empty(65536, device="cuda"), torch.empty(65536, device="cuda")
+    L.raise_for(L.load().fp8lin_debug_silu(g.data_ptr(), fast.data_ptr(), divided.data_ptr(), g.numel(),
+                                           torch.cuda.current_stream().cuda_stream), "fp8lin_debug_silu")
+    nan = divided.isnan()
+    assert torch.equal(nan, fast.isnan())
+    assert torch.equal(fast[~nan].view(torch.int32), divided[~nan].view(torch.int32))
+    x = g.double()
+    want = x / (1 + torch.exp(-x))
+    ok = torch.isfinite(want) & (want.abs() > 1e-30)
+    assert ((divided.double() - want).abs() <= 4e-7 * want.abs())[ok].all()              # 3 ulps: expf, the sum, the quotient
