@@ -1020,7 +1020,7 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
     w.off_chunks = take((size_t)(E + rows / 16 + 2) * 16);
     w.off_meta = take(16);
     w.off_inv = take((size_t)(rows > 0 ? rows : 1) * 4);
-    w.off_gu = take((size_t)rows * 2 * I * 2);
+    w.off_gu = take(g_tune.moe_fused == 0 ? (size_t)rows * 2 * I * 2 : 0);      // bf16 gate_up rows: only the separate pass reads them
     w.off_hq = take((size_t)rows * I);
     w.off_xq = take(rows >= kMoePrequantRows ? (size_t)rows * H : 0);
     w.total = o;

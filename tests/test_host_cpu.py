@@ -201,6 +201,22 @@ def test_routing_of_large_shapes(pkg):
     assert small >= L.WS_HEADER_BYTES + 16 * 18944 * 5
 
 
+def test_expert_scratch_holds_what_the_route_writes(pkg):
+    """Grouping tables, e4m3 rows in expert order and e4m3 activations; bf16 gate_up rows only for the separate activation pass."""
+    lib = pkg._lib.load()
+    rows, e, h, i = 16384, 60, 2048, 1408
+    need = lib.fp8lin_moe_workspace_bytes(rows, e, h, i)
+    used = rows * (h + i) + rows * 4 * 2 + (e + 1) * 4 + (e + rows // 16 + 2) * 16
+    assert used <= need - pkg._lib.WS_HEADER_BYTES <= used + 8 * 256
+    try:
+        assert lib.fp8lin_set_tuning(b"moe_fused", 0) == 0
+        assert lib.fp8lin_moe_workspace_bytes(rows, e, h, i) >= need + rows * 4 * i
+    finally:
+        lib.fp8lin_set_tuning(b"moe_fused", -1)
+    block = lib.fp8lin_moe_block_workspace_bytes(rows // 4, 4, e, h, i)
+    assert block == need + rows * h * 2                              # + the routed rows that the combine reads
+
+
 def test_gate_up_interleave_is_a_tile_row_permutation():
     """interleave_gate_up(pack(W)) == pack(W with its 128-row blocks alternating gate / up)."""
     from importlib import import_module
