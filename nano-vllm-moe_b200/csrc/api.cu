@@ -264,11 +264,10 @@ bool swap_prequant(int64_t M) {
 // times K blocks, a cluster's hand-over or a last round cut in two where the plan has them; large calls of the CTA-pair GEMM
 // are bound by power (0.385 us per pair tile and K block).  Fitted to the same row counts and shapes as that plan.
 double umma_cost(const UmmaPlan& pl, int64_t K, int64_t N) {
-    static const int max_clusters[9] = {148, 148, 74, 45, 33, 26, 22, 15, 15};
     const double kblocks = (double)pack_kblocks(K), block = pl.bn == 256 ? 0.45 : (pl.bn == 128 ? 0.254 : 0.185);
     const int64_t tiles = (int64_t)pl.m_tiles * pl.n_tiles, sms = sm_count();
     if (pl.splits > 1) {
-        const int64_t waves = (tiles + max_clusters[pl.splits] - 1) / max_clusters[pl.splits];
+        const int64_t waves = (tiles + pl.slots - 1) / pl.slots;
         return (double)waves * (pl.kblocks_per_split * block + 1.17) + 1.81 * pl.bn / 128 + 3.14;
     }
     const double hbm = (double)K * (double)N / 5.5e6;                           // the weights, for few rows

@@ -113,6 +113,7 @@ struct UmmaPlan {
     int kblocks_per_split;
     int m_tiles, n_tiles;
     int grid;          // persistent CTAs
+    int slots;         // splits > 1: clusters resident at once
     int tail_tiles;    // last tiles finished by a second, cluster split-K launch (0 = none)
     int tail_splits, tail_kps;
     int narrow_tiles;  // last tiles of a 256-wide persistent launch run as two 128-column halves each (0 = none)

@@ -641,11 +641,12 @@ UmmaPlan plan_umma(int64_t M, int64_t K, int64_t N, int force_bn, int force_spli
         splits = (kblocks + kps - 1) / kps;                           // no empty K slice
         const long work = tiles * splits;
         long waves = (work + (sm_count() - 1)) / sm_count();
+        int slots = 0;
         if (splits > 1) {
             const void* kern = bn == 256 ? (const void*)umma_gemm_kernel<256, true>
                              : bn == 128 ? (const void*)umma_gemm_kernel<128, true> : (const void*)umma_gemm_kernel<64, true>;
             const size_t smem = bn == 256 ? UmmaCfg<256>::kSmemBytes : bn == 128 ? UmmaCfg<128>::kSmemBytes : UmmaCfg<64>::kSmemBytes;
-            int slots = max_active_clusters(kern, kThreads, smem, splits);
+            slots = max_active_clusters(kern, kThreads, smem, splits);
             if (slots < 1) slots = 1;
             waves = (tiles + slots - 1) / slots;
         }
@@ -659,7 +660,7 @@ UmmaPlan plan_umma(int64_t M, int64_t K, int64_t N, int force_bn, int force_spli
         if (cost < best_cost) {
             best_cost = cost;
             best.bn = bn; best.splits = splits; best.kblocks_per_split = kps;
-            best.m_tiles = m_tiles; best.n_tiles = n_tiles;
+            best.m_tiles = m_tiles; best.n_tiles = n_tiles; best.slots = slots;
             best.grid = splits > 1 ? (int)work : (int)(work < sm_count() ? work : sm_count());
             best.partial_bytes = 0;
         }

@@ -518,6 +518,16 @@ SwapPlan plan_swap(int64_t M, int64_t K, int64_t N, int force_splits, bool preq)
     const int kblocks = (int)((K + kKB - 1) / kKB);
     int best_s = 1;
     double best_cost = 1e30;
+    // Clusters of s resident at once.  The occupancy query answers as if one CTA had an SM to itself (74 clusters of two, 15 of
+    // eight) whatever the kernel's shared memory; two CTAs of the 16-row kernel do share an SM (86 clusters of two run as one
+    // wave: 7.9 us against 10.9 us unsplit on 2048 -> 11008), so for that kernel the figure is doubled.
+    auto resident_clusters = [&](int s) {
+        int n = sm_count();
+        if (s > 1 && preq) n = pl.mp == 16 ? swap_max_clusters<16, true>(s) : (pl.mp == 32 ? swap_max_clusters<32, true>(s) : swap_max_clusters<64, true>(s));
+        else if (s > 1) n = pl.mp == 16 ? swap_max_clusters<16, false>(s) : (pl.mp == 32 ? swap_max_clusters<32, false>(s) : swap_max_clusters<64, false>(s));
+        if (pl.mp == 16) n *= 2;
+        return n < 1 ? 1 : n;
+    };
     for (int s = 1; s <= 8; ++s) {
         if (force_splits > 0 && s != (force_splits > 8 ? 8 : force_splits)) continue;
         if (s > kblocks) break;
@@ -527,16 +537,7 @@ SwapPlan plan_swap(int64_t M, int64_t K, int64_t N, int force_splits, bool preq)
         if (force_splits <= 0 && s > 1 && kblocks / s < min_blocks) break;
         const int kps = (kblocks + s - 1) / s;
         if ((kblocks + kps - 1) / kps != s) continue;                        // would leave an empty slice
-        int slots = sm_count() * (pl.mp == 16 ? 2 : 1);
-        if (s > 1) {
-            if (preq) slots = pl.mp == 16 ? swap_max_clusters<16, true>(s) : (pl.mp == 32 ? swap_max_clusters<32, true>(s) : swap_max_clusters<64, true>(s));
-            else slots = pl.mp == 16 ? swap_max_clusters<16, false>(s) : (pl.mp == 32 ? swap_max_clusters<32, false>(s) : swap_max_clusters<64, false>(s));
-        }
-        // The occupancy query answers as if one CTA had an SM to itself (74 clusters of two, 15 of eight) whatever the
-        // kernel's shared memory; two CTAs of the 16-row kernel do share an SM (86 clusters of two run as one wave:
-        // 7.9 us against 10.9 us unsplit on 2048 -> 11008), so for that kernel the figure is doubled.
-        if (s > 1 && pl.mp == 16) slots *= 2;
-        if (slots < 1) slots = 1;
+        const int slots = resident_clusters(s);
         // The slice count fixes the order in which the products of an output are added, so it is part of the result: another
         // count moves a few bf16 results by their last bit, and a stack of layers spreads that through the e4m3 codes
         // between its linears (four layers end 2 to 3 % apart).  So the counts stay what this model of the time of a wave has
@@ -565,8 +566,7 @@ SwapPlan plan_swap(int64_t M, int64_t K, int64_t N, int force_splits, bool preq)
     }
     // what a call takes, microseconds: fitted like plan_w8a8_pair, against which it is weighed
     {
-        static const int max_clusters[9] = {148, 148, 74, 45, 33, 26, 22, 15, 15};
-        const int kps = (kblocks + best_s - 1) / best_s, slots = max_clusters[best_s] * (pl.mp == 16 ? 2 : 1);
+        const int kps = (kblocks + best_s - 1) / best_s, slots = resident_clusters(best_s);
         const int ctas = pl.n_tiles * best_s, resident = ctas < slots * best_s ? ctas : slots * best_s, waves = (pl.n_tiles + slots - 1) / slots;
         const double alone = pl.mp == 16 ? 0.261 : (pl.mp == 32 ? 0.179 : 0.184), shared = 16384.0 * resident / 5.33e6;
         const double t_block = shared > alone ? shared : alone;
