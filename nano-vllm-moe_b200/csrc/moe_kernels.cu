@@ -37,7 +37,12 @@ moe_route_kernel(const LogitT* __restrict__ logits, int64_t ld, int T, int E, in
     }
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
 #pragma unroll
-    for (int i = 0; i < kMaxPerLane; ++i) v[i] = (lane + 32 * i) < E ? v[i] / sum : -1.f;
+    for (int i = 0; i < kMaxPerLane; ++i) {
+        // a NaN logit makes every probability of the row a NaN: it ranks above all others, as in torch's topk, so that the
+        // picks stay experts of this router
+        const float pr = v[i] / sum;
+        v[i] = (lane + 32 * i) < E ? (pr == pr ? pr : INFINITY) : -1.f;
+    }
 
     float picked_w = 0.f;     // lane j keeps the j-th pick
     int picked_id = 0;
@@ -55,8 +60,9 @@ moe_route_kernel(const LogitT* __restrict__ logits, int64_t ld, int T, int E, in
             const int oe = __shfl_xor_sync(0xffffffffu, best_e, o);
             if (ob > best || (ob == best && oe < best_e)) { best = ob; best_e = oe; }
         }
-        if (lane == j) { picked_w = best; picked_id = best_e; }
-        wsum += best;
+        const float w = best < INFINITY ? best : __int_as_float(0x7fffffff);
+        if (lane == j) { picked_w = w; picked_id = best_e; }
+        wsum += w;
         if ((best_e & 31) == lane) v[best_e >> 5] = -1.f;     // remove it from the next round
     }
     if (lane < top_k) {

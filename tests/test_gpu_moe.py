@@ -71,6 +71,24 @@ def test_router_large_and_bf16(moe):
         np.testing.assert_allclose(w.cpu().numpy(), w_ref, rtol=1e-5)
 
 
+@pytest.mark.parametrize("E,k", [(60, 4), (7, 7), (300, 5), (1000, 3)])
+def test_router_picks_experts_for_a_row_of_nans(moe, E, k):
+    """Weights are NaN then (the softmax is), ids distinct experts of the router; the other rows do not notice."""
+    logits = torch.randn(9, E, device="cuda")
+    want_w, want_ids = moe.SoftmaxTopKRouter(k, False).select_experts(None, logits)
+    bad = logits.clone()
+    bad[2, E // 2] = float("nan")
+    bad[5] = float("nan")
+    bad[7, 0] = float("inf")                     # inf - inf
+    w, ids = moe.SoftmaxTopKRouter(k, False).select_experts(None, bad)
+    rows = [2, 5, 7]
+    assert w[rows].isnan().all()
+    for row in ids[rows].tolist():
+        assert len(set(row)) == k and all(0 <= e < E for e in row)
+    keep = [r for r in range(9) if r not in rows]
+    assert torch.equal(w[keep], want_w[keep]) and torch.equal(ids[keep], want_ids[keep])
+
+
 @pytest.mark.parametrize("T,H,I,E,k", [(1, 256, 128, 8, 2), (16, 512, 256, 12, 4), (64, 2048, 1408, 60, 4),
                                        (300, 256, 128, 6, 2), (1024, 512, 384, 8, 4),
                                        (48, 2048, 704, 15, 4), (700, 512, 704, 5, 2)])     # 704 = a TP-2 slice of 1408
