@@ -190,8 +190,9 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 
 // Tensor memory of a CTA pair, from warp 1 of every CTA.  The allocation and its release reach into the partner CTA, so the
 // first waits until every CTA of the cluster runs, and none ends before all are through the second.  Between the two, every
-// CTA's mbarriers exist (initialised before the call) and its tensor memory is allocated before a leader's MMA writes there;
-// nobody releases while a partner may still signal its barriers or the leader's MMAs may still use its memory.
+// CTA's mbarriers exist (initialised before the call); a leader's MMA writes its partner's tensor memory only after operands
+// have arrived that the partner's producer loads behind this call, hence behind its allocation.  Nobody releases while a
+// partner may still signal its barriers or the leader's MMAs may still use its memory.
 __device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_base, uint32_t cols) {
     cluster_sync_all();
     if (warp == 1) {
@@ -200,7 +201,6 @@ __device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();
     tc_fence_after();
     return *s_base;
 }

@@ -21,7 +21,7 @@ def test_pair_tensor_memory_is_taken_and_released_between_cluster_barriers():
     """tcgen05.alloc / dealloc of a CTA pair are collective over both CTAs: the partner has to run, and has to be there still."""
     common = SOURCES["umma_common.cuh"]
     begin, end = body(common, "pair_tmem_begin"), body(common, "pair_tmem_end")
-    assert begin.index("cluster_sync_all") < begin.index("tmem_alloc_pair") < begin.rindex("cluster_sync_all")
+    assert begin.index("cluster_sync_all") < begin.index("tmem_alloc_pair") < begin.index("__syncthreads")
     assert end.index("cluster_sync_all") < end.index("tmem_dealloc_pair") < end.rindex("cluster_sync_all")
     for name, text in SOURCES.items():
         rest = text.replace(begin, "").replace(end, "")
