@@ -190,11 +190,16 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 
 // Tensor memory of a CTA pair, from warp 1 of every CTA.  The allocation and its release reach into the partner CTA, so the
 // first waits until every CTA of the cluster runs, and none ends before all are through the second.  Between the two, every
-// CTA's mbarriers exist (initialised before the call); a leader's MMA writes its partner's tensor memory only after operands
-// have arrived that the partner's producer loads behind this call, hence behind its allocation.  Nobody releases while a
+// CTA's mbarriers exist (initialised before the first call); a leader's MMA writes its partner's tensor memory only after rows
+// have arrived that the partner's producer loads behind pair_tmem_begin, hence behind its allocation.  Nobody releases while a
 // partner may still signal its barriers or the leader's MMAs may still use its memory.
+//   pair_enter       every CTA of the cluster runs, and its barriers exist: loads may be signalled on them
+//   pair_tmem_begin  ... and the tensor memory is there; between the two the producers send the first weights
+//   pair_tmem_end    the last thing a thread does with the cluster.  All threads take part in both of its barriers: with the
+//                    other warps ending in front of the second one, kernels stopped there, although a thread that has
+//                    ended should count as arrived.
+__device__ __forceinline__ void pair_enter() { cluster_sync_all(); }
 __device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_base, uint32_t cols) {
-    cluster_sync_all();
     if (warp == 1) {
         __syncwarp();
         tmem_alloc_pair(smem_u32(s_base), cols);

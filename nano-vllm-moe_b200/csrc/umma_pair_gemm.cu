@@ -100,6 +100,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    pair_enter();
     const uint32_t tmem_base = pair_tmem_begin(warp, &s_tmem_base, kTmemCols);
     pdl_launch_dependents();
     static_assert(!kFuseQ || !kF16, "in-kernel quantisation: e4m3 operands only");

@@ -197,6 +197,17 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    auto load_weights = [&](uint32_t elected, int item, int kb, int slot) {
+        const uint32_t full = smem_u32(&bar_wfull[slot]);
+        mbar_expect_tx(elected, full, kWBytes);
+        tma_load_2d(elected, wring + slot * kWBytes, &tmap_w, 0, ((2 * (item / sched.m_tiles) + (int)rank) * sched.kblocks + kb) * kTile, full);
+    };
+    pair_enter();
+    const int w_pre = min(kb1 - kb0, nw);              // K blocks of the weight ring's first pass
+    if (warp == 2 + kConvWarps + kEpiWarps) {
+        const uint32_t el = elect_one();
+        for (int i = 0; i < w_pre; ++i) load_weights(el, first_item, kb0 + i, i);
+    }
     const uint32_t tmem_base = pair_tmem_begin(warp, &s_tmem_base, kTmemCols);
     pdl_launch_dependents();
 
@@ -267,17 +278,14 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         // Its own thread: the weights do not depend on the predecessor, and a slot is refilled as soon as its tile has been
         // widened, up to n_a blocks ahead of the tensor core.
         const uint32_t el = elect_one();
-        int slot = 0;
-        uint32_t phase = 1;
+        int slot = w_pre == nw ? 0 : w_pre;
+        uint32_t phase = w_pre == nw ? 0 : 1;
         bool ok = true;
         for (int item = first_item; item < items && ok; item += item_step) {
-            const int wtile = 2 * (item / sched.m_tiles) + (int)rank;
-            for (int kb = kb0; kb < kb1; ++kb) {
+            for (int kb = item == first_item ? kb0 + w_pre : kb0; kb < kb1; ++kb) {
                 ok = !s_abort && warp_wait(smem_u32(&bar_wempty[slot]), phase, p.status, kDevTimeoutEmpty);
                 if (!__all_sync(0xffffffffu, ok)) { ok = false; s_abort = 1; break; }
-                const uint32_t full = smem_u32(&bar_wfull[slot]);
-                mbar_expect_tx(el, full, kWBytes);
-                tma_load_2d(el, wring + slot * kWBytes, &tmap_w, 0, (wtile * sched.kblocks + kb) * kTile, full);
+                load_weights(el, item, kb, slot);
                 if (++slot == nw) { slot = 0; phase ^= 1; }
             }
         }

@@ -140,31 +140,33 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    const uint32_t el = elect_one();
+    auto load_weights = [&](const Item& it, int kb, int slot) {
+        const uint32_t full_local = smem_u32(&bar_full[slot]);
+        mbar_expect_tx(leader ? el : 0u, full_local, 2u * (kWBytes + (uint32_t)it.half * kKB));
+        const uint32_t full = map_to_cta(full_local, leader_cta);
+        const uint32_t ws = smem_base + slot * slot_bytes;
+        if (kMlp) {
+            const int row = (2 * it.nt * sched.kblocks + kb) * kTile + (int)rank * 64;
+            tma_load_2d_pair(el, ws, &maps.w, 0, row, full);
+            tma_load_2d_pair(el, ws + kWBytes / 2, &maps.w, 0, row + sched.kblocks * kTile, full);
+        } else {
+            tma_load_2d_pair(el, ws, &maps.w, 0, ((2 * it.nt + (int)rank) * sched.kblocks + kb) * kTile, full);
+        }
+    };
+    pair_enter();
+    const int pre = min(kb1 - kb0, n_slots);               // K blocks of the first ring pass
+    if (warp == 0)
+        for (int i = 0; i < pre; ++i) load_weights(it0, kb0 + i, i);
     const uint32_t tmem_base = pair_tmem_begin(warp, &s_tmem_base, kTmemCols);
     pdl_launch_dependents();
 
     if (warp == 0) {
         // ================= TMA producer (both CTAs) =================
-        const uint32_t el = elect_one();
-        auto load_weights = [&](const Item& it, int kb, int slot) {
-            const uint32_t full_local = smem_u32(&bar_full[slot]);
-            mbar_expect_tx(leader ? el : 0u, full_local, 2u * (kWBytes + (uint32_t)it.half * kKB));
-            const uint32_t full = map_to_cta(full_local, leader_cta);
-            const uint32_t ws = smem_base + slot * slot_bytes;
-            if (kMlp) {
-                const int row = (2 * it.nt * sched.kblocks + kb) * kTile + (int)rank * 64;
-                tma_load_2d_pair(el, ws, &maps.w, 0, row, full);
-                tma_load_2d_pair(el, ws + kWBytes / 2, &maps.w, 0, row + sched.kblocks * kTile, full);
-            } else {
-                tma_load_2d_pair(el, ws, &maps.w, 0, ((2 * it.nt + (int)rank) * sched.kblocks + kb) * kTile, full);
-            }
-        };
         auto load_rows = [&](const Item& it, int kb, int slot) {
             const uint32_t full = map_to_cta(smem_u32(&bar_full[slot]), leader_cta);
             tma_load_2d_pair(el, smem_base + slot * slot_bytes + kWBytes, it.last ? &maps.x_last : &maps.x, kb * kKB, it.m0 + (int)rank * it.half, full);
         };
-        const int pre = min(kb1 - kb0, n_slots);
-        for (int i = 0; i < pre; ++i) load_weights(it0, kb0 + i, i);
         pdl_wait();
         for (int i = 0; i < pre; ++i) load_rows(it0, kb0 + i, i);
         int slot = pre == n_slots ? 0 : pre;
@@ -187,7 +189,6 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     } else if (warp == 1) {
         // ================= MMA issuer (leader CTA only) =================
         if (leader) {
-            const uint32_t el = elect_one();
             const uint16_t both = (uint16_t)(3u << crank);                      // this CTA and its partner
             int tl = 0, slot = 0;
             uint32_t phase = 0;

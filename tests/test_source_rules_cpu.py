@@ -21,13 +21,19 @@ def test_pair_tensor_memory_is_taken_and_released_between_cluster_barriers():
     """tcgen05.alloc / dealloc of a CTA pair are collective over both CTAs: the partner has to run, and has to be there still."""
     common = SOURCES["umma_common.cuh"]
     begin, end = body(common, "pair_tmem_begin"), body(common, "pair_tmem_end")
-    assert begin.index("cluster_sync_all") < begin.index("tmem_alloc_pair") < begin.index("__syncthreads")
+    assert "cluster_sync_all" in body(common, "pair_enter")
+    assert begin.index("tmem_alloc_pair") < begin.index("__syncthreads")
     assert end.index("cluster_sync_all") < end.index("tmem_dealloc_pair") < end.rindex("cluster_sync_all")
     for name, text in SOURCES.items():
         rest = text.replace(begin, "").replace(end, "")
         calls = re.findall(r"(?<!void )tmem_(?:de)?alloc_pair\(", rest)
         assert not calls, f"{name} takes or releases a pair's tensor memory by itself"
         assert text.count("pair_tmem_begin(") == text.count("pair_tmem_end("), name
+        if "= pair_tmem_begin(" in text:
+            assert text.index("mbar_init(") < text.index("pair_enter();") < text.index("= pair_tmem_begin("), name
+            # the partner's rows, which a leader's MMA waits for, are loaded behind the partner's own allocation
+            rows = {"umma_pair_gemm.cu": "&tmap_a, kb", "umma_w8a8_pair.cu": "load_rows(it0", "umma_w8a16_pair.cu": "&tmap_x, kb"}[name]
+            assert text.index("= pair_tmem_begin(") < text.index(rows), name
     assert sum(t.count("= pair_tmem_begin(") for t in SOURCES.values()) == 3
 
 
