@@ -181,12 +181,20 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+// Whole warps come here, and they are brought together first: code in front may have been skipped by a part of the warp, and
+// the barrier counts warps.
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    cluster_arrive();
+    cluster_wait();
+}
 
 // Tensor memory of a CTA pair, from warp 1 of every CTA.  The allocation and its release reach into the partner CTA, so the
 // first waits until every CTA of the cluster runs, and none ends before all are through the second.  Between the two, every
@@ -195,9 +203,9 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 // partner may still signal its barriers or the leader's MMAs may still use its memory.
 //   pair_enter       every CTA of the cluster runs, and its barriers exist: loads may be signalled on them
 //   pair_tmem_begin  ... and the tensor memory is there; between the two the producers send the first weights
-//   pair_tmem_end    the last thing a thread does with the cluster.  All threads take part in both of its barriers: with the
-//                    other warps ending in front of the second one, kernels stopped there, although a thread that has
-//                    ended should count as arrived.
+//   pair_tmem_end    the last thing a thread does with the cluster.  All threads take part in both of its barriers, from a
+//                    __syncthreads on: without it, and with the other warps ending in front of the second barrier, kernels
+//                    stopped there.
 __device__ __forceinline__ void pair_enter() { cluster_sync_all(); }
 __device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_base, uint32_t cols) {
     if (warp == 1) {

@@ -76,3 +76,15 @@ def test_tensor_memory_is_handed_over_at_cluster_scope():
         for bar in remote:
             waits = re.findall(r"(mbar_wait(?:<true>)?)\(smem_u32\(&" + bar, SOURCES[name])
             assert waits and set(waits) == {"mbar_wait<true>"}, (name, bar, waits)
+
+
+def test_cluster_barriers_are_reached_by_warps_that_are_together():
+    """The two instructions stand in one place each, behind a __syncwarp: a loop that part of a warp skips may end at the call."""
+    for name, text in SOURCES.items():
+        found = re.findall(r"barrier\.cluster\.\w+[.\w]*", text)
+        if name != "umma_common.cuh":
+            assert not found, (name, found)
+    for function, instruction in (("cluster_arrive", "barrier.cluster.arrive.release.aligned"), ("cluster_wait", "barrier.cluster.wait.acquire.aligned")):
+        code = body(SOURCES["umma_common.cuh"], function)
+        assert code.index("__syncwarp()") < code.index(instruction)
+    assert len(re.findall(r"barrier\.cluster\.", SOURCES["umma_common.cuh"])) == 2
