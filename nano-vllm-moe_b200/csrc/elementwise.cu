@@ -62,7 +62,7 @@ cudaError_t launch_act_quant(const __nv_bfloat16* x, int64_t ldx, const float* i
     const int64_t total = M * (K / 16);
     if (total == 0) return cudaSuccess;
     int64_t blocks = (total + 511) / 512;
-    const int64_t cap = sm_count() * 16;
+    const int64_t cap = sm_count() * 15;           // five blocks an SM at a time (48 registers a thread): three whole rounds
     if (blocks > cap) blocks = cap;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
