@@ -17,8 +17,9 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
     const int64_t total = M * vec_per_row;
     int64_t base = (int64_t)blockIdx.x * 512;
     uint4 a[2][2];
-    unsigned char* dst[2];
-    auto load = [&]() {
+    const uint4* src[2];
+    unsigned char* dst[2];                // nullptr: past the end
+    auto locate = [&]() {
         const int64_t row0 = base / vec_per_row;
         const int col0 = (int)(base - row0 * vec_per_row);
 #pragma unroll
@@ -30,14 +31,16 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
             if (col < 0) { --dr; col += vec_per_row; }
             else if (col >= vec_per_row) { ++dr; col -= vec_per_row; }
             const int64_t row = row0 + dr;
+            src[u] = reinterpret_cast<const uint4*>(x + row * ldx + (int64_t)col * 16);
             dst[u] = base + u * 256 + threadIdx.x < total ? xq + row * K + (int64_t)col * 16 : nullptr;
-            if (dst[u]) {
-                const uint4* src = reinterpret_cast<const uint4*>(x + row * ldx + (int64_t)col * 16);
-                a[u][0] = __ldg(src);
-                a[u][1] = __ldg(src + 1);
-            }
         }
     };
+    auto load = [&]() {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (dst[u]) { a[u][0] = __ldg(src[u]); a[u][1] = __ldg(src[u] + 1); }
+    };
+    locate();
     pdl_wait();                    // x may come from the kernel before, the scale too
     if (base >= total) return;
     const float scale = fmaxf(__ldg(input_scale), 1e-12f);
@@ -53,6 +56,7 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
         }
         base += (int64_t)gridDim.x * 512;
         if (base >= total) break;
+        locate();
         load();
     }
 }

@@ -181,12 +181,15 @@ stream_linear_kernel(StreamArgs p) {
     for (int s = 0; s < 4; ++s) load_w_step(0, s);       // weights first: they do not depend on the predecessor
     pdl_launch_dependents();
     pdl_wait();                                           // x, y and the split-K scratch may belong to the predecessor, scales and bias too
+    if (SCHEME == FP8LIN_W8A8_STATIC) in_scale = __ldg(p.input_scale);
+    load_x(0, 0);                                         // (in flight beside the scale, which the first quotient needs)
     if (SCHEME == FP8LIN_W8A8_STATIC) {
-        in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
+        in_scale = fmaxf(in_scale, 1e-12f);
         div_scale = ExactDiv(in_scale);
     }
+    store_x(0, 0);
 #pragma unroll
-    for (int part = 0; part < kParts; ++part) { load_x(0, part); store_x(0, part); }
+    for (int part = 1; part < kParts; ++part) { load_x(0, part); store_x(0, part); }
     __syncthreads();
 
     for (int c = 0; c < n_chunks; ++c) {
