@@ -196,38 +196,6 @@ __device__ __forceinline__ void cluster_sync_all() {
     cluster_wait();
 }
 
-// Tensor memory of a CTA pair, from warp 1 of every CTA.  The allocation and its release reach into the partner CTA, so the
-// first waits until every CTA of the cluster runs, and none ends before all are through the second.  Between the two, every
-// CTA's mbarriers exist (initialised before the first call); a leader's MMA writes its partner's tensor memory only after rows
-// have arrived that the partner's producer loads behind pair_tmem_begin, hence behind its allocation.  Nobody releases while a
-// partner may still signal its barriers or the leader's MMAs may still use its memory.
-//   pair_enter       every CTA of the cluster runs, and its barriers exist: loads may be signalled on them
-//   pair_tmem_begin  ... and the tensor memory is there; between the two the producers send the first weights
-//   pair_tmem_end    the last thing a thread does with the cluster.  All threads take part in both of its barriers, from a
-//                    __syncthreads on: without it, and with the other warps ending in front of the second barrier, kernels
-//                    stopped there.
-__device__ __forceinline__ void pair_enter() { cluster_sync_all(); }
-__device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_base, uint32_t cols) {
-    if (warp == 1) {
-        __syncwarp();
-        tmem_alloc_pair(smem_u32(s_base), cols);
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    return *s_base;
-}
-__device__ __forceinline__ void pair_tmem_end(int warp, uint32_t tmem_base, uint32_t cols) {
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync_all();
-    if (warp == 1) {
-        __syncwarp();
-        tc_fence_after();
-        tmem_dealloc_pair(tmem_base, cols);
-    }
-    cluster_sync_all();
-}
 // 16 bytes into a CTA of the cluster (dst and bar are shared::cluster addresses of the same CTA); the store is
 // asynchronous and counts its bytes on that CTA's barrier when it lands
 //
@@ -254,6 +222,45 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
     float4 v;
     asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
     return v;
+}
+
+// Tensor memory of a CTA pair, from warp 1 of every CTA.  The allocation and its release reach into the partner CTA, so the
+// first waits until every CTA of the cluster runs, and none ends before all are through the second.  Between the two, every
+// CTA's mbarriers exist (initialised before the first call); a leader's MMA writes its partner's tensor memory only after rows
+// have arrived that the partner's producer loads behind pair_tmem_begin, hence behind its allocation.
+//   pair_enter         every CTA of the cluster runs, and its barriers exist: loads may be signalled on them
+//   pair_tmem_begin    ... and the tensor memory is there; between the two the producers send the first weights
+//   pair_tmem_done     every warp but those of the producers and the MMA issuer, when it has made its last tensor-memory access
+//                      (an epilogue warp has then seen the last MMA end, or given up a second ago): arrives in both CTAs
+//   pair_tmem_release  warp 1: releases when the warps of both CTAs are done, under the epilogues' last stores
+//   pair_leave         nobody ends while its partner may still signal its barriers, or before both have released.  From a
+//                      __syncthreads on and by all threads: without it, and with most warps ending in front of a second cluster
+//                      barrier, kernels stopped there.
+__device__ __forceinline__ void pair_enter() { cluster_sync_all(); }
+__device__ __forceinline__ uint32_t pair_tmem_begin(int warp, const uint32_t* s_base, uint32_t cols) {
+    if (warp == 1) {
+        __syncwarp();
+        tmem_alloc_pair(smem_u32(s_base), cols);
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    return *s_base;
+}
+__device__ __forceinline__ void pair_tmem_done(uint32_t bar, uint32_t leader_cta, int lane) {
+    tc_fence_before();
+    __syncwarp();
+    if (lane < 2) mbar_arrive_remote(map_to_cta(bar, leader_cta + (uint32_t)lane));
+}
+__device__ __forceinline__ void pair_tmem_release(uint32_t bar, uint32_t tmem_base, uint32_t cols, int* status) {
+    mbar_wait<true>(bar, 0, status, kDevTimeoutTmemEmpty, 8 * kWaitCycles);      // (the waits it waits for are bounded themselves)
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, cols);
+}
+__device__ __forceinline__ void pair_leave() {
+    __syncthreads();
+    cluster_sync_all();
 }
 
 // ---- named barriers ------------------------------------------------------------------------------------------

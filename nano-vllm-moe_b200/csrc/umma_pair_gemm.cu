@@ -80,6 +80,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     __shared__ __align__(8) uint64_t bar_empty[S];
     __shared__ __align__(8) uint64_t bar_tfull[2];
     __shared__ __align__(8) uint64_t bar_tempty[2];
+    __shared__ __align__(8) uint64_t bar_done;       // tensor memory of both CTAs has been read for the last time
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
     __shared__ __align__(16) float s_scale[kBN];
@@ -96,6 +97,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     if (threadIdx.x == 0) {
         for (int i = 0; i < S; ++i) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_empty[i]), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bar_tfull[i]), 1); mbar_init(smem_u32(&bar_tempty[i]), 2 * kEpiWarps); }
+        mbar_init(smem_u32(&bar_done), 2 * kEpiWarps);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -195,6 +197,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (ok) umma_commit_both(el, smem_u32(&bar_tfull[as]), both);
             }
         }
+        pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
     } else {
         // ================= epilogue (warps 2..9 of both CTAs) =================
         // Warp (q, h): TMEM lanes [32q, 32q+32) = 32 rows of this CTA's half of the tile; of every 64
@@ -325,10 +328,11 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive_remote(map_to_cta(smem_u32(&bar_tempty[as]), 0));
         }
+        pair_tmem_done(smem_u32(&bar_done), 0, lane);
         if (lane == 0) tma_store_wait_all();
     }
 
-    pair_tmem_end(warp, tmem_base, kTmemCols);
+    pair_leave();
     if (kFuseQ && threadIdx.x == 0) quant_ctrl_release(qjob, p.M);
 }
 

@@ -148,6 +148,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     __shared__ __align__(8) uint64_t bar_empty[kMaxA];    // the MMAs that read the widened weights are done (both CTAs')
     __shared__ __align__(8) uint64_t bar_tfull[2];
     __shared__ __align__(8) uint64_t bar_tempty[2];    // leader's
+    __shared__ __align__(8) uint64_t bar_done;         // tensor memory of both CTAs has been used for the last time
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
 
@@ -193,6 +194,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             mbar_init(smem_u32(&bar_empty[i]), 1);
         }
         for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bar_tfull[i]), 1); mbar_init(smem_u32(&bar_tempty[i]), 2 * kEpiWarps); }
+        mbar_init(smem_u32(&bar_done), 2 * (kConvWarps + kEpiWarps));
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -273,6 +275,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 if (ok) umma_commit_both(el, smem_u32(&bar_tfull[as]), both);
             }
         }
+        if (!kSplit) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
     } else if (warp == 2 + kConvWarps + kEpiWarps) {
         // ================= weight producer (both CTAs) =================
         // Its own thread: the weights do not depend on the predecessor, and a slot is refilled as soon as its tile has been
@@ -333,6 +336,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 if (++aslot == n_a) { aslot = 0; aphase ^= 1; }
             }
         }
+        pair_tmem_done(smem_u32(&bar_done), leader_cta, lane);
     } else {
         // ================= epilogue (warps 10..17 of both CTAs) =================
         pdl_wait();                                        // y may still be in use by the predecessor
@@ -396,6 +400,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 }
             }
         }
+        pair_tmem_done(smem_u32(&bar_done), leader_cta, lane);
     }
 
     if constexpr (kSplit) {
@@ -403,13 +408,14 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         __syncwarp();
         pdl_wait();
         cluster_sync_all();                                // every CTA's sums are parked
+        if (warp == 1) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
         if (!s_abort) {
             finish_parked_band(p, smem_base, sched.splits, (int)rank, slice_rank * band, band_rows, m_valid,
                                (2 * (first_item / sched.m_tiles) + (int)rank) * kTile, (first_item % sched.m_tiles) * T, 1.f, 1.f, kThreads);
         }
     }
 
-    pair_tmem_end(warp, tmem_base, kTmemCols);
+    pair_leave();
 }
 
 bool encode_x_tokens(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes, uint32_t box_rows) {

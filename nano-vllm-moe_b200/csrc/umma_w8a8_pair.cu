@@ -100,6 +100,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     __shared__ __align__(8) uint64_t bar_empty[kMaxSlots];     // the MMAs that read the slot are done (both CTAs')
     __shared__ __align__(8) uint64_t bar_tfull[2];
     __shared__ __align__(8) uint64_t bar_tempty[2];            // leader's
+    __shared__ __align__(8) uint64_t bar_done;                 // tensor memory of both CTAs has been read for the last time
     __shared__ uint32_t s_tmem_base;
     __shared__ volatile int s_abort;
 
@@ -136,6 +137,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxSlots; ++i) { mbar_init(smem_u32(&bar_full[i]), 1); mbar_init(smem_u32(&bar_empty[i]), 1); }
         for (int i = 0; i < 2; ++i) { mbar_init(smem_u32(&bar_tfull[i]), 1); mbar_init(smem_u32(&bar_tempty[i]), 2 * kEpiWarps); }
+        mbar_init(smem_u32(&bar_done), 2 * kEpiWarps);
         s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -221,6 +223,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                 if (ok) umma_commit_both(el, smem_u32(&bar_tfull[as]), both);
             }
         }
+        if (!kSplit) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
     } else {
         // ================= epilogue (warps 2..9 of both CTAs) =================
         pdl_wait();                                        // the output may still be in use by the predecessor
@@ -320,6 +323,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                 }
             }
         }
+        pair_tmem_done(smem_u32(&bar_done), leader_cta, lane);
     }
 
     if constexpr (kSplit) {
@@ -327,6 +331,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         __syncwarp();
         pdl_wait();
         cluster_sync_all();                                // every CTA's sums are parked
+        if (warp == 1) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
         if (!s_abort) {
             float pre;
             const float in_scale = channel_factor(p, pre);
@@ -335,7 +340,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         }
     }
 
-    pair_tmem_end(warp, tmem_base, kTmemCols);
+    pair_leave();
 }
 
 template <bool kSplit, bool kMlp>

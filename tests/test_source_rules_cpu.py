@@ -17,24 +17,32 @@ def body(source, function):
     raise AssertionError(f"{function} does not end")
 
 
-def test_pair_tensor_memory_is_taken_and_released_between_cluster_barriers():
+def test_pair_tensor_memory_is_taken_and_released_while_both_ctas_are_there():
     """tcgen05.alloc / dealloc of a CTA pair are collective over both CTAs: the partner has to run, and has to be there still."""
     common = SOURCES["umma_common.cuh"]
-    begin, end = body(common, "pair_tmem_begin"), body(common, "pair_tmem_end")
+    begin, release, leave = (body(common, f) for f in ("pair_tmem_begin", "pair_tmem_release", "pair_leave"))
     assert "cluster_sync_all" in body(common, "pair_enter")
     assert begin.index("tmem_alloc_pair") < begin.index("__syncthreads")
-    assert end.index("cluster_sync_all") < end.index("tmem_dealloc_pair") < end.rindex("cluster_sync_all")
+    assert release.index("mbar_wait<true>") < release.index("__syncwarp") < release.index("tmem_dealloc_pair")
+    assert leave.index("__syncthreads") < leave.index("cluster_sync_all")
+    rows = {"umma_pair_gemm.cu": "&tmap_a, kb", "umma_w8a8_pair.cu": "load_rows(it0", "umma_w8a16_pair.cu": "&tmap_x, kb"}
     for name, text in SOURCES.items():
-        rest = text.replace(begin, "").replace(end, "")
-        calls = re.findall(r"(?<!void )tmem_(?:de)?alloc_pair\(", rest)
-        assert not calls, f"{name} takes or releases a pair's tensor memory by itself"
-        assert text.count("pair_tmem_begin(") == text.count("pair_tmem_end("), name
-        if "= pair_tmem_begin(" in text:
-            assert text.index("mbar_init(") < text.index("pair_enter();") < text.index("= pair_tmem_begin("), name
-            # the partner's rows, which a leader's MMA waits for, are loaded behind the partner's own allocation
-            rows = {"umma_pair_gemm.cu": "&tmap_a, kb", "umma_w8a8_pair.cu": "load_rows(it0", "umma_w8a16_pair.cu": "&tmap_x, kb"}[name]
-            assert text.index("= pair_tmem_begin(") < text.index(rows), name
-    assert sum(t.count("= pair_tmem_begin(") for t in SOURCES.values()) == 3
+        rest = text.replace(begin, "").replace(release, "")
+        assert not re.findall(r"(?<!void )tmem_(?:de)?alloc_pair\(", rest), f"{name} takes or releases a pair's tensor memory by itself"
+        assert ("= pair_tmem_begin(" in text) == (name in rows)
+    for name, load in rows.items():
+        text = SOURCES[name]
+        order = ["mbar_init(", "pair_enter();", "= pair_tmem_begin(", "pair_tmem_release(", "pair_leave();"]
+        at = [text.index(o) for o in order]
+        assert at == sorted(at) and all(text.count(o) == 1 for o in order if o not in ("mbar_init(", "pair_tmem_release(")), (name, at)
+        # once per launch: split-K releases under its band of sums, the others in the issuer's role
+        assert text.count("if (!kSplit) pair_tmem_release(") == text.count("pair_tmem_release(") - 1, name
+        # the partner's rows, which a leader's MMA waits for, are loaded behind the partner's own allocation
+        assert at[2] < text.index(load), name
+        # every role that uses tensor memory says when it is done, once per warp: epilogue, and converters where there are any
+        users = 2 if "kConvWarps" in text else 1
+        assert text.count("pair_tmem_done(") == users, name
+        assert ("2 * (kConvWarps + kEpiWarps)" if users == 2 else "2 * kEpiWarps") + ");\n        s_abort" in text, name
 
 
 def test_named_barriers_do_not_ask_for_a_converged_warp():
