@@ -55,6 +55,7 @@ void need_cuda(const at::Tensor& t) {
 struct StreamScratch {
     at::Tensor buffer;
     at::Tensor gave_up;          // pinned int
+    volatile int* word = nullptr;        // ... its address
 };
 struct Scratch {
     std::mutex lock;
@@ -64,13 +65,11 @@ struct Scratch {
 constexpr int64_t kHostWordAt = 8;           // byte of the header that names the host's word
 Scratch& scratch() { static Scratch* s = new Scratch; return *s; }      // (outlives the CUDA context's teardown)
 
-// Raises when a kernel of an earlier call on this stream gave up a wait, and forgets it.
-void raise_if_given_up(StreamScratch& e) {
-    volatile int* word = e.gave_up.mutable_data_ptr<int>();
-    const int code = *word;
-    if (code == 0) return;
+// A kernel of an earlier call on this stream gave up a wait: forgets it and raises.
+[[noreturn]] void raise_given_up(StreamScratch& e) {
+    const int code = *e.word;
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
-        *word = 0;
+        *e.word = 0;
         const c10::InferenceMode any_tensor(true);      // (the buffer may have been made in inference mode)
         e.buffer.narrow(0, 0, (int64_t)sizeof(int)).zero_();
     }
@@ -86,7 +85,7 @@ at::Tensor workspace(c10::cuda::CUDAStream stream, size_t nbytes, bool raise = t
     std::lock_guard<std::mutex> guard(s.lock);
     auto it = s.live.find(key);
     if (it != s.live.end()) {
-        if (raise) raise_if_given_up(it->second);
+        if (raise && *it->second.word != 0) raise_given_up(it->second);
         if ((size_t)it->second.buffer.numel() >= nbytes) return it->second.buffer;
     }
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
@@ -101,7 +100,8 @@ at::Tensor workspace(c10::cuda::CUDAStream stream, size_t nbytes, bool raise = t
     StreamScratch fresh;
     fresh.buffer = at::zeros({(int64_t)size}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, stream.device_index()));
     fresh.gave_up = it != s.live.end() ? it->second.gave_up : at::zeros({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-    fresh.buffer.narrow(0, kHostWordAt, (int64_t)sizeof(int64_t)).view(at::kLong).fill_((int64_t)(intptr_t)fresh.gave_up.mutable_data_ptr());
+    fresh.word = fresh.gave_up.mutable_data_ptr<int>();
+    fresh.buffer.narrow(0, kHostWordAt, (int64_t)sizeof(int64_t)).view(at::kLong).fill_((int64_t)(intptr_t)fresh.word);
     if (it != s.live.end()) s.retired.push_back(it->second.buffer);
     s.live[key] = fresh;
     return fresh.buffer;
@@ -488,7 +488,7 @@ PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t na) {
             stream.synchronize();
             Scratch& s = scratch();
             std::lock_guard<std::mutex> lock(s.lock);
-            *s.live[std::make_pair((int)stream.device_index(), (void*)stream.stream())].gave_up.mutable_data_ptr<int>() = 0;
+            *s.live.at(std::make_pair((int)stream.device_index(), (void*)stream.stream())).word = 0;
         }
         return THPVariable_Wrap(t);
     });
