@@ -27,9 +27,10 @@
  *              tile is exactly one TMA box.  Produce it once per layer with
  *              fp8lin_prepack_weight (from "kn") or fp8lin_pack_weight_nk (from "nk").
  *              In the prototypes below `w_nk` names this packed buffer.  A call may read it
- *              while the kernel in front of it in the stream is still ending, so what writes it
- *              has to be complete before the first call that uses it is made: synchronise once
- *              after packing.  (Everything else a call reads is ordered by the stream.)
+ *              while the kernel directly in front of it in the stream is still ending, so a kernel
+ *              of the caller's that writes it (a copy, a permutation) must not be that one: any
+ *              other ordinary launch or a synchronisation between the two will do.  The two packing
+ *              calls see to it themselves.  (Everything else a call reads is ordered by the stream.)
  *
  * Return value: 0 on success, otherwise one of the FP8LIN_ERR_* codes;
  * fp8lin_last_error() returns a thread-local description of the last failure.

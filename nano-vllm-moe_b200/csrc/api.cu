@@ -436,6 +436,7 @@ static int pack_common(const void* src, void* dst, int64_t K, int64_t N, bool sr
     if (!src || !dst) return fail(FP8LIN_ERR_NULL, "source and destination must not be NULL");
     if (!aligned16(dst)) return fail(FP8LIN_ERR_ALIGN, "w_packed must be 16-byte aligned");
     cudaError_t e = launch_pack_tiles((const unsigned char*)src, (unsigned char*)dst, K, N, src_is_kn, (cudaStream_t)stream);
+    if (e == cudaSuccess) e = launch_order((cudaStream_t)stream);       // (a linear behind this reads the weights before it waits)
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "prepack launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
 }

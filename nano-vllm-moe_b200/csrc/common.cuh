@@ -69,7 +69,7 @@ __host__ __device__ inline size_t pack_offset(int64_t n, int64_t k, int64_t KB) 
 // writing or reading (activations, outputs, scratch, and scales or biases, which a
 // caller may have converted just before), waits for the predecessors to finish
 // (pdl_wait).  Only packed weights are read before the wait: they are packed once,
-// and who packs them waits until that is done before handing them out.
+// and a kernel that waits for the packing in full is launched behind it.
 // Both are no-ops when the launch carries no such dependency.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -73,6 +73,10 @@ cudaError_t launch_abs_max(const __nv_bfloat16* x, int64_t ldx, int64_t M, int64
 cudaError_t launch_pack_tiles(const unsigned char* src, unsigned char* dst, int64_t K, int64_t N, bool src_is_kn,
                               cudaStream_t stream);
 
+// An empty kernel launched the ordinary way: it starts when everything in front of it is complete and visible.  Behind it, a
+// dependent launch may read what was written in front of it without waiting (packed weights).
+cudaError_t launch_order(cudaStream_t stream);
+
 // RMSNorm (+ residual add) fused with the static activation quantiser (rmsnorm_quant.cu).  residual (in/out), xq and y
 // may each be nullptr; H <= 8192, a multiple of 8.
 cudaError_t launch_rmsnorm_quant(const __nv_bfloat16* x, int64_t ldx, __nv_bfloat16* residual, int64_t ld_res,

@@ -49,8 +49,8 @@ class Fp8ExpertWeights:
             i = il
         if w2_q.shape != (e, h, i):
             raise ValueError(f"w2 must be [E, H, I] = {(e, h, i)}, got {tuple(w2_q.shape)}")
-        w13_p = torch.cat([kernels.pack_weight_nk(w13_q[x], wait=False) for x in range(e)])
-        w2_p = torch.cat([kernels.pack_weight_nk(w2_q[x], wait=False) for x in range(e)])
+        w13_p = torch.cat([kernels.pack_weight_nk(w13_q[x]) for x in range(e)])
+        w2_p = torch.cat([kernels.pack_weight_nk(w2_q[x]) for x in range(e)])
         dev = w13_q.device
         kernels.weights_written(dev)
         return cls(w13_p, w13_scale.to(dev, torch.float32).contiguous(), w13_input_scale.to(dev, torch.float32).reshape(()),

@@ -97,14 +97,13 @@ def packed_bytes(k: int, n: int) -> int:
 
 
 def weights_written(device: torch.device) -> None:
-    """Wait until packed weights that this stream has just written are complete (load time).  The linears read packed weights
-    before they wait for the kernel in front of them, so stream order alone does not protect them.  During a stream capture
-    there is nothing to wait for: the packing runs when the graph does, and that replay has to end first."""
-    if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
-        torch.cuda.current_stream(device).synchronize()
+    """Behind a torch kernel that has just written packed weights on this stream (a copy, a permutation): the linears read packed
+    weights before they wait for the kernel in front of them, so that one must not be it.  Puts a launch between."""
+    if device.type == "cuda":
+        torch.zeros(1, dtype=torch.uint8, device=device)
 
 
-def _pack(src: torch.Tensor, k: int, n: int, from_kn: bool, wait: bool = True) -> torch.Tensor:
+def _pack(src: torch.Tensor, k: int, n: int, from_kn: bool) -> torch.Tensor:
     _require_cuda(src)
     if src.dtype not in (torch.uint8, torch.float8_e4m3fn) or src.dim() != 2:
         raise ValueError("weight codes must be a 2-D uint8/float8_e4m3fn tensor")
@@ -114,8 +113,6 @@ def _pack(src: torch.Tensor, k: int, n: int, from_kn: bool, wait: bool = True) -
     with torch.cuda.device(src.device):
         rc = fn(src.data_ptr(), out.data_ptr(), k, n, _stream_ptr(src.device))
     _lib.raise_for(rc, "fp8lin_prepack_weight" if from_kn else "fp8lin_pack_weight_nk")
-    if wait:
-        weights_written(src.device)
     return out
 
 
@@ -125,11 +122,10 @@ def prepack_weight(qweight_kn: torch.Tensor) -> torch.Tensor:
     return _pack(qweight_kn, k, n, True)
 
 
-def pack_weight_nk(qweight_nk: torch.Tensor, wait: bool = True) -> torch.Tensor:
-    """e4m3 codes [N, K] (the checkpoint layout) -> the kernels' packed tile layout.  ``wait=False``: the caller sees to
-    ``weights_written`` (after packing several)."""
+def pack_weight_nk(qweight_nk: torch.Tensor) -> torch.Tensor:
+    """e4m3 codes [N, K] (the checkpoint layout) -> the kernels' packed tile layout."""
     n, k = qweight_nk.shape
-    return _pack(qweight_nk, k, n, False, wait)
+    return _pack(qweight_nk, k, n, False)
 
 
 def _check_linear_args(x, w_packed, weight_scale, bias):
