@@ -72,20 +72,7 @@ __host__ __device__ inline size_t pack_offset(int64_t n, int64_t k, int64_t KB) 
 // and a kernel that waits for the packing in full is launched behind it.
 // Both are no-ops when the launch carries no such dependency.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-//
-// The wait names every pointer that is read behind it with ordinary loads.  A load through the read-only path (__ldg, or a
-// const __restrict__ parameter) promises that nobody writes the memory while the kernel runs, so the compiler may move it in
-// front of the wait, memory clobber or not; it did, in the streaming kernel, as soon as a branch stood there, and only a
-// replayed graph of single rows was fast enough to show it.  A pointer that comes out of the wait is a new value, and nothing
-// can be loaded through it earlier.  (TMA loads are volatile statements and stay where they are.)
-// pdl_renew names one later, where it would only occupy registers in between.
-template <class P>
-__device__ __forceinline__ void pdl_renew(P& pointer) { asm volatile("" : "+l"(pointer) :: "memory"); }
-template <class... P>
-__device__ __forceinline__ void pdl_wait(P&... pointers) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    (pdl_renew(pointers), ...);
-}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---- small numeric helpers ----------------------------------------------------
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }

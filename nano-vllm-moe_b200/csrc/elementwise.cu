@@ -41,7 +41,7 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
             if (dst[u]) { a[u][0] = __ldg(src[u]); a[u][1] = __ldg(src[u] + 1); }
     };
     locate();
-    pdl_wait(x, src[0], src[1], input_scale);                    // x may come from the kernel before, the scale too
+    pdl_wait();                    // x may come from the kernel before, the scale too
     if (base >= total) return;
     const float scale = fmaxf(__ldg(input_scale), 1e-12f);
     load();                        // (in flight beside the scale, which the first quotient needs)
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256)
 sum_slots_kernel(const __nv_bfloat16* __restrict__ slots, int n_slots, int64_t slot_stride, __nv_bfloat16* __restrict__ y,
                  int64_t ldy, int64_t M, int64_t N, int64_t ld_slot) {
     pdl_launch_dependents();
-    pdl_wait(slots);
+    pdl_wait();
     const int64_t vec_per_row = N / 8;
     const int64_t total = M * vec_per_row;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(256)
 sum_slots_gather_kernel(const __nv_bfloat16* __restrict__ slots, int n_slots, int64_t slot_stride, int64_t ld_slot, SumDst dst,
                         int64_t ld_dst, int64_t M, int64_t N) {
     pdl_launch_dependents();
-    pdl_wait(slots);
+    pdl_wait();
     const int64_t vec_per_row = N / 8;
     const int64_t total = M * vec_per_row;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -157,7 +157,7 @@ cudaError_t launch_sum_slots_gather(const __nv_bfloat16* slots, int n_slots, int
 __global__ void __launch_bounds__(256)
 x_to_f16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __half* __restrict__ x16, int64_t M, int64_t K) {
     pdl_launch_dependents();
-    pdl_wait(x);
+    pdl_wait();
     const int64_t vec_per_row = K / 8;
     const int64_t total = M * vec_per_row;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -190,7 +190,7 @@ cudaError_t launch_x_to_f16(const __nv_bfloat16* x, int64_t ldx, void* x16, int6
 __global__ void __launch_bounds__(256)
 dequant_tiles_f16_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst, int64_t src_bytes) {
     pdl_launch_dependents();
-    pdl_wait(src);                    // the GEMM before this pass may still read the destination
+    pdl_wait();                    // the GEMM before this pass may still read the destination
     const int64_t total = src_bytes / 16;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t off = i * 16;
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256)
 silu_mul_quant_interleaved_kernel(const __nv_bfloat16* __restrict__ gu, const float* __restrict__ h_scale,
                                   unsigned char* __restrict__ hq, int64_t M, int64_t I) {
     pdl_launch_dependents();
-    pdl_wait(gu, h_scale);
+    pdl_wait();
     const ExactDiv div_scale(fmaxf(__ldg(h_scale), 1e-12f));
     const int64_t vec_per_row = I / 8;
     const int64_t total = M * vec_per_row;

@@ -14,7 +14,7 @@ __global__ void __launch_bounds__(256)
 moe_route_kernel(const LogitT* __restrict__ logits, int64_t ld, int T, int E, int top_k, int renormalize,
                  float* __restrict__ out_w, IdT* __restrict__ out_ids) {
     pdl_launch_dependents();
-    pdl_wait(logits);
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int token = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (token >= T) return;
@@ -146,7 +146,7 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
             e[i] = id >= 0 && id < E ? (int)id : -1;
         }
     };
-    pdl_wait(ids);
+    pdl_wait();
     __syncthreads();
     if (warp < kWarps) {
         int* mine = count + warp * E;
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256)
 moe_scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ inv, int rows,
                          const float* __restrict__ input_scale, unsigned char* __restrict__ xq, int H) {
     pdl_launch_dependents();
-    pdl_wait(x, inv, input_scale);
+    pdl_wait();
     const ExactDiv div_scale(fmaxf(__ldg(input_scale), 1e-12f));
     const int vec_per_row = H / 16;
     const int tokens = (rows + x_div - 1) / x_div;
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(256)
 silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, const float* __restrict__ input_scale,
                       unsigned char* __restrict__ hq, const int* __restrict__ meta, int I) {
     pdl_launch_dependents();
-    pdl_wait(gu, input_scale, meta);
+    pdl_wait();
     const int rows = meta[1];
     const ExactDiv div_scale(fmaxf(__ldg(input_scale), 1e-12f));
     const int vec_per_row = I / 8;
@@ -323,7 +323,7 @@ __global__ void __launch_bounds__(256)
 moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, const int* __restrict__ inv, __nv_bfloat16* __restrict__ y, int64_t ld_y, int T,
                    int top_k, int H) {
     pdl_launch_dependents();
-    pdl_wait(routed, inv);
+    pdl_wait();
     const int vec = H / 8;
     for (int64_t t = blockIdx.x; t < T; t += gridDim.x) {
         const __nv_bfloat16* src = routed + (size_t)t * top_k * H;

@@ -32,7 +32,7 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     // A decode-sized call is one dependent chain: predecessor's end -> row -> sum of squares -> quantised row.  All loads, of
     // the row and of the operands it meets later, are in flight together, and every thread adds the warps' partial sums itself
     // (one barrier instead of two).
-    pdl_wait(x, residual, weight, input_scale);                                     // x and the residual come from the kernels before, perhaps a copy of the weight too
+    pdl_wait();                                     // x and the residual come from the kernels before, perhaps a copy of the weight too
     const float scale = quant ? fmaxf(__ldg(input_scale), 1e-12f) : 1.f;
     const int64_t row = blockIdx.x;
     const __nv_bfloat16* xr = x + row * ldx;

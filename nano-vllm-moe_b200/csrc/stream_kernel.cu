@@ -180,7 +180,7 @@ stream_linear_kernel(StreamArgs p) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) load_w_step(0, s);       // weights first: they do not depend on the predecessor
     pdl_launch_dependents();
-    pdl_wait(x, p.input_scale);                                           // x, y and the split-K scratch may belong to the predecessor, scales and bias too
+    pdl_wait();                                           // x, y and the split-K scratch may belong to the predecessor, scales and bias too
     if (SCHEME == FP8LIN_W8A8_STATIC) in_scale = __ldg(p.input_scale);
     load_x(0, 0);                                         // (in flight beside the scale, which the first quotient needs)
     if (SCHEME == FP8LIN_W8A8_STATIC) {
@@ -285,7 +285,6 @@ stream_linear_kernel(StreamArgs p) {
         __syncthreads();
         if (!s_last) return;
         __threadfence();
-        pdl_renew(p.partial);
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) { acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f; }
         for (int s = 0; s < n_splits; ++s) {
@@ -307,8 +306,6 @@ stream_linear_kernel(StreamArgs p) {
 
     __nv_bfloat16* y = p.y + (size_t)m_base * p.ldy;
     float sa = 0.f, sb = 0.f, ba = 0.f, bb = 0.f;
-    pdl_renew(p.w_scale);
-    pdl_renew(p.bias);
     if (n_a < p.N) { sa = __ldg(p.w_scale + n_a); if (p.bias) ba = __bfloat162float(p.bias[n_a]); }
     if (n_b < p.N) { sb = __ldg(p.w_scale + n_b); if (p.bias) bb = __bfloat162float(p.bias[n_b]); }
 #pragma unroll

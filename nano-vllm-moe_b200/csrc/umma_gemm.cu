@@ -176,7 +176,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 
     if (kFuseQ && warp >= 2 + kEpiWarps) {
         // ================= activation quantiser (warps 10..13) =================
-        pdl_wait(qjob.x, p.input_scale);                    // x comes from the kernel before; xq may still be read by it
+        pdl_wait();                    // x comes from the kernel before; xq may still be read by it
         quant_worker(qjob, p.input_scale, p.M, p.K, lane);
     } else if (warp == 0) {
         // ================= TMA producer =================
@@ -295,7 +295,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     } else {
         // ================= epilogue (warps 2..9) =================
         // Warp (q, h): TMEM lanes [32q, 32q+32) = 32 rows of the tile, column half h.
-        pdl_wait(p.input_scale, p.w_scale, p.bias);                                            // y may still be in use by the predecessor
+        pdl_wait();                                            // y may still be in use by the predecessor
         const int ew = warp - 2;
         const int q = warp & 3;
         const int h = ew >> 2;

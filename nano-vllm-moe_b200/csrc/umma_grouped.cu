@@ -95,7 +95,7 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     pdl_launch_dependents();
-    pdl_wait(p.meta, p.chunks, p.sorted_rows, p.topk_w, p.x, p.w_scale, p.input_scale, p.h_scale);                                   // the chunk list, the rows and the outputs all come from predecessors
+    pdl_wait();                                   // the chunk list, the rows and the outputs all come from predecessors
 
     const int n_chunks = uniform(p.meta[0]);
     const int total = n_chunks * p.n_tiles;       // item w = chunk * n_tiles + tile

@@ -66,7 +66,7 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     tc_fence_after();
     const uint32_t tmem_base = s_tmem_base;
     pdl_launch_dependents();
-    pdl_wait(p.meta, p.chunks, p.sorted_rows, p.topk_w, p.w_scale, p.input_scale, p.h_scale);                                   // the chunk list, the rows and the outputs all come from predecessors
+    pdl_wait();                                   // the chunk list, the rows and the outputs all come from predecessors
 
     const int n_chunks = uniform(p.meta[0]);
     const int n_items = p.n_tiles;                // channel items per chunk (set by the launcher)

@@ -111,7 +111,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 
     if (kFuseQ && warp >= 2 + kEpiWarps) {
         // ================= activation quantiser (warps 10..13 of both CTAs) =================
-        pdl_wait(qjob.x, p.input_scale);
+        pdl_wait();
         quant_worker(qjob, p.input_scale, p.M, p.K, lane);
     } else if (warp == 0) {
         // ================= TMA producer (both CTAs) =================
@@ -202,7 +202,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         // ================= epilogue (warps 2..9 of both CTAs) =================
         // Warp (q, h): TMEM lanes [32q, 32q+32) = 32 rows of this CTA's half of the tile; of every 64
         // columns warp h converts [32h, 32h + 32) into its half of the pair's staging box.
-        pdl_wait(p.input_scale, p.w_scale, p.bias, h_scale);                                            // y may still be in use by the predecessor
+        pdl_wait();                                            // y may still be in use by the predecessor
         const int ew = warp - 2;
         const int q = warp & 3;
         const int h = ew >> 2;

@@ -174,7 +174,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (kSplit || kGateUp) cluster_arrive();                 // (waited for before the first remote access: the peers' barriers exist)
     // Everything but the packed weights may come from the kernel in front -- the rows, but also a bias or a scale that the
     // caller has just converted.  The producer warp waits by itself, between the weights and the rows.
-    if (warp != 0) pdl_wait(p.input_scale, p.w_scale, p.bias, p.h_scale);
+    if (warp != 0) pdl_wait();
     // scale and bias of the first channel this thread finishes, fetched long before they are needed
     float ws0 = 0.f, bs0 = 0.f, in_scale0 = 0.f;
     auto fetch_first = [&]() {
@@ -209,7 +209,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                     tma_load_2d(el, smem_base + i * Cfg::kStageBytes, &tmap_w, 0,
                                 (first_tile * sched.kblocks_total + kb0 + i) * kTileN, full);   // one packed tile
                 }
-                pdl_wait(p.input_scale, p.w_scale, p.bias);
+                pdl_wait();
                 for (int i = 0; i < first_kb; ++i)
                     tma_load_2d(el, smem_base + i * Cfg::kStageBytes + kXDst, &tmap_x,
                                 (kb0 + i) * kKB, 0, smem_u32(&bar_full[i]));

@@ -339,7 +339,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         pair_tmem_done(smem_u32(&bar_done), leader_cta, lane);
     } else {
         // ================= epilogue (warps 10..17 of both CTAs) =================
-        pdl_wait(p.w_scale, p.bias);                                        // y may still be in use by the predecessor
+        pdl_wait();                                        // y may still be in use by the predecessor
         const int q = warp & 3;
         const int h = (warp - 2 - kConvWarps) >> 2;        // which half of the tile's tokens
         const uint32_t t_lane = tmem_base + ((uint32_t)(q * 32) << 16) + h * half;
@@ -406,7 +406,7 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     if constexpr (kSplit) {
         // ---- this CTA finishes its band: slices added in rank order, scaled, stored ----
         __syncwarp();
-        pdl_wait(p.w_scale, p.bias);
+        pdl_wait();
         cluster_sync_all();                                // every CTA's sums are parked
         if (warp == 1) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
         if (!s_abort) {

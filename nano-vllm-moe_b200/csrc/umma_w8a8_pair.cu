@@ -226,7 +226,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         if (!kSplit) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
     } else {
         // ================= epilogue (warps 2..9 of both CTAs) =================
-        pdl_wait(p.input_scale, p.w_scale, p.bias, p.h_scale);                                        // the output may still be in use by the predecessor
+        pdl_wait();                                        // the output may still be in use by the predecessor
         const int q = warp & 3;                            // TMEM lane quarter
         const int h = (warp - 2) >> 2;                     // which half of the tile's tokens
         float pre;
@@ -329,7 +329,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     if constexpr (kSplit) {
         // ---- this CTA finishes its band: slices added in rank order, scaled, stored ----
         __syncwarp();
-        pdl_wait(p.input_scale, p.w_scale, p.bias);
+        pdl_wait();
         cluster_sync_all();                                // every CTA's sums are parked
         if (warp == 1) pair_tmem_release(smem_u32(&bar_done), tmem_base, kTmemCols, p.status);
         if (!s_abort) {
