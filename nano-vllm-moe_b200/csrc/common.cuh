@@ -74,6 +74,48 @@ __host__ __device__ inline size_t pack_offset(int64_t n, int64_t k, int64_t KB) 
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Loads of what a kernel in front may have written.  Never through the read-only path (__ldg, ld.global.nc, or a plain read of a
+// const __restrict__ parameter): it promises that nobody writes the memory while this kernel runs, which a kernel that starts
+// early cannot promise, and the assembler moves such loads in front of the wait.  It did with the rows of the streaming
+// kernel when a branch stood in front of the wait: every replay of a graph of single-row steps read stale rows, eager calls
+// were too far apart to show it.
+__device__ __forceinline__ uint4 ld_dep(const uint4* p) {
+    uint4 r;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float ld_dep(const float* p) {
+    float r;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ int ld_dep(const int* p) {
+    int r;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ long long ld_dep(const long long* p) {
+    long long r;
+    asm volatile("ld.global.s64 %0, [%1];" : "=l"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float ld_dep(const __nv_bfloat16* p) {
+    unsigned short r;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(r) : "l"(p));
+    return __uint_as_float((uint32_t)r << 16);
+}
+// ... past L1: what other SMs (or peers) write while the kernel runs
+__device__ __forceinline__ uint4 ld_dep_l2(const uint4* p) {
+    uint4 r;
+    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+    return r;
+}
+__device__ __forceinline__ float2 ld_dep_l2(const float2* p) {
+    float2 r;
+    asm volatile("ld.global.cg.v2.f32 {%0,%1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(p) : "memory");
+    return r;
+}
+
 // ---- small numeric helpers ----------------------------------------------------
 __device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
@@ -199,16 +241,12 @@ __device__ __forceinline__ uint4 bf16x8_to_f16x8(uint4 v) {
     return r;
 }
 
-// Streaming 16-byte load that does not pollute L1 (weights are read once).
+// Streaming 16-byte load that does not pollute L1 (weights are read once).  The read-only path: packed weights only.
 __device__ __forceinline__ uint4 ld_stream16(const void* p) {
     uint4 r;
     asm volatile("ld.global.nc.L1::no_allocate.L2::128B.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
     return r;
-}
-
-__device__ __forceinline__ uint4 ld_cached16(const void* p) {
-    return __ldg(reinterpret_cast<const uint4*>(p));
 }
 
 }  // namespace fp8lin

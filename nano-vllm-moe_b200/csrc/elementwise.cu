@@ -38,12 +38,12 @@ act_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const float* 
     auto load = [&]() {
 #pragma unroll
         for (int u = 0; u < 2; ++u)
-            if (dst[u]) { a[u][0] = __ldg(src[u]); a[u][1] = __ldg(src[u] + 1); }
+            if (dst[u]) { a[u][0] = ld_dep(src[u]); a[u][1] = ld_dep(src[u] + 1); }
     };
     locate();
     pdl_wait();                    // x may come from the kernel before, the scale too
     if (base >= total) return;
-    const float scale = fmaxf(__ldg(input_scale), 1e-12f);
+    const float scale = fmaxf(ld_dep(input_scale), 1e-12f);
     load();                        // (in flight beside the scale, which the first quotient needs)
     const ExactDiv s(scale);
     for (;;) {
@@ -93,7 +93,7 @@ sum_slots_kernel(const __nv_bfloat16* __restrict__ slots, int n_slots, int64_t s
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int r = 0; r < n_slots; ++r) {
             // peers wrote these lines: read them past L1
-            const uint4 v = __ldcg(reinterpret_cast<const uint4*>(slots + r * slot_stride + m * ld_slot + c));
+            const uint4 v = ld_dep_l2(reinterpret_cast<const uint4*>(slots + r * slot_stride + m * ld_slot + c));
             acc[0] += bf16_lo(v.x); acc[1] += bf16_hi(v.x); acc[2] += bf16_lo(v.y); acc[3] += bf16_hi(v.y);
             acc[4] += bf16_lo(v.z); acc[5] += bf16_hi(v.z); acc[6] += bf16_lo(v.w); acc[7] += bf16_hi(v.w);
         }
@@ -129,7 +129,7 @@ sum_slots_gather_kernel(const __nv_bfloat16* __restrict__ slots, int n_slots, in
         const int64_t c = (i - m * vec_per_row) * 8;
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         for (int r = 0; r < n_slots; ++r) {
-            const uint4 v = __ldcg(reinterpret_cast<const uint4*>(slots + r * slot_stride + m * ld_slot + c));
+            const uint4 v = ld_dep_l2(reinterpret_cast<const uint4*>(slots + r * slot_stride + m * ld_slot + c));
             acc[0] += bf16_lo(v.x); acc[1] += bf16_hi(v.x); acc[2] += bf16_lo(v.y); acc[3] += bf16_hi(v.y);
             acc[4] += bf16_lo(v.z); acc[5] += bf16_hi(v.z); acc[6] += bf16_lo(v.w); acc[7] += bf16_hi(v.w);
         }
@@ -163,7 +163,7 @@ x_to_f16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __half* __rest
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / vec_per_row;
         const int64_t c = (i - r * vec_per_row) * 8;
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + r * ldx + c));
+        const uint4 v = ld_dep(reinterpret_cast<const uint4*>(x + r * ldx + c));
         *reinterpret_cast<uint4*>(x16 + r * K + c) = bf16x8_to_f16x8(v);
     }
 }
@@ -233,15 +233,15 @@ silu_mul_quant_interleaved_kernel(const __nv_bfloat16* __restrict__ gu, const fl
                                   unsigned char* __restrict__ hq, int64_t M, int64_t I) {
     pdl_launch_dependents();
     pdl_wait();
-    const ExactDiv div_scale(fmaxf(__ldg(h_scale), 1e-12f));
+    const ExactDiv div_scale(fmaxf(ld_dep(h_scale), 1e-12f));
     const int64_t vec_per_row = I / 8;
     const int64_t total = M * vec_per_row;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / vec_per_row;
         const int64_t c = (i - r * vec_per_row) * 8;
         const int64_t gcol = (c >> 7) * 256 + (c & 127);
-        const uint4 g = __ldg(reinterpret_cast<const uint4*>(gu + r * 2 * I + gcol));
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(gu + r * 2 * I + gcol + 128));
+        const uint4 g = ld_dep(reinterpret_cast<const uint4*>(gu + r * 2 * I + gcol));
+        const uint4 u = ld_dep(reinterpret_cast<const uint4*>(gu + r * 2 * I + gcol + 128));
         const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
         uint4 h;
         uint32_t* hw = reinterpret_cast<uint32_t*>(&h);
@@ -289,7 +289,7 @@ quantize_weight_kernel(const void* __restrict__ w_, int64_t ldw, unsigned char* 
     float amax = 0.f;
     if (vec) {
         for (int64_t k = 8 * (int64_t)threadIdx.x; k < K; k += 8 * 256) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(wb + k));
+            const uint4 v = ld_dep(reinterpret_cast<const uint4*>(wb + k));
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(bf16_lo(v.x)), fabsf(bf16_hi(v.x))), fmaxf(fabsf(bf16_lo(v.y)), fabsf(bf16_hi(v.y)))));
             amax = fmaxf(amax, fmaxf(fmaxf(fabsf(bf16_lo(v.z)), fabsf(bf16_hi(v.z))), fmaxf(fabsf(bf16_lo(v.w)), fabsf(bf16_hi(v.w)))));
         }
@@ -308,7 +308,7 @@ quantize_weight_kernel(const void* __restrict__ w_, int64_t ldw, unsigned char* 
     unsigned char* out = q + n * K;
     if (vec) {
         for (int64_t k = 8 * (int64_t)threadIdx.x; k < K; k += 8 * 256)
-            *reinterpret_cast<uint2*>(out + k) = quant8_e4m3(__ldg(reinterpret_cast<const uint4*>(wb + k)), d);
+            *reinterpret_cast<uint2*>(out + k) = quant8_e4m3(ld_dep(reinterpret_cast<const uint4*>(wb + k)), d);
         return;
     }
     for (int64_t k = 2 * (int64_t)threadIdx.x; k < K; k += 512) {          // K is even: two codes per store
@@ -337,7 +337,7 @@ abs_max_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int64_t M, int6
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / vec_per_row;
         const int64_t c = (i - r * vec_per_row) * 8;
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + r * ldx + c));
+        const uint4 v = ld_dep(reinterpret_cast<const uint4*>(x + r * ldx + c));
         m = fmaxf(m, fmaxf(fmaxf(fabsf(bf16_lo(v.x)), fabsf(bf16_hi(v.x))), fmaxf(fabsf(bf16_lo(v.y)), fabsf(bf16_hi(v.y)))));
         m = fmaxf(m, fmaxf(fmaxf(fabsf(bf16_lo(v.z)), fabsf(bf16_hi(v.z))), fmaxf(fabsf(bf16_lo(v.w)), fabsf(bf16_hi(v.w)))));
     }

@@ -24,7 +24,7 @@ moe_route_kernel(const LogitT* __restrict__ logits, int64_t ld, int T, int E, in
 #pragma unroll
     for (int i = 0; i < kMaxPerLane; ++i) {
         const int e = lane + 32 * i;
-        v[i] = e < E ? (float)row[e] : -INFINITY;
+        v[i] = e < E ? ld_dep(row + e) : -INFINITY;
         mx = fmaxf(mx, v[i]);
     }
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
@@ -142,7 +142,7 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
     auto load_ids = [&](int r, int end, int* e) {
 #pragma unroll
         for (int i = 0; i < kBatch; ++i) {
-            const long long id = r + 32 * i < end ? (long long)__ldg(ids + r + 32 * i) : -1;
+            const long long id = r + 32 * i < end ? (long long)ld_dep(ids + r + 32 * i) : -1;
             e[i] = id >= 0 && id < E ? (int)id : -1;
         }
     };
@@ -243,7 +243,7 @@ moe_scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x
                          const float* __restrict__ input_scale, unsigned char* __restrict__ xq, int H) {
     pdl_launch_dependents();
     pdl_wait();
-    const ExactDiv div_scale(fmaxf(__ldg(input_scale), 1e-12f));
+    const ExactDiv div_scale(fmaxf(ld_dep(input_scale), 1e-12f));
     const int vec_per_row = H / 16;
     const int tokens = (rows + x_div - 1) / x_div;
     // a block walks whole tokens, so no element needs a division to find its row
@@ -255,12 +255,12 @@ moe_scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x
         if (t >= tokens) continue;
         for (int c = per > 1 ? (int)threadIdx.x - sub * vec_per_row : (int)threadIdx.x; c < vec_per_row; c += per > 1 ? vec_per_row : 256) {
             const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)t * ldx + c * 16);
-            const uint2 qa = quant8_e4m3(__ldg(src), div_scale);
-            const uint2 qb = quant8_e4m3(__ldg(src + 1), div_scale);
+            const uint2 qa = quant8_e4m3(ld_dep(src), div_scale);
+            const uint2 qb = quant8_e4m3(ld_dep(src + 1), div_scale);
             const uint4 o = make_uint4(qa.x, qa.y, qb.x, qb.y);
             for (int j = 0; j < x_div; ++j) {
                 const int64_t r = t * x_div + j;
-                const int pos = r < rows ? __ldg(inv + r) : -1;
+                const int pos = r < rows ? ld_dep(inv + r) : -1;
                 if (pos >= 0) *reinterpret_cast<uint4*>(xq + (size_t)pos * H + c * 16) = o;
             }
         }
@@ -285,15 +285,15 @@ silu_mul_quant_kernel(const __nv_bfloat16* __restrict__ gu, const float* __restr
                       unsigned char* __restrict__ hq, const int* __restrict__ meta, int I) {
     pdl_launch_dependents();
     pdl_wait();
-    const int rows = meta[1];
-    const ExactDiv div_scale(fmaxf(__ldg(input_scale), 1e-12f));
+    const int rows = ld_dep(meta + 1);
+    const ExactDiv div_scale(fmaxf(ld_dep(input_scale), 1e-12f));
     const int vec_per_row = I / 8;
     const int64_t total = (int64_t)rows * vec_per_row;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = i / vec_per_row;
         const int c = (int)(i - r * vec_per_row) * 8;
-        const uint4 g = __ldg(reinterpret_cast<const uint4*>(gu + r * 2 * I + c));
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(gu + r * 2 * I + I + c));
+        const uint4 g = ld_dep(reinterpret_cast<const uint4*>(gu + r * 2 * I + c));
+        const uint4 u = ld_dep(reinterpret_cast<const uint4*>(gu + r * 2 * I + I + c));
         const uint32_t gw[4] = {g.x, g.y, g.z, g.w}, uw[4] = {u.x, u.y, u.z, u.w};
         uint4 h;
         uint32_t* hw = reinterpret_cast<uint32_t*>(&h);
@@ -334,8 +334,8 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ routed, const int* __restri
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     v[j] = make_uint4(0u, 0u, 0u, 0u);
-                    if (j0 + j < top_k && (!inv || __ldg(inv + t * top_k + j0 + j) >= 0))
-                        v[j] = __ldg(reinterpret_cast<const uint4*>(src + (size_t)(j0 + j) * H + c * 8));
+                    if (j0 + j < top_k && (!inv || ld_dep(inv + t * top_k + j0 + j) >= 0))
+                        v[j] = ld_dep(reinterpret_cast<const uint4*>(src + (size_t)(j0 + j) * H + c * 8));
                 }
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {

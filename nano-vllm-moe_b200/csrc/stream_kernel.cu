@@ -140,7 +140,7 @@ stream_linear_kernel(StreamArgs p) {
             const int r = v / XS::kVecPerRow;
             const int k = k0 + (v % XS::kVecPerRow) * 8;
             xr[i] = make_uint4(0, 0, 0, 0);
-            if (v < XS::kVecs && r < m_valid && k < k_end) xr[i] = ld_cached16(x + (size_t)r * p.ldx + k);
+            if (v < XS::kVecs && r < m_valid && k < k_end) xr[i] = ld_dep(reinterpret_cast<const uint4*>(x + (size_t)r * p.ldx + k));
         }
     };
     auto store_x = [&](int buf, int part) {
@@ -181,7 +181,7 @@ stream_linear_kernel(StreamArgs p) {
     for (int s = 0; s < 4; ++s) load_w_step(0, s);       // weights first: they do not depend on the predecessor
     pdl_launch_dependents();
     pdl_wait();                                           // x, y and the split-K scratch may belong to the predecessor, scales and bias too
-    if (SCHEME == FP8LIN_W8A8_STATIC) in_scale = __ldg(p.input_scale);
+    if (SCHEME == FP8LIN_W8A8_STATIC) in_scale = ld_dep(p.input_scale);
     load_x(0, 0);                                         // (in flight beside the scale, which the first quotient needs)
     if (SCHEME == FP8LIN_W8A8_STATIC) {
         in_scale = fmaxf(in_scale, 1e-12f);
@@ -293,11 +293,11 @@ stream_linear_kernel(StreamArgs p) {
             for (int mt = 0; mt < MT; ++mt) {
                 const int m = mt * 8 + 2 * t;
                 if (n_a < p.N) {
-                    const float2 v = __ldcg(reinterpret_cast<const float2*>(ps + (size_t)n_a * MP + m));
+                    const float2 v = ld_dep_l2(reinterpret_cast<const float2*>(ps + (size_t)n_a * MP + m));
                     acc[mt][0] += v.x; acc[mt][1] += v.y;
                 }
                 if (n_b < p.N) {
-                    const float2 v = __ldcg(reinterpret_cast<const float2*>(ps + (size_t)n_b * MP + m));
+                    const float2 v = ld_dep_l2(reinterpret_cast<const float2*>(ps + (size_t)n_b * MP + m));
                     acc[mt][2] += v.x; acc[mt][3] += v.y;
                 }
             }
@@ -306,8 +306,8 @@ stream_linear_kernel(StreamArgs p) {
 
     __nv_bfloat16* y = p.y + (size_t)m_base * p.ldy;
     float sa = 0.f, sb = 0.f, ba = 0.f, bb = 0.f;
-    if (n_a < p.N) { sa = __ldg(p.w_scale + n_a); if (p.bias) ba = __bfloat162float(p.bias[n_a]); }
-    if (n_b < p.N) { sb = __ldg(p.w_scale + n_b); if (p.bias) bb = __bfloat162float(p.bias[n_b]); }
+    if (n_a < p.N) { sa = ld_dep(p.w_scale + n_a); if (p.bias) ba = ld_dep(p.bias + n_a); }
+    if (n_b < p.N) { sb = ld_dep(p.w_scale + n_b); if (p.bias) bb = ld_dep(p.bias + n_b); }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
         const int m = mt * 8 + 2 * t;

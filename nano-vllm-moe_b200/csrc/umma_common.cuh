@@ -335,8 +335,8 @@ __device__ __forceinline__ void finish_parked_band(const UmmaArgs& p, uint32_t s
         float4 a = u[0];
 #pragma unroll
         for (int sl = 1; sl < 4; ++sl) { a.x += u[sl].x; a.y += u[sl].y; a.z += u[sl].z; a.w += u[sl].w; }
-        const float ws = factor * __ldg(p.w_scale + n);
-        const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
+        const float ws = factor * ld_dep(p.w_scale + n);
+        const float bs = p.bias ? ld_dep(p.bias + n) : 0.f;
         const float o[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j)
@@ -468,7 +468,7 @@ __device__ __forceinline__ bool quant_probe_block(const QuantJob& j, int M, int 
 
 // One quantiser warp: take units until none are left.
 __device__ __forceinline__ void quant_worker(const QuantJob& j, const float* input_scale, int M, int K, int lane) {
-    const ExactDiv div(fmaxf(__ldg(input_scale), 1e-12f));
+    const ExactDiv div(fmaxf(ld_dep(input_scale), 1e-12f));
     const int total_units = M > j.row_start ? (M - j.row_start + kQuantRows - 1) / kQuantRows : 0;
     const int vec_per_row = K >> 4;
     for (;;) {
@@ -497,8 +497,8 @@ __device__ __forceinline__ void quant_worker(const QuantJob& j, const float* inp
                 uint4 a[4][2];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
-                    a[q][0] = ld_stream16(src[q] + v * 16);
-                    a[q][1] = ld_stream16(src[q] + v * 16 + 8);
+                    a[q][0] = ld_dep(reinterpret_cast<const uint4*>(src[q] + v * 16));
+                    a[q][1] = ld_dep(reinterpret_cast<const uint4*>(src[q] + v * 16 + 8));
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {

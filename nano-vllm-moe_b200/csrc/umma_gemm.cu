@@ -301,7 +301,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         const int h = ew >> 2;
         const int et = threadIdx.x - 64;                            // 0..255 among the epilogue threads
         constexpr int kPiece = Cfg::kPiece;
-        const float in_scale = p.input_scale ? fmaxf(__ldg(p.input_scale), 1e-12f) : 1.f;   // W8A16: weights' scale only
+        const float in_scale = p.input_scale ? fmaxf(ld_dep(p.input_scale), 1e-12f) : 1.f;   // W8A16: weights' scale only
         const uint32_t box = smem_base + Cfg::kRingBytes + ew * Cfg::kBoxBytes;
         const uint32_t row_off = lane * (kPiece * 2);
         const uint32_t sw = kPiece == 64 ? (lane & 7) : ((lane >> 1) & 3);   // 128-byte / 64-byte swizzle
@@ -314,7 +314,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             const WorkItem f = decode_work<BN, kNarrow>(sched, work);
             const int n = f.n0 + et;
             const bool in = et < f.bn && n < p.N;
-            next_scale = in ? in_scale * __ldg(p.w_scale + n) : 0.f;
+            next_scale = in ? in_scale * ld_dep(p.w_scale + n) : 0.f;
             next_bias = (in && p.bias) ? p.bias[n] : __float2bfloat16(0.f);
         };
         if (first_work < sched.total_work) fetch_columns(first_work);

@@ -185,7 +185,7 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
             constexpr int kTeams = kGrpConvWarps / Cfg::kTeam;
             const int team = (warp - 2) / Cfg::kTeam;       // a ring slot always belongs to the same team
             const int member = (warp - 2) % Cfg::kTeam;
-            const ExactDiv div_scale(fmaxf(__ldg(p.input_scale), 1e-12f));
+            const ExactDiv div_scale(fmaxf(ld_dep(p.input_scale), 1e-12f));
             uint32_t it = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
@@ -204,10 +204,10 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
                         const int k = kb * kGrpKB + c * 16;
                         uint2 qa = make_uint2(0u, 0u), qb = make_uint2(0u, 0u);
                         if (r < ch.z && k < p.K) {
-                            const int src_row = __ldg(p.sorted_rows + ch.y + r) / p.x_div;
+                            const int src_row = ld_dep(p.sorted_rows + ch.y + r) / p.x_div;
                             const uint4* src = reinterpret_cast<const uint4*>(p.x + (size_t)src_row * p.ldx + k);
-                            qa = quant8_e4m3(__ldg(src), div_scale);
-                            qb = quant8_e4m3(__ldg(src + 1), div_scale);
+                            qa = quant8_e4m3(ld_dep(src), div_scale);
+                            qb = quant8_e4m3(ld_dep(src + 1), div_scale);
                         }
                         const uint32_t dst = xq + r * 128 + (((uint32_t)c ^ (uint32_t)(r & 7)) << 4);
                         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(qa.x), "r"(qa.y), "r"(qb.x),
@@ -222,7 +222,7 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
     } else {
         // ================= epilogue (warps 10..13) =================
         const int q = warp & 3;
-        const float in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
+        const float in_scale = fmaxf(ld_dep(p.input_scale), 1e-12f);
         int tl = 0;
         bool ok = true;
         for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++tl) {
@@ -234,7 +234,7 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
             // of quarters 0, 1)
             const bool up = kFused && q >= 2;
             const int n = kFused ? t * 64 + (q & 1) * 32 + lane : t * kGrpTile + q * 32 + lane;
-            const float ws = n < p.N ? in_scale * __ldg(p.w_scale + (kFused ? (size_t)ch.x * 2 * p.N + (up ? p.N : 0) : (size_t)ch.x * p.N) + n) : 0.f;
+            const float ws = n < p.N ? in_scale * ld_dep(p.w_scale + (kFused ? (size_t)ch.x * 2 * p.N + (up ? p.N : 0) : (size_t)ch.x * p.N) + n) : 0.f;
             // routed-row index and routing weight of the chunk's rows, one row per lane and piece;
             // the inner loop gets them by shuffle instead of two dependent global loads per row
             int my_routed[(MP + 31) / 32];
@@ -244,8 +244,8 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
                 const int r = i * 32 + lane;
                 my_routed[i] = 0; my_w[i] = 0.f;
                 if (p.scatter && r < ch.z) {
-                    my_routed[i] = __ldg(p.sorted_rows + ch.y + r);
-                    my_w[i] = __ldg(p.topk_w + my_routed[i]);
+                    my_routed[i] = ld_dep(p.sorted_rows + ch.y + r);
+                    my_w[i] = ld_dep(p.topk_w + my_routed[i]);
                 }
             }
             bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull);
@@ -255,7 +255,7 @@ grouped_w8a8_kernel(const __grid_constant__ GroupedMaps maps, GroupedArgs p) {
             const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + as * Cfg::kAccCols;
             if constexpr (kFused) {
                 constexpr int kP = Cfg::kPiece, kH = kP / 4;      // rows per step; column pairs each warp of a pair finishes
-                const ExactDiv div_h(fmaxf(__ldg(p.h_scale), 1e-12f));
+                const ExactDiv div_h(fmaxf(ld_dep(p.h_scale), 1e-12f));
                 const uint32_t swap_buf = smem_u32(s_swap) + (uint32_t)(q & 1) * (kP * 64);
                 const uint32_t code_buf = smem_u32(s_code) + (uint32_t)(q & 1) * (kP * 32);
 #pragma unroll 1

@@ -147,8 +147,8 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         const int q = warp & 3;                   // TMEM lane quarter = rows [32q, 32q + 32) of the item
         const int h = ew >> 2;                    // column half of the item
         const int et = threadIdx.x - 64;          // 0..255 among the epilogue threads: stages column et's multiplier
-        const float in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
-        const ExactDiv div_h(kFusedAct ? fmaxf(__ldg(p.h_scale), 1e-12f) : 1.f);
+        const float in_scale = fmaxf(ld_dep(p.input_scale), 1e-12f);
+        const ExactDiv div_h(kFusedAct ? fmaxf(ld_dep(p.h_scale), 1e-12f) : 1.f);
         int tl = 0;
         bool ok = true;
         auto column_scale = [&](int work) -> float {
@@ -156,10 +156,10 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             const int t = work % n_items;
             if (kFusedAct) {                      // columns [0,128) gate channels 128 t + c, [128,256) the up channels of the same c
                 const int ch_idx = t * 128 + (et & 127);
-                return ch_idx < p.N ? in_scale * __ldg(p.w_scale + (size_t)c.x * 2 * p.N + (et >> 7) * p.N + ch_idx) : 0.f;
+                return ch_idx < p.N ? in_scale * ld_dep(p.w_scale + (size_t)c.x * 2 * p.N + (et >> 7) * p.N + ch_idx) : 0.f;
             }
             const int n = t * kColsN + et;
-            return n < p.N ? in_scale * __ldg(p.w_scale + (size_t)c.x * p.N + n) : 0.f;
+            return n < p.N ? in_scale * ld_dep(p.w_scale + (size_t)c.x * p.N + n) : 0.f;
         };
         float next_scale = blockIdx.x < total ? column_scale(blockIdx.x) : 0.f;
         for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++tl) {
@@ -175,8 +175,8 @@ grouped_rows_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             int routed = 0;
             float rw = 0.f;
             if (!kFusedAct && live) {
-                routed = __ldg(p.sorted_rows + ch.y + r);
-                rw = __ldg(p.topk_w + routed);
+                routed = ld_dep(p.sorted_rows + ch.y + r);
+                rw = ld_dep(p.topk_w + routed);
             }
             const bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull);
             if (named_sync_any(1, 256, !arrived)) { s_abort = 1; ok = false; break; }

@@ -207,7 +207,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int q = warp & 3;
         const int h = ew >> 2;
         const int et = threadIdx.x - 64;                            // 0..255 among the epilogue threads
-        const float in_scale = p.input_scale ? fmaxf(__ldg(p.input_scale), 1e-12f) : 1.f;
+        const float in_scale = p.input_scale ? fmaxf(ld_dep(p.input_scale), 1e-12f) : 1.f;
         const uint32_t pbox = smem_base + kRingBytes + q * kBoxBytes;
         int tl = 0;
         bool ok = true;
@@ -218,7 +218,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             decode_pair_tile(sched, tile, ftmp, ftn);
             const int n = ftn * kBN + et;
             const bool in = n < p.N;
-            next_scale = in ? in_scale * __ldg(p.w_scale + n) : 0.f;
+            next_scale = in ? in_scale * ld_dep(p.w_scale + n) : 0.f;
             next_bias = (in && p.bias) ? p.bias[n] : __float2bfloat16(0.f);
         };
         if (first_tile < sched.total) fetch_columns(first_tile);
@@ -240,7 +240,7 @@ umma_pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if (kMlp) {
                 // warp h owns output bytes [64h, 64h + 64) of the tile's 128: two steps of 32 columns, each from
                 // 32 gate accumulators (columns c..) and the 32 up accumulators 128 columns further on
-                const ExactDiv div_h(fmaxf(__ldg(h_scale), 1e-12f));
+                const ExactDiv div_h(fmaxf(ld_dep(h_scale), 1e-12f));
                 const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + as * kBN;
                 if (n0 < p.N) {
 #pragma unroll 1

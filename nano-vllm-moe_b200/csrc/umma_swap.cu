@@ -178,12 +178,12 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // scale and bias of the first channel this thread finishes, fetched long before they are needed
     float ws0 = 0.f, bs0 = 0.f, in_scale0 = 0.f;
     auto fetch_first = [&]() {
-        in_scale0 = fmaxf(__ldg(p.input_scale), 1e-12f);
+        in_scale0 = fmaxf(ld_dep(p.input_scale), 1e-12f);
         if (band_rows > 0 && (int)threadIdx.x < band_rows * m_groups) {
             const int n0 = first_tile * kTileN + split_rank * band + (int)threadIdx.x % band_rows;
             if (n0 < p.N) {
-                ws0 = __ldg(p.w_scale + n0);
-                if (p.bias) bs0 = __bfloat162float(p.bias[n0]);
+                ws0 = ld_dep(p.w_scale + n0);
+                if (p.bias) bs0 = ld_dep(p.bias + n0);
             }
         }
     };
@@ -276,7 +276,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const int kTeams = kConvWarps / team_sz;
         const int team = (warp - 2) / team_sz;               // a ring slot always belongs to the same team
         const int member = (warp - 2) % team_sz;
-        const ExactDiv div_scale(fmaxf(__ldg(p.input_scale), 1e-12f));
+        const ExactDiv div_scale(fmaxf(ld_dep(p.input_scale), 1e-12f));
         const int items = p.M * 8;                          // (row, 16-element chunk) pairs of the real rows
         uint32_t it = 0;
         bool ok = true;
@@ -314,11 +314,11 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     } else {
         // ================= epilogue (warps 10..13) =================
         const int q = warp & 3;
-        const float in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
+        const float in_scale = fmaxf(ld_dep(p.input_scale), 1e-12f);
         bool ok = true;
         if constexpr (kGateUp) {
             // ---- pairs of tiles: h = silu(gate) * up, quantised for the down projection ----
-            const ExactDiv div_h(fmaxf(__ldg(p.h_scale), 1e-12f));
+            const ExactDiv div_h(fmaxf(ld_dep(p.h_scale), 1e-12f));
             const int inter = p.N >> 1;
             const int groups = (p.M + 7) >> 3;                                     // rows travel in groups of eight bf16
             const uint32_t recv = smem_base + Cfg::kRingBytes + (uint32_t)(q * 32 + lane) * (MP * 2);
@@ -330,8 +330,8 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 const int as = tl & 1;
                 const uint32_t aph = (tl >> 1) & 1;
                 const int n = t * kTileN + q * 32 + lane;                           // (N is a multiple of 256: in range)
-                const float ws = __ldg(p.w_scale + n);
-                const float bs = p.bias ? __bfloat162float(p.bias[n]) : 0.f;
+                const float ws = ld_dep(p.w_scale + n);
+                const float bs = p.bias ? ld_dep(p.bias + n) : 0.f;
                 uint32_t v[MP];
                 if (!mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull)) { s_abort = 1; ok = false; break; }
                 tc_fence_after();
@@ -399,8 +399,8 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             const int n = t * kTileN + q * 32 + lane;
             float ws = 0.f, bs = 0.f;
             if (!kSplit && n < p.N) {
-                ws = __ldg(p.w_scale + n);
-                if (p.bias) bs = __bfloat162float(p.bias[n]);
+                ws = ld_dep(p.w_scale + n);
+                if (p.bias) bs = ld_dep(p.bias + n);
             }
             if (!mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull)) { s_abort = 1; ok = false; break; }
             tc_fence_after();
@@ -463,8 +463,8 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
                 }
             }
             const bool first = i == (int)threadIdx.x;
-            const float ws = first ? ws0 : __ldg(p.w_scale + n);
-            const float bs = first ? bs0 : (p.bias ? __bfloat162float(p.bias[n]) : 0.f);
+            const float ws = first ? ws0 : ld_dep(p.w_scale + n);
+            const float bs = first ? bs0 : (p.bias ? ld_dep(p.bias + n) : 0.f);
             const float o[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j)

@@ -162,8 +162,8 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         if (band_rows > 0 && (int)threadIdx.x < band_rows * m_groups) {
             const int n0 = first_tile * kS16Tile + split_rank * band + (int)threadIdx.x % band_rows;
             if (n0 < p.N) {
-                ws0 = __ldg(p.w_scale + n0);
-                if (p.bias) bs0 = __bfloat162float(p.bias[n0]);
+                ws0 = ld_dep(p.w_scale + n0);
+                if (p.bias) bs0 = ld_dep(p.bias + n0);
             }
         }
     };
@@ -306,8 +306,8 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             const int n = t * kS16Tile + q * 32 + lane;
             float ws = 0.f, bs = 0.f;
             if (!kSplit && n < p.N) {
-                ws = __ldg(p.w_scale + n);
-                if (p.bias) bs = __bfloat162float(p.bias[n]);
+                ws = ld_dep(p.w_scale + n);
+                if (p.bias) bs = ld_dep(p.bias + n);
             }
             if (!mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull)) { s_abort = 1; ok = false; break; }
             tc_fence_after();
@@ -367,8 +367,8 @@ swap_w8a16_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                 }
             }
             const bool first = i == (int)threadIdx.x;
-            const float ws = first ? ws0 : __ldg(p.w_scale + n);
-            const float bs = first ? bs0 : (p.bias ? __bfloat162float(p.bias[n]) : 0.f);
+            const float ws = first ? ws0 : ld_dep(p.w_scale + n);
+            const float bs = first ? bs0 : (p.bias ? ld_dep(p.bias + n) : 0.f);
             const float o[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
             for (int j = 0; j < 4; ++j)

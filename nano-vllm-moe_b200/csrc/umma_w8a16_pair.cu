@@ -353,8 +353,8 @@ w8a16_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             const int m0 = (item % sched.m_tiles) * T + h * half;
             float ws = 0.f, bs = 0.f;
             if (!kSplit && n < p.N) {
-                ws = __ldg(p.w_scale + n);
-                if (p.bias) bs = __bfloat162float(p.bias[n]);
+                ws = ld_dep(p.w_scale + n);
+                if (p.bias) bs = ld_dep(p.bias + n);
             }
             if (!mbar_wait(smem_u32(&bar_tfull[as]), aph, p.status, kDevTimeoutTmemFull)) { s_abort = 1; ok = false; break; }
             tc_fence_after();

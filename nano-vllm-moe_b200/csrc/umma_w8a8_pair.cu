@@ -86,7 +86,7 @@ __device__ __forceinline__ Item decode_item(const PairSched8& s, int item) {
 // product of the scales above, as the 256-row kernels do.  The bf16 results of a row count are the same bits whichever kernel
 // takes it.  Returns the factor of the channel's scale; `pre` multiplies the sum.
 __device__ __forceinline__ float channel_factor(const UmmaArgs& p, float& pre) {
-    const float in_scale = fmaxf(__ldg(p.input_scale), 1e-12f);
+    const float in_scale = fmaxf(ld_dep(p.input_scale), 1e-12f);
     pre = p.M <= 64 ? in_scale : 1.f;
     return p.M <= 64 ? 1.f : in_scale;
 }
@@ -231,7 +231,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         const int h = (warp - 2) >> 2;                     // which half of the tile's tokens
         float pre;
         const float in_scale = channel_factor(p, pre);
-        const ExactDiv div_h(kMlp ? fmaxf(__ldg(p.h_scale), 1e-12f) : 1.f);
+        const ExactDiv div_h(kMlp ? fmaxf(ld_dep(p.h_scale), 1e-12f) : 1.f);
         const bool odd = lane & 1;
         const bool up = kMlp && q >= 2;
         const int pair = (q & 1) + 2 * h;                  // kMlp: the warps of quarters q and q ^ 2 share 32 channels
@@ -245,8 +245,8 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
             const int n = kMlp ? it.nt * 256 + (up ? 128 : 0) + (int)rank * 64 + (q & 1) * 32 + lane : (2 * it.nt + (int)rank) * kTile + q * 32 + lane;
             float ws = 0.f, bs = 0.f;
             if (!kSplit && n < p.N) {
-                ws = in_scale * __ldg(p.w_scale + n);
-                if (p.bias) bs = __bfloat162float(p.bias[n]);
+                ws = in_scale * ld_dep(p.w_scale + n);
+                if (p.bias) bs = ld_dep(p.bias + n);
             }
             bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1), p.status, kDevTimeoutTmemFull);
             if (kMlp) arrived = !named_sync_any(5, 256, !arrived);        // warps that meet at barriers below leave together

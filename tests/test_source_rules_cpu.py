@@ -56,20 +56,42 @@ def test_named_barriers_do_not_ask_for_a_converged_warp():
             assert not asm, f"{name}: {asm}"
 
 
+def waiting_kernels():
+    """(file, name, signature, body) of every kernel that waits for the one in front of it."""
+    for name, text in SOURCES.items():
+        for head in re.finditer(r"__global__[^{;]*?\b(\w+_kernel)\(", text):
+            rest = " " + text[head.end(1) - len(head.group(1)):]
+            code = body(rest, head.group(1))
+            if "pdl_wait(" in code:
+                yield name, head.group(1), rest[:rest.index("{")], code
+
+
 def test_only_packed_weights_are_read_before_the_wait_for_the_kernel_in_front():
     """A bias or a norm's weight may be a copy that the caller's last kernel wrote; only griddepcontrol.wait orders it."""
     early = re.compile(r"\b(bias|weight|w_scale|input_scale|h_scale|topk_w|residual)\b")
-    kernels = 0
+    found = {}
+    for file, kernel, _, code in waiting_kernels():
+        before = re.sub(r"if \([^;{]*\) prefetch_l2\([^;]*;|prefetch_l2\([^;]*;", "", code[:code.index("pdl_wait(")])
+        found[file, kernel] = early.findall(before)
+    assert len(found) > 15 and not any(found.values()), {k: v for k, v in found.items() if v}
+
+
+def test_nothing_but_weights_goes_through_the_read_only_path():
+    """Read-only loads promise that nobody writes the memory while the kernel runs, and the assembler moves them in front of the
+    wait for the kernel that does: packed weights alone may take that path."""
+    weights = {"stream_kernel.cu": ["wa + tile_off(k)", "wb + tile_off(k)"], "elementwise.cu": ["src + off"]}
     for name, text in SOURCES.items():
-        for head in re.finditer(r"__global__[^{;]*?\b(\w+_kernel)\(", text):
-            code = body(text[head.start():], head.group(1)) if f" {head.group(1)}(" in text[head.start():] else \
-                body(" " + text[head.start():].replace("\n" + head.group(1) + "(", "\n " + head.group(1) + "(", 1), head.group(1))
-            if "pdl_wait()" not in code:
-                continue
-            kernels += 1
-            found = early.findall(code[:code.index("pdl_wait()")])
-            assert not found, f"{name}: {head.group(1)} reads {found} too early"
-    assert kernels > 15
+        if name == "common.cuh":
+            assert len(re.findall(r"ld\.global\.nc", text)) == 1 and "ld.global.nc" in body(text, "ld_stream16")
+            text = text.replace(body(text, "ld_stream16"), "")
+            assert "ld.global.nc" not in text
+        else:
+            assert re.findall(r"ld_stream16\(([^;]*)\);", text) == weights.get(name, []), name
+            assert "ld.global" not in text, name
+        assert not re.search(r"__ld(?:g|cg|ca|cs|lu|cv)\(", text), name
+    for file, kernel, signature, code in waiting_kernels():
+        for pointer in re.findall(r"const (?:\w+|\w+ \w+)\* __restrict__ (\w+)", signature):
+            assert not re.search(rf"\b{pointer}\[|\*{pointer}\b", code), f"{file}: {kernel} reads {pointer} plainly"
 
 
 def test_tensor_memory_is_handed_over_at_cluster_scope():
