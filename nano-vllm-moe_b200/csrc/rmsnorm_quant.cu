@@ -33,7 +33,6 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     // the row and of the operands it meets later, are in flight together, and every thread adds the warps' partial sums itself
     // (one barrier instead of two).
     pdl_wait();                                     // x and the residual come from the kernels before, perhaps a copy of the weight too
-    const float scale = quant ? fmaxf(ld_dep(input_scale), 1e-12f) : 1.f;
     const int64_t row = blockIdx.x;
     const __nv_bfloat16* xr = x + row * ldx;
     __nv_bfloat16* rr = residual ? residual + row * ld_res : nullptr;
@@ -47,7 +46,7 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
             w[j] = ld_dep(reinterpret_cast<const uint4*>(weight + vec * 8));
         }
     }
-    const ExactDiv div(scale);
+    const ExactDiv div(quant ? fmaxf(ld_dep(input_scale), 1e-12f) : 1.f);    // behind the row's loads: its use holds the warp
     float v[kNormMaxVec][8];
     float ss = 0.f;
 #pragma unroll

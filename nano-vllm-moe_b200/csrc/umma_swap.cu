@@ -175,10 +175,11 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     // Everything but the packed weights may come from the kernel in front -- the rows, but also a bias or a scale that the
     // caller has just converted.  The producer warp waits by itself, between the weights and the rows.
     if (warp != 0) pdl_wait();
-    // scale and bias of the first channel this thread finishes, fetched long before they are needed
+    // Scale and bias of the first channel this thread finishes, fetched long before they are needed.  Nothing is computed from
+    // the first load before the others are out: a value that is needed at once holds the warp, and they would come one by one.
     float ws0 = 0.f, bs0 = 0.f, in_scale0 = 0.f;
     auto fetch_first = [&]() {
-        in_scale0 = fmaxf(ld_dep(p.input_scale), 1e-12f);
+        in_scale0 = ld_dep(p.input_scale);
         if (band_rows > 0 && (int)threadIdx.x < band_rows * m_groups) {
             const int n0 = first_tile * kTileN + split_rank * band + (int)threadIdx.x % band_rows;
             if (n0 < p.N) {
@@ -276,7 +277,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const int kTeams = kConvWarps / team_sz;
         const int team = (warp - 2) / team_sz;               // a ring slot always belongs to the same team
         const int member = (warp - 2) % team_sz;
-        const ExactDiv div_scale(fmaxf(ld_dep(p.input_scale), 1e-12f));
+        const ExactDiv div_scale(fmaxf(kSplit ? in_scale0 : ld_dep(p.input_scale), 1e-12f));
         const int items = p.M * 8;                          // (row, 16-element chunk) pairs of the real rows
         uint32_t it = 0;
         bool ok = true;
@@ -446,7 +447,7 @@ swap_w8a8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         }
         if ((int)threadIdx.x >= band_rows * m_groups) return;
         if (s_abort || !mbar_wait(smem_u32(&bar_recv), 0, p.status, kDevTimeoutPeer)) return;
-        const float in_scale = in_scale0;
+        const float in_scale = fmaxf(in_scale0, 1e-12f);
         // consecutive threads take consecutive channels, so the stores of one token coalesce
         for (int i = threadIdx.x; i < band_rows * m_groups; i += kSwapThreads) {
             const int rl = i % band_rows;
