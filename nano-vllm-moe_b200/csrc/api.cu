@@ -1,4 +1,5 @@
 // extern "C" surface of libfp8lin.so (declared in include/fp8lin.h).
+#include <math.h>
 #include <stdarg.h>
 #include <atomic>
 #include <stdio.h>
@@ -45,6 +46,7 @@ struct Tuning {
     int fuse_quant = -1;        // large-M W8A8: <= 0 (default) = quantise x in a separate pass; 1 = the pass takes the rows
                                 // of the first round of tiles, the GEMM's own quantiser warps the rest; n > 1 = the pass
                                 // takes the first n rows (rounded up to 128)
+    int moe_pair = -1;          // 0 = prefill-sized expert batches never on CTA pairs; 32..320 = always, with chunks of at most so many rows
     int moe_rows_major = -1;    // 0 = prefill-sized expert batches stay on the channel-major grouped kernel
     int mlp_decode_fused = -1;  // 1 = the fused MLP on up to 16 pre-quantised rows computes silu * up in the gate_up kernel (study knob)
     int moe_fused = -1;         // 0 = the expert FFN keeps its separate silu-multiply-quantise pass for every batch size
@@ -996,6 +998,7 @@ int fp8lin_set_tuning(const char* knob, int value) {
     else if (!strcmp(knob, "stream_push")) set_stream_push(value != 0);
     else if (!strcmp(knob, "mlp_decode_fused")) g_tune.mlp_decode_fused = value;
     else if (!strcmp(knob, "moe_fused")) g_tune.moe_fused = value;
+    else if (!strcmp(knob, "moe_pair")) g_tune.moe_pair = value;
     else if (!strcmp(knob, "moe_rows_major")) g_tune.moe_rows_major = value;
     else if (!strcmp(knob, "pair_stages")) set_pair_stages(value);
     else if (!strcmp(knob, "pdl")) set_pdl_enabled(value != 0);
@@ -1025,6 +1028,28 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
     w.off_xq = take(rows >= kMoePrequantRows ? (size_t)rows * H : 0);
     w.total = o;
     return w;
+}
+}  // namespace
+
+// Expert batches on CTA pairs (umma_grouped_pair.cu): the most rows of a chunk, 0 = one CTA's kernels.
+//   The line: more than 32 rows per expert, of at least kMoePrequantRows.  Measured (us per block in a loop, one CTA / pairs): 60
+//   experts 2048 -> 1408, 34 rows each 119 / 110, 68 rows 129 / 124, 136 rows 175 / 150, 273 rows 258 / 207; 64 experts 1024 -> 512,
+//   40 rows 57 / 49; 8 experts 1024 -> 512, 4096 rows 132 / 116; but 30 experts 1152 -> 1200, 26 rows 47.0 / 48.5.  Up to 128 rows a pair
+//   has to have two work items of either projection: 16 experts 2048 -> 1024, 75 rows 43.7 / 47.0 (128 items, 74 pairs); a chunk of more
+//   can be cut (8 experts 1024 -> 1408, 175 rows, 88 items 41.4 / 38.6).
+//   The chunk: a busy expert's rows, should the tokens choose at random (mean and three deviations), where that is 320 or less:
+//   273 rows on average 207 in chunks of up to 320, 215 of 288 (a sixth of the experts in two), 238 of 256; 256 above (512 rows
+//   112 / 113.5 in chunks of up to 320, 4096 rows 116 / 119).  Shorter chunks leave room for more slots, but below 192 rows that buys nothing.
+namespace {
+int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, int64_t ld_out) {
+    if (g_tune.moe_pair == 0 || g_tune.moe_fused == 0 || g_tune.moe_rows_major >= 0 || rows < kMoePrequantRows || E > 1024) return 0;
+    if (ld_out % 2 != 0 || (reinterpret_cast<uintptr_t>(out) & 3) != 0) return 0;                      // (two channels per store)
+    if (g_tune.moe_pair > 0) return (int)align_up((size_t)(g_tune.moe_pair < kGroupedPairMaxRows ? g_tune.moe_pair : kGroupedPairMaxRows), 32);
+    const int64_t avg = (rows + E - 1) / E;
+    const int64_t items = E * (pack_ntiles(I) < (pack_ntiles(H) + 1) / 2 ? pack_ntiles(I) : (pack_ntiles(H) + 1) / 2);
+    if (avg <= 32 || (avg <= 128 && items < sm_count())) return 0;
+    const int64_t busy = (int64_t)align_up((size_t)((double)avg + 3.0 * sqrt((double)avg)), 32);
+    return busy < 192 ? 192 : busy <= kGroupedPairMaxRows || avg <= 288 ? (int)(busy < kGroupedPairMaxRows ? busy : kGroupedPairMaxRows) : 256;
 }
 }  // namespace
 
@@ -1059,7 +1084,7 @@ int fp8lin_moe_align(const int32_t* ids, int64_t rows, int E, int chunk_rows, in
         return fail(FP8LIN_ERR_ARG, "chunk_rows must be 16, 32, 64 or 128");
     if (!ids || !expert_offsets || !sorted_rows || !chunks || !meta) return fail(FP8LIN_ERR_NULL, "a required pointer is NULL");
     if (!aligned16(chunks)) return fail(FP8LIN_ERR_ALIGN, "chunks must be 16-byte aligned");
-    cudaError_t e = launch_moe_align(ids, false, (int)rows, E, chunk_rows, expert_offsets, sorted_rows, (int4*)chunks, meta, nullptr,
+    cudaError_t e = launch_moe_align(ids, false, (int)rows, E, chunk_rows, false, expert_offsets, sorted_rows, (int4*)chunks, meta, nullptr,
                                      (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
@@ -1099,11 +1124,12 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     int* inv = (int*)(ws + L.off_inv);
     __nv_bfloat16* gu = (__nv_bfloat16*)(ws + L.off_gu);
     unsigned char* hq = ws + L.off_hq;
-    const int mp = grouped_chunk_rows(rows, E);
-    // Prefill-sized batches whose experts fill 128-row chunks: the rows are the MMA M dimension (umma_grouped_rows.cu), in
+    const int pair_rows = moe_pair_rows(rows, E, H, I, out_routed, ld_out);
+    const int mp = pair_rows ? pair_rows : grouped_chunk_rows(rows, E);
+    // Few work items whose experts fill 128-row chunks: the rows are the MMA M dimension (umma_grouped_rows.cu), in
     // gate_up where the up channels start at a tile.
-    const bool rows_major = rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
-    cudaError_t e = launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
+    const bool rows_major = !pair_rows && rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
+    cudaError_t e = launch_moe_align(ids, ids_i64, (int)rows, E, mp, pair_rows != 0, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
     GroupedArgs a;
@@ -1119,7 +1145,8 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
         unsigned char* xq = ws + L.off_xq;
         e = launch_moe_scatter_quant((const __nv_bfloat16*)x, ldx, x_div, inv, (int)rows, w13_input_scale, xq, (int)H, st);
         if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row quantiser launch: %s", cudaGetErrorString(e));
-        e = rows_major && fused_act && I % 128 == 0 ? launch_grouped_rows_w8a8(g, w13_packed, E, xq, rows, st, &why)
+        e = pair_rows ? launch_grouped_pair_w8a8(g, pair_rows, w13_packed, E, xq, rows, st, &why)
+          : rows_major && fused_act && I % 128 == 0 ? launch_grouped_rows_w8a8(g, w13_packed, E, xq, rows, st, &why)
                                                     : launch_grouped_w8a8(false, mp, g, w13_packed, E, xq, rows, st, &why);
     } else {
         e = launch_grouped_w8a8(true, mp, g, w13_packed, E, nullptr, 0, st, &why);
@@ -1131,7 +1158,8 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     }
     a.w_scale = w2_scale; a.input_scale = w2_input_scale; a.out = (__nv_bfloat16*)out_routed; a.ld_out = (int)ld_out;
     a.N = (int)H; a.K = (int)I; a.scatter = 1;
-    e = rows_major && ld_out % 8 == 0 && aligned16(out_routed) ? launch_grouped_rows_w8a8(a, w2_packed, E, hq, rows, st, &why)
+    e = pair_rows ? launch_grouped_pair_w8a8(a, pair_rows, w2_packed, E, hq, rows, st, &why)
+      : rows_major && ld_out % 8 == 0 && aligned16(out_routed) ? launch_grouped_rows_w8a8(a, w2_packed, E, hq, rows, st, &why)
                                                                : launch_grouped_w8a8(false, mp, a, w2_packed, E, hq, rows, st, &why);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "down grouped GEMM launch: %s (%s)", cudaGetErrorString(e), why ? why : "");
     return FP8LIN_OK;

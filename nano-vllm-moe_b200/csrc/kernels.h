@@ -189,7 +189,10 @@ cudaError_t launch_swap_w8a8(const SwapPlan& plan, const UmmaArgs& a, const void
 // ---- MoE expert FFN (moe_kernels.cu, umma_grouped.cu) ------------------------------
 cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, int T, int E, int top_k, int renormalize,
                              float* out_w, void* out_ids, bool ids_i64, cudaStream_t stream);
-cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
+// even: the rows of an expert are cut into as few chunks of at most chunk_rows as they fill, all of the same size up to the next
+// multiple of 32 (chunk_rows is one), chunk.w = the costs (grouped_pair_cost) of all chunks in front of it, meta[2] = of all; else
+// into chunks of chunk_rows and a rest, chunk.w = 0.
+cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even, int* expert_offsets, int* sorted_rows,
                              int4* chunks, int* meta, int* inv, cudaStream_t stream);
 cudaError_t launch_moe_scatter_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* inv, int rows,
                                      const float* input_scale, unsigned char* xq, int H, cudaStream_t stream);
@@ -224,6 +227,14 @@ int grouped_chunk_rows(int64_t rows, int num_experts);
 // the down projection (scatter to routed rows, times the routing weight).  Needs the chunk list made with 128-row chunks and
 // rows already e4m3.
 cudaError_t launch_grouped_rows_w8a8(GroupedArgs args, const void* w_packed, int num_experts, const void* xq_sorted,
+                                     int64_t xq_rows, cudaStream_t stream, const char** why);
+// The same on CTA pairs with the channels as the MMA's M (umma_grouped_pair.cu): needs even chunks of at most max_rows rows, a
+// multiple of 32 up to kGroupedPairMaxRows; any widths that are multiples of 16; for down a 4-byte aligned out and an even ld_out.
+constexpr int kGroupedPairMaxRows = 320;
+// What a work item of `groups` groups of 32 rows costs that kernel, per K block in units of 32 SM cycles: the tensor core's time, or
+// the way of the weights and rows into shared memory where that is longer.
+__host__ __device__ constexpr int grouped_pair_cost(int groups) { return groups < 8 ? 8 + groups : 2 * groups; }
+cudaError_t launch_grouped_pair_w8a8(GroupedArgs args, int max_rows, const void* w_packed, int num_experts, const void* xq_sorted,
                                      int64_t xq_rows, cudaStream_t stream, const char** why);
 cudaError_t launch_grouped_w8a8(bool gather, int mp, GroupedArgs a, const void* w_packed, int num_experts,
                                 const void* xq_sorted, int64_t xq_rows, cudaStream_t stream, const char** why);

@@ -111,7 +111,8 @@ cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, in
 
 // ---- grouping of routed rows by expert ------------------------------------------------------
 // One CTA.  counts -> exclusive scan -> scatter.  Also writes the chunk list the grouped GEMM
-// walks: every expert's rows are cut into chunks of `chunk_rows`.
+// walks: every expert's rows are cut into chunks of `chunk_rows`, or (even) into as few chunks of at most that as they fill, of
+// the same size up to the next multiple of 32.
 //   sorted_rows[pos]     routed-row index at sorted position pos (rows of one expert are adjacent)
 //   expert_offsets[e]    first sorted position of expert e (E+1 entries)
 //   chunks[c]            {expert, first sorted position, rows in chunk, 0}
@@ -126,14 +127,20 @@ cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, in
 // few thousand rows on (16384 rows: 14.7 us).
 template <typename IdT, int kWarps>
 __global__ void __launch_bounds__(1024)
-moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, int* __restrict__ expert_offsets,
+moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, int even, int* __restrict__ expert_offsets,
                  int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta, int* __restrict__ inv) {
     pdl_launch_dependents();
+    auto chunk_size = [&](int n) {         // rows of an expert's chunks but the last
+        if (!even || n <= 0) return chunk_rows;
+        const int k = (n + chunk_rows - 1) / chunk_rows;
+        return ((n + k - 1) / k + 31) & ~31;
+    };
     extern __shared__ int sh[];
     int* count = sh;                       // [kWarps][E]: rows of expert e in warp w's share, then their next position
     int* total = sh + kWarps * E;          // [E]
     int* start = total + E;                // [E + 1]
     int* cstart = start + E + 1;           // [E + 1] chunk prefix
+    int* coststart = cstart + E + 1;       // [E] cost prefix; there only where `even`
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < kWarps * E; i += blockDim.x) count[i] = 0;
     const int share = ((rows + kWarps * 32 - 1) / (kWarps * 32)) * 32;
@@ -167,22 +174,29 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
     }
     __syncthreads();
     if (warp == 0) {                       // exclusive scans of rows and chunks over the experts
-        int row_base = 0, chunk_base = 0;
+        int row_base = 0, chunk_base = 0, cost_base = 0;
         for (int e0 = 0; e0 < E; e0 += 32) {
             const int n = e0 + lane < E ? total[e0 + lane] : 0;
-            const int c = (n + chunk_rows - 1) / chunk_rows;
-            int sn = n, sc = c;
+            const int size = chunk_size(n), c = (n + size - 1) / size;
+            const int cost = even && c ? (c - 1) * grouped_pair_cost(size >> 5) + grouped_pair_cost((n - (c - 1) * size + 31) >> 5) : 0;
+            int sn = n, sc = c, sw = cost;
             for (int o = 1; o < 32; o <<= 1) {
-                const int pn = __shfl_up_sync(0xffffffffu, sn, o), pc = __shfl_up_sync(0xffffffffu, sc, o);
-                if (lane >= o) { sn += pn; sc += pc; }
+                const int pn = __shfl_up_sync(0xffffffffu, sn, o), pc = __shfl_up_sync(0xffffffffu, sc, o), pw = __shfl_up_sync(0xffffffffu, sw, o);
+                if (lane >= o) { sn += pn; sc += pc; sw += pw; }
             }
-            if (e0 + lane < E) { start[e0 + lane] = row_base + sn - n; cstart[e0 + lane] = chunk_base + sc - c; }
+            if (e0 + lane < E) {
+                start[e0 + lane] = row_base + sn - n;
+                cstart[e0 + lane] = chunk_base + sc - c;
+                if (even) coststart[e0 + lane] = cost_base + sw - cost;
+            }
             row_base += __shfl_sync(0xffffffffu, sn, 31);
             chunk_base += __shfl_sync(0xffffffffu, sc, 31);
+            cost_base += __shfl_sync(0xffffffffu, sw, 31);
         }
         if (lane == 0) {
             start[E] = row_base; cstart[E] = chunk_base;
             meta[0] = chunk_base; meta[1] = row_base;
+            if (even) meta[2] = cost_base;
         }
     }
     __syncthreads();
@@ -206,28 +220,28 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
         }
     }
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int n = total[e];
-        for (int c = 0, pos = 0; pos < n; ++c, pos += chunk_rows)
-            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(chunk_rows, n - pos), 0);
+        const int n = total[e], size = chunk_size(n);
+        for (int c = 0, pos = 0; pos < n; ++c, pos += size)
+            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(size, n - pos), even ? coststart[e] + c * grouped_pair_cost(size >> 5) : 0);
     }
 }
 
 template <typename IdT>
-static cudaError_t launch_align(const IdT* ids, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows, int4* chunks,
+static cudaError_t launch_align(const IdT* ids, int rows, int E, int chunk_rows, int even, int* expert_offsets, int* sorted_rows, int4* chunks,
                                 int* meta, int* inv, cudaStream_t stream) {
     // counters per warp: 32 sets where they fit the 48 KB of shared memory (E <= 340), one set beyond (E <= 3071)
-    auto smem = [&](int sets) { return (size_t)((sets + 3) * E + 2) * sizeof(int); };
+    auto smem = [&](int sets) { return (size_t)((sets + (even ? 4 : 3)) * E + 2) * sizeof(int); };
     if (rows > 1024 && smem(32) <= 48 * 1024)
-        return launch_dependent(moe_align_kernel<IdT, 32>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+        return launch_dependent(moe_align_kernel<IdT, 32>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv);
     if (smem(8) <= 48 * 1024)
-        return launch_dependent(moe_align_kernel<IdT, 8>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
-    return launch_dependent(moe_align_kernel<IdT, 1>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+        return launch_dependent(moe_align_kernel<IdT, 8>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv);
+    return launch_dependent(moe_align_kernel<IdT, 1>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv);
 }
 
-cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
+cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even, int* expert_offsets, int* sorted_rows,
                              int4* chunks, int* meta, int* inv, cudaStream_t stream) {
-    return ids_i64 ? launch_align((const long long*)ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv, stream)
-                   : launch_align((const int*)ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv, stream);
+    return ids_i64 ? launch_align((const long long*)ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv, stream)
+                   : launch_align((const int*)ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv, stream);
 }
 
 // (Within an expert the rows land in the arrival order of the atomics.  Every routed row is an

@@ -1,0 +1,111 @@
+"""Expert batches on CTA pairs: the bits of the kernels that one CTA runs, at the edges of groups, MMA tiles, chunks and stretches."""
+import importlib
+
+import numpy as np
+import pytest
+import torch
+
+from helpers import kernels, to_bf16_cuda
+from test_gpu_moe import make_moe_case, upload_weights
+
+pytestmark = pytest.mark.gpu
+
+
+def block(E, I, T, H, seed):
+    moe = importlib.import_module("nano-vllm-moe_b200.executor.moe")
+    cfg = moe.make_moe_parallel_config(tp_group=None, ep_group=None, global_num_experts=E, intermediate_size=I)
+    kern = moe.MoEKernel(prepare_finalize=moe.NoEPPrepareFinalize(cfg), experts=moe.Fp8Experts(), parallel_config=cfg)
+    c = make_moe_case(seed, T, H, I, E, 1)
+    return moe, kern, c
+
+
+@pytest.mark.parametrize("counts,H,I,rows", [
+    ([256, 257, 0, 33], 272, 144, 320),           # one MMA tile, two, a group and a row; up rows inside a weight tile
+    ([320, 321, 31, 32, 1], 512, 192, 320),       # the longest chunk, two even ones; 64-row steps of the up channels
+    ([700, 320], 256, 128, 320),                  # three work items for all pairs: cut between groups
+    ([200, 500, 90], 144, 16, 32),                # one group per chunk, the narrowest intermediate size
+    ([60] * 12 + [64, 65], 272, 272, 64),         # a lone last weight tile in down
+    ([5, 17, 96, 40, 300] * 9, 144, 1040, 192),   # many work items, dealt out in turn
+    ([290, 310, 320, 280] * 10, 128, 1024, 320),  # ... whose sums do not fit beside each other in tensor memory
+])
+def test_pairs_give_the_bits_of_one_cta(counts, H, I, rows):
+    Kn = kernels()
+    E, T = len(counts), sum(counts)
+    _, kern, c = block(E, I, T, H, T + I)
+    wts, x = upload_weights(importlib.import_module("nano-vllm-moe_b200.executor.moe"), c), to_bf16_cuda(c["x"])
+    ids = torch.from_numpy(np.random.default_rng(I).permutation(np.repeat(np.arange(E), counts)).astype(np.int64)[:, None]).cuda()
+    w = torch.rand((T, 1), device="cuda") + 0.2
+    try:
+        Kn.set_tuning("moe_pair", 0)
+        want = kern(x, w, ids, wts, model_dtype=torch.bfloat16)
+        Kn.set_tuning("moe_pair", rows)
+        got = [kern(x, w, ids, wts, model_dtype=torch.bfloat16) for _ in range(3)]
+    finally:
+        Kn.set_tuning("moe_pair", -1)
+    assert want.float().abs().max() > 0
+    assert all(torch.equal(y, want) for y in got)
+    assert Kn.read_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("pad,offset", [(0, 0), (2, 2), (1, 0), (0, 1)])       # the last two: no place for a 4-byte store
+def test_output_rows_of_any_pitch_and_alignment(pkg, pad, offset):
+    L, Kn = pkg._lib, kernels()
+    lib = L.load()
+    E, H, I, counts = 3, 256, 128, [300, 200, 100]
+    T = sum(counts)
+    moe, _, c = block(E, I, T, H, 11)
+    wts, x = upload_weights(moe, c), to_bf16_cuda(c["x"])
+    ids = torch.from_numpy(np.repeat(np.arange(E), counts).astype(np.int32)).cuda()
+    w = torch.rand(T, device="cuda") + 0.2
+    ws = torch.zeros(lib.fp8lin_moe_workspace_bytes(T, E, H, I), dtype=torch.uint8, device="cuda")
+
+    def run(pad, offset):
+        out = torch.full((offset + T * (H + pad),), 7.0, dtype=torch.bfloat16, device="cuda")
+        rc = lib.fp8lin_moe_experts_w8a8(x.data_ptr(), H, 1, ids.data_ptr(), w.data_ptr(), T, wts.w13_packed.data_ptr(), wts.w13_scale.data_ptr(),
+                                         wts.w13_input_scale.data_ptr(), wts.w2_packed.data_ptr(), wts.w2_scale.data_ptr(),
+                                         wts.w2_input_scale.data_ptr(), E, H, I, out.data_ptr() + 2 * offset, H + pad, ws.data_ptr(), ws.numel(),
+                                         torch.cuda.current_stream().cuda_stream)
+        L.raise_for(rc, "fp8lin_moe_experts_w8a8")
+        rows = out[offset:].view(T, H + pad)
+        assert (out[:offset] == 7).all() and (rows[:, H:] == 7).all()
+        return rows[:, :H].clone()
+
+    try:
+        Kn.set_tuning("moe_pair", 0)
+        want = run(0, 0)
+        Kn.set_tuning("moe_pair", 320)
+        assert torch.equal(run(pad, offset), want)
+    finally:
+        Kn.set_tuning("moe_pair", -1)
+
+
+@pytest.mark.parametrize("gate", [0.0, 30.0, 79.0, 81.0, 300.0, 1e30, float("inf"), float("nan")])
+def test_gates_of_any_size_in_the_epilogue(gate):
+    """Gates that overflow the exponential, zeros, infinities and NaN: the values of the separate activation pass."""
+    Kn = kernels()
+    E, H, I, counts = 3, 256, 144, [300, 290, 10]
+    T = sum(counts)
+    moe, kern, c = block(E, I, T, H, 5)
+    wts, x = upload_weights(moe, c), to_bf16_cuda(c["x"])
+    # the gates of expert 0's first channels, of either sign, grow by orders of magnitude; the others stay as they are
+    wts.w13_scale[0, :16] *= gate
+    wts.w13_scale[0, I:I + 8] *= gate                 # ... and half of their up values
+    ids = torch.from_numpy(np.random.default_rng(3).permutation(np.repeat(np.arange(E), counts)).astype(np.int64)[:, None]).cuda()
+    w = torch.rand((T, 1), device="cuda") + 0.2
+    out = {}
+    try:
+        for name, knobs in {"pair": {"moe_pair": 320}, "one": {"moe_pair": 0}, "separate": {"moe_fused": 0}}.items():
+            for k, v in knobs.items():
+                Kn.set_tuning(k, v)
+            out[name] = kern(x, w, ids, wts, model_dtype=torch.bfloat16)
+            for k in knobs:
+                Kn.set_tuning(k, -1)
+    finally:
+        Kn.set_tuning("moe_pair", -1)
+        Kn.set_tuning("moe_fused", -1)
+    for name in ("pair", "one"):
+        assert torch.equal(out[name].isnan(), out["separate"].isnan()), name
+        assert torch.equal(out[name].nan_to_num(0.0), out["separate"].nan_to_num(0.0)), name
+    other = ids[:, 0] != 0
+    assert torch.isfinite(out["pair"][other].float()).all()
+    assert Kn.read_status(torch.device("cuda", 0)) == 0

@@ -118,3 +118,14 @@ def test_cluster_barriers_are_reached_by_warps_that_are_together():
         code = body(SOURCES["umma_common.cuh"], function)
         assert code.index("__syncwarp()") < code.index(instruction)
     assert len(re.findall(r"barrier\.cluster\.", SOURCES["umma_common.cuh"])) == 2
+
+
+def test_grouped_pairs_take_and_release_tensor_memory_as_the_other_pair_kernels_do():
+    text = SOURCES["umma_grouped_pair.cu"]
+    order = ["mbar_init(", "pair_enter();", "pair_tmem_begin(", "pdl_wait();", "&maps.w, 0, wr.a", "pair_tmem_release(", "pair_tmem_done(", "pair_leave();"]
+    at = [text.index(o) for o in order]
+    assert at == sorted(at) and all(text.count(o) == 1 for o in order if o != "mbar_init("), at
+    assert "2 * kEpiWarps);\n        s_abort" in text
+    # every item's tensor memory is handed on at cluster scope: arrivals of both CTAs, one wait
+    assert re.findall(r"(mbar_wait(?:<true>)?)\(smem_u32\(&bar_tfree", text) == ["mbar_wait<true>"]
+    assert text.count("mbar_arrive_remote(free_bar)") == 2 and "map_to_cta(smem_u32(&bar_tfree[side]), 0)" in text
