@@ -24,7 +24,7 @@
 // one CTA (umma_grouped_rows.cu), 207 here; 8192 rows 175 / 150; 2048 rows 119 / 110.  Five or six slots of loads in flight: asking
 // weights beyond them into L2 in front was slower the further (192 us without, 196 six blocks ahead, 206 sixteen).
 //
-// Sixteen epilogue warps: eight take longer over an item of gate_up (49 instructions per value then) than its MMAs do.
+// Sixteen epilogue warps: eight take longer over an item of gate_up than its MMAs do.
 //
 // Work: the items of all chunks in a row, chunk after chunk, are dealt out to the pairs, so that those at work at one time share a
 // few chunks' rows, which stay in L2 (a stretch of the row per pair, each on chunks of its own: 85 MB more from memory, gate_up of 16384
