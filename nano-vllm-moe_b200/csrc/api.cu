@@ -1012,13 +1012,14 @@ namespace {
 // instead of inside the gate_up GEMM (where every channel tile would redo it)
 constexpr int64_t kMoePrequantRows = 512;
 struct MoeWs {
-    size_t off_offsets, off_sorted, off_chunks, off_meta, off_inv, off_gu, off_hq, off_xq, total;
+    size_t off_offsets, off_counts, off_sorted, off_chunks, off_meta, off_inv, off_gu, off_hq, off_xq, total;
 };
 MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
     MoeWs w;
     size_t o = FP8LIN_WS_HEADER_BYTES;
     auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return at; };
     w.off_offsets = take((size_t)(E + 1) * 4);
+    w.off_counts = take(rows >= kMoePrequantRows ? moe_count_ints(rows, E) * 4 : 0);
     w.off_sorted = take((size_t)(rows > 0 ? rows : 1) * 4);
     w.off_chunks = take((size_t)(E + rows / 16 + 2) * 16);
     w.off_meta = take(16);
@@ -1084,7 +1085,7 @@ int fp8lin_moe_align(const int32_t* ids, int64_t rows, int E, int chunk_rows, in
         return fail(FP8LIN_ERR_ARG, "chunk_rows must be 16, 32, 64 or 128");
     if (!ids || !expert_offsets || !sorted_rows || !chunks || !meta) return fail(FP8LIN_ERR_NULL, "a required pointer is NULL");
     if (!aligned16(chunks)) return fail(FP8LIN_ERR_ALIGN, "chunks must be 16-byte aligned");
-    cudaError_t e = launch_moe_align(ids, false, (int)rows, E, chunk_rows, false, expert_offsets, sorted_rows, (int4*)chunks, meta, nullptr,
+    cudaError_t e = launch_moe_align(ids, false, (int)rows, E, chunk_rows, expert_offsets, sorted_rows, (int4*)chunks, meta, nullptr,
                                      (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
@@ -1129,7 +1130,10 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     // Few work items whose experts fill 128-row chunks: the rows are the MMA M dimension (umma_grouped_rows.cu), in
     // gate_up where the up channels start at a tile.
     const bool rows_major = !pair_rows && rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
-    cudaError_t e = launch_moe_align(ids, ids_i64, (int)rows, E, mp, pair_rows != 0, offsets, sorted, chunks, meta, inv, st);
+    unsigned char* xq = ws + L.off_xq;
+    cudaError_t e = rows >= kMoePrequantRows ? launch_moe_group_quant((const __nv_bfloat16*)x, ldx, x_div, ids, ids_i64, (int)rows, E, mp, pair_rows != 0,
+                                                                      w13_input_scale, (int*)(ws + L.off_counts), sorted, chunks, meta, inv, xq, (int)H, st)
+                                             : launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
     GroupedArgs a;
@@ -1142,9 +1146,6 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     GroupedArgs g = a;
     if (fused_act) { g.N = (int)I; g.hq = hq; g.h_scale = w2_input_scale; g.out = nullptr; }
     if (rows >= kMoePrequantRows) {
-        unsigned char* xq = ws + L.off_xq;
-        e = launch_moe_scatter_quant((const __nv_bfloat16*)x, ldx, x_div, inv, (int)rows, w13_input_scale, xq, (int)H, st);
-        if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row quantiser launch: %s", cudaGetErrorString(e));
         e = pair_rows ? launch_grouped_pair_w8a8(g, pair_rows, w13_packed, E, xq, rows, st, &why)
           : rows_major && fused_act && I % 128 == 0 ? launch_grouped_rows_w8a8(g, w13_packed, E, xq, rows, st, &why)
                                                     : launch_grouped_w8a8(false, mp, g, w13_packed, E, xq, rows, st, &why);

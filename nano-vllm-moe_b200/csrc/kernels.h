@@ -189,13 +189,17 @@ cudaError_t launch_swap_w8a8(const SwapPlan& plan, const UmmaArgs& a, const void
 // ---- MoE expert FFN (moe_kernels.cu, umma_grouped.cu) ------------------------------
 cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, int T, int E, int top_k, int renormalize,
                              float* out_w, void* out_ids, bool ids_i64, cudaStream_t stream);
+cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
+                             int4* chunks, int* meta, int* inv, cudaStream_t stream);
+// Grouping as launch_moe_align's and the rows in that order as e4m3, for batches that one CTA takes too long to group (two kernels).
+// counts: moe_count_ints(rows, E) ints of scratch; inv[r]: not negative where routed row r has an expert here.
 // even: the rows of an expert are cut into as few chunks of at most chunk_rows as they fill, all of the same size up to the next
 // multiple of 32 (chunk_rows is one), chunk.w = the costs (grouped_pair_cost) of all chunks in front of it, meta[2] = of all; else
 // into chunks of chunk_rows and a rest, chunk.w = 0.
-cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even, int* expert_offsets, int* sorted_rows,
-                             int4* chunks, int* meta, int* inv, cudaStream_t stream);
-cudaError_t launch_moe_scatter_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* inv, int rows,
-                                     const float* input_scale, unsigned char* xq, int H, cudaStream_t stream);
+size_t moe_count_ints(int64_t rows, int E);
+cudaError_t launch_moe_group_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even,
+                                   const float* input_scale, int* counts, int* sorted_rows, int4* chunks, int* meta, int* inv, unsigned char* xq, int H,
+                                   cudaStream_t stream);
 cudaError_t launch_silu_mul_quant(const __nv_bfloat16* gu, const float* input_scale, unsigned char* hq, const int* meta,
                                   int max_rows, int I, cudaStream_t stream);
 cudaError_t launch_moe_combine(const __nv_bfloat16* routed, const int* inv, __nv_bfloat16* y, int64_t ld_y, int T, int top_k, int H,

@@ -111,8 +111,8 @@ cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, in
 
 // ---- grouping of routed rows by expert ------------------------------------------------------
 // One CTA.  counts -> exclusive scan -> scatter.  Also writes the chunk list the grouped GEMM
-// walks: every expert's rows are cut into chunks of `chunk_rows`, or (even) into as few chunks of at most that as they fill, of
-// the same size up to the next multiple of 32.
+// walks: every expert's rows are cut into chunks of `chunk_rows`, or (even: moe_place_kernel's) into as few chunks of at most that as
+// they fill, of the same size up to the next multiple of 32.
 //   sorted_rows[pos]     routed-row index at sorted position pos (rows of one expert are adjacent)
 //   expert_offsets[e]    first sorted position of expert e (E+1 entries)
 //   chunks[c]            {expert, first sorted position, rows in chunk, 0}
@@ -125,22 +125,69 @@ cudaError_t launch_moe_route(const void* logits, int logits_bf16, int64_t ld, in
 // (scan over experts, inside an expert over warps) and the warps place their rows.  Against one set of E counters and a
 // serial scan by one thread: 5.7 -> 2.8 us for 256 rows of 60 experts.  A single SM's shared memory atomics bound it from a
 // few thousand rows on (16384 rows: 14.7 us).
+
+// rows of an expert's chunks but the last, of n rows in all
+__device__ __forceinline__ int chunk_size(int n, int chunk_rows, int even) {
+    if (!even || n <= 0) return chunk_rows;
+    const int k = (n + chunk_rows - 1) / chunk_rows;
+    return ((n + k - 1) / k + 31) & ~31;
+}
+// One warp: exclusive scans of rows, chunks and (even) costs over the experts; start and cstart have E + 1 entries.  All but start may
+// be left out (null).
+__device__ __forceinline__ void scan_experts(const int* total, int E, int chunk_rows, int even, int* start, int* cstart, int* coststart, int* meta) {
+    const int lane = threadIdx.x & 31;
+    int row_base = 0, chunk_base = 0, cost_base = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+        const int n = e0 + lane < E ? total[e0 + lane] : 0;
+        int sn = n, c = 0, cost = 0;
+        if (cstart) {
+            const int size = chunk_size(n, chunk_rows, even);
+            c = (n + size - 1) / size;
+            cost = even && c ? (c - 1) * grouped_pair_cost(size >> 5) + grouped_pair_cost((n - (c - 1) * size + 31) >> 5) : 0;
+        }
+        int sc = c, sw = cost;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int pn = __shfl_up_sync(0xffffffffu, sn, o);
+            if (lane >= o) sn += pn;
+            if (cstart) {
+                const int pc = __shfl_up_sync(0xffffffffu, sc, o), pw = __shfl_up_sync(0xffffffffu, sw, o);
+                if (lane >= o) { sc += pc; sw += pw; }
+            }
+        }
+        if (e0 + lane < E) {
+            start[e0 + lane] = row_base + sn - n;
+            if (cstart) cstart[e0 + lane] = chunk_base + sc - c;
+            if (cstart && even) coststart[e0 + lane] = cost_base + sw - cost;
+        }
+        row_base += __shfl_sync(0xffffffffu, sn, 31);
+        chunk_base += __shfl_sync(0xffffffffu, sc, 31);
+        cost_base += __shfl_sync(0xffffffffu, sw, 31);
+    }
+    if (lane == 0 && cstart) {
+        start[E] = row_base; cstart[E] = chunk_base;
+        meta[0] = chunk_base; meta[1] = row_base;
+        if (even) meta[2] = cost_base;
+    }
+}
+__device__ __forceinline__ void write_chunks(const int* total, int E, int chunk_rows, int even, const int* start, const int* cstart,
+                                             const int* coststart, int4* chunks) {
+    for (int e = threadIdx.x; e < E; e += blockDim.x) {
+        const int n = total[e], size = chunk_size(n, chunk_rows, even);
+        for (int c = 0, pos = 0; pos < n; ++c, pos += size)
+            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(size, n - pos), even ? coststart[e] + c * grouped_pair_cost(size >> 5) : 0);
+    }
+}
+
 template <typename IdT, int kWarps>
 __global__ void __launch_bounds__(1024)
-moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, int even, int* __restrict__ expert_offsets,
+moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, int* __restrict__ expert_offsets,
                  int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta, int* __restrict__ inv) {
     pdl_launch_dependents();
-    auto chunk_size = [&](int n) {         // rows of an expert's chunks but the last
-        if (!even || n <= 0) return chunk_rows;
-        const int k = (n + chunk_rows - 1) / chunk_rows;
-        return ((n + k - 1) / k + 31) & ~31;
-    };
     extern __shared__ int sh[];
     int* count = sh;                       // [kWarps][E]: rows of expert e in warp w's share, then their next position
     int* total = sh + kWarps * E;          // [E]
     int* start = total + E;                // [E + 1]
     int* cstart = start + E + 1;           // [E + 1] chunk prefix
-    int* coststart = cstart + E + 1;       // [E] cost prefix; there only where `even`
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int i = threadIdx.x; i < kWarps * E; i += blockDim.x) count[i] = 0;
     const int share = ((rows + kWarps * 32 - 1) / (kWarps * 32)) * 32;
@@ -173,32 +220,7 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
         total[e] = acc;
     }
     __syncthreads();
-    if (warp == 0) {                       // exclusive scans of rows and chunks over the experts
-        int row_base = 0, chunk_base = 0, cost_base = 0;
-        for (int e0 = 0; e0 < E; e0 += 32) {
-            const int n = e0 + lane < E ? total[e0 + lane] : 0;
-            const int size = chunk_size(n), c = (n + size - 1) / size;
-            const int cost = even && c ? (c - 1) * grouped_pair_cost(size >> 5) + grouped_pair_cost((n - (c - 1) * size + 31) >> 5) : 0;
-            int sn = n, sc = c, sw = cost;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int pn = __shfl_up_sync(0xffffffffu, sn, o), pc = __shfl_up_sync(0xffffffffu, sc, o), pw = __shfl_up_sync(0xffffffffu, sw, o);
-                if (lane >= o) { sn += pn; sc += pc; sw += pw; }
-            }
-            if (e0 + lane < E) {
-                start[e0 + lane] = row_base + sn - n;
-                cstart[e0 + lane] = chunk_base + sc - c;
-                if (even) coststart[e0 + lane] = cost_base + sw - cost;
-            }
-            row_base += __shfl_sync(0xffffffffu, sn, 31);
-            chunk_base += __shfl_sync(0xffffffffu, sc, 31);
-            cost_base += __shfl_sync(0xffffffffu, sw, 31);
-        }
-        if (lane == 0) {
-            start[E] = row_base; cstart[E] = chunk_base;
-            meta[0] = chunk_base; meta[1] = row_base;
-            if (even) meta[2] = cost_base;
-        }
-    }
+    if (warp == 0) scan_experts(total, E, chunk_rows, 0, start, cstart, nullptr, meta);
     __syncthreads();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = start[e];
     if (warp < kWarps) {
@@ -219,75 +241,162 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
             }
         }
     }
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        const int n = total[e], size = chunk_size(n);
-        for (int c = 0, pos = 0; pos < n; ++c, pos += size)
-            chunks[cstart[e] + c] = make_int4(e, start[e] + pos, min(size, n - pos), even ? coststart[e] + c * grouped_pair_cost(size >> 5) : 0);
-    }
+    write_chunks(total, E, chunk_rows, 0, start, cstart, nullptr, chunks);
 }
 
 template <typename IdT>
-static cudaError_t launch_align(const IdT* ids, int rows, int E, int chunk_rows, int even, int* expert_offsets, int* sorted_rows, int4* chunks,
+static cudaError_t launch_align(const IdT* ids, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows, int4* chunks,
                                 int* meta, int* inv, cudaStream_t stream) {
     // counters per warp: 32 sets where they fit the 48 KB of shared memory (E <= 340), one set beyond (E <= 3071)
-    auto smem = [&](int sets) { return (size_t)((sets + (even ? 4 : 3)) * E + 2) * sizeof(int); };
+    auto smem = [&](int sets) { return (size_t)((sets + 3) * E + 2) * sizeof(int); };
     if (rows > 1024 && smem(32) <= 48 * 1024)
-        return launch_dependent(moe_align_kernel<IdT, 32>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv);
+        return launch_dependent(moe_align_kernel<IdT, 32>, 1, 1024, smem(32), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
     if (smem(8) <= 48 * 1024)
-        return launch_dependent(moe_align_kernel<IdT, 8>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv);
-    return launch_dependent(moe_align_kernel<IdT, 1>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv);
+        return launch_dependent(moe_align_kernel<IdT, 8>, 1, 256, smem(8), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
+    return launch_dependent(moe_align_kernel<IdT, 1>, 1, 256, smem(1), stream, ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv);
 }
 
-cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even, int* expert_offsets, int* sorted_rows,
+cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int chunk_rows, int* expert_offsets, int* sorted_rows,
                              int4* chunks, int* meta, int* inv, cudaStream_t stream) {
-    return ids_i64 ? launch_align((const long long*)ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv, stream)
-                   : launch_align((const int*)ids, rows, E, chunk_rows, even, expert_offsets, sorted_rows, chunks, meta, inv, stream);
+    return ids_i64 ? launch_align((const long long*)ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv, stream)
+                   : launch_align((const int*)ids, rows, E, chunk_rows, expert_offsets, sorted_rows, chunks, meta, inv, stream);
 }
 
 // (Within an expert the rows land in the arrival order of the atomics.  Every routed row is an
 // independent column of the grouped GEMM, so the order does not change a single output bit.)
 
-// ---- quantise the rows once and place them in expert order (prefill-sized batches) -------------
-// xq[inv[r]][:] = e4m3(x[r / x_div][:] / scale) for every routed row r with a valid expert; the grouped GEMM then takes its
-// rows by TMA instead of re-quantising them for every channel tile.  A thread converts 16 elements of a token once and
-// stores them to the positions of its x_div slots: 2 + x_div bytes of traffic per token element instead of the 3 x_div of
-// a gather per sorted position, and one conversion instead of x_div (16384 rows x 2048, four slots: 19.2 -> 9 us).
-__global__ void __launch_bounds__(256)
-moe_scatter_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ inv, int rows,
-                         const float* __restrict__ input_scale, unsigned char* __restrict__ xq, int H) {
+// ---- group, quantise and place the rows of a large batch ------------------------------------------------------
+// From a few hundred rows on the grouping above is one SM's shared-memory atomics (16384 rows: 14.7 us), so it is spread out.
+// moe_count_kernel: a block counts its share of the rows by expert and leaves each row's expert and rank inside the share;
+// moe_place_kernel: a block sums up what it needs of the counts (every block the same few kilobytes from L2), which gives its rows'
+// places in expert order, and quantises its tokens there: xq[place][:] = e4m3(x[r / x_div][:] / scale) for every routed row r with a
+// valid expert.  The grouped GEMM then takes its rows by TMA instead of re-quantising them for every channel tile.  A thread converts 16
+// elements of a token once and stores them to the places of its x_div slots: 2 + x_div bytes of traffic per token element.  The
+// first block also writes the chunk list.  Launch times of 16384 rows x 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before,
+// 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); 4096 tokens, 4 of 60 experts 222 -> 217.
+constexpr int kMoeShares = 128;                    // at most (see moe_count_ints)
+constexpr int kRankBits = 18;                      // a row's rank inside its share (of 2^24 / 128 rows and a token's); the expert (E <= 3071) above it
+static_assert((1 << 24) / kMoeShares < 1 << kRankBits, "2^24 routed rows at most");
+
+// tokens of a share: all slots of a token lie in the same one
+__host__ __device__ inline int share_tokens(int rows, int x_div) {
+    const int tokens = (rows + x_div - 1) / x_div, least = (512 + x_div - 1) / x_div, even = (tokens + kMoeShares - 1) / kMoeShares;
+    return least > even ? least : even;
+}
+
+template <typename IdT>
+__global__ void __launch_bounds__(512)
+moe_count_kernel(const IdT* __restrict__ ids, int rows, int E, int share_rows, int* __restrict__ counts, int* __restrict__ inv) {
     pdl_launch_dependents();
+    extern __shared__ int sh[];                    // [E]
+    for (int e = threadIdx.x; e < E; e += blockDim.x) sh[e] = 0;
     pdl_wait();
-    const ExactDiv div_scale(fmaxf(ld_dep(input_scale), 1e-12f));
+    __syncthreads();
+    const int64_t r0 = (int64_t)blockIdx.x * share_rows;
+    const int r1 = (int)(r0 + share_rows < rows ? r0 + share_rows : rows);
+    for (int r = (int)r0 + (int)threadIdx.x; r < r1; r += blockDim.x) {
+        const long long e = (long long)ld_dep(ids + r);
+        inv[r] = e >= 0 && e < E ? (int)e << kRankBits | atomicAdd(&sh[e], 1) : -1;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += blockDim.x) counts[(size_t)blockIdx.x * E + e] = sh[e];
+}
+
+__global__ void __launch_bounds__(256)
+moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ inv, int rows, const float* __restrict__ input_scale,
+                 unsigned char* __restrict__ xq, int H, const int* __restrict__ counts, int shares, int share_tok, int parts, int E, int chunk_rows, int even,
+                 int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta) {
+    pdl_launch_dependents();
+    extern __shared__ int sh[];
+    int* before = sh;                              // [E] rows of the expert in the shares in front
+    int* total = sh + E;                           // [E]
+    int* start = total + E;                        // [E + 1]
+    int* cstart = start + E + 1;                   // [E + 1]: the first block only
+    int* coststart = cstart + E + 1;               // [E]: there only where `even`
+    for (int e = threadIdx.x; e < 2 * E; e += blockDim.x) sh[e] = 0;
+    const int share = (int)blockIdx.x / parts, part = (int)blockIdx.x - share * parts;
+    // this block's tokens; it walks whole ones, `per` at a time, so that no element needs a division to find its row
+    const int64_t tokens = ((int64_t)rows + x_div - 1) / x_div;
+    const int part_tok = (share_tok + parts - 1) / parts;
+    const int64_t t_first = (int64_t)share * share_tok + (int64_t)part * part_tok;
+    const int64_t t_last = min(min(tokens, (int64_t)(share + 1) * share_tok), t_first + part_tok);
     const int vec_per_row = H / 16;
-    const int tokens = (rows + x_div - 1) / x_div;
-    // a block walks whole tokens, so no element needs a division to find its row
-    const int per = vec_per_row < 256 ? 256 / vec_per_row : 1;             // tokens a block takes at a time
-    const int sub = threadIdx.x / vec_per_row < per ? threadIdx.x / vec_per_row : per;
-    for (int64_t t0 = (int64_t)blockIdx.x * per; t0 < tokens; t0 += (int64_t)gridDim.x * per) {
-        const int64_t t = t0 + (per > 1 ? sub : 0);
-        if (sub >= per && per > 1) continue;
-        if (t >= tokens) continue;
-        for (int c = per > 1 ? (int)threadIdx.x - sub * vec_per_row : (int)threadIdx.x; c < vec_per_row; c += per > 1 ? vec_per_row : 256) {
-            const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)t * ldx + c * 16);
-            const uint2 qa = quant8_e4m3(ld_dep(src), div_scale);
-            const uint2 qb = quant8_e4m3(ld_dep(src + 1), div_scale);
+    const int per = vec_per_row < 256 ? 256 / vec_per_row : 1;
+    const int sub = per > 1 ? (int)threadIdx.x / vec_per_row : 0;
+    const int c_first = per > 1 ? (int)threadIdx.x - sub * vec_per_row : (int)threadIdx.x, c_step = per > 1 ? vec_per_row : 256;
+    const int64_t t_mine = sub < per ? t_first + sub : t_last;
+    auto source = [&](int64_t t, int c) { return reinterpret_cast<const uint4*>(x + (size_t)t * ldx + c * 16); };
+    pdl_wait();
+    uint4 va = make_uint4(0u, 0u, 0u, 0u), vb = va;                        // the first piece is on its way beside the counts
+    if (t_mine < t_last && c_first < vec_per_row) {
+        va = ld_dep(source(t_mine, c_first));
+        vb = ld_dep(source(t_mine, c_first) + 1);
+    }
+    __syncthreads();
+    // a warp sums up every eighth share, a lane every 32nd expert; four loads in flight
+    for (int e = threadIdx.x & 31; e < E; e += 32) {
+        int all = 0, front = 0;
+        for (int b = threadIdx.x >> 5; b < shares; b += 32) {
+            int n[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) n[i] = b + 8 * i < shares ? ld_dep(counts + (size_t)(b + 8 * i) * E + e) : 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                all += n[i];
+                if (b + 8 * i < share) front += n[i];
+            }
+        }
+        if (all) atomicAdd(&total[e], all);
+        if (front) atomicAdd(&before[e], front);
+    }
+    __syncthreads();
+    const bool first = blockIdx.x == 0;
+    if (threadIdx.x < 32) scan_experts(total, E, chunk_rows, even, start, first ? cstart : nullptr, first ? coststart : nullptr, meta);
+    __syncthreads();
+    if (first) write_chunks(total, E, chunk_rows, even, start, cstart, coststart, chunks);
+
+    const ExactDiv div_scale(fmaxf(ld_dep(input_scale), 1e-12f));
+    for (int64_t t = t_mine; t < t_last; t += per)
+        for (int c = c_first; c < vec_per_row; c += c_step) {
+            if (t != t_mine || c != c_first) {
+                va = ld_dep(source(t, c));
+                vb = ld_dep(source(t, c) + 1);
+            }
+            const uint2 qa = quant8_e4m3(va, div_scale), qb = quant8_e4m3(vb, div_scale);
             const uint4 o = make_uint4(qa.x, qa.y, qb.x, qb.y);
             for (int j = 0; j < x_div; ++j) {
                 const int64_t r = t * x_div + j;
-                const int pos = r < rows ? ld_dep(inv + r) : -1;
-                if (pos >= 0) *reinterpret_cast<uint4*>(xq + (size_t)pos * H + c * 16) = o;
+                const int code = r < rows ? ld_dep(inv + r) : -1;
+                if (code < 0) continue;
+                const int e = code >> kRankBits, place = start[e] + before[e] + (code & ((1 << kRankBits) - 1));
+                *reinterpret_cast<uint4*>(xq + (size_t)place * H + c * 16) = o;
+                if (c == 0) sorted_rows[place] = (int)r;
             }
         }
-    }
 }
 
-cudaError_t launch_moe_scatter_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const int* inv, int rows,
-                                     const float* input_scale, unsigned char* xq, int H, cudaStream_t stream) {
+size_t moe_count_ints(int64_t rows, int E) {
+    const int64_t shares = (rows + 511) / 512;     // (a share has 512 rows at least)
+    return (size_t)(shares < kMoeShares ? shares : kMoeShares) * E;
+}
+
+cudaError_t launch_moe_group_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even,
+                                   const float* input_scale, int* counts, int* sorted_rows, int4* chunks, int* meta, int* inv, unsigned char* xq, int H,
+                                   cudaStream_t stream) {
+    const int share_tok = share_tokens(rows, x_div), tokens = (rows + x_div - 1) / x_div;
+    const int shares = (tokens + share_tok - 1) / share_tok;
+    const size_t smem = (size_t)E * sizeof(int);
+    cudaError_t e = ids_i64 ? launch_dependent(moe_count_kernel<long long>, shares, 512, smem, stream, (const long long*)ids, rows, E, share_tok * x_div, counts, inv)
+                            : launch_dependent(moe_count_kernel<int>, shares, 512, smem, stream, (const int*)ids, rows, E, share_tok * x_div, counts, inv);
+    if (e != cudaSuccess) return e;
+    // parts of a share: about eight blocks per SM in all, but whole turns of a block
     const int vec = H / 16, per = vec < 256 ? 256 / vec : 1;
-    int64_t blocks = ((int64_t)(rows + x_div - 1) / x_div + per - 1) / per;
-    if (blocks > sm_count() * 8) blocks = sm_count() * 8;
-    if (blocks < 1) blocks = 1;
-    return launch_dependent(moe_scatter_quant_kernel, (unsigned)blocks, 256, 0, stream, x, ldx, x_div, inv, rows, input_scale, xq, H);
+    int parts = sm_count() * 8 / shares;
+    if (parts > (share_tok + per - 1) / per) parts = (share_tok + per - 1) / per;
+    if (parts < 1) parts = 1;
+    // (E <= 3071, with even chunks <= 1024: 48 KB)
+    return launch_dependent(moe_place_kernel, (unsigned)(shares * parts), 256, (size_t)((even ? 5 : 4) * E + 2) * sizeof(int), stream, x, ldx, x_div, inv, rows,
+                            input_scale, xq, H, counts, shares, share_tok, parts, E, chunk_rows, even, sorted_rows, chunks, meta);
 }
 
 // ---- h = silu(gate) * up, quantised for the down projection ----------------------------------

@@ -5,7 +5,7 @@
 //
 // The expert's weight tile is the 128-row MMA "A" operand (TMA, packed layout, one 16 KiB box
 // per K block); the routed rows are the MMA "N" dimension.  Work items (chunk, tile) come from
-// the chunk list moe_align_kernel leaves in device memory, so no host synchronisation is needed;
+// the chunk list that the grouping (moe_kernels.cu) leaves in device memory, so no host synchronisation is needed;
 // the grid is persistent (one CTA per SM) and every CTA strides over the items.
 //
 // Source of the rows (template flag kGather):
@@ -13,7 +13,7 @@
 //          token matrix through the sorted row index and quantised on the fly (static scale,
 //          exact division) by converter warps straight into the swizzled MMA "B" tile.
 //   false  the rows are already e4m3 and contiguous in sorted order (down projection always;
-//          gate_up after moe_scatter_quant_kernel for prefill-sized batches): one TMA box.
+//          gate_up after moe_place_kernel for prefill-sized batches): one TMA box.
 // Epilogue (run-time flag `scatter`):
 //   0      gu[sorted position][channel] = bf16(acc * in_scale * w_scale[e][channel])
 //   1      out[routed row][channel] = bf16(acc * in_scale * w_scale[e][channel] * topk_w[routed row])

@@ -2,7 +2,7 @@
 //
 //   D[256 channels, R rows] = W_e[256 channels, K] . xq[rows of one chunk, K]^T        R = the chunk's rows, rounded up to 32
 //
-// for every chunk of at most 320 routed rows that share an expert e (even chunks, moe_align_kernel; the rows already e4m3 and in
+// for every chunk of at most 320 routed rows that share an expert e (even chunks, moe_place_kernel; the rows already e4m3 and in
 // sorted order) and every item of 256 channels:
 //   gate_up (kDown = false)  an item is gate tile t and up tile t of the expert (128 channels each).  CTA r of the pair takes
 //             channels [64 r, 64 r + 64) of BOTH, so that a gate value and its up value meet in one CTA: warps of the gate

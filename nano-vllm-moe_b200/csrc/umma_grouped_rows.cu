@@ -15,7 +15,7 @@
 //                      bf16 first -- the same values and roundings as the separate activation pass.
 //   kFusedAct = false  down: out[routed row][n] = bf16( acc * in_scale * w_scale[e][n] * topk_w[routed row] ).
 //
-// Chunks are the 128-row chunks of moe_align_kernel's list; rows of a chunk's 128-row box beyond its own rows belong
+// Chunks are the 128-row chunks of the grouping (moe_kernels.cu); rows of a chunk's 128-row box beyond its own rows belong
 // to the next chunk (or lie past the end and read as zeros): they are multiplied but never stored.  Persistent, one CTA
 // per SM, TMA producer / MMA issuer / 8 epilogue warps, two accumulator stages in TMEM; every mbarrier wait is bounded.
 #include "umma_common.cuh"

@@ -109,3 +109,44 @@ def test_gates_of_any_size_in_the_epilogue(gate):
     other = ids[:, 0] != 0
     assert torch.isfinite(out["pair"][other].float()).all()
     assert Kn.read_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("rows,x_div,E", [(512, 1, 3), (513, 5, 60), (1031, 4, 7), (70000, 3, 9), (2000, 600, 3000)])
+def test_grouping_of_large_batches(pkg, rows, x_div, E):
+    """Shares of whole tokens, a last one that is cut short, more than 128 times 512 rows, as many experts as there may be: every
+    routed row gets what it gets in a batch that one CTA groups."""
+    L, Kn = pkg._lib, kernels()
+    lib = L.load()
+    H = I = 16
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    tokens = -(-rows // x_div)
+    x = torch.randn(tokens, H, generator=gen, device="cuda").bfloat16()
+    ids = torch.randint(-1, E + 1, (rows,), generator=gen, device="cuda", dtype=torch.int32)       # some of them no expert's here
+    w = torch.rand(rows, generator=gen, device="cuda") + 0.2
+    code = lambda *s: (torch.randn(*s, generator=gen, device="cuda") * 0.5).to(torch.float8_e4m3fn).view(torch.uint8)
+    w13 = torch.cat([Kn.pack_weight_nk(code(2 * I, H)) for _ in range(min(E, 64))])
+    w2 = torch.cat([Kn.pack_weight_nk(code(H, I)) for _ in range(min(E, 64))])
+    if E > 64:                                                     # (the same 64 experts again and again)
+        w13, w2 = (t.view(64, -1).repeat(-(-E // 64), 1)[:E].contiguous().view(-1) for t in (w13, w2))
+    s13, s2 = torch.rand(E, 2 * I, generator=gen, device="cuda") + 0.5, torch.rand(E, H, generator=gen, device="cuda") + 0.5
+    in13, in2 = torch.tensor(0.01, device="cuda"), torch.tensor(0.05, device="cuda")
+
+    def run(x, x_div, ids, w):
+        n = ids.numel()
+        out = torch.zeros(n, H, dtype=torch.bfloat16, device="cuda")
+        ws = torch.zeros(lib.fp8lin_moe_workspace_bytes(n, E, H, I), dtype=torch.uint8, device="cuda")
+        L.raise_for(lib.fp8lin_moe_experts_w8a8(x.data_ptr(), H, x_div, ids.data_ptr(), w.data_ptr(), n, w13.data_ptr(), s13.data_ptr(), in13.data_ptr(), w2.data_ptr(),
+                                                s2.data_ptr(), in2.data_ptr(), E, H, I, out.data_ptr(), H, ws.data_ptr(), ws.numel(),
+                                                torch.cuda.current_stream().cuda_stream), "fp8lin_moe_experts_w8a8")
+        torch.cuda.synchronize()
+        return out
+
+    got = run(x, x_div, ids, w)
+    picked = torch.arange(rows, device="cuda")
+    if rows > 4000:
+        picked = torch.cat([picked[:511], picked[rows // 2:rows // 2 + 511], picked[-511:]])
+    for part in picked.split(511):
+        r = part.long()
+        want = run(x[r // x_div].contiguous(), 1, ids[r].contiguous(), w[r].contiguous())
+        assert torch.equal(got[r], want)
+    assert (got[(ids < 0) | (ids >= E)] == 0).all() and got.float().abs().max() > 0
