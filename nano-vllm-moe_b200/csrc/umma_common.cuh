@@ -440,10 +440,10 @@ EncodeTiledFn get_encode_fn();     // defined in umma_gemm.cu
 int max_active_clusters(const void* kernel, int threads, size_t smem_bytes, int cluster);
 // 2-D byte tensor [rows][cols] (cols contiguous), box = 128 bytes x box_rows, 128-byte swizzle.
 bool encode_u8_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
-// Output map: bf16 [rows][cols] with a row pitch in bytes, box = box_cols x 32 rows, swizzle span = the
+// Output map: bf16 [rows][cols] with a row pitch in bytes, box = box_cols x box_rows, swizzle span = the
 // box's row length (128 or 64 bytes).
 bool encode_out_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes,
-                   uint32_t box_cols);
+                   uint32_t box_cols, uint32_t box_rows = 32);
 
 // ---- activation quantisation inside the large-M GEMM ------------------------------------------------
 // The GEMM kernels that take bf16 activations carry kQuantWarps extra warps.  Those warps turn rows

@@ -11,8 +11,7 @@
 //   warp 0        TMA producer: 16 KB of weights and T/2 x 128 bytes of xq per slot; the weights of the first ring pass go
 //                 out before the wait for the kernel that writes xq
 //   warp 1        MMA issuer (leader CTA): four tcgen05.mma.cta_group::2.kind::f8f6f4 (256 x T x 32) per K block
-//   warps 2..9    epilogue: lane = channel, y[m][n] = bf16(acc * in_scale * w_scale[n] + bias[n]); two lanes swap halves so
-//                 that a lane stores two channels of one token
+//   warps 2..9    epilogue: lane = channel, y[m][n] = bf16(acc * in_scale * w_scale[n] + bias[n]), turned to rows in shared memory
 //
 // kMlp (gate_up of the fused MLP, gate and up channels in alternating tiles of 128): a CTA stages 64 gate channels and the
 // 64 up channels of the same indices, and the epilogue writes e4m3 h = bf16(silu(g) * u) / h_scale; the warps of the gate
@@ -44,11 +43,13 @@ constexpr int kWBytes = kTile * kKB;
 constexpr int kMaxSlots = 12;
 constexpr int kMaxT = 256;                     // columns of an accumulator stage
 constexpr int kTmemCols = 512;
-constexpr int kRingBytes = 210 * 1024;         // 16 KB + 64 T bytes per slot
+template <bool kStored> constexpr int kRingBytes = (kStored ? 200 : 210) * 1024;       // 16 KB + 64 T bytes per slot; kStored: beside boxes
+constexpr int kBoxBytes = 32 * 128;            // results of 32 tokens x 64 channels on their way out, one box per two epilogue warps
 constexpr int kSwapBytes = 32 * 64;            // kMlp: bf16 values of 32 rows x 32 channels, one buffer per warp pair
 constexpr int kCodeBytes = 32 * 32;            // ... and their e4m3 results
-template <bool kMlp> constexpr int kSmemBytes = kRingBytes + (kMlp ? 4 * (kSwapBytes + kCodeBytes) : 0) + 1024;
-static_assert(kTile * 256 * 4 <= kRingBytes, "the parked sums must fit in the ring");
+template <bool kSplit, bool kMlp>
+constexpr int kSmemBytes = kRingBytes<!kSplit && !kMlp> + 4 * (kMlp ? kSwapBytes + kCodeBytes : kSplit ? 0 : kBoxBytes) + 1024;
+static_assert(kTile * 256 * 4 <= kRingBytes<false>, "the parked sums must fit in the ring");
 
 struct PairSched8 {
     int n_tiles;              // 256-channel tiles
@@ -59,9 +60,9 @@ struct PairSched8 {
     int kblocks, kblocks_per_slice;
 };
 
-// weights (boxes of 128 rows, kMlp 64) and xq (boxes of half a full and half a last token tile)
+// weights (boxes of 128 rows, kMlp 64), xq (boxes of half a full and half a last token tile) and y (16 tokens x 64 channels)
 struct PairMaps8 {
-    CUtensorMap w, x, x_last;
+    CUtensorMap w, x, x_last, y;
 };
 
 struct Item {
@@ -95,6 +96,7 @@ template <bool kSplit, bool kMlp>
 __global__ void __launch_bounds__(kThreads, 1)
 w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 sched) {
     static_assert(!(kSplit && kMlp), "the activation epilogue takes whole sums");
+    constexpr int kRing = kRingBytes<!kSplit && !kMlp>;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_full[kMaxSlots];      // leader's: both CTAs' weights and rows landed
     __shared__ __align__(8) uint64_t bar_empty[kMaxSlots];     // the MMAs that read the slot are done (both CTAs')
@@ -122,7 +124,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
     const int acc_cols = n_acc * sched.tokens;
     const int acc_stages = 2 * acc_cols <= kTmemCols ? 2 : 1;
     const uint32_t slot_bytes = kWBytes + (uint32_t)sched.tokens * 64u;
-    const int n_slots = min(kMaxSlots, (int)(kRingBytes / slot_bytes));
+    const int n_slots = min(kMaxSlots, (int)(kRing / slot_bytes));
     // split-K: band r of this CTA's 128 channels is finished by slice r's CTA of the same pair rank
     const int band = kSplit ? (kTile + sched.splits - 1) / sched.splits : kTile;
     const int band_rows = kSplit ? max(0, min(kTile, (slice_rank + 1) * band) - slice_rank * band) : 0;
@@ -235,7 +237,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
         const bool odd = lane & 1;
         const bool up = kMlp && q >= 2;
         const int pair = (q & 1) + 2 * h;                  // kMlp: the warps of quarters q and q ^ 2 share 32 channels
-        const uint32_t swap_buf = smem_base + kRingBytes + pair * (kSwapBytes + kCodeBytes);
+        const uint32_t swap_buf = smem_base + kRing + pair * (kSwapBytes + kCodeBytes);
         const uint32_t code_buf = swap_buf + kSwapBytes;
         int tl = 0;
         for (int item = first_item; item < items; item += item_step, ++tl) {
@@ -249,7 +251,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                 if (p.bias) bs = ld_dep(p.bias + n);
             }
             bool arrived = mbar_wait(smem_u32(&bar_tfull[as]), acc_stages == 2 ? ((tl >> 1) & 1) : (tl & 1), p.status, kDevTimeoutTmemFull);
-            if (kMlp) arrived = !named_sync_any(5, 256, !arrived);        // warps that meet at barriers below leave together
+            if (!kSplit) arrived = !named_sync_any(5, 256, !arrived);      // warps that meet at barriers below leave together
             if (!arrived) { s_abort = 1; break; }
             tc_fence_after();
             const int m0 = it.m0 + h * it.half;
@@ -293,19 +295,37 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
                         *reinterpret_cast<float4*>(p.hq + (size_t)m * ld + hc + (i & 1) * 16) = ld_shared_f4(code_buf + (i >> 1) * 32 + (i & 1) * 16);
                 }
             } else if constexpr (!kSplit) {
-                // a lane stores two channels of one token: even lanes the even tokens, odd lanes the odd ones
-                __nv_bfloat16* yp = p.y + (size_t)m0 * p.ldy + (n & ~1) + (odd ? p.ldy : 0);
-                const bool in = (n & ~1) < p.N;                // (N is even)
+                // Two warps (64 channels) fill a box of 32 tokens, which leaves by TMA in whole 128-byte lines, clipped at M and N
+                // (stored by the lanes, 64 bytes of a row at a time, the tile of T = 224 took 6600 SM cycles behind the last MMA, 2500 of
+                // them for the stores: 1031 rows on 3584 -> 4608 19.1 -> 18.2 us, in a loop on 3584 -> 37888 131 -> 114; four 7B decoder layers
+                // of 64 rows 241.8 -> 238.4).  Two lanes swap halves, so that a lane writes two channels of a token: even lanes token j, odd lanes j + 4, whose
+                // swizzled places lie in the other banks.
+                const uint32_t box = smem_base + kRing + ((q >> 1) + 2 * h) * kBoxBytes;
+                const bool issuer = (q & 1) == 0 && lane == 0;
+                const int n_box = (2 * it.nt + (int)rank) * kTile + (q >> 1) * 64;
+                const uint32_t at = box + (odd ? 512u : 0u) + (uint32_t)(lane & 6) * 2u, chunk = (uint32_t)((q & 1) * 4 + (lane >> 3)), sel = odd ? 0x3276u : 0x5410u;
                 for (int c = 0; c < it.half; c += 32) {
                     uint32_t v[32];
                     read32(c, v);
+                    uint32_t o[16];
 #pragma unroll
-                    for (int j = 0; j < 32; j += 2) {
-                        if (j == 16 && c + 16 >= it.half) break;
-                        const float a0 = fmaf(__uint_as_float(v[j]) * pre, ws, bs), a1 = fmaf(__uint_as_float(v[j + 1]) * pre, ws, bs);
-                        const float other = __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 1);
-                        const uint32_t o = odd ? pack_bf16x2(other, a1) : pack_bf16x2(a0, other);
-                        if (in && m0 + c + j + (odd ? 1 : 0) < p.M) *reinterpret_cast<uint32_t*>(yp + (size_t)(c + j) * p.ldy) = o;
+                    for (int j = 0; j < 16; ++j) {
+                        const int k = 8 * (j >> 2) + (j & 3);
+                        o[j] = pack_bf16x2(fmaf(__uint_as_float(v[k]) * pre, ws, bs), fmaf(__uint_as_float(v[k + 4]) * pre, ws, bs));
+                        o[j] = __byte_perm(o[j], __shfl_xor_sync(0xffffffffu, o[j], 1), sel);
+                    }
+                    if (issuer) tma_store_wait_read();         // the previous store has read the box
+                    named_sync(1 + (q >> 1) + 2 * h, 64);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {             // row 8 (j / 4) + j % 4, odd lanes four further on
+                        const uint32_t r = (uint32_t)(j & 3) + (odd ? 4u : 0u);
+                        asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + (uint32_t)(8 * (j >> 2) + (j & 3)) * 128u + ((chunk ^ r) << 4)), "r"(o[j]) : "memory");
+                    }
+                    fence_async_smem();
+                    named_sync(1 + (q >> 1) + 2 * h, 64);
+                    if (issuer && n_box < p.N) {
+                        if (m0 + c < p.M) tma_store_2d(&maps.y, box, n_box, m0 + c);
+                        if (c + 16 < it.half && m0 + c + 16 < p.M) tma_store_2d(&maps.y, box + kBoxBytes / 2, n_box, m0 + c + 16);
                     }
                 }
             } else {
@@ -324,6 +344,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
             }
         }
         pair_tmem_done(smem_u32(&bar_done), leader_cta, lane);
+        if (!kSplit && !kMlp && lane == 0) tma_store_wait_all();
     }
 
     if constexpr (kSplit) {
@@ -347,7 +368,7 @@ template <bool kSplit, bool kMlp>
 cudaError_t launch_kernel(const W8a8PairPlan& pl, const UmmaArgs& a, const PairMaps8& maps, cudaStream_t stream) {
     auto kern = w8a8_pair_kernel<kSplit, kMlp>;
     static SmemOptIn opted;
-    cudaError_t e = ensure_dynamic_smem((const void*)kern, kSmemBytes<kMlp>, opted);
+    cudaError_t e = ensure_dynamic_smem((const void*)kern, kSmemBytes<kSplit, kMlp>, opted);
     if (e != cudaSuccess) return e;
     PairSched8 s;
     s.n_tiles = pl.n_tiles; s.m_tiles = pl.m_tiles; s.tokens = pl.tokens; s.last_tokens = pl.last_tokens; s.splits = pl.splits; s.slices = pl.slices;
@@ -355,7 +376,7 @@ cudaError_t launch_kernel(const W8a8PairPlan& pl, const UmmaArgs& a, const PairM
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)pl.grid);
     cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kSmemBytes<kMlp>;
+    cfg.dynamicSmemBytes = kSmemBytes<kSplit, kMlp>;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int na = pdl_attribute(attr);
@@ -392,7 +413,7 @@ W8a8PairPlan plan_w8a8_pair(int64_t M, int64_t K, int64_t N, bool mlp, int slice
         if (force_splits > 0 && splits != force_splits) continue;
         const void* kern = splits > 1 ? (const void*)w8a8_pair_kernel<true, false>
                          : mlp ? (const void*)w8a8_pair_kernel<false, true> : (const void*)w8a8_pair_kernel<false, false>;
-        const int slots = max_active_clusters(kern, kThreads, mlp ? kSmemBytes<true> : kSmemBytes<false>, 2 * splits);
+        const int slots = max_active_clusters(kern, kThreads, splits > 1 ? kSmemBytes<true, false> : mlp ? kSmemBytes<false, true> : kSmemBytes<false, false>, 2 * splits);
         if (slots < 1) continue;
         const int blocks = splits > 1 ? kps : kblocks;                        // K blocks of a pair
         for (int tokens = 32; tokens <= kMaxT; tokens += 32) {
@@ -436,9 +457,13 @@ W8a8PairPlan plan_w8a8_pair(int64_t M, int64_t K, int64_t N, bool mlp, int slice
 cudaError_t launch_w8a8_pair(const W8a8PairPlan& pl, const UmmaArgs& a, cudaStream_t stream, const char** why) {
     const bool mlp = a.hq != nullptr;
     PairMaps8 maps;
-    if (pl.tokens < 32 || !encode_u8_2d(&maps.w, a.w, (uint64_t)(pack_ntiles(a.N) * pack_kblocks(a.K) * 128), 128, mlp ? kTile / 2 : kTile) ||
-        !encode_u8_2d(&maps.x, a.xq, (uint64_t)a.M, (uint64_t)a.K, (uint32_t)pl.tokens / 2) ||
-        !encode_u8_2d(&maps.x_last, a.xq, (uint64_t)a.M, (uint64_t)a.K, (uint32_t)pl.last_tokens / 2)) {
+    bool ok = pl.tokens >= 32 && encode_u8_2d(&maps.w, a.w, (uint64_t)(pack_ntiles(a.N) * pack_kblocks(a.K) * 128), 128, mlp ? kTile / 2 : kTile) &&
+              encode_u8_2d(&maps.x_last, a.xq, (uint64_t)a.M, (uint64_t)a.K, (uint32_t)pl.last_tokens / 2);
+    maps.x = maps.x_last;                                  // (a map costs the host 0.1 us: only what the kernel reads)
+    if (ok && pl.m_tiles > 1 && pl.tokens != pl.last_tokens) ok = encode_u8_2d(&maps.x, a.xq, (uint64_t)a.M, (uint64_t)a.K, (uint32_t)pl.tokens / 2);
+    maps.y = maps.x_last;
+    if (ok && !mlp && pl.splits == 1) ok = encode_out_2d(&maps.y, a.y, (uint64_t)a.M, (uint64_t)a.N, (uint64_t)a.ldy * 2, 64, 16);
+    if (!ok) {
         if (why) *why = "no plan, or cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
     }

@@ -56,3 +56,19 @@ def test_mlp_epilogue_equals_the_other_kernels(m, h, inter, tokens):
     Kn.set_tuning("w8a8_pair", 1)
     Kn.set_tuning("w8a8_pair_tokens", tokens)
     np.testing.assert_array_equal(run_fused(d), want)
+
+
+@pytest.mark.parametrize("m,n,tokens", [(17, 72, 32), (47, 264, 32), (81, 584, 96), (160, 8, 160), (300, 648, 224)])
+def test_results_stay_inside_the_output_matrix(m, n, tokens):
+    """Boxes of 16 tokens and 64 channels, clipped at the last token and channel: rows of a wider, longer matrix keep what was there."""
+    Kn = kernels()
+    d = upload_case(O.make_case(m + n, m, 272, n))
+    Kn.set_tuning("w8a8_pair", 0)
+    want = Kn.launch_w8a8_gemm(d["x"], d["w_nk"], d["input_scale"], d["w_scale"], d["bias"])
+    Kn.set_tuning("w8a8_pair", 1)
+    Kn.set_tuning("w8a8_pair_tokens", tokens)
+    around = torch.full((m + 40, n + 136), 7.0, dtype=torch.bfloat16, device="cuda")
+    Kn.launch_w8a8_gemm(d["x"], d["w_nk"], d["input_scale"], d["w_scale"], d["bias"], out=around[:m, 64:64 + n])
+    assert torch.equal(around[:m, 64:64 + n], want)
+    around[:m, 64:64 + n] = 7.0
+    assert (around == 7.0).all()
