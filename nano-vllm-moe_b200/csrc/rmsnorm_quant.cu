@@ -21,6 +21,10 @@ namespace fp8lin {
 constexpr int kNormThreads = 256;
 constexpr int kNormMaxVec = 4;          // 8-element vectors per thread: H <= 256 * 8 * 4 = 8192
 
+// kVec: vectors that a thread may hold.  The row stays in registers, so a prompt's rows run in as many turns as registers allow CTAs: with
+// room for four vectors whatever H was, two CTAs per SM took 9 to 10.6 us for 1031 rows of 3584 beside power-limited GEMMs, with room for
+// two four of them take 7 to 8.6 (two 7B decoder layers of 1031 rows 491.7 -> 489.0 us, four of 64 rows 238.6 -> 237.2).
+template <int kVec>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bfloat16* __restrict__ residual, int64_t ld_res,
                      const __nv_bfloat16* __restrict__ weight, float eps, const float* __restrict__ input_scale,
@@ -36,9 +40,9 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     const int64_t row = blockIdx.x;
     const __nv_bfloat16* xr = x + row * ldx;
     __nv_bfloat16* rr = residual ? residual + row * ld_res : nullptr;
-    uint4 xa[kNormMaxVec], ra[kNormMaxVec], w[kNormMaxVec];
+    uint4 xa[kVec], ra[kVec], w[kVec];
 #pragma unroll
-    for (int j = 0; j < kNormMaxVec; ++j) {
+    for (int j = 0; j < kVec; ++j) {
         const int vec = threadIdx.x + j * kNormThreads;
         if (vec < nvec) {
             xa[j] = ld_dep(reinterpret_cast<const uint4*>(xr + vec * 8));
@@ -47,10 +51,10 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
         }
     }
     const ExactDiv div(quant ? fmaxf(ld_dep(input_scale), 1e-12f) : 1.f);    // behind the row's loads: its use holds the warp
-    float v[kNormMaxVec][8];
+    float v[kVec][8];
     float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < kNormMaxVec; ++j) {
+    for (int j = 0; j < kVec; ++j) {
         const int vec = threadIdx.x + j * kNormThreads;
         if (vec < nvec) {
             const uint32_t aw[4] = {xa[j].x, xa[j].y, xa[j].z, xa[j].w};
@@ -80,7 +84,7 @@ rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bflo
     for (int i = 0; i < kNormThreads / 32; ++i) t += s_part[i];
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(t, (float)H), eps)));
 #pragma unroll
-    for (int j = 0; j < kNormMaxVec; ++j) {
+    for (int j = 0; j < kVec; ++j) {
         const int vec = threadIdx.x + j * kNormThreads;
         if (vec < nvec) {
             const uint32_t ww[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
@@ -108,7 +112,9 @@ cudaError_t launch_rmsnorm_quant(const __nv_bfloat16* x, int64_t ldx, __nv_bfloa
     cudaLaunchAttribute attr[1];
     cfg.numAttrs = pdl_attribute(attr);
     cfg.attrs = attr;
-    return counted(cudaLaunchKernelEx(&cfg, rmsnorm_quant_kernel, x, ldx, residual, ld_res, weight, eps, input_scale, xq, y, ldy, (int)H));
+    const int64_t per_thread = (H / 8 + kNormThreads - 1) / kNormThreads;
+    auto kern = per_thread <= 1 ? rmsnorm_quant_kernel<1> : per_thread <= 2 ? rmsnorm_quant_kernel<2> : rmsnorm_quant_kernel<kNormMaxVec>;
+    return counted(cudaLaunchKernelEx(&cfg, kern, x, ldx, residual, ld_res, weight, eps, input_scale, xq, y, ldy, (int)H));
 }
 
 }  // namespace fp8lin
