@@ -9,7 +9,7 @@
 // written back widened, and no pass over x is needed (the earlier route for more than 64 rows re-read the weights for
 // every 64 rows on mma.sync, and from 256 rows wrote f16 copies of weights and activations to scratch first).
 //
-// What bounds it: per 128-element K block a CTA widens 16 KB of weights (about 450 SM cycles on the ALU and FMA pipes,
+// What bounds it: per 128-element K block a CTA widens 16 KB of weights (about 400 SM cycles on the ALU and FMA pipes,
 // eight warps) and the tensor core works 4 T cycles, so up to T = 160 the weight stream (690 cycles per 16 KB at 6.5 TB/s
 // over 148 SMs) or the widening is the limit and above it the tensor core.  Against one CTA with the same T the pair
 // halves the activation bytes each SM stages and feeds to its tensor core, which shared memory could not carry (a 128 x
@@ -89,15 +89,17 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* v) {
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Two e4m3 codes, zero-extended in the two halves of p, -> bf16x2, exact.  The magnitude bits go to bits 4..10 of a bf16
-// and the sign to bit 15 (b * 16 + (b & 0x80) * 240, no carry between the halves); that bf16 is the code's value times
-// 2^-120 (e4m3 subnormals become bf16 subnormals), so one multiplication by 2^120 finishes it.  Two IMADs and one HMUL2
-// run beside the two ALU instructions: 430 cycles per 16 KB tile and SM against 490 for the shift-and-mask form.  The NaN
-// codes 0x7f / 0xff come out as +-480; the caller tests for them.
-__device__ __forceinline__ uint32_t e4m3_pair_to_bf16(uint32_t p) {
-    const uint32_t t = p * 16u + (p & 0x00800080u) * 240u;
-    uint32_t r;
-    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(t), "r"(0x7b807b80u));
+// Two e4m3 codes of a word -> bf16x2, exact.  The magnitude bits go to bits 4..10 of a bf16 and the sign stays in bit 15; that bf16 is
+// the code's value times 2^-120 (e4m3 subnormals become bf16 subnormals), so one multiplication by 2^120 finishes it.  The byte
+// permutation replicates the sign bit, so that a shift (as a product: the ALU is the busier pipe) and a mask are all there is between.
+// With the sign put in by a second product instead, 64 rows on 3584 -> 37888 32.1 -> 30.3 us, 100 rows 37.5 -> 35.4.  (Four teams
+// of converters instead of two: the same; the sums of the NaN test as products too: slower.)  The NaN codes 0x7f / 0xff come out as
+// +-480; the caller tests for them.
+template <uint32_t kSelector>                      // 0x9180: codes 0 and 1 of the word, 0xb3a2: 2 and 3 (bit 3 of a digit: the byte's sign)
+__device__ __forceinline__ uint32_t e4m3_pair_to_bf16(uint32_t codes) {
+    uint32_t q, r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(q) : "r"(codes), "n"(kSelector));
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"((q * 16u) & 0x87f087f0u), "r"(0x7b807b80u));
     return r;
 }
 
@@ -116,8 +118,8 @@ __device__ __forceinline__ void widen_half_row(uint32_t row_addr, uint32_t swizz
         const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            v[8 * c + 2 * j] = e4m3_pair_to_bf16(__byte_perm(u[j], 0, 0x4140));
-            v[8 * c + 2 * j + 1] = e4m3_pair_to_bf16(__byte_perm(u[j], 0, 0x4342));
+            v[8 * c + 2 * j] = e4m3_pair_to_bf16<0x9180>(u[j]);
+            v[8 * c + 2 * j + 1] = e4m3_pair_to_bf16<0xb3a2>(u[j]);
             bad |= (u[j] & 0x7f7f7f7fu) + 0x01010101u;               // bit 7 of a byte: its code was a NaN
         }
     }
