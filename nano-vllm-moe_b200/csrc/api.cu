@@ -296,11 +296,12 @@ bool other_w8a8_route_forced() {
 //   17 to 64 rows: where the one-CTA decode kernel does not split K (a pair's CTAs then stage half of the rows each: 64 rows
 //     on 2048 -> 11008 6.7 us against 7.8, 3584 -> 37888 23.1 / 24.2), and where the pairs are modelled faster (64 rows on
 //     2048 -> 2048 4.5 / 4.8, 3584 -> 3584 6.2 / 6.8; not 18944 -> 3584 14.9 / 14.8, 8192 -> 1024 6.6 / 5.6).
-//   65 to 4096 rows: where modelled faster than both kernels with fixed tiles.  Over twelve layer shapes (1280 -> 1536 ..
-//     18944 -> 3584, 3584 -> 37888) and nineteen row counts the choice is 0.4 % slower than the best of the three; it is this
-//     kernel for most counts below 1500, e.g. (us, this / the other two) 256 rows on 3584 -> 3584 8.3 / 10.0, 700 on 18944 ->
-//     3584 40 / 51, 1031 on 3584 -> 37888 102 / 111, 3584 -> 4608 16.7 / 20.1; not 512 on 2560 -> 9472 13.9 / 12.6, 2048 on 3584
-//     -> 4608 25.6 / 24.5.  Above 4096 rows the 256-row tiles are as good as full and store whole lines.
+//   65 to 4096 rows: where modelled faster than both kernels with fixed tiles.  The model was fitted while the lanes stored the
+//     results; since they leave by TMA a call with whole sums takes 0.86 of it.  Over eleven layer shapes (2048 -> 2048 .. 3584 ->
+//     18944, 18944 -> 3584, 8192 -> 1024) and eighteen row counts from 17 on the choice is 0.2 % slower than the faster kernel, with the model as
+//     it was 1.3 %: e.g. (us, this / the other two) 700 rows on 3584 -> 4608 12.3 / 14.0, 1031 on 3584 -> 3584 12.8 / 13.4, 1500 on 11008
+//     -> 2048 24.9 / 31.4, 256 on 3584 -> 18944 14.5 / 16.2, 4096 on 3584 -> 3584 37.0 / 39.6; not 512 on 2560 -> 9472 12.0 / 11.4, 160 on
+//     8192 -> 1024 12.1 / 10.4.  Above 4096 rows the 256-row tiles are as good as full.
 const W8a8PairPlan* w8a8_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
     if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (two channels per store)
     if (g_tune.w8a8_pair < 0 && (M < 17 || M > 4096 || other_w8a8_route_forced())) return nullptr;
@@ -323,7 +324,7 @@ const W8a8PairPlan* w8a8_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy
             if (pl.splits == 1 && other > umma_pair_cost(M, K, N)) other = umma_pair_cost(M, K, N);
         }
         n.plan = plan_w8a8_pair(M, K, N, false, slices, g_tune.w8a8_pair_tokens, g_tune.w8a8_pair_splits);
-        n.pair = n.plan.cost < (g_tune.w8a8_pair > 0 ? 1e30 : other);
+        n.pair = n.plan.cost * (n.plan.slices == 1 ? 0.86 : 1.0) < (g_tune.w8a8_pair > 0 ? 1e29 : other);
         return n;
     });
     return r.pair ? &r.plan : nullptr;
