@@ -150,8 +150,12 @@ __device__ __forceinline__ void scan_experts(const int* total, int E, int chunk_
             const int pn = __shfl_up_sync(0xffffffffu, sn, o);
             if (lane >= o) sn += pn;
             if (cstart) {
-                const int pc = __shfl_up_sync(0xffffffffu, sc, o), pw = __shfl_up_sync(0xffffffffu, sw, o);
-                if (lane >= o) { sc += pc; sw += pw; }
+                const int pc = __shfl_up_sync(0xffffffffu, sc, o);
+                if (lane >= o) sc += pc;
+            }
+            if (cstart && even) {                  // (no shuffles of zeros in the chain of a decode step's grouping: 0.2 us)
+                const int pw = __shfl_up_sync(0xffffffffu, sw, o);
+                if (lane >= o) sw += pw;
             }
         }
         if (e0 + lane < E) {
@@ -161,7 +165,7 @@ __device__ __forceinline__ void scan_experts(const int* total, int E, int chunk_
         }
         row_base += __shfl_sync(0xffffffffu, sn, 31);
         chunk_base += __shfl_sync(0xffffffffu, sc, 31);
-        cost_base += __shfl_sync(0xffffffffu, sw, 31);
+        if (cstart && even) cost_base += __shfl_sync(0xffffffffu, sw, 31);
     }
     if (lane == 0 && cstart) {
         start[E] = row_base; cstart[E] = chunk_base;
