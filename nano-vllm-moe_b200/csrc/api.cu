@@ -1013,20 +1013,22 @@ namespace {
 // instead of inside the gate_up GEMM (where every channel tile would redo it)
 constexpr int64_t kMoePrequantRows = 512;
 struct MoeWs {
-    size_t off_offsets, off_counts, off_sorted, off_chunks, off_meta, off_inv, off_gu, off_hq, off_xq, total;
+    size_t off_offsets, off_sorted, off_chunks, off_meta, off_inv, off_gu, off_hq, off_xq, total;
 };
 MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
     MoeWs w;
     size_t o = FP8LIN_WS_HEADER_BYTES;
     auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return at; };
     w.off_offsets = take((size_t)(E + 1) * 4);
-    w.off_counts = take(rows >= kMoePrequantRows ? moe_count_ints(rows, E) * 4 : 0);
     w.off_sorted = take((size_t)(rows > 0 ? rows : 1) * 4);
     w.off_chunks = take((size_t)(E + rows / 16 + 2) * 16);
     w.off_meta = take(16);
     w.off_inv = take((size_t)(rows > 0 ? rows : 1) * 4);
     w.off_gu = take(g_tune.moe_fused == 0 ? (size_t)rows * 2 * I * 2 : 0);      // bf16 gate_up rows: only the separate pass reads them
-    w.off_hq = take((size_t)rows * I);
+    // The activations.  The grouping's counts lie there first: the GEMM that writes activations waits for the pass that reads the counts
+    // last, and the counting kernel waits for whatever read the activations of a call before.
+    const size_t counts = rows >= kMoePrequantRows ? moe_count_ints(rows, E) * 4 : 0;
+    w.off_hq = take((size_t)rows * I > counts ? (size_t)rows * I : counts);
     w.off_xq = take(rows >= kMoePrequantRows ? (size_t)rows * H : 0);
     w.total = o;
     return w;
@@ -1133,7 +1135,7 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     const bool rows_major = !pair_rows && rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
     unsigned char* xq = ws + L.off_xq;
     cudaError_t e = rows >= kMoePrequantRows ? launch_moe_group_quant((const __nv_bfloat16*)x, ldx, x_div, ids, ids_i64, (int)rows, E, mp, pair_rows != 0,
-                                                                      w13_input_scale, (int*)(ws + L.off_counts), sorted, chunks, meta, inv, xq, (int)H, st)
+                                                                      w13_input_scale, (int*)hq, sorted, chunks, meta, inv, xq, (int)H, st)
                                              : launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
