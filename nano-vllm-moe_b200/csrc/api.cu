@@ -142,7 +142,7 @@ bool w8a16_pair_wanted(int64_t M, int64_t K, int64_t N) {
 }
 // null: another kernel's
 const W8a16PairPlan* w8a16_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
-    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (two channels per store)
+    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (whole sums leave by TMA, slices two channels per store)
     const W8a16Route& r = route_of<W8a16Route>(M, K, N, 0, [&] {
         W8a16Route n;
         n.pair = w8a16_pair_wanted(M, K, N);
@@ -303,7 +303,7 @@ bool other_w8a8_route_forced() {
 //     -> 2048 24.9 / 31.4, 256 on 3584 -> 18944 14.5 / 16.2, 4096 on 3584 -> 3584 37.0 / 39.6; not 512 on 2560 -> 9472 12.0 / 11.4, 160 on
 //     8192 -> 1024 12.1 / 10.4.  Above 4096 rows the 256-row tiles are as good as full.
 const W8a8PairPlan* w8a8_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
-    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (two channels per store)
+    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (whole sums leave by TMA, slices two channels per store)
     if (g_tune.w8a8_pair < 0 && (M < 17 || M > 4096 || other_w8a8_route_forced())) return nullptr;
     const W8a8Route& r = route_of<W8a8Route>(M, K, N, 0, [&] {
         W8a8Route n;
@@ -1047,7 +1047,7 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 namespace {
 int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, int64_t ld_out) {
     if (g_tune.moe_pair == 0 || g_tune.moe_fused == 0 || g_tune.moe_rows_major >= 0 || rows < kMoePrequantRows || E > 1024) return 0;
-    if (ld_out % 2 != 0 || (reinterpret_cast<uintptr_t>(out) & 3) != 0) return 0;                      // (two channels per store)
+    if (ld_out % 2 != 0 || (reinterpret_cast<uintptr_t>(out) & 3) != 0) return 0;                      // (whole sums leave by TMA, slices two channels per store)
     if (g_tune.moe_pair > 0) return (int)align_up((size_t)(g_tune.moe_pair < kGroupedPairMaxRows ? g_tune.moe_pair : kGroupedPairMaxRows), 32);
     const int64_t avg = (rows + E - 1) / E;
     const int64_t items = E * (pack_ntiles(I) < (pack_ntiles(H) + 1) / 2 ? pack_ntiles(I) : (pack_ntiles(H) + 1) / 2);
