@@ -347,6 +347,10 @@ int fp8lin_debug_wait_timeout(void* workspace, int64_t limit_us, void* stream);
  * division, both fp32, for n bf16 values g. */
 int fp8lin_debug_silu(const void* g, float* fast, float* divided, int64_t n, void* stream);
 
+/* For tests: the routed rows that a block of the expert batches' grouping ranks (all slots of its tokens), 0 where the batch
+ * is grouped by one CTA. */
+int64_t fp8lin_debug_moe_share_rows(int64_t rows, int x_div);
+
 #ifdef __cplusplus
 }
 #endif

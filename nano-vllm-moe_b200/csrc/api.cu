@@ -1010,7 +1010,7 @@ int fp8lin_set_tuning(const char* knob, int value) {
 // ---- MoE -------------------------------------------------------------------------------------
 namespace {
 // from this many routed rows on, the rows are gathered and quantised once by a separate pass
-// instead of inside the gate_up GEMM (where every channel tile would redo it)
+// instead of inside the gate_up GEMM (where every channel tile would redo it), if that pass can rank them (moe_share_rows)
 constexpr int64_t kMoePrequantRows = 512;
 struct MoeWs {
     size_t off_offsets, off_sorted, off_chunks, off_meta, off_inv, off_gu, off_hq, off_xq, total;
@@ -1128,15 +1128,17 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     int* inv = (int*)(ws + L.off_inv);
     __nv_bfloat16* gu = (__nv_bfloat16*)(ws + L.off_gu);
     unsigned char* hq = ws + L.off_hq;
-    const int pair_rows = moe_pair_rows(rows, E, H, I, out_routed, ld_out);
+    // grouped and quantised by kernels that spread over the chip; else one CTA groups and gate_up quantises the rows it gathers
+    const bool spread = rows >= kMoePrequantRows && moe_share_rows(rows, x_div) > 0;
+    const int pair_rows = !spread ? 0 : moe_pair_rows(rows, E, H, I, out_routed, ld_out);
     const int mp = pair_rows ? pair_rows : grouped_chunk_rows(rows, E);
     // Few work items whose experts fill 128-row chunks: the rows are the MMA M dimension (umma_grouped_rows.cu), in
     // gate_up where the up channels start at a tile.
-    const bool rows_major = !pair_rows && rows >= kMoePrequantRows && mp == 128 && g_tune.moe_rows_major != 0;
+    const bool rows_major = spread && !pair_rows && mp == 128 && g_tune.moe_rows_major != 0;
     unsigned char* xq = ws + L.off_xq;
-    cudaError_t e = rows >= kMoePrequantRows ? launch_moe_group_quant((const __nv_bfloat16*)x, ldx, x_div, ids, ids_i64, (int)rows, E, mp, pair_rows != 0,
-                                                                      w13_input_scale, (int*)hq, sorted, chunks, meta, inv, xq, (int)H, st)
-                                             : launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
+    cudaError_t e = spread ? launch_moe_group_quant((const __nv_bfloat16*)x, ldx, x_div, ids, ids_i64, (int)rows, E, mp, pair_rows != 0, w13_input_scale,
+                                                    (int*)hq, sorted, chunks, meta, inv, xq, (int)H, st)
+                           : launch_moe_align(ids, ids_i64, (int)rows, E, mp, offsets, sorted, chunks, meta, inv, st);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "row grouping launch: %s", cudaGetErrorString(e));
     const char* why = nullptr;
     GroupedArgs a;
@@ -1148,7 +1150,7 @@ static int moe_experts_impl(const void* x, int64_t ldx, int x_div, const void* i
     const bool fused_act = g_tune.moe_fused != 0;
     GroupedArgs g = a;
     if (fused_act) { g.N = (int)I; g.hq = hq; g.h_scale = w2_input_scale; g.out = nullptr; }
-    if (rows >= kMoePrequantRows) {
+    if (spread) {
         e = pair_rows ? launch_grouped_pair_w8a8(g, pair_rows, w13_packed, E, xq, rows, st, &why)
           : rows_major && fused_act && I % 128 == 0 ? launch_grouped_rows_w8a8(g, w13_packed, E, xq, rows, st, &why)
                                                     : launch_grouped_w8a8(false, mp, g, w13_packed, E, xq, rows, st, &why);
@@ -1225,6 +1227,10 @@ int fp8lin_debug_wait_timeout(void* workspace, int64_t limit_us, void* stream) {
     cudaError_t e = launch_wait_timeout_probe((int*)workspace, (long long)limit_us * 2000, nullptr, (cudaStream_t)stream);
     if (e != cudaSuccess) return fail(FP8LIN_ERR_LAUNCH, "probe launch: %s", cudaGetErrorString(e));
     return FP8LIN_OK;
+}
+
+int64_t fp8lin_debug_moe_share_rows(int64_t rows, int x_div) {
+    return rows >= kMoePrequantRows && rows <= (1ll << 24) && x_div > 0 ? moe_share_rows(rows, x_div) : 0;
 }
 
 int fp8lin_debug_silu(const void* g, float* fast, float* divided, int64_t n, void* stream) {

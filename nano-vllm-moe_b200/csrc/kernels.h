@@ -197,6 +197,9 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // multiple of 32 (chunk_rows is one), chunk.w = the costs (grouped_pair_cost) of all chunks in front of it, meta[2] = of all; else
 // into chunks of chunk_rows and a rest, chunk.w = 0.
 size_t moe_count_ints(int64_t rows, int E);
+// The routed rows (at most 2^24, x_div to a token) that a block of it ranks, all slots of its tokens; 0: more than a rank's bits
+// hold, such a batch is launch_moe_align's.
+int64_t moe_share_rows(int64_t rows, int x_div);
 cudaError_t launch_moe_group_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even,
                                    const float* input_scale, int* counts, int* sorted_rows, int4* chunks, int* meta, int* inv, unsigned char* xq, int H,
                                    cudaStream_t stream);

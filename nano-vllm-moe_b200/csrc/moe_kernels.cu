@@ -279,13 +279,16 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // first block also writes the chunk list.  Launch times of 16384 rows x 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before,
 // 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); 4096 tokens, 4 of 60 experts 222 -> 217.
 constexpr int kMoeShares = 128;                    // at most (see moe_count_ints)
-constexpr int kRankBits = 18;                      // a row's rank inside its share (of 2^24 / 128 rows and a token's); the expert (E <= 3071) above it
-static_assert((1 << 24) / kMoeShares < 1 << kRankBits, "2^24 routed rows at most");
+constexpr int kRankBits = 18;                      // a row's rank inside its share (see moe_share_rows); the expert (E <= 3071) above it
 
 // tokens of a share: all slots of a token lie in the same one
-__host__ __device__ inline int share_tokens(int rows, int x_div) {
+static int share_tokens(int rows, int x_div) {
     const int tokens = (rows + x_div - 1) / x_div, least = (512 + x_div - 1) / x_div, even = (tokens + kMoeShares - 1) / kMoeShares;
     return least > even ? least : even;
+}
+int64_t moe_share_rows(int64_t rows, int x_div) {
+    const int64_t n = (int64_t)share_tokens((int)rows, x_div) * x_div;
+    return n <= 1 << kRankBits ? n : 0;
 }
 
 template <typename IdT>

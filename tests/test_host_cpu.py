@@ -217,6 +217,23 @@ def test_expert_scratch_holds_what_the_route_writes(pkg):
     assert block == need + rows * h * 2                              # + the routed rows that the combine reads
 
 
+def test_ranks_of_grouped_rows_fit_their_bits(pkg):
+    """A routed row's place is kept as its expert above an 18-bit rank inside a share of whole tokens: a batch whose shares are
+    longer (from some 131072 slots of one token on) has to be grouped the other way."""
+    share = pkg._lib.load().fp8lin_debug_moe_share_rows
+    bits, most = 18, 1 << 24
+    rng = np.random.default_rng(5)
+    cases = [(most, d) for d in (1, 4, 32, 131072, 262144, 262145)]
+    cases += [(300000, d) for d in (1, 262143, 262144, 262145, 300000)] + [(1 << 18, 1 << 18), ((1 << 18) + 1, (1 << 18) + 1)]
+    cases += [(int(2 ** rng.uniform(9, 24)), int(2 ** rng.uniform(0, 24))) for _ in range(2000)]
+    for rows, d in cases:
+        n = share(rows, d)
+        # tokens of a share: 512 rows at least, 128 shares at most
+        whole = d * max(-(-512 // d), -(-(-(-rows // d)) // 128))
+        assert n == (whole if whole <= 1 << bits else 0), (rows, d, n)
+    assert share(511, 1) == 0 and share(512, 1) == 512 and share(most, 1) == most // 128 and share(most, 32) == most // 128
+
+
 def test_gate_up_interleave_is_a_tile_row_permutation():
     """interleave_gate_up(pack(W)) == pack(W with its 128-row blocks alternating gate / up)."""
     from importlib import import_module
