@@ -281,13 +281,10 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 constexpr int kMoeShares = 128;                    // at most (see moe_count_ints)
 constexpr int kRankBits = 18;                      // a row's rank inside its share (see moe_share_rows); the expert (E <= 3071) above it
 
-// tokens of a share: all slots of a token lie in the same one
-static int share_tokens(int rows, int x_div) {
-    const int tokens = (rows + x_div - 1) / x_div, least = (512 + x_div - 1) / x_div, even = (tokens + kMoeShares - 1) / kMoeShares;
-    return least > even ? least : even;
-}
+// all slots of a token lie in the same share
 int64_t moe_share_rows(int64_t rows, int x_div) {
-    const int64_t n = (int64_t)share_tokens((int)rows, x_div) * x_div;
+    const int64_t tokens = (rows + x_div - 1) / x_div, least = (512 + (int64_t)x_div - 1) / x_div, even = (tokens + kMoeShares - 1) / kMoeShares;
+    const int64_t n = (least > even ? least : even) * x_div;
     return n <= 1 << kRankBits ? n : 0;
 }
 
@@ -390,7 +387,8 @@ size_t moe_count_ints(int64_t rows, int E) {
 cudaError_t launch_moe_group_quant(const __nv_bfloat16* x, int64_t ldx, int x_div, const void* ids, bool ids_i64, int rows, int E, int chunk_rows, bool even,
                                    const float* input_scale, int* counts, int* sorted_rows, int4* chunks, int* meta, int* inv, unsigned char* xq, int H,
                                    cudaStream_t stream) {
-    const int share_tok = share_tokens(rows, x_div), tokens = (rows + x_div - 1) / x_div;
+    const int share_tok = (int)(moe_share_rows(rows, x_div) / x_div), tokens = (rows + x_div - 1) / x_div;
+    if (share_tok == 0) return cudaErrorInvalidValue;
     const int shares = (tokens + share_tok - 1) / share_tok;
     const size_t smem = (size_t)E * sizeof(int);
     cudaError_t e = ids_i64 ? launch_dependent(moe_count_kernel<long long>, shares, 512, smem, stream, (const long long*)ids, rows, E, share_tok * x_div, counts, inv)

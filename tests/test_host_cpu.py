@@ -225,7 +225,8 @@ def test_ranks_of_grouped_rows_fit_their_bits(pkg):
     rng = np.random.default_rng(5)
     cases = [(most, d) for d in (1, 4, 32, 131072, 262144, 262145)]
     cases += [(300000, d) for d in (1, 262143, 262144, 262145, 300000)] + [(1 << 18, 1 << 18), ((1 << 18) + 1, (1 << 18) + 1)]
-    cases += [(int(2 ** rng.uniform(9, 24)), int(2 ** rng.uniform(0, 24))) for _ in range(2000)]
+    cases += [(rows, (1 << 31) - d) for rows in (512, 600, most) for d in (1, 2, 511, 512, 513, 600, most)]       # x_div is any int
+    cases += [(int(2 ** rng.uniform(9, 24)), int(2 ** rng.uniform(0, 31)) - 1 | 1) for _ in range(2000)]
     for rows, d in cases:
         n = share(rows, d)
         # tokens of a share: 512 rows at least, 128 shares at most
