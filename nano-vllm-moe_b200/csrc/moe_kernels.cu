@@ -132,18 +132,48 @@ __device__ __forceinline__ int chunk_size(int n, int chunk_rows, int even) {
     const int k = (n + chunk_rows - 1) / chunk_rows;
     return ((n + k - 1) / k + 31) & ~31;
 }
-// One warp: exclusive scans of rows, chunks and (even) costs over the experts; start and cstart have E + 1 entries.  All but start may
-// be left out (null).
+// Exclusive scans of rows, chunks and (even) costs over the experts by one warp or by a block of kWarps, a stretch of the experts
+// each, behind what each adds up of the stretches in front; start and cstart have E + 1 entries.  All but start may be left out (null).
+template <int kWarps>
 __device__ __forceinline__ void scan_experts(const int* total, int E, int chunk_rows, int even, int* start, int* cstart, int* coststart, int* meta) {
-    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int stretch = (E + 32 * kWarps - 1) / (32 * kWarps) * 32;
+    const int first = kWarps == 1 ? 0 : min(E, warp * stretch), last = min(E, first + stretch);
+    auto chunks_of = [&](int n, int& c, int& cost) {
+        const int size = chunk_size(n, chunk_rows, even);
+        c = (n + size - 1) / size;
+        cost = even && c ? (c - 1) * grouped_pair_cost(size >> 5) + grouped_pair_cost((n - (c - 1) * size + 31) >> 5) : 0;
+    };
     int row_base = 0, chunk_base = 0, cost_base = 0;
-    for (int e0 = 0; e0 < E; e0 += 32) {
-        const int n = e0 + lane < E ? total[e0 + lane] : 0;
-        int sn = n, c = 0, cost = 0;
+    if constexpr (kWarps > 1) {
+        if (cstart) {                              // (the divisions once per expert; the scans take them from their own places)
+            for (int e = threadIdx.x; e < E; e += 32 * kWarps) {
+                int c, cost;
+                chunks_of(total[e], c, cost);
+                cstart[e] = c;
+                if (even) coststart[e] = cost;
+            }
+            __syncthreads();
+        }
+        for (int e = lane; e < first; e += 32) {
+            row_base += total[e];
+            if (cstart) chunk_base += cstart[e];
+            if (cstart && even) cost_base += coststart[e];
+        }
+        row_base = __reduce_add_sync(0xffffffffu, row_base);
         if (cstart) {
-            const int size = chunk_size(n, chunk_rows, even);
-            c = (n + size - 1) / size;
-            cost = even && c ? (c - 1) * grouped_pair_cost(size >> 5) + grouped_pair_cost((n - (c - 1) * size + 31) >> 5) : 0;
+            chunk_base = __reduce_add_sync(0xffffffffu, chunk_base);
+            cost_base = __reduce_add_sync(0xffffffffu, cost_base);
+            __syncthreads();
+        }
+    }
+    for (int e0 = first; e0 < last; e0 += 32) {
+        const int n = e0 + lane < last ? total[e0 + lane] : 0;
+        int sn = n, c = 0, cost = 0;
+        if (cstart && kWarps == 1) chunks_of(n, c, cost);
+        if (cstart && kWarps > 1 && e0 + lane < last) {
+            c = cstart[e0 + lane];
+            if (even) cost = coststart[e0 + lane];
         }
         int sc = c, sw = cost;
         for (int o = 1; o < 32; o <<= 1) {
@@ -158,7 +188,7 @@ __device__ __forceinline__ void scan_experts(const int* total, int E, int chunk_
                 if (lane >= o) sw += pw;
             }
         }
-        if (e0 + lane < E) {
+        if (e0 + lane < last) {
             start[e0 + lane] = row_base + sn - n;
             if (cstart) cstart[e0 + lane] = chunk_base + sc - c;
             if (cstart && even) coststart[e0 + lane] = cost_base + sw - cost;
@@ -167,7 +197,7 @@ __device__ __forceinline__ void scan_experts(const int* total, int E, int chunk_
         chunk_base += __shfl_sync(0xffffffffu, sc, 31);
         if (cstart && even) cost_base += __shfl_sync(0xffffffffu, sw, 31);
     }
-    if (lane == 0 && cstart) {
+    if (warp == kWarps - 1 && lane == 0 && cstart) {
         start[E] = row_base; cstart[E] = chunk_base;
         meta[0] = chunk_base; meta[1] = row_base;
         if (even) meta[2] = cost_base;
@@ -224,7 +254,7 @@ moe_align_kernel(const IdT* __restrict__ ids, int rows, int E, int chunk_rows, i
         total[e] = acc;
     }
     __syncthreads();
-    if (warp == 0) scan_experts(total, E, chunk_rows, 0, start, cstart, nullptr, meta);
+    if (warp == 0) scan_experts<1>(total, E, chunk_rows, 0, start, cstart, nullptr, meta);
     __syncthreads();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) expert_offsets[e] = start[e];
     if (warp < kWarps) {
@@ -278,6 +308,11 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // elements of a token once and stores them to the places of its x_div slots: 2 + x_div bytes of traffic per token element.  The
 // first block also writes the chunk list.  Launch times of 16384 rows x 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before,
 // 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); 4096 tokens, 4 of 60 experts 222 -> 217.
+// What grows with the experts is every block's: the counts of a share are read beside each other by as many threads as there are
+// experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
+// experts (512 rows; 14 now, one CTA's grouping and the rows 17).  Blocks in a loop, us, one CTA's grouping and a pass over the rows / here:
+// 60 experts 2048 -> 1408, 512 rows 97.7 / 96.5, 2048 rows 115.4 / 103.2; 512 experts 2048 -> 512, 512 rows 183.9 / 180.2, 4096 rows
+// 297.5 / 289.3; 1024 experts 1024 -> 256, 512 rows 89.9 / 89.3, 4096 rows 191.0 / 181.4.
 constexpr int kMoeShares = 128;                    // at most (see moe_count_ints)
 constexpr int kRankBits = 18;                      // a row's rank inside its share (see moe_share_rows); the expert (E <= 3071) above it
 
@@ -337,17 +372,18 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
         vb = ld_dep(source(t_mine, c_first) + 1);
     }
     __syncthreads();
-    // a warp sums up every eighth share, a lane every 32nd expert; four loads in flight
-    for (int e = threadIdx.x & 31; e < E; e += 32) {
+    // threads beside each other sum up experts beside each other, eight shares in flight; what is left of the block divides the shares
+    const int across = E <= 32 ? 32 : E <= 64 ? 64 : E <= 128 ? 128 : 256, groups = 256 / across;
+    for (int e = (int)threadIdx.x & (across - 1); e < E; e += across) {
         int all = 0, front = 0;
-        for (int b = threadIdx.x >> 5; b < shares; b += 32) {
-            int n[4];
+        for (int b = (int)threadIdx.x / across; b < shares; b += 8 * groups) {
+            int n[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) n[i] = b + 8 * i < shares ? ld_dep(counts + (size_t)(b + 8 * i) * E + e) : 0;
+            for (int i = 0; i < 8; ++i) n[i] = b + i * groups < shares ? ld_dep(counts + (size_t)(b + i * groups) * E + e) : 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < 8; ++i) {
                 all += n[i];
-                if (b + 8 * i < share) front += n[i];
+                if (b + i * groups < share) front += n[i];
             }
         }
         if (all) atomicAdd(&total[e], all);
@@ -355,7 +391,7 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
     }
     __syncthreads();
     const bool first = blockIdx.x == 0;
-    if (threadIdx.x < 32) scan_experts(total, E, chunk_rows, even, start, first ? cstart : nullptr, first ? coststart : nullptr, meta);
+    scan_experts<8>(total, E, chunk_rows, even, start, first ? cstart : nullptr, first ? coststart : nullptr, meta);
     __syncthreads();
     if (first) write_chunks(total, E, chunk_rows, even, start, cstart, coststart, chunks);
 
