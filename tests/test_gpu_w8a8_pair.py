@@ -58,6 +58,34 @@ def test_mlp_epilogue_equals_the_other_kernels(m, h, inter, tokens):
     np.testing.assert_array_equal(run_fused(d), want)
 
 
+@pytest.mark.parametrize("tokens", [32, 64])
+@pytest.mark.parametrize("gate", [0.0, 30.0, 300.0, 1e4, 1e30, 3e38, float("inf"), float("nan")])
+def test_mlp_epilogue_on_gates_of_any_size(gate, tokens):
+    """Gates that overflow the exponential, zeros, infinities and NaN beside ordinary ones: the codes of the separate activation pass.  The
+    rows lie orders of magnitude apart, so that those beside a row with a NaN stay finite."""
+    Kn = kernels()
+    m, h, inter = 64, 272, 256
+    gu, down = make_mlp_case(23, m, h, inter, 264)
+    gu["x"] = O.bf16_round((gu["x"] * 2.0 ** -(np.arange(m) % 8)[:, None]).astype(np.float32))
+    gu["x"][5] = 0.0
+    if np.isnan(gate):
+        gu["x"][9::16, 3] = np.nan
+    else:                                             # of the first channels, half of their up values with them
+        gu["w_scale"][:16] *= np.float32(gate)
+        gu["w_scale"][inter:inter + 8] *= np.float32(gate)
+    d = upload_mlp(gu, down, inter)
+    Kn.set_tuning("w8a8_pair", 0)
+    want = run_fused(d)
+    Kn.set_tuning("w8a8_pair", 1)
+    Kn.set_tuning("w8a8_pair_tokens", tokens)
+    got = run_fused(d)
+    np.testing.assert_array_equal(got, want)          # (NaN equals NaN here)
+    if np.isnan(gate):
+        assert np.isnan(want[9::16]).all() and np.isfinite(np.delete(want, np.s_[9::16], 0)).all()
+    elif np.isfinite(gate):
+        assert np.isfinite(want[5]).all() and np.abs(want).max() > 0
+
+
 @pytest.mark.parametrize("m,n,tokens", [(17, 72, 32), (47, 264, 32), (81, 584, 96), (160, 8, 160), (300, 648, 224)])
 def test_results_stay_inside_the_output_matrix(m, n, tokens):
     """Boxes of 16 tokens and 64 channels, clipped at the last token and channel: rows of a wider, longer matrix keep what was there."""
