@@ -142,7 +142,7 @@ bool w8a16_pair_wanted(int64_t M, int64_t K, int64_t N) {
 }
 // null: another kernel's
 const W8a16PairPlan* w8a16_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
-    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (whole sums leave by TMA, slices two channels per store)
+    if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (the lanes store two channels at once; 8 and 16 bytes as in the other routes)
     const W8a16Route& r = route_of<W8a16Route>(M, K, N, 0, [&] {
         W8a16Route n;
         n.pair = w8a16_pair_wanted(M, K, N);
@@ -293,15 +293,18 @@ bool other_w8a8_route_forced() {
 
 // W8A8 on CTA pairs with the rows as the MMA's N (umma_w8a8_pair.cu), K in as many slices as the sums of the other kernels
 // have (see plan_swap); where the one-CTA GEMM would cut only its last tiles (its tail launch), the call stays there.
+// Figures: us per call on rows that are codes, in a loop over weights from memory, this / the kernels it stands in for.
 //   17 to 64 rows: where the one-CTA decode kernel does not split K (a pair's CTAs then stage half of the rows each: 64 rows
-//     on 2048 -> 11008 6.7 us against 7.8, 3584 -> 37888 23.1 / 24.2), and where the pairs are modelled faster (64 rows on
-//     2048 -> 2048 4.5 / 4.8, 3584 -> 3584 6.2 / 6.8; not 18944 -> 3584 14.9 / 14.8, 8192 -> 1024 6.6 / 5.6).
+//     on 2048 -> 11008 6.2 / 7.8, 3584 -> 37888 23.1 / 24.2), and where the pairs are modelled faster (64 rows on 2048 -> 2048
+//     4.84 / 4.96, 3584 -> 3584 6.92 / 7.07, 18944 -> 3584 14.7 / 15.3; not 8192 -> 1024 12.1 / 5.8).  Where K is split and bf16 rows bring a
+//     quantiser in front, the decode kernel hides more of it (64 rows on 3584 -> 3584 8.6 / 7.9, 2048 -> 2048 6.4 / 6.3), which
+//     this line does not weigh.
 //   65 to 4096 rows: where modelled faster than both kernels with fixed tiles.  The model was fitted while the lanes stored the
 //     results; since they leave by TMA a call with whole sums takes 0.86 of it.  Over eleven layer shapes (2048 -> 2048 .. 3584 ->
 //     18944, 18944 -> 3584, 8192 -> 1024) and eighteen row counts from 17 on the choice is 0.2 % slower than the faster kernel, with the model as
-//     it was 1.3 %: e.g. (us, this / the other two) 700 rows on 3584 -> 4608 12.3 / 14.0, 1031 on 3584 -> 3584 12.8 / 13.4, 1500 on 11008
-//     -> 2048 24.9 / 31.4, 256 on 3584 -> 18944 14.5 / 16.2, 4096 on 3584 -> 3584 37.0 / 39.6; not 512 on 2560 -> 9472 12.0 / 11.4, 160 on
-//     8192 -> 1024 12.1 / 10.4.  Above 4096 rows the 256-row tiles are as good as full.
+//     it was 1.3 %: e.g. 700 rows on 3584 -> 4608 12.0 / 14.5, 1031 on 3584 -> 3584 13.0 / 14.2, 1500 on 11008 -> 2048 27.8 / 33.5, 256 on
+//     3584 -> 18944 18.2 / 19.2, 512 on 2560 -> 9472 12.7 / 13.3, 4096 on 3584 -> 3584 40.3 / 45.1; not 160 on 8192 -> 1024 12.1 / 10.8.
+//     Above 4096 rows the 256-row tiles are as good as full.
 const W8a8PairPlan* w8a8_pair_route(int64_t M, int64_t K, int64_t N, int64_t ldy, const void* y) {
     if (N % 8 != 0 || ldy % 8 != 0 || !aligned16(y)) return nullptr;           // (whole sums leave by TMA, slices two channels per store)
     if (g_tune.w8a8_pair < 0 && (M < 17 || M > 4096 || other_w8a8_route_forced())) return nullptr;
@@ -1040,17 +1043,18 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 
 // Expert batches on CTA pairs (umma_grouped_pair.cu): the most rows of a chunk, 0 = one CTA's kernels.
 //   The line: more than 32 rows per expert, of at least kMoePrequantRows.  Measured (us per block in a loop, one CTA / pairs): 60
-//   experts 2048 -> 1408, 34 rows each 119 / 110, 68 rows 129 / 124, 136 rows 175 / 150, 273 rows 258 / 207; 64 experts 1024 -> 512,
-//   40 rows 57 / 49; 8 experts 1024 -> 512, 4096 rows 132 / 116; but 30 experts 1152 -> 1200, 26 rows 47.0 / 48.5.  Up to 128 rows a pair
-//   has to have two work items of either projection: 16 experts 2048 -> 1024, 75 rows 43.7 / 47.0 (128 items, 74 pairs); a chunk of more
-//   can be cut (8 experts 1024 -> 1408, 175 rows, 88 items 41.4 / 38.6).
+//   experts 2048 -> 1408, 34 rows each 115 / 105, 68 rows 124.6 / 122.5, 136 rows 180 / 148, 273 rows 278 / 219; 64 experts 1024 -> 512,
+//   40 rows 48.8 / 39.6; 8 experts 1024 -> 512, 4096 rows 128 / 120; but 30 experts 1152 -> 1200, 26 rows 41.4 / 43.8.  Up to 128 rows a pair
+//   has to have two work items of either projection: 16 experts 2048 -> 1024, 75 rows 36.9 / 38.4 (128 items, 74 pairs); a chunk of more
+//   can be cut (8 experts 1024 -> 1408, 175 rows, 88 items 33.4 / 31.0).  Of a hundred sizes (8 to 60 experts, 512 to 16384 rows) one is
+//   known to lose by it: 8 experts 1024 -> 512, 512 rows each 28.9 / 32.3.
 //   The chunk: a busy expert's rows, should the tokens choose at random (mean and three deviations), where that is 320 or less:
-//   273 rows on average 207 in chunks of up to 320, 215 of 288 (a sixth of the experts in two), 238 of 256; 256 above (512 rows
-//   112 / 113.5 in chunks of up to 320, 4096 rows 116 / 119).  Shorter chunks leave room for more slots, but below 192 rows that buys nothing.
+//   273 rows on average 219 in chunks of up to 320, 221 of 288 (a sixth of the experts in two), 241 of 256; 256 above (8 experts 1024 ->
+//   512, 512 rows each 32.3, in chunks of up to 320 31.8, 4096 rows 120.6 / 118: little either way).  Shorter chunks leave room for more slots, but below 192 rows that buys nothing.
 namespace {
 int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, int64_t ld_out) {
     if (g_tune.moe_pair == 0 || g_tune.moe_fused == 0 || g_tune.moe_rows_major >= 0 || rows < kMoePrequantRows || E > 1024) return 0;
-    if (ld_out % 2 != 0 || (reinterpret_cast<uintptr_t>(out) & 3) != 0) return 0;                      // (whole sums leave by TMA, slices two channels per store)
+    if (ld_out % 2 != 0 || (reinterpret_cast<uintptr_t>(out) & 3) != 0) return 0;   // (down stores two channels, 4 bytes, at once)
     if (g_tune.moe_pair > 0) return (int)align_up((size_t)(g_tune.moe_pair < kGroupedPairMaxRows ? g_tune.moe_pair : kGroupedPairMaxRows), 32);
     const int64_t avg = (rows + E - 1) / E;
     const int64_t items = E * (pack_ntiles(I) < (pack_ntiles(H) + 1) / 2 ? pack_ntiles(I) : (pack_ntiles(H) + 1) / 2);

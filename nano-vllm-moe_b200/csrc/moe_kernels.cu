@@ -307,7 +307,7 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // valid expert.  The grouped GEMM then takes its rows by TMA instead of re-quantising them for every channel tile.  A thread converts 16
 // elements of a token once and stores them to the places of its x_div slots: 2 + x_div bytes of traffic per token element.  The
 // first block also writes the chunk list.  Launch times of 16384 rows x 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before,
-// 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); 4096 tokens, 4 of 60 experts 222 -> 217.
+// 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); the block of 4096 tokens, 4 of 60 experts, takes 2 % less.
 // What grows with the experts is every block's: the counts of a share are read beside each other by as many threads as there are
 // experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
 // experts (512 rows; 14 now, one CTA's grouping and the rows 17).  Blocks in a loop, us, one CTA's grouping and a pass over the rows / here:

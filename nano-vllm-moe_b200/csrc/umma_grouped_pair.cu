@@ -20,8 +20,8 @@
 // of 60 experts 2048 -> 2 x 1408, its MMAs 576 SM cycles per K block of 288 rows), memory alone below.  So a chunk holds all
 // rows of an expert where it can (its weights come once), rows are the MMA's N (273 rows of an expert on average are multiplied as
 // 288, in 128-row tiles as 384), and a K block of 256 channels x 288 rows moves 34 KB into each SM where 128 x 256 tiles move 48 KB
-// for a third of the products.  16384 rows of 60 experts, in a loop under the power limit: the block 258 us with 128 x 256 tiles on
-// one CTA (umma_grouped_rows.cu), 207 here; 8192 rows 175 / 150; 2048 rows 119 / 110.  Five or six slots of loads in flight: asking
+// for a third of the products.  16384 rows of 60 experts, in a loop under the power limit: the block 278 us with 128 x 256 tiles on
+// one CTA (umma_grouped_rows.cu), 219 here; 8192 rows 180 / 148; 2048 rows 115 / 105.  Five or six slots of loads in flight: asking
 // weights beyond them into L2 in front was slower the further (192 us without, 196 six blocks ahead, 206 sixteen).
 //
 // Sixteen epilogue warps: eight take longer over an item of gate_up than its MMAs do.

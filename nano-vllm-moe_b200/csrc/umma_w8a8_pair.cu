@@ -25,10 +25,11 @@
 //   and park their sums in shared memory; slice r's CTA adds up band r of its pair rank's channels
 //
 // What bounds it: up to T = 64 the way of 16 KB of weights per CTA and K block into shared memory (0.09 us when few SMs load,
-// 0.16 when all do), above that the tensor core (512 cycles per K block at T = 256), for large calls its power.  Per call back
-// to back, before (decode kernel, one-CTA GEMM or 256-row pairs, whichever was chosen) -> now: 3584 -> 3584 64 rows 7.2 -> 6.2
-// us, 256 rows 10.0 -> 8.3; 3584 -> 4608 1031 rows 20.1 -> 16.7; 3584 -> 37888 1031 rows 111 -> 102; 18944 -> 3584 700 rows
-// 51 -> 40, 1031 rows 59 -> 54.  Four 7B layers of 64 rows: 271 -> 239 us, two of 1031 rows: 527 -> 484.  All waits are bounded.
+// 0.16 when all do), above that the tensor core (512 cycles per K block at T = 256), for large calls its power.  Per call on
+// codes, in a loop over weights from memory, us: decode kernel, one-CTA GEMM or 256-row pairs, whichever would be chosen / here
+// with the lanes storing the results / here: 3584 -> 3584 64 rows 7.07 / 7.25 / 6.92, 256 rows 9.8 / 8.5 / 8.2; 3584 -> 4608 1031 rows 19.9 / 16.8
+// / 16.1; 3584 -> 37888 1031 rows 122 / 110 / 107 (power: 5 % from run to run); 18944 -> 3584 700 rows 54 / 41.3 / 40.9, 1031 rows
+// 60 / 54.6 / 53.7.  All waits are bounded.
 #include "umma_common.cuh"
 
 namespace fp8lin {
@@ -297,8 +298,7 @@ w8a8_pair_kernel(const __grid_constant__ PairMaps8 maps, UmmaArgs p, PairSched8 
             } else if constexpr (!kSplit) {
                 // Two warps (64 channels) fill a box of 32 tokens, which leaves by TMA in whole 128-byte lines, clipped at M and N
                 // (stored by the lanes, 64 bytes of a row at a time, the tile of T = 224 took 6600 SM cycles behind the last MMA, 2500 of
-                // them for the stores: 1031 rows on 3584 -> 4608 19.1 -> 18.2 us, in a loop on 3584 -> 37888 131 -> 114; four 7B decoder layers
-                // of 64 rows 241.8 -> 238.4).  Two lanes swap halves, so that a lane writes two channels of a token: even lanes token j, odd lanes j + 4, whose
+                // them for the stores).  Two lanes swap halves, so that a lane writes two channels of a token: even lanes token j, odd lanes j + 4, whose
                 // swizzled places lie in the other banks.
                 const uint32_t box = smem_base + kRing + ((q >> 1) + 2 * h) * kBoxBytes;
                 const bool issuer = (q & 1) == 0 && lane == 0;
@@ -394,7 +394,8 @@ cudaError_t launch_kernel(const W8a8PairPlan& pl, const UmmaArgs& a, const PairM
 
 // Tokens per tile, and whether a cluster takes the slices: the cheapest by a model of the kernel in microseconds, fitted to
 // back-to-back calls with every T and 1 to 4 slices over twelve layer shapes (1280 -> 1536 .. 2048 -> 11008 .. 18944 -> 3584, 3584
-// -> 37888) at 16 to 4096 rows; the choice is 1 % slower than the best of the sweep on average.  A K block takes the longer
+// -> 37888) at 16 to 4096 rows while the lanes stored the results; with the results by TMA the choice of T is 0.3 % slower than the best of
+// the sweep on average where the kernel is routed to (eleven shapes, 17 to 3000 rows), 0.7 % over all of them.  A K block takes the longer
 // of the way of the operands into shared memory (0.09 + 0.0003 T: 16 KB of weights whatever T is; more when every SM loads)
 // and the tensor core's (0.03 + 0.0013 T); all blocks together at least what the power limit allows.  A call starts later the
 // more SMs it needs at once (the kernel before it is still on them), and clusters add the hand-over of the sums and their
