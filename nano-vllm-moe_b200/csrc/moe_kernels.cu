@@ -310,9 +310,11 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); the block of 4096 tokens, 4 of 60 experts, takes 2 % less.
 // What grows with the experts is every block's: the counts of a share are read beside each other by as many threads as there are
 // experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
-// experts (512 rows; 14 now, one CTA's grouping and the rows 17).  Blocks in a loop, us, one CTA's grouping and a pass over the rows / here:
-// 60 experts 2048 -> 1408, 512 rows 97.7 / 96.5, 2048 rows 115.4 / 103.2; 512 experts 2048 -> 512, 512 rows 183.9 / 180.2, 4096 rows
-// 297.5 / 289.3; 1024 experts 1024 -> 256, 512 rows 89.9 / 89.3, 4096 rows 191.0 / 181.4.
+// experts (512 rows; 10 now, one CTA's grouping and the rows 17).  The slots of a token are one thread's, one behind the other: from some 256
+// of them on that shows (16384 rows, 256 of a token 252 us per block, 4096 622, one token 1978; one at a time 252, 696 and 2273).
+// Blocks in a loop, us, one CTA's grouping and a pass over the rows / here: 60 experts 2048 -> 1408, 512 rows 97.1 / 95.7, 2048 rows
+// 115.6 / 103.1; 512 experts 2048 -> 512, 512 rows 183.0 / 179.9, 4096 rows 297.3 / 291.8; 1024 experts 1024 -> 256, 512 rows 89.5 / 89.7, 4096
+// rows 190.5 / 181.7.
 constexpr int kMoeShares = 128;                    // at most (see moe_count_ints)
 constexpr int kRankBits = 18;                      // a row's rank inside its share (see moe_share_rows); the expert (E <= 3071) above it
 
@@ -404,13 +406,20 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
             }
             const uint2 qa = quant8_e4m3(va, div_scale), qb = quant8_e4m3(vb, div_scale);
             const uint4 o = make_uint4(qa.x, qa.y, qb.x, qb.y);
-            for (int j = 0; j < x_div; ++j) {
-                const int64_t r = t * x_div + j;
-                const int code = r < rows ? ld_dep(inv + r) : -1;
-                if (code < 0) continue;
-                const int e = code >> kRankBits, place = start[e] + before[e] + (code & ((1 << kRankBits) - 1));
-                *reinterpret_cast<uint4*>(xq + (size_t)place * H + c * 16) = o;
-                if (c == 0) sorted_rows[place] = (int)r;
+            for (int j0 = 0; j0 < x_div; j0 += 4) {            // four slots' codes in flight
+                int code[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int64_t r = t * x_div + j0 + j;
+                    code[j] = j0 + j < x_div && r < rows ? ld_dep(inv + r) : -1;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (code[j] < 0) continue;
+                    const int e = code[j] >> kRankBits, place = start[e] + before[e] + (code[j] & ((1 << kRankBits) - 1));
+                    *reinterpret_cast<uint4*>(xq + (size_t)place * H + c * 16) = o;
+                    if (c == 0) sorted_rows[place] = (int)(t * x_div + j0 + j);
+                }
             }
         }
 }
