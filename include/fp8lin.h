@@ -351,6 +351,9 @@ int fp8lin_debug_silu(const void* g, float* fast, float* divided, int64_t n, voi
  * is grouped by one CTA. */
 int64_t fp8lin_debug_moe_share_rows(int64_t rows, int x_div);
 
+/* For tests: the most rows of a work item where an expert batch (of aligned outputs) runs on CTA pairs, 0 where it does not. */
+int fp8lin_debug_moe_pair_rows(int64_t rows, int num_experts, int64_t H, int64_t I);
+
 #ifdef __cplusplus
 }
 #endif

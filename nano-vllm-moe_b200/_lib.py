@@ -61,6 +61,7 @@ SIGNATURES = {
     "fp8lin_moe_block_w8a8": (c_int, [c_void_p, c_int64, c_void_p, c_int, c_void_p, c_int64, c_int, c_void_p, c_void_p, c_void_p,
                                       c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_size_t, c_void_p]),
     "fp8lin_debug_moe_share_rows": (c_int64, [c_int64, c_int]),
+    "fp8lin_debug_moe_pair_rows": (c_int, [c_int64, c_int, c_int64, c_int64]),
     "fp8lin_debug_silu": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
     "fp8lin_debug_wait_timeout": (c_int, [c_void_p, c_int64, c_void_p]),
     "fp8lin_moe_align": (c_int, [c_void_p, c_int64, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p]),

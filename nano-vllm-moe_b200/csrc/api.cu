@@ -1048,9 +1048,19 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 //   has to have two work items of either projection: 16 experts 2048 -> 1024, 75 rows 36.9 / 38.4 (128 items, 74 pairs); a chunk of more
 //   can be cut (8 experts 1024 -> 1408, 175 rows, 88 items 33.4 / 31.0).  Of a hundred sizes (8 to 60 experts, 512 to 16384 rows) one is
 //   known to lose by it: 8 experts 1024 -> 512, 512 rows each 28.9 / 32.3.
-//   The chunk: a busy expert's rows, should the tokens choose at random (mean and three deviations), where that is 320 or less:
-//   273 rows on average 219 in chunks of up to 320, 221 of 288 (a sixth of the experts in two), 241 of 256; 256 above (8 experts 1024 ->
-//   512, 512 rows each 32.3, in chunks of up to 320 31.8, 4096 rows 120.6 / 118: little either way).  Shorter chunks leave room for more slots, but below 192 rows that buys nothing.
+//   The chunk: a busy expert's rows, should the tokens choose at random (mean and three deviations), up to 320.  Above that an expert in two
+//   chunks has its weights loaded twice, but items of up to 256 rows lie in tensor memory beside each other, which longer ones do not: up
+//   to 320 as long as most experts fit into one chunk (mean and half a deviation, 311 rows; with K of 512 or less, where the epilogues are the
+//   longer part, nearly all of them: mean and two, 286 rows), 256 beyond.  Time with chunks of up to 320 over that of 256, three routings each:
+//       rows per expert         276   284   292   300   308   316   330   480   530   590   640
+//       60, 2048 -> 1408       0.87  0.88  0.91  0.90  0.94  0.97  0.99  0.99  0.89  0.98  1.03
+//       48, 1280 -> 1280       0.92  0.91  0.93  0.99  0.99  1.01  1.05  1.00  0.96  0.98  1.01
+//       16, 2048 -> 1024       0.88  0.89  0.90  0.91  0.92  0.96  1.02  1.01  1.07  1.02  1.00
+//       20, 3584 -> 1024       0.98  0.95  0.99  1.00  0.99  1.03  1.07  1.02  1.01  1.03  1.07
+//       64, 1536 ->  640       0.95  0.97  0.94  0.96  1.01  0.99  1.04  1.00  0.95  1.00  1.01
+//       64, 1024 ->  512       0.95  0.97  1.00  1.00  1.08  1.04  1.06  0.95  0.95  0.98
+//        8, 1024 ->  512       0.95  1.05  1.05  1.05  1.01  1.03  1.05  1.00  0.96  0.96  0.97
+//   Shorter chunks leave room for more slots, but below 192 rows that buys nothing.
 namespace {
 int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, int64_t ld_out) {
     if (g_tune.moe_pair == 0 || g_tune.moe_fused == 0 || g_tune.moe_rows_major >= 0 || rows < kMoePrequantRows || E > 1024) return 0;
@@ -1059,8 +1069,10 @@ int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, in
     const int64_t avg = (rows + E - 1) / E;
     const int64_t items = E * (pack_ntiles(I) < (pack_ntiles(H) + 1) / 2 ? pack_ntiles(I) : (pack_ntiles(H) + 1) / 2);
     if (avg <= 32 || (avg <= 128 && items < sm_count())) return 0;
-    const int64_t busy = (int64_t)align_up((size_t)((double)avg + 3.0 * sqrt((double)avg)), 32);
-    return busy < 192 ? 192 : busy <= kGroupedPairMaxRows || avg <= 288 ? (int)(busy < kGroupedPairMaxRows ? busy : kGroupedPairMaxRows) : 256;
+    const double mean = (double)avg, deviation = sqrt(mean);
+    const int most = mean + (H <= 512 || I <= 512 ? 2.0 : 0.5) * deviation <= kGroupedPairMaxRows ? kGroupedPairMaxRows : 256;
+    const int64_t busy = (int64_t)align_up((size_t)(mean + 3.0 * deviation), 32);
+    return busy < 192 ? 192 : busy < most ? (int)busy : most;
 }
 }  // namespace
 
@@ -1238,6 +1250,10 @@ int fp8lin_debug_wait_timeout(void* workspace, int64_t limit_us, void* stream) {
 
 int64_t fp8lin_debug_moe_share_rows(int64_t rows, int x_div) {
     return rows >= kMoePrequantRows && rows <= (1ll << 24) && x_div > 0 ? moe_share_rows(rows, x_div) : 0;
+}
+
+int fp8lin_debug_moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I) {
+    return rows > 0 && E > 0 && H > 0 && I > 0 ? moe_pair_rows(rows, E, H, I, nullptr, H) : 0;
 }
 
 int fp8lin_debug_silu(const void* g, float* fast, float* divided, int64_t n, void* stream) {
