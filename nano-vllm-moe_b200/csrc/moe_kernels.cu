@@ -308,8 +308,8 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // elements of a token once and stores them to the places of its x_div slots: 2 + x_div bytes of traffic per token element.  The
 // first block also writes the chunk list.  Launch times of 16384 rows x 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before,
 // 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); the block of 4096 tokens, 4 of 60 experts, takes 2 % less.
-// What grows with the experts is every block's: the counts of a share are read beside each other by as many threads as there are
-// experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
+// What grows with the experts is every block's: from 33 experts on the counts of a share are read beside each other by as many threads as
+// there are experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
 // experts (512 rows; 10 now, one CTA's grouping and the rows 17).  The slots of a token are one thread's, one behind the other: from some 256
 // of them on that shows (16384 rows, 256 of a token 252 us per block, 4096 622, one token 1978; one at a time 252, 696 and 2273).
 // Blocks in a loop, us, one CTA's grouping and a pass over the rows / here: 60 experts 2048 -> 1408, 512 rows 97.1 / 95.7, 2048 rows
@@ -343,7 +343,12 @@ moe_count_kernel(const IdT* __restrict__ ids, int rows, int E, int share_rows, i
     for (int e = threadIdx.x; e < E; e += blockDim.x) counts[(size_t)blockIdx.x * E + e] = sh[e];
 }
 
-__global__ void __launch_bounds__(256)
+// kMany: the form for more than 32 experts, or more slots of a token than the router gives.  Up to there a warp's lanes hold all experts,
+// and fewer loads in flight leave room for five blocks per SM instead of four (48 registers; blocks us, that form / kMany: 8 experts 1024 ->
+// 512, 4800 rows, 640 blocks of this kernel, 29.1 / 30.8, 1600 rows 23.0 / 23.3; 32 experts, 9600 rows 42.9 / 44.3, 2240 rows 26.6 / 26.2; 60 experts
+// 2048 -> 512, 2400 rows 53.7 / 52.8; 96 experts 1024 -> 512, 3840 rows 46.6 / 44.2; 256 experts 1024 -> 256, 2048 rows 63.3 / 57.3).
+template <bool kMany>
+__global__ void __launch_bounds__(256, kMany ? 4 : 5)
 moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ inv, int rows, const float* __restrict__ input_scale,
                  unsigned char* __restrict__ xq, int H, const int* __restrict__ counts, int shares, int share_tok, int parts, int E, int chunk_rows, int even,
                  int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta) {
@@ -374,16 +379,17 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
         vb = ld_dep(source(t_mine, c_first) + 1);
     }
     __syncthreads();
-    // threads beside each other sum up experts beside each other, eight shares in flight; what is left of the block divides the shares
-    const int across = E <= 32 ? 32 : E <= 64 ? 64 : E <= 128 ? 128 : 256, groups = 256 / across;
+    // threads beside each other sum up experts beside each other, some shares in flight; what is left of the block divides the shares
+    constexpr int kFlight = kMany ? 8 : 4;
+    const int across = !kMany || E <= 32 ? 32 : E <= 64 ? 64 : E <= 128 ? 128 : 256, groups = 256 / across;
     for (int e = (int)threadIdx.x & (across - 1); e < E; e += across) {
         int all = 0, front = 0;
-        for (int b = (int)threadIdx.x / across; b < shares; b += 8 * groups) {
-            int n[8];
+        for (int b = (int)threadIdx.x / across; b < shares; b += kFlight * groups) {
+            int n[kFlight];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) n[i] = b + i * groups < shares ? ld_dep(counts + (size_t)(b + i * groups) * E + e) : 0;
+            for (int i = 0; i < kFlight; ++i) n[i] = b + i * groups < shares ? ld_dep(counts + (size_t)(b + i * groups) * E + e) : 0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
+            for (int i = 0; i < kFlight; ++i) {
                 all += n[i];
                 if (b + i * groups < share) front += n[i];
             }
@@ -393,10 +399,11 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
     }
     __syncthreads();
     const bool first = blockIdx.x == 0;
-    scan_experts<8>(total, E, chunk_rows, even, start, first ? cstart : nullptr, first ? coststart : nullptr, meta);
+    if (kMany || threadIdx.x < 32) scan_experts<kMany ? 8 : 1>(total, E, chunk_rows, even, start, first ? cstart : nullptr, first ? coststart : nullptr, meta);
     __syncthreads();
     if (first) write_chunks(total, E, chunk_rows, even, start, cstart, coststart, chunks);
 
+    constexpr int kSlots = kMany ? 4 : 1;                                  // codes in flight
     const ExactDiv div_scale(fmaxf(ld_dep(input_scale), 1e-12f));
     for (int64_t t = t_mine; t < t_last; t += per)
         for (int c = c_first; c < vec_per_row; c += c_step) {
@@ -406,15 +413,15 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
             }
             const uint2 qa = quant8_e4m3(va, div_scale), qb = quant8_e4m3(vb, div_scale);
             const uint4 o = make_uint4(qa.x, qa.y, qb.x, qb.y);
-            for (int j0 = 0; j0 < x_div; j0 += 4) {            // four slots' codes in flight
-                int code[4];
+            for (int j0 = 0; j0 < x_div; j0 += kSlots) {
+                int code[kSlots];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < kSlots; ++j) {
                     const int64_t r = t * x_div + j0 + j;
-                    code[j] = j0 + j < x_div && r < rows ? ld_dep(inv + r) : -1;
+                    code[j] = (kSlots == 1 || j0 + j < x_div) && r < rows ? ld_dep(inv + r) : -1;
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
+                for (int j = 0; j < kSlots; ++j) {
                     if (code[j] < 0) continue;
                     const int e = code[j] >> kRankBits, place = start[e] + before[e] + (code[j] & ((1 << kRankBits) - 1));
                     *reinterpret_cast<uint4*>(xq + (size_t)place * H + c * 16) = o;
@@ -445,7 +452,8 @@ cudaError_t launch_moe_group_quant(const __nv_bfloat16* x, int64_t ldx, int x_di
     if (parts > (share_tok + per - 1) / per) parts = (share_tok + per - 1) / per;
     if (parts < 1) parts = 1;
     // (E <= 3071, with even chunks <= 1024: 48 KB)
-    return launch_dependent(moe_place_kernel, (unsigned)(shares * parts), 256, (size_t)((even ? 5 : 4) * E + 2) * sizeof(int), stream, x, ldx, x_div, inv, rows,
+    const auto place = E > 32 || x_div > 32 ? moe_place_kernel<true> : moe_place_kernel<false>;
+    return launch_dependent(place, (unsigned)(shares * parts), 256, (size_t)((even ? 5 : 4) * E + 2) * sizeof(int), stream, x, ldx, x_div, inv, rows,
                             input_scale, xq, H, counts, shares, share_tok, parts, E, chunk_rows, even, sorted_rows, chunks, meta);
 }
 
