@@ -1051,7 +1051,8 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 //   The chunk: a busy expert's rows, should the tokens choose at random (mean and three deviations), up to 320.  Above that an expert in two
 //   chunks has its weights loaded twice, but items of up to 256 rows lie in tensor memory beside each other, which longer ones do not: up
 //   to 320 as long as most experts fit into one chunk (mean and half a deviation, 311 rows; with K of 512 or less, where the epilogues are the
-//   longer part, nearly all of them: mean and two, 286 rows), 256 beyond.  Time with chunks of up to 320 over that of 256, three routings each:
+//   longer part, or with gate_up items for less than two thirds of the pairs, where all are cut between groups of rows anyway, nearly all of
+//   them: mean and two, 286 rows), 256 beyond.  Time with chunks of up to 320 over that of 256, three routings each:
 //       rows per expert         276   284   292   300   308   316   330   480   530   590   640
 //       60, 2048 -> 1408       0.87  0.88  0.91  0.90  0.94  0.97  0.99  0.99  0.89  0.98  1.03
 //       48, 1280 -> 1280       0.92  0.91  0.93  0.99  0.99  1.01  1.05  1.00  0.96  0.98  1.01
@@ -1060,6 +1061,8 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 //       64, 1536 ->  640       0.95  0.97  0.94  0.96  1.01  0.99  1.04  1.00  0.95  1.00  1.01
 //       64, 1024 ->  512       0.95  0.97  1.00  1.00  1.08  1.04  1.06  0.95  0.95  0.98
 //        8, 1024 ->  512       0.95  1.05  1.05  1.05  1.01  1.03  1.05  1.00  0.96  0.96  0.97
+//   and, four routings, 292 and 300 rows: 8 experts 3584 -> 1408 0.94 0.94; 8, 2048 -> 1280 0.96 0.97; 5, 2048 -> 1408 (55 items of gate_up)
+//   0.97 0.97; 4, 2048 -> 1408 (44) 1.00 1.00; 4, 2048 -> 1024 (32) 1.05 1.05; 2, 2048 -> 1408 (22) 1.00 1.01.
 //   Shorter chunks leave room for more slots, but below 192 rows that buys nothing.
 namespace {
 int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, int64_t ld_out) {
@@ -1070,7 +1073,7 @@ int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, in
     const int64_t items = E * (pack_ntiles(I) < (pack_ntiles(H) + 1) / 2 ? pack_ntiles(I) : (pack_ntiles(H) + 1) / 2);
     if (avg <= 32 || (avg <= 128 && items < sm_count())) return 0;
     const double mean = (double)avg, deviation = sqrt(mean);
-    const int most = mean + (H <= 512 || I <= 512 ? 2.0 : 0.5) * deviation <= kGroupedPairMaxRows ? kGroupedPairMaxRows : 256;
+    const int most = mean + (H <= 512 || I <= 512 || 3 * E * pack_ntiles(I) < 2 * (sm_count() / 2) ? 2.0 : 0.5) * deviation <= kGroupedPairMaxRows ? kGroupedPairMaxRows : 256;
     const int64_t busy = (int64_t)align_up((size_t)(mean + 3.0 * deviation), 32);
     return busy < 192 ? 192 : busy < most ? (int)busy : most;
 }
