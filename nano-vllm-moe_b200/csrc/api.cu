@@ -1046,8 +1046,12 @@ MoeWs moe_ws_layout(int64_t rows, int E, int64_t H, int64_t I) {
 //   experts 2048 -> 1408, 34 rows each 115 / 105, 68 rows 124.6 / 122.5, 136 rows 180 / 148, 273 rows 278 / 219; 64 experts 1024 -> 512,
 //   40 rows 48.8 / 39.6; 8 experts 1024 -> 512, 4096 rows 128 / 120; but 30 experts 1152 -> 1200, 26 rows 41.4 / 43.8.  Up to 128 rows a pair
 //   has to have two work items of either projection: 16 experts 2048 -> 1024, 75 rows 36.9 / 38.4 (128 items, 74 pairs); a chunk of more
-//   can be cut (8 experts 1024 -> 1408, 175 rows, 88 items 33.4 / 31.0).  Of a hundred sizes (8 to 60 experts, 512 to 16384 rows) one is
-//   known to lose by it: 8 experts 1024 -> 512, 512 rows each 28.9 / 32.3.
+//   can be cut (8 experts 1024 -> 1408, 175 rows, 88 items 33.4 / 31.0).
+//   Nor pairs where one CTA each does the 128 x 256 items of either projection in one round that fills more than two thirds of the chip, with
+//   more than 192 rows per expert (one CTA / pairs): 8 experts 1024 -> 512, 450 rows 25.1 / 25.9, 512 rows 25.2 / 27.7, but 600 rows (1.1 rounds)
+//   34.8 / 31.1; 4 experts 2048 -> 1024, 500 rows 29.1 / 31.6; 12 experts 1024 -> 512, 300 rows 25.6 / 28.1; 2 experts 3584 -> 1408, 600 rows
+//   38.7 / 42.5; 6 experts 1536 -> 640, 500 rows 31.4 / 31.4.  With half of the chip or fewer rows the cuts between pairs pay for more: 8 experts
+//   1024 -> 512, 300 rows 24.2 / 22.6, 16 experts (128 items) 160 rows 25.4 / 24.4, 2 experts 2048 -> 2048, 350 rows (96 items) 28.4 / 27.1.
 //   The chunk: a busy expert's rows, should the tokens choose at random (mean and three deviations), up to 320.  Above that an expert in two
 //   chunks has its weights loaded twice, but items of up to 256 rows lie in tensor memory beside each other, which longer ones do not: up
 //   to 320 as long as most experts fit into one chunk (mean and half a deviation, 311 rows; with K of 512 or less, where the epilogues are the
@@ -1073,6 +1077,11 @@ int moe_pair_rows(int64_t rows, int E, int64_t H, int64_t I, const void* out, in
     const int64_t items = E * (pack_ntiles(I) < (pack_ntiles(H) + 1) / 2 ? pack_ntiles(I) : (pack_ntiles(H) + 1) / 2);
     if (avg <= 32 || (avg <= 128 && items < sm_count())) return 0;
     const double mean = (double)avg, deviation = sqrt(mean);
+    // chunks of 128 rows (grouped_rows_kernel's), should the tokens choose at random: the mean over four equal parts of that distribution
+    double chunks = 0.0;
+    for (const double d : {-1.15, -0.32, 0.32, 1.15}) chunks += 0.25 * (double)E * ceil((mean + d * deviation) / 128.0);
+    const double gate_up = chunks * (double)pack_ntiles(I), down = chunks * (double)((H + 255) / 256), sms = (double)sm_count();
+    if (avg > 192 && I % 128 == 0 && ld_out % 8 == 0 && aligned16(out) && gate_up <= sms && down <= sms && 3.0 * gate_up > 2.0 * sms) return 0;
     const int most = mean + (H <= 512 || I <= 512 || 3 * E * pack_ntiles(I) < 2 * (sm_count() / 2) ? 2.0 : 0.5) * deviation <= kGroupedPairMaxRows ? kGroupedPairMaxRows : 256;
     const int64_t busy = (int64_t)align_up((size_t)(mean + 3.0 * deviation), 32);
     return busy < 192 ? 192 : busy < most ? (int)busy : most;

@@ -245,12 +245,26 @@ def test_experts_stay_in_one_chunk_while_most_of_them_fit(pkg):
         for avg in range(129, 2000):
             n = rule(avg * e, e, h, i)
             spread = avg ** 0.5 * (0.5 if min(h, i) > 512 and e * -(-i // 128) > 49 else 2)
+            if n == 0:
+                continue                                             # one CTA's
             assert n % 32 == 0 and 192 <= n <= most
             if avg + spread <= most:
                 assert n >= min(avg + spread, most) and n >= last, (e, h, i, avg, n)
                 last = n
             else:
                 assert n == 256, (e, h, i, avg, n)
+
+
+def test_expert_batches_of_one_full_round_stay_on_one_cta(pkg):
+    """128 x 256 items of either projection that fill most of one round of the chip, rows per expert that fill whole tiles: pairs have
+    nothing to share out.  The items are those of tokens that choose at random, not of the mean alone."""
+    rule = pkg._lib.load().fp8lin_debug_moe_pair_rows
+    alone = {(8, 1024, 512): [450, 512], (4, 2048, 1024): [400, 500], (12, 1024, 512): [300, 350], (2, 3584, 1408): [512, 600], (16, 1024, 512): [200]}
+    pairs = {(8, 1024, 512): [192, 256, 300, 600], (4, 2048, 1024): [256, 350, 600], (12, 1024, 512): [400], (2, 3584, 1408): [430, 640],
+             (16, 1024, 512): [256, 300], (8, 1024, 528): [512], (8, 2048, 512): [512]}         # 528: up channels inside a tile
+    assert all(rule(e * n, e, h, i) == 0 for (e, h, i), rows in alone.items() for n in rows)
+    assert all(rule(e * n, e, h, i) > 0 for (e, h, i), rows in pairs.items() for n in rows)
+    assert all((rule(60 * n, 60, 2048, 1408) > 0) == (n > 32) for n in range(9, 400))
 
 
 def test_gate_up_interleave_is_a_tile_row_permutation():
