@@ -310,8 +310,9 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); the block of 4096 tokens, 4 of 60 experts, takes 2 % less.
 // What grows with the experts is every block's: from 33 experts on the counts of a share are read beside each other by as many threads as
 // there are experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
-// experts (512 rows; 10 now, one CTA's grouping and the rows 17).  The slots of a token are one thread's, one behind the other: from some 256
-// of them on that shows (16384 rows, 256 of a token 252 us per block, 4096 622, one token 1978; one at a time 252, 696 and 2273).
+// experts (512 rows; 10 now, one CTA's grouping and the rows 17).  The slots of a token are one thread's, one behind the other; where tokens
+// have more than the router gives, blocks share them out (16384 rows x 2048, 60 experts, us per block, all slots one thread's / shared out: 64 of a
+// token 165 / 162, 1024 274 / 155, 4096 667 / 157, one token 2250 / 163).
 // Blocks in a loop, us, one CTA's grouping and a pass over the rows / here: 60 experts 2048 -> 1408, 512 rows 97.1 / 95.7, 2048 rows
 // 115.6 / 103.1; 512 experts 2048 -> 512, 512 rows 183.0 / 179.9, 4096 rows 297.3 / 291.8; 1024 experts 1024 -> 256, 512 rows 89.5 / 89.7, 4096
 // rows 190.5 / 181.7.
@@ -350,8 +351,8 @@ moe_count_kernel(const IdT* __restrict__ ids, int rows, int E, int share_rows, i
 template <bool kMany>
 __global__ void __launch_bounds__(256, kMany ? 4 : 5)
 moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, const int* __restrict__ inv, int rows, const float* __restrict__ input_scale,
-                 unsigned char* __restrict__ xq, int H, const int* __restrict__ counts, int shares, int share_tok, int parts, int E, int chunk_rows, int even,
-                 int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta) {
+                 unsigned char* __restrict__ xq, int H, const int* __restrict__ counts, int shares, int share_tok, int parts, int slot_parts, int E,
+                 int chunk_rows, int even, int* __restrict__ sorted_rows, int4* __restrict__ chunks, int* __restrict__ meta) {
     pdl_launch_dependents();
     extern __shared__ int sh[];
     int* before = sh;                              // [E] rows of the expert in the shares in front
@@ -360,7 +361,11 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
     int* cstart = start + E + 1;                   // [E + 1]: the first block only
     int* coststart = cstart + E + 1;               // [E]: there only where `even`
     for (int e = threadIdx.x; e < 2 * E; e += blockDim.x) sh[e] = 0;
-    const int share = (int)blockIdx.x / parts, part = (int)blockIdx.x - share * parts;
+    const int block = kMany ? (int)blockIdx.x / slot_parts : (int)blockIdx.x;
+    const int share = block / parts, part = block - share * parts;
+    // this block's slots of a token (slot_parts > 1: blocks that quantise the same tokens)
+    const int slots = kMany ? ((x_div + slot_parts - 1) / slot_parts + 3) & ~3 : x_div;
+    const int j_first = kMany ? ((int)blockIdx.x - block * slot_parts) * slots : 0, j_last = kMany ? min(x_div, j_first + slots) : x_div;
     // this block's tokens; it walks whole ones, `per` at a time, so that no element needs a division to find its row
     const int64_t tokens = ((int64_t)rows + x_div - 1) / x_div;
     const int part_tok = (share_tok + parts - 1) / parts;
@@ -413,12 +418,12 @@ moe_place_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, int x_div, co
             }
             const uint2 qa = quant8_e4m3(va, div_scale), qb = quant8_e4m3(vb, div_scale);
             const uint4 o = make_uint4(qa.x, qa.y, qb.x, qb.y);
-            for (int j0 = 0; j0 < x_div; j0 += kSlots) {
+            for (int j0 = j_first; j0 < j_last; j0 += kSlots) {
                 int code[kSlots];
 #pragma unroll
                 for (int j = 0; j < kSlots; ++j) {
                     const int64_t r = t * x_div + j0 + j;
-                    code[j] = (kSlots == 1 || j0 + j < x_div) && r < rows ? ld_dep(inv + r) : -1;
+                    code[j] = (kSlots == 1 || j0 + j < j_last) && r < rows ? ld_dep(inv + r) : -1;
                 }
 #pragma unroll
                 for (int j = 0; j < kSlots; ++j) {
@@ -451,10 +456,14 @@ cudaError_t launch_moe_group_quant(const __nv_bfloat16* x, int64_t ldx, int x_di
     int parts = sm_count() * 8 / shares;
     if (parts > (share_tok + per - 1) / per) parts = (share_tok + per - 1) / per;
     if (parts < 1) parts = 1;
+    // where that leaves blocks and a token has more slots than the router gives: stretches of at least 64 slots of it
+    int slot_parts = x_div > 32 ? sm_count() * 8 / (shares * parts) : 1;
+    if (slot_parts > (x_div + 63) / 64) slot_parts = (x_div + 63) / 64;
+    if (slot_parts < 1) slot_parts = 1;
     // (E <= 3071, with even chunks <= 1024: 48 KB)
     const auto place = E > 32 || x_div > 32 ? moe_place_kernel<true> : moe_place_kernel<false>;
-    return launch_dependent(place, (unsigned)(shares * parts), 256, (size_t)((even ? 5 : 4) * E + 2) * sizeof(int), stream, x, ldx, x_div, inv, rows,
-                            input_scale, xq, H, counts, shares, share_tok, parts, E, chunk_rows, even, sorted_rows, chunks, meta);
+    return launch_dependent(place, (unsigned)(shares * parts * slot_parts), 256, (size_t)((even ? 5 : 4) * E + 2) * sizeof(int), stream, x, ldx, x_div, inv, rows,
+                            input_scale, xq, H, counts, shares, share_tok, parts, slot_parts, E, chunk_rows, even, sorted_rows, chunks, meta);
 }
 
 // ---- h = silu(gate) * up, quantised for the down projection ----------------------------------

@@ -111,7 +111,7 @@ def test_gates_of_any_size_in_the_epilogue(gate):
     assert Kn.read_status(torch.device("cuda", 0)) == 0
 
 
-@pytest.mark.parametrize("rows,x_div,E", [(512, 1, 3), (513, 5, 60), (1031, 4, 7), (70000, 3, 9), (2000, 600, 3000), (700, 2, 3071), (1500, 3, 1024), (9000, 1, 257), (300000, 300000, 3)])
+@pytest.mark.parametrize("rows,x_div,E", [(512, 1, 3), (513, 5, 60), (1031, 4, 7), (70000, 3, 9), (2000, 600, 3000), (700, 2, 3071), (1500, 3, 1024), (9000, 1, 257), (300000, 300000, 3), (3000, 33, 5), (5000, 5000, 7), (20011, 1999, 40)])
 def test_grouping_of_large_batches(pkg, rows, x_div, E):
     """Shares of whole tokens, a last one that is cut short, more than 128 times 512 rows, as many experts as there may be, one token with more
     slots than a rank inside a share can count: every routed row gets what it gets in a batch that one CTA groups."""
