@@ -121,7 +121,9 @@ def test_fused_activation_epilogue_equals_the_separate_pass(moe, T, H, I, E, k):
     w, ids = moe.SoftmaxTopKRouter(k, False).select_experts(None, torch.from_numpy(c["logits"]).cuda())
     x = to_bf16_cuda(c["x"])
     try:
-        y_rows = kern(x, w, ids, wts, model_dtype=torch.bfloat16)          # default: rows as the MMA M dimension where chunks are 128 rows
+        y_default = kern(x, w, ids, wts, model_dtype=torch.bfloat16)       # CTA pairs, or few rows per expert on one CTA
+        Kn.set_tuning("moe_pair", 0)                                       # one CTA: rows as the MMA M dimension where chunks are 128 rows
+        y_rows = kern(x, w, ids, wts, model_dtype=torch.bfloat16)
         Kn.set_tuning("moe_rows_major", 0)                                 # the channel-major grouped kernel, activation fused ...
         y_fused = kern(x, w, ids, wts, model_dtype=torch.bfloat16)
         Kn.set_tuning("moe_fused", 0)                                      # ... and with the separate activation pass
@@ -129,15 +131,37 @@ def test_fused_activation_epilogue_equals_the_separate_pass(moe, T, H, I, E, k):
     finally:
         Kn.set_tuning("moe_fused", -1)
         Kn.set_tuning("moe_rows_major", -1)
+        Kn.set_tuning("moe_pair", -1)
     assert torch.equal(y_fused, y_plain)
+    assert torch.equal(y_default, y_rows)                                  # whole sums over K in the same order, whatever the tiles
     assert y_fused.float().abs().max() > 0
     # the other orientation multiplies the same codes; only the accumulation order inside the MMA may differ
     assert_parity(from_bf16(y_rows), from_bf16(y_plain), "rows-major vs channel-major grouped GEMM", ulps=2.0, min_cos=0.99999)
     w_ref, ids_ref = O.softmax_topk(c["logits"], k, False)
     if T * k * H * I <= 2e9:
         ref = O.moe_experts_w8a8(c["x"], ids_ref, w_ref, c["w13_q"], c["w13_s"], c["in13"], c["w2_q"], c["w2_s"], c["in2"])
-        assert_parity(from_bf16(y_rows), ref, f"rows-major moe T={T} E={E}", ulps=3.0, min_cos=0.9999)
+        for name, y in {"default": y_default, "one CTA": y_rows}.items():
+            assert_parity(from_bf16(y), ref, f"{name} moe T={T} E={E}", ulps=3.0, min_cos=0.9999)
     assert Kn.read_status(torch.device("cuda", 0)) == 0
+
+
+@pytest.mark.parametrize("E,H,I,avg,pairs", [(40, 1024, 512, 32, False), (40, 1024, 512, 33, True), (16, 512, 256, 75, False),
+                                             (8, 256, 128, 128, False), (8, 256, 128, 129, True),
+                                             (25, 512, 256, 200, False), (25, 512, 256, 300, True)])
+def test_default_dispatch_on_both_sides_of_its_lines(pkg, moe, E, H, I, avg, pairs):
+    """Rows per expert where prefill-sized batches change kernels: 32 rows, 128 rows of few work items, one full round of one-CTA items."""
+    assert (pkg._lib.load().fp8lin_debug_moe_pair_rows(E * avg, E, H, I) > 0) == pairs
+    T = E * avg
+    c = make_moe_case(avg + E, T, H, I, E, 1)
+    wts = upload_weights(moe, c)
+    rng = np.random.default_rng(avg)
+    ids, w = rng.permutation(np.arange(T) % E)[:, None].astype(np.int64), (rng.random((T, 1)) + 0.2).astype(np.float32)
+    cfg = moe.make_moe_parallel_config(tp_group=None, ep_group=None, global_num_experts=E, intermediate_size=I)
+    kern = moe.MoEKernel(prepare_finalize=moe.NoEPPrepareFinalize(cfg), experts=moe.Fp8Experts(), parallel_config=cfg)
+    y = from_bf16(kern(to_bf16_cuda(c["x"]), torch.from_numpy(w).cuda(), torch.from_numpy(ids).cuda(), wts, model_dtype=torch.bfloat16))
+    ref = O.moe_experts_w8a8(c["x"], ids, w, c["w13_q"], c["w13_s"], c["in13"], c["w2_q"], c["w2_s"], c["in2"])
+    assert_parity(y, ref, f"moe {avg} rows of {E} experts", ulps=3.0, min_cos=0.9999)
+    assert kernels().read_status(torch.device("cuda", 0)) == 0
 
 
 def test_expert_rows_outside_local_range_are_skipped(moe):
