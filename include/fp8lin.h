@@ -203,7 +203,7 @@ int fp8lin_quantize_activation(const void* x, int64_t ldx, const float* input_sc
  * The gate_up grouped GEMM applies silu(g) * u and the down projection's quantiser in its epilogue.  From 512 routed rows
  * on (of at most some 131072 to a token, x_div) the rows are quantised once, into expert order, before it; with more than 32 rows per expert on average the grouped
  * GEMMs then run on CTA pairs, 256 channels x up to 320 rows per work item (out_routed 4-byte aligned, ld_out even; a few
- * work items of up to 128 rows each stay on one CTA).
+ * work items of up to 128 rows each, or items that fill one round of the chip, stay on one CTA).
  * fp8lin_moe_route replaces SoftmaxTopKRouter.select_experts (executor/moe/router.py:24-34):
  * fp32 softmax over E logits (logits_dtype 0 = f32, 1 = bf16), top-k, optional
  * renormalisation; topk_w f32 [T][k], topk_ids i32 [T][k]. */

@@ -300,7 +300,9 @@ bool other_w8a8_route_forced() {
 //     quantiser in front, the decode kernel hides more of it (64 rows on 3584 -> 3584 8.6 / 7.9, 2048 -> 2048 6.4 / 6.3), which
 //     this line does not weigh.
 //   65 to 4096 rows: where modelled faster than both kernels with fixed tiles.  The model was fitted while the lanes stored the
-//     results; since they leave by TMA a call with whole sums takes 0.86 of it.  Over eleven layer shapes (2048 -> 2048 .. 3584 ->
+//     results; since they leave by TMA a call of one K slice takes 0.86 of it.  (Several slices in one pair leave the same way and are weighed as they
+//     were: up to 64 bf16 rows the decode kernel would lose its better cover of the quantiser by it, above that up to 10 % stays there, 128 rows
+//     on 4096 -> 4096 9.3 / 10.2.)  Over eleven layer shapes (2048 -> 2048 .. 3584 ->
 //     18944, 18944 -> 3584, 8192 -> 1024) and eighteen row counts from 17 on the choice is 0.2 % slower than the faster kernel, with the model as
 //     it was 1.3 %: e.g. 700 rows on 3584 -> 4608 12.0 / 14.5, 1031 on 3584 -> 3584 13.0 / 14.2, 1500 on 11008 -> 2048 27.8 / 33.5, 256 on
 //     3584 -> 18944 18.2 / 19.2, 512 on 2560 -> 9472 12.7 / 13.3, 4096 on 3584 -> 3584 40.3 / 45.1; not 160 on 8192 -> 1024 12.1 / 10.8.

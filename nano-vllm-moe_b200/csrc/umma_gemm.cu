@@ -598,7 +598,7 @@ bool encode_u8_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t co
     return r == CUDA_SUCCESS;
 }
 
-// Output map: bf16 [rows][cols] with a row pitch in bytes, box = box_cols x 32 rows,
+// Output map: bf16 [rows][cols] with a row pitch in bytes, box = box_cols x box_rows,
 // swizzle span = the box's row length (128 or 64 bytes).
 bool encode_out_2d(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t pitch_bytes,
                    uint32_t box_cols, uint32_t box_rows) {

@@ -16,8 +16,8 @@
 //   warp 1      MMA issuer (leader): four tcgen05.mma 256 x N x 32 per K block, twice that where R > 256 (N <= 256 each)
 //   warps 2..17 epilogue: warp (q, h) owns TMEM lanes [32 q, 32 q + 32) and every fourth piece of 16 rows
 //
-// What bounds it: memory and the tensor core about equally at some 270 rows per expert (weights once from memory: 59 us for gate_up
-// of 60 experts 2048 -> 2 x 1408, its MMAs 576 SM cycles per K block of 288 rows), memory alone below.  So a chunk holds all
+// What bounds it: memory and the tensor core about equally at some 270 rows per expert (weights and rows once from memory: 59 us for
+// gate_up of 60 experts 2048 -> 2 x 1408, its MMAs 576 SM cycles per K block of 288 rows), memory alone below.  So a chunk holds all
 // rows of an expert where it can (its weights come once), rows are the MMA's N (273 rows of an expert on average are multiplied as
 // 288, in 128-row tiles as 384), and a K block of 256 channels x 288 rows moves 34 KB into each SM where 128 x 256 tiles move 48 KB
 // for a third of the products.  16384 rows of 60 experts, in a loop under the power limit: the block 278 us with 128 x 256 tiles on
