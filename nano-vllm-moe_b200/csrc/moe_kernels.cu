@@ -302,12 +302,13 @@ cudaError_t launch_moe_align(const void* ids, bool ids_i64, int rows, int E, int
 // ---- group, quantise and place the rows of a large batch ------------------------------------------------------
 // From a few hundred rows on the grouping above is one SM's shared-memory atomics (16384 rows: 14.7 us), so it is spread out.
 // moe_count_kernel: a block counts its share of the rows by expert and leaves each row's expert and rank inside the share;
-// moe_place_kernel: a block sums up what it needs of the counts (every block all of them from L2, 4 bytes per share and expert: 8 KB of 16384
-// rows and 60 experts, 512 KB of 65536 rows and 1024), which gives its rows' places in expert order, and quantises its tokens there: xq[place][:] = e4m3(x[r / x_div][:] / scale) for every routed row r with a
-// valid expert.  The grouped GEMM then takes its rows by TMA instead of re-quantising them for every channel tile.  A thread converts 16
-// elements of a token once and stores them to the places of its x_div slots: 2 + x_div bytes of traffic per token element.  The
-// first block also writes the chunk list.  Launch times of 16384 rows x 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before,
-// 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel summing up for all); the block of 4096 tokens, 4 of 60 experts, takes 2 % less.
+// moe_place_kernel: a block sums up what it needs of the counts (every block all of them from L2, 4 bytes per share and expert: 8 KB of
+// 16384 rows and 60 experts, 512 KB of 65536 rows and 1024), which gives its rows' places in expert order, and quantises its tokens there:
+// xq[place][:] = e4m3(x[r / x_div][:] / scale) for every routed row r with a valid expert.  The grouped GEMM then takes its rows by TMA
+// instead of re-quantising them for every channel tile.  A thread converts 16 elements of a token once and stores them to the places of its
+// x_div slots: 2 + x_div bytes of traffic per token element.  The first block also writes the chunk list.  Launch times of 16384 rows x
+// 2048, 60 experts: 16.4 us on one CTA and 10.2 for the rows before, 3.0 + 16.7 here (6.9 + 12.6 with the last block of the first kernel
+// summing up for all); the block of 4096 tokens, 4 of 60 experts, takes 2 % less.
 // What grows with the experts is every block's: from 33 experts on the counts of a share are read beside each other by as many threads as
 // there are experts, and eight warps scan them.  With a warp for 32 experts at a time and one warp's scan the second kernel took 38 us with 1024
 // experts (512 rows; 10 now, one CTA's grouping and the rows 17).  The slots of a token are one thread's, one behind the other; where tokens
