@@ -407,8 +407,13 @@ cudaError_t launch_grouped_pair_w8a8(GroupedArgs a, int max_rows, const void* w_
     }
     GroupedPairMaps maps;
     const uint64_t w_rows = (uint64_t)num_experts * a.w_tiles * a.kblocks * 128;
-    bool ok = encode_u8_2d(&maps.w, w_packed, w_rows, 128, gate_up ? 64 : 128) && encode_u8_2d(&maps.w16, w_packed, w_rows, 128, 16);
-    for (int i = 0; i < 8 && ok; ++i) ok = encode_u8_2d(&maps.x[i], xq_sorted, (uint64_t)xq_rows, (uint64_t)a.K, 16 * (i + 1));
+    bool ok = encode_u8_2d(&maps.w, w_packed, w_rows, 128, gate_up ? 64 : 128);
+    // (a map costs the host 0.1 us: only what the kernel reads.  Up rows inside a tile; halves of an MMA tile of up to max_rows, 256 at most)
+    maps.w16 = maps.w;
+    if (ok && gate_up && (a.N & 63) != 0) ok = encode_u8_2d(&maps.w16, w_packed, w_rows, 128, 16);
+    const int boxes = max_rows <= 256 ? max_rows / 32 : 8;
+    for (int i = 0; i < boxes && ok; ++i) ok = encode_u8_2d(&maps.x[i], xq_sorted, (uint64_t)xq_rows, (uint64_t)a.K, 16 * (i + 1));
+    for (int i = boxes; i < 8; ++i) maps.x[i] = maps.w;
     if (!ok) {
         if (why) *why = "cuTensorMapEncodeTiled failed";
         return cudaErrorInvalidValue;
