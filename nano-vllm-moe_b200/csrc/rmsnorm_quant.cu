@@ -23,7 +23,9 @@ constexpr int kNormMaxVec = 4;          // 8-element vectors per thread: H <= 25
 
 // kVec: vectors that a thread may hold.  The row stays in registers, so a prompt's rows run in as many turns as registers allow CTAs: with
 // room for four vectors whatever H was, two CTAs per SM took 9 to 10.6 us for 1031 rows of 3584 beside power-limited GEMMs, with room for
-// two four of them take 7 to 8.6 (two 7B decoder layers of 1031 rows 491.7 -> 489.0 us, four of 64 rows 238.6 -> 237.2).
+// two four of them take 7 to 8.6 (two 7B decoder layers of 1031 rows 491.7 -> 489.0 us, four of 64 rows 238.6 -> 237.2).  Behind another
+// kernel no size of 1 to 4096 rows x 1024 to 5120 is slower for it (384 rows x 2048 behind an elementwise kernel 3.98 -> 3.87 us for both, 1031 rows
+// 7.05 -> 6.03); a row of nothing but norms is for 320 to 384 rows, whose blocks then crowd on the SMs that the one in front left first (2.45 -> 2.8).
 template <int kVec>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_quant_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, __nv_bfloat16* __restrict__ residual, int64_t ld_res,
